@@ -176,6 +176,24 @@ def test_linear_fp32_is_true_fp32(m, n, k):
     torch.testing.assert_close(got.double(), want, atol=2e-5 * (k ** 0.5), rtol=1e-5)
 
 
+@pytest.mark.parametrize("n,k", [(31, 33), (33, 64), (65, 130), (4096, 260), (1024, 1028)])
+def test_linear_fp32_tiles_give_the_same_bits(n, k):
+    """Every tile the row count and the width may choose adds in one order: the row's bits are those of the
+    row alone, at the edges of the tiles; against 64 bits the error is that of eight chains of k / 8."""
+    torch.manual_seed(16)
+    x = torch.randn(400, k, device="cuda")
+    w = torch.randn(n, k, device="cuda")
+    rows = [ops().linear(x[r:r + 1], w) for r in (0, 7, 8, 16, 33)]
+    for m in (7, 8, 9, 16, 17, 32, 33, 63, 64, 65, 129, 400):
+        got = ops().linear(x[:m], w)
+        for r, one in zip((0, 7, 8, 16, 33), rows):
+            if r < m:
+                assert torch.equal(got[r], one[0]), (m, r)
+        # a chain of c terms: at most c * 2^-24 of the sum of the terms' sizes, and 8 partials more
+        bound = (k / 8 + 16) * 2.0 ** -24 * (x[:m].abs().double() @ w.abs().double().T)
+        assert ((got.double() - x[:m].double() @ w.double().T).abs() <= bound).all(), m
+
+
 def test_linear_fp32_row_does_not_depend_on_batch():
     """A row gives the same bits alone and among 333 rows (the reference checks its
     batch-invariant product the same way, tests/test_10_batch_invariant.py:32-43)."""
