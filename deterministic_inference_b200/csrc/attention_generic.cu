@@ -1,8 +1,7 @@
-// Generic paged attention: one warp per (token, query head), float32 arithmetic
-// throughout (expf, not the fast intrinsic), any head_dim up to 256, any number
-// of heads and groups, any page size, optional window.  It is the attention of
-// the 32-bit path, and the fallback of the bfloat16 path for head sizes the
-// tensor-core kernels refuse.
+// Generic paged attention: float32 arithmetic throughout (expf, not the fast
+// intrinsic), any head_dim up to 256, any number of heads and groups, any page size,
+// optional window.  It is the attention of the 32-bit path, and the fallback of the
+// bfloat16 path for head sizes the tensor-core kernels refuse.
 //
 // Every token of the step is one query: token t belongs to sequence
 // token_seq[t], stands at absolute position positions[t] and sees the keys
@@ -13,92 +12,294 @@
 // the same token gives the same bits however the prompt was cut into steps,
 // whatever else is in the batch and whichever pages hold its keys.
 //
+// A block has 16 neighbouring (token, head of the group) queries of one key-value head,
+// or those of them that belong to one sequence: block (x, y) takes the y-th run of equal
+// sequences among the 16 and ends at once where there is none.  So the tile of keys and
+// values is read into shared memory once (the next one's copies are in flight meanwhile)
+// for up to 16 queries, four a warp: a prompt's queries share it, a decoding token has
+// a block of its own.  One warp per query with its keys read from global memory, a
+// 512-byte stride between lanes, was bound by the cache lines of those reads (4 decoding tokens and a
+// prompt's 200, up to 600 keys, 16 heads of 128: some 1,000 us a layer; so 22 us).
+// Bound now: the FMA and the shared-memory reads of its operands.
+//
 // Cache layout of a layer: [num_pages, 2, num_kv_heads, page_size, head_dim].
 #include "common.cuh"
+
+#include <type_traits>
 
 namespace {
 
 constexpr int MAX_D = 256;
-constexpr int WARPS = 4;
+constexpr int WARPS = 4, THREADS = WARPS * 32;
+constexpr int NQ = 4, ITEMS = WARPS * NQ;      // queries a warp, a block
+constexpr int KEYS = 32;
 constexpr float NEG_BIG = -1e30f;
 
-template <typename T>
-__global__ void __launch_bounds__(WARPS * 32)
+// floats between rows of a tile: rows padded to whole vectors, an odd number of vectors apart (the
+// lanes' rows then start in different banks)
+__host__ __device__ __forceinline__ int row_stride(int D) {
+  const int v = (D + 3) / 4;
+  return 4 * (v + 1 + (v & 1));
+}
+__host__ __device__ __forceinline__ int smem_floats(int D) {
+  return 4 * KEYS * row_stride(D) + ITEMS * row_stride(D) + ITEMS * KEYS;
+}
+
+// dot products of the lane's key with N queries, d in index order
+template <int N>
+__device__ __forceinline__ void dots(const float* krow, const float* q, int ld, int vecs, float (&s)[NQ]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) s[i] = 0.f;
+#pragma unroll 4
+  for (int v = 0; v < vecs; ++v) {
+    const float4 k = *reinterpret_cast<const float4*>(krow + 4 * v);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const float4 x = *reinterpret_cast<const float4*>(q + i * ld + 4 * v);
+      s[i] = fmaf(x.x, k.x, s[i]);
+      s[i] = fmaf(x.y, k.y, s[i]);
+      s[i] = fmaf(x.z, k.z, s[i]);
+      s[i] = fmaf(x.w, k.w, s[i]);
+    }
+  }
+}
+
+// NV: vectors of four dimensions a lane owns (1: D <= 128).  ASYNC: float32 rows on 16 bytes.
+template <typename T, int NV, bool ASYNC>
+__global__ void __launch_bounds__(THREADS)
 paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
                                const T* __restrict__ kv_cache,
                                const int* __restrict__ block_table, int max_blocks,
                                const int* __restrict__ token_seq,
                                const int* __restrict__ positions, int T_tokens, int Hq, int Hkv,
                                int D, int page_size, float scale, int window) {
+  extern __shared__ __align__(16) float smem[];
   pdl_prologue(q, kv_cache, block_table, token_seq, positions);
-  __shared__ float sq[WARPS][MAX_D];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long item = (long long)blockIdx.x * WARPS + warp;
-  if (item >= (long long)T_tokens * Hq) return;
-  const int t = (int)(item / Hq), h = (int)(item % Hq);
-  const int group = Hq / Hkv;
-  const int kvh = h / group;
-  const int seq = token_seq[t];
-  const int pos = positions[t];
-  const int* bt = block_table + (size_t)seq * max_blocks;
+  const int group = Hq / Hkv, kvh = blockIdx.x % Hkv;
+  const long long item0 = (long long)(blockIdx.x / Hkv) * ITEMS, items = (long long)T_tokens * group;
 
-  const T* qrow = q + ((size_t)t * Hq + h) * D;
-  for (int d = lane; d < D; d += 32) sq[warp][d] = Elem<T>::load(qrow + d);
-  __syncwarp();
-
-  const int first = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
-  float m = NEG_BIG, l = 0.f;
-  float acc[MAX_D / 32];
+  // the block's run of queries
+  const long long item = item0 + lane;
+  const bool there = lane < ITEMS && item < items;
+  const int my_t = there ? (int)(item / group) : 0;
+  const int my_seq = there ? token_seq[my_t] : -1;
+  const int my_pos = there ? positions[my_t] : -1;
+  const int before = __shfl_up_sync(0xffffffffu, my_seq, 1);
+  const unsigned starts = __ballot_sync(0xffffffffu, there && (lane == 0 || my_seq != before));
+  const int run = __popc(starts & (0xffffffffu >> (31 - lane))) - 1;
+  const unsigned mine = __ballot_sync(0xffffffffu, there && run == (int)blockIdx.y);
+  if (mine == 0u) return;                                // (the same for the whole block)
+  const int lane0 = __ffs(mine) - 1, count = __popc(mine);
+  const int seq = __shfl_sync(0xffffffffu, my_seq, lane0);
+  const bool in_run = (mine >> lane) & 1u;
+  const int my_first = window > 0 && my_pos - window + 1 > 0 ? my_pos - window + 1 : 0;
+  int lo = in_run ? my_first : 0x7fffffff, hi = in_run ? my_pos : -1;   // keys the run sees
 #pragma unroll
-  for (int i = 0; i < MAX_D / 32; ++i) acc[i] = 0.f;
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
 
+  const int ld = row_stride(D), vecs = (D + 3) / 4;
+  float* sk = smem;                                      // [2][KEYS][ld]
+  float* sv = sk + 2 * KEYS * ld;
+  float* sq = sv + 2 * KEYS * ld + warp * NQ * ld;       // this warp's queries
+  float* sp = smem + 4 * KEYS * ld + ITEMS * ld + warp * NQ * KEYS;
+
+  // queries number warp, warp + WARPS, ... of the run are this warp's
+  int nq = 0, first[NQ], pos[NQ];
+  long long row[NQ];
+#pragma unroll
+  for (int i = 0; i < NQ; ++i) {
+    const int n = warp + i * WARPS;
+    const int src = lane0 + (n < count ? n : 0);
+    first[i] = __shfl_sync(0xffffffffu, my_first, src);
+    pos[i] = __shfl_sync(0xffffffffu, my_pos, src);
+    const int t = __shfl_sync(0xffffffffu, my_t, src);
+    row[i] = ((long long)t * Hq + kvh * group + (int)((item0 + src) % group)) * D;
+    if (n < count) nq = i + 1;
+    for (int d = lane; d < 4 * vecs; d += 32)
+      sq[i * ld + d] = n < count && d < D ? Elem<T>::load(q + row[i] + d) : 0.f;
+  }
+
+  const int* bt = block_table + (size_t)seq * max_blocks;
   const size_t head_stride = (size_t)page_size * D;          // one head inside a page
   const size_t kv_stride = (size_t)Hkv * head_stride;        // keys -> values inside a page
   const size_t page_stride = 2 * kv_stride;
+  const int row0 = threadIdx.x / vecs, col0 = threadIdx.x % vecs;
+  const int row_step = THREADS / vecs, col_step = THREADS % vecs;
 
-  for (int k0 = (first / 32) * 32; k0 <= pos; k0 += 32) {
+  auto fetch = [&](int k0, int buf) {
     const int key = k0 + lane;
-    const bool visible = key >= first && key <= pos;
-    float s = NEG_BIG;
-    const T* vrow = nullptr;
-    if (visible) {
-      const int page = bt[key / page_size];
-      const T* krow = kv_cache + (size_t)page * page_stride + (size_t)kvh * head_stride +
-                      (size_t)(key % page_size) * D;
-      vrow = krow + kv_stride;
-      float dot = 0.f;
-      for (int d = 0; d < D; ++d) dot = fmaf(sq[warp][d], Elem<T>::load(krow + d), dot);
-      s = dot * scale;
-    }
-    const float tile_max = warp_max(s);
-    const float m_new = fmaxf(m, tile_max);   // the tile holds at least one visible key
-    const float p = visible ? expf(s - m_new) : 0.f;
-    const float alpha = expf(m - m_new);
-    l = l * alpha + warp_sum(p);
+    long long off = -1;                                  // of the lane's key; rows nobody sees become zeros
+    if (key >= lo && key <= hi)
+      off = (long long)((size_t)bt[key / page_size] * page_stride + (size_t)kvh * head_stride +
+                        (size_t)(key % page_size) * D);
+    float* dk = sk + buf * KEYS * ld;
+    float* dv = sv + buf * KEYS * ld;
+    int r = row0, c = col0;
+    for (int i = threadIdx.x; i < KEYS * vecs; i += THREADS) {   // (whole warps: KEYS * vecs is a multiple of 32)
+      const long long o = __shfl_sync(0xffffffffu, off, r);
+      if constexpr (ASYNC) {
+        const T* src = kv_cache + (o < 0 ? 0 : o + 4 * c);
+        const unsigned n = o < 0 ? 0u : 16u;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::
+                         "r"((unsigned)__cvta_generic_to_shared(dk + r * ld + 4 * c)), "l"(src), "r"(n) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::
+                         "r"((unsigned)__cvta_generic_to_shared(dv + r * ld + 4 * c)), "l"(o < 0 ? src : src + kv_stride),
+                         "r"(n) : "memory");
+      } else {
 #pragma unroll
-    for (int i = 0; i < MAX_D / 32; ++i) acc[i] *= alpha;
-    // P.V: keys in order, each lane owns dims lane, lane+32, ...
-    const unsigned long long vaddr = (unsigned long long)vrow;
-    for (int j = 0; j < 32; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, p, j);
-      const unsigned long long va = __shfl_sync(0xffffffffu, vaddr, j);
-      if (va == 0ull) continue;   // warp-uniform
-      const T* vr = (const T*)va;
-#pragma unroll
-      for (int i = 0; i < MAX_D / 32; ++i) {
-        const int d = lane + 32 * i;
-        if (d < D) acc[i] = fmaf(pj, Elem<T>::load(vr + d), acc[i]);
+        for (int e = 0; e < 4; ++e) {
+          const int d = 4 * c + e;
+          const bool in = o >= 0 && d < D;
+          dk[r * ld + d] = in ? Elem<T>::load(kv_cache + o + d) : 0.f;
+          dv[r * ld + d] = in ? Elem<T>::load(kv_cache + o + kv_stride + d) : 0.f;
+        }
+      }
+      r += row_step;
+      c += col_step;
+      if (c >= vecs) {
+        c -= vecs;
+        ++r;
       }
     }
-    m = m_new;
-  }
-  const float inv = 1.0f / l;
-  T* orow = out + ((size_t)t * Hq + h) * D;
+    if constexpr (ASYNC) asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  float m[NQ], l[NQ];
+  float4 acc[NQ][NV];
 #pragma unroll
-  for (int i = 0; i < MAX_D / 32; ++i) {
-    const int d = lane + 32 * i;
-    if (d < D) Elem<T>::store(orow + d, acc[i] * inv);
+  for (int i = 0; i < NQ; ++i) {
+    m[i] = NEG_BIG;
+    l[i] = 0.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) acc[i][n] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
+
+  const int begin = lo / KEYS * KEYS;
+  fetch(begin, 0);
+  int buf = 0;
+  for (int k0 = begin; k0 <= hi; k0 += KEYS, buf ^= 1) {
+    if constexpr (ASYNC) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                     // tile k0 is there; the other buffer has been read
+    if (k0 + KEYS <= hi) fetch(k0 + KEYS, buf ^ 1);
+    if (nq == 0) continue;
+    const float* krow = sk + (buf * KEYS + lane) * ld;
+    float s[NQ];
+    if (nq == 1) dots<1>(krow, sq, ld, vecs, s);
+    else dots<NQ>(krow, sq, ld, vecs, s);
+    const int key = k0 + lane;
+    bool whole = true;                                   // every query of the warp sees the whole tile
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      if (i >= nq) break;
+      whole = whole && first[i] <= k0 && pos[i] >= k0 + KEYS - 1;
+      if (first[i] > k0 + KEYS - 1 || pos[i] < k0) continue;          // it sees none of it
+      const bool visible = key >= first[i] && key <= pos[i];
+      const float x = visible ? s[i] * scale : NEG_BIG;
+      const float m_new = fmaxf(m[i], warp_max(x));      // the tile holds at least one visible key
+      const float p = visible ? expf(x - m_new) : 0.f;
+      const float alpha = expf(m[i] - m_new);
+      l[i] = fmaf(l[i], alpha, warp_sum(p));
+#pragma unroll
+      for (int n = 0; n < NV; ++n) {
+        acc[i][n].x *= alpha;
+        acc[i][n].y *= alpha;
+        acc[i][n].z *= alpha;
+        acc[i][n].w *= alpha;
+      }
+      m[i] = m_new;
+      sp[i * KEYS + lane] = p;
+    }
+    __syncwarp();
+    // P.V: keys in order, a lane owns the dimensions 4 * lane ..
+    const float* vt = sv + buf * KEYS * ld + 4 * lane;
+    auto add = [&](int i, float p, const float4 (&v)[NV]) {
+#pragma unroll
+      for (int n = 0; n < NV; ++n) {
+        acc[i][n].x = fmaf(p, v[n].x, acc[i][n].x);
+        acc[i][n].y = fmaf(p, v[n].y, acc[i][n].y);
+        acc[i][n].z = fmaf(p, v[n].z, acc[i][n].z);
+        acc[i][n].w = fmaf(p, v[n].w, acc[i][n].w);
+      }
+    };
+    auto value = [&](int j, float4 (&v)[NV]) {
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+        v[n] = lane + 32 * n < vecs ? *reinterpret_cast<const float4*>(vt + j * ld + 128 * n)
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if (whole) {
+#pragma unroll 2
+      for (int j = 0; j < KEYS; j += 4) {
+        float4 v0[NV], v1[NV], v2[NV], v3[NV];
+        value(j, v0);
+        value(j + 1, v1);
+        value(j + 2, v2);
+        value(j + 3, v3);
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+          if (i >= nq) break;
+          const float4 p = *reinterpret_cast<const float4*>(sp + i * KEYS + j);
+          add(i, p.x, v0);
+          add(i, p.y, v1);
+          add(i, p.z, v2);
+          add(i, p.w, v3);
+        }
+      }
+    } else {
+      const int j1 = min(KEYS - 1, hi - k0);
+      for (int j = 0; j <= j1; ++j) {
+        float4 v[NV];
+        value(j, v);
+#pragma unroll
+        for (int i = 0; i < NQ; ++i)      // (a key that a query does not see adds nothing, not even 0 times its value)
+          if (i < nq && k0 + j >= first[i] && k0 + j <= pos[i]) add(i, sp[i * KEYS + j], v);
+      }
+    }
+    __syncwarp();                                        // sp is written again in the next tile
+  }
+#pragma unroll
+  for (int i = 0; i < NQ; ++i) {
+    if (i >= nq) break;
+    const float inv = 1.0f / l[i];
+    T* orow = out + row[i];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+      const int d = 4 * (lane + 32 * n);
+      if (d < D) Elem<T>::store(orow + d, acc[i][n].x * inv);
+      if (d + 1 < D) Elem<T>::store(orow + d + 1, acc[i][n].y * inv);
+      if (d + 2 < D) Elem<T>::store(orow + d + 2, acc[i][n].z * inv);
+      if (d + 3 < D) Elem<T>::store(orow + d + 3, acc[i][n].w * inv);
+    }
+  }
+}
+
+template <typename T, int NV, bool ASYNC>
+int launch(const T* q, T* out, const T* kv, const int* bt, int max_blocks, const int* token_seq, const int* positions,
+           int tokens, int Hq, int Hkv, int D, int page_size, float scale, int window, cudaStream_t st) {
+  static DeviceOnce once;
+  if (!once.done()) {
+    if (cudaFuncSetAttribute(paged_attention_generic_kernel<T, NV, ASYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             4 * smem_floats(MAX_D)) != cudaSuccess) {
+      cudaGetLastError();
+      return DIB_LAUNCH_FAILED;
+    }
+    once.mark();
+  }
+  const int group = Hq / Hkv;
+  const long long blocks = ((long long)tokens * group + ITEMS - 1) / ITEMS;
+  // 16 neighbouring queries touch at most this many tokens, and as many sequences
+  int runs = (ITEMS + group - 2) / group + 1;
+  if (runs > ITEMS) runs = ITEMS;
+  if (runs > tokens) runs = tokens;
+  dib_launch(paged_attention_generic_kernel<T, NV, ASYNC>, dim3((unsigned)(blocks * Hkv), runs), dim3(THREADS),
+             4 * smem_floats(D), st, q, out, kv, bt, max_blocks, token_seq, positions, tokens, Hq, Hkv, D, page_size,
+             scale, window);
+  DIB_CHECK_LAUNCH();
+  return DIB_OK;
 }
 
 }  // namespace
@@ -110,17 +311,18 @@ extern "C" int dib_paged_attention_generic(const void* q, void* out, const void*
                                            int window, int dtype, cudaStream_t st) {
   if (T == 0) return DIB_OK;
   if (D < 1 || D > MAX_D || Hkv < 1 || Hq % Hkv != 0 || page_size < 1) return DIB_BAD_SIZE;
-  const long long items = (long long)T * Hq;
-  const int blocks = ceil_div_host(items, WARPS);
-  if (dtype == 0)
-    dib_launch(paged_attention_generic_kernel<float>, dim3(blocks), dim3(WARPS * 32), 0, st, 
-        (const float*)q, (float*)out, (const float*)kv_cache, block_table, max_blocks, token_seq,
-        positions, T, Hq, Hkv, D, page_size, scale, window);
-  else if (dtype == 1)
-    dib_launch(paged_attention_generic_kernel<__nv_bfloat16>, dim3(blocks), dim3(WARPS * 32), 0, st, 
-        (const __nv_bfloat16*)q, (__nv_bfloat16*)out, (const __nv_bfloat16*)kv_cache, block_table,
-        max_blocks, token_seq, positions, T, Hq, Hkv, D, page_size, scale, window);
-  else return DIB_BAD_DTYPE;
-  DIB_CHECK_LAUNCH();
-  return DIB_OK;
+  if (((long long)T * (Hq / Hkv) + ITEMS - 1) / ITEMS * Hkv > 0x7fffffffll) return DIB_BAD_SIZE;
+  auto go = [&](auto* tag, auto async) {
+    using E = std::remove_pointer_t<decltype(tag)>;
+    constexpr bool A = decltype(async)::value;
+    return D <= 128 ? launch<E, 1, A>((const E*)q, (E*)out, (const E*)kv_cache, block_table, max_blocks, token_seq,
+                                      positions, T, Hq, Hkv, D, page_size, scale, window, st)
+                    : launch<E, 2, A>((const E*)q, (E*)out, (const E*)kv_cache, block_table, max_blocks, token_seq,
+                                      positions, T, Hq, Hkv, D, page_size, scale, window, st);
+  };
+  if (dtype == 0)     // (rows of the cache start on 16 bytes when D is a multiple of 4)
+    return D % 4 == 0 && ((uintptr_t)kv_cache & 15) == 0 ? go((float*)nullptr, std::true_type{})
+                                                         : go((float*)nullptr, std::false_type{});
+  if (dtype == 1) return go((__nv_bfloat16*)nullptr, std::false_type{});
+  return DIB_BAD_DTYPE;
 }

@@ -678,6 +678,41 @@ def test_paged_attention_cut_and_batch_invariance(dtype):
     assert torch.equal(again, whole)
 
 
+@pytest.mark.parametrize("dtype,hq,hkv,d,window", [
+    (torch.float32, 4, 2, 128, 0), (torch.float32, 3, 1, 20, 0), (torch.float32, 2, 2, 33, 40),
+    (torch.float32, 40, 2, 132, 0), (torch.float32, 1, 1, 256, 33), (torch.bfloat16, 17, 1, 64, 0),
+    (torch.bfloat16, 2, 1, 250, 31)])
+def test_generic_attention_runs_of_queries(dtype, hq, hkv, d, window):
+    """Blocks of 16 neighbouring queries that belong to several sequences, one query or a whole tile of them,
+    rows that are no whole vectors; keys behind a query do not reach it, whatever their values are."""
+    lens = [1, 32, 33, 150, 64, 97]
+    case = PagedCase(lens, hkv, d, 16, dtype, seed=61)
+    cuts = {0: (0, 1), 1: (31, 1), 2: (32, 1), 5: (96, 1), 3: (63, 87), 4: (0, 64)}
+    g = torch.Generator().manual_seed(62)
+    q = torch.randn(sum(n for _, n in cuts.values()), hq, d, generator=g).to(device="cuda", dtype=dtype)
+    scale = d ** -0.5
+    meta = case.meta(list(cuts), list(cuts.values()))
+    got = ops().paged_attention(q, case.cache, meta, scale, window or None)
+    # values of the prompt's last keys become infinite: only queries that see them change
+    pages = torch.tensor(case.tables[3], device="cuda")
+    spoilt = case.cache.clone()
+    for p in range(140, 150):
+        spoilt[pages[p // 16], 1, :, p % 16] = float("inf")
+    again = ops().paged_attention(q, spoilt, meta, scale, window or None)
+    at = 0
+    for s, (first, n) in cuts.items():
+        want = dense_reference(q[at:at + n], case.k[s], case.v[s], scale, range(first, first + n), window)
+        # d roundings in a score, one per key in the sums; bfloat16 results add their own rounding
+        size = scale * (q[at:at + n].abs().float().amax() * case.k[s].abs().float().amax()) * d
+        err = (2 * d * 2.0 ** -24 * size + (lens[s] + 8) * 2.0 ** -24) * 2 * case.v[s].abs().float().amax()
+        err = err + (2.0 ** -8 * want.abs() if dtype == torch.bfloat16 else 0)
+        assert ((got[at:at + n].float() - want).abs() <= err).all(), s
+        for i, p in enumerate(range(first, first + n)):
+            if s != 3 or p < 140:
+                assert torch.equal(again[at + i], got[at + i]), (s, p)
+        at += n
+
+
 # ------------------------------------------------------------------ sampling
 
 def test_argmax_lowest_index_on_ties():
