@@ -286,10 +286,9 @@ moe_product_mma_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __re
       *reinterpret_cast<uint4*>(As + r * as + c8 * 8) = v;
     }
     __syncthreads();
-    // The weight loads of AHEAD steps are issued before the first step's products (tiles of 16 rows are
-    // bound by the loads in flight).  No load has a condition: past the run's end it reads the row's
-    // first elements, which meet the zeros staged there.
-    constexpr int AHEAD = MT == 1 ? 16 / NJ : 2;
+    // The weight loads of AHEAD steps are issued before the first step's products.  No load has a
+    // condition: past the run's end it reads the row's first elements, which meet the zeros staged there.
+    constexpr int AHEAD = 2;
     for (int k0 = 0; k0 < kpad; k0 += 32 * AHEAD) {
       uint4 b[AHEAD][NJ];
 #pragma unroll
@@ -353,6 +352,110 @@ moe_product_mma_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __re
           }
       }
     }
+}
+
+// The same for tiles of 16 rows (decoded tokens), where an expert's weights are read for a few rows
+// and the time is that of their bytes.  A CTA takes 32 rows of B (mode 0: 16 of the gate and the same
+// 16 of up), a warp 8 of them, and brings them and the tile's A rows into shared memory in runs of
+// ST_K k, ST_STAGES - 1 runs ahead by asynchronous copies of whole 512-byte pieces of a row: at
+// K = 1024 all of a CTA's 64 KB are asked for at once, by two CTAs an SM, while others multiply.  A
+// row's sum is the same as above: steps of 32 k, ascending, in the same permutation.
+// (8 tokens, 2 of 16 experts each, 1024 x 1536, 66 MB and 33 MB of weights: gate and up 22 .. 27 us, down
+// 13 .. 15 us; weights loaded into registers 16 loads ahead, four warps of 32 columns a CTA: 50 and
+// 59 .. 75 us.)
+constexpr int ST_THREADS = 128, ST_B = 32, ST_A = 16, ST_K = 256, ST_STAGES = 4;
+constexpr int ST_LD = ST_K + GP_PAD;
+constexpr int ST_STAGE = (ST_B + ST_A) * ST_LD;                    // elements
+__global__ void __launch_bounds__(ST_THREADS, 2)
+moe_product_stream_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __restrict__ order, int max_tiles,
+                          int top, const __nv_bfloat16* __restrict__ w, void* out, int K, int N, int mode, float limit,
+                          float alpha) {
+  extern __shared__ __align__(16) unsigned char gp_smem[];
+  __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(gp_smem);
+  __shared__ float up_sums[2][32][4];
+  pdl_prologue(a_rows, order);
+  const int tl = blockIdx.x % max_tiles;
+  const int expert = order[(long long)max_tiles * ST_A + tl];
+  if (expert < 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+  const int cols = mode == 0 ? ST_B / 2 : ST_B;
+  const int n0 = (int)(blockIdx.x / max_tiles) * cols;
+  const int* pairs = order + (long long)tl * ST_A;
+  // this warp copies rows warp, warp + 4, ... of a run: 32 lanes of 16 bytes each
+  constexpr int ROWS = (ST_B + ST_A) / 4;
+  const __nv_bfloat16* from[ROWS];                       // null: a row of zeros
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const int r = warp + 4 * i;
+    from[i] = nullptr;
+    if (r < ST_B) {
+      const int n = n0 + (mode == 0 ? r % (ST_B / 2) : r);
+      const long long rb = (mode == 0 && r >= ST_B / 2 ? (long long)N : 0ll) + n;
+      if (n < N) from[i] = w + ((long long)expert * (mode == 0 ? 2 * N : N) + rb) * K + lane * 8;
+    } else {
+      const int pair = pairs[r - ST_B];
+      const long long arow = mode != 1 ? pair / top : (long long)tl * ST_A + r - ST_B;
+      if (pair >= 0) from[i] = a_rows + arow * K + lane * 8;
+    }
+  }
+  const int runs = (K + ST_K - 1) / ST_K;
+  auto fetch = [&](int run) {
+    if (run < runs) {
+      const bool in = run * ST_K + lane * 8 < K;
+      __nv_bfloat16* to = ring + (run % ST_STAGES) * ST_STAGE + warp * ST_LD + lane * 8;
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const bool there = in && from[i] != nullptr;
+        const __nv_bfloat16* src = there ? from[i] + run * ST_K : w;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::
+                         "r"((unsigned)__cvta_generic_to_shared(to + 4 * i * ST_LD)), "l"(src), "r"(there ? 16 : 0)
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int k = 0; k < ST_STAGES - 1; ++k) fetch(k);
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int run = 0; run < runs; ++run) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(ST_STAGES - 2) : "memory");
+    __syncthreads();                 // the run is there for all; the one before has been read by all
+    fetch(run + ST_STAGES - 1);
+    const __nv_bfloat16* b = ring + (run % ST_STAGES) * ST_STAGE + (warp * 8 + g) * ST_LD + tig * 8;
+    const __nv_bfloat16* a = ring + (run % ST_STAGES) * ST_STAGE + (ST_B + g) * ST_LD + tig * 8;
+    const int klen = min(ST_K, K - run * ST_K);
+#pragma unroll 4
+    for (int k = 0; k < klen; k += 32) {
+      const uint4 lo = *reinterpret_cast<const uint4*>(a + k);
+      const uint4 hi = *reinterpret_cast<const uint4*>(a + 8 * ST_LD + k);
+      const uint4 x = *reinterpret_cast<const uint4*>(b + k);
+      mma_bf16_16816(acc, lo.x, hi.x, lo.y, hi.y, x.x, x.y);
+      mma_bf16_16816(acc, lo.z, hi.z, lo.w, hi.w, x.z, x.w);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (mode == 0) {                   // the warps of up hand their sums to those of the gate
+    if (warp >= 2) *reinterpret_cast<float4*>(up_sums[warp - 2][lane]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    __syncthreads();
+    if (warp >= 2) return;
+  }
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    const int r = g + 8 * hh;
+    const int pair = pairs[r];
+    if (pair < 0) continue;
+    const long long row = mode == 1 ? pair : (long long)tl * ST_A + r;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int n = n0 + warp * 8 + tig * 2 + e;
+      const float v = acc[2 * hh + e];
+      if (n >= N) continue;
+      if (mode == 1) reinterpret_cast<float*>(out)[row * N + n] = v;
+      else
+        reinterpret_cast<__nv_bfloat16*>(out)[row * N + n] =
+            __float2bfloat16_rn(mode == 0 ? expert_gate(v, up_sums[warp][lane][2 * hh + e], limit, alpha) : gelu_erf(v));
+    }
+  }
 }
 
 // CUDA-core form: any type, any sizes.  A CTA takes 16 rows of a tile (blockIdx.z picks them) and 128
@@ -458,10 +561,9 @@ __global__ void moe_combine_kernel(const float* __restrict__ per_pair, const flo
 template <int MT, int NJ>
 int launch_product_mma(const void* a_rows, const int* order, int max_tiles, int tile, int top, const void* w, void* out,
                        int K, int N, int mode, float limit, float alpha, cudaStream_t st) {
-  // the A rows' k are staged in runs of KC (a multiple of 64) that fit 64 KB; tiles of 16 rows (decoded
-  // tokens: the product is bound by how many weight loads an SM keeps in flight) in runs that fit 16 KB,
-  // so that an SM holds many CTAs.  The runs do not change the order of a sum.
-  int KC = ((MT == 1 ? 16 : 64) * 1024 / (MT * 16 * 2) - GP_PAD) / 64 * 64;
+  // the A rows' k are staged in runs of KC (a multiple of 64) that fit 64 KB.  The runs do not change the
+  // order of a sum.
+  int KC = (64 * 1024 / (MT * 16 * 2) - GP_PAD) / 64 * 64;
   if (KC > (K + 63) / 64 * 64) KC = (K + 63) / 64 * 64;
   const size_t smem = (size_t)MT * 16 * (KC + GP_PAD) * 2;
   static DeviceOnce once;
@@ -478,13 +580,31 @@ int launch_product_mma(const void* a_rows, const int* order, int max_tiles, int 
   return DIB_OK;
 }
 
+int launch_product_stream(const void* a_rows, const int* order, int max_tiles, int top, const void* w, void* out, int K,
+                          int N, int mode, float limit, float alpha, cudaStream_t st) {
+  constexpr size_t smem = sizeof(__nv_bfloat16) * ST_STAGES * ST_STAGE;      // 108 KB
+  static DeviceOnce once;
+  if (!once.done()) {
+    if (cudaFuncSetAttribute(moe_product_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return DIB_LAUNCH_FAILED;
+    once.mark();
+  }
+  const int cols = mode == 0 ? ST_B / 2 : ST_B;
+  const long long blocks = (long long)max_tiles * ((N + cols - 1) / cols);
+  if (blocks > 0x7fffffffll) return DIB_BAD_SIZE;
+  dib_launch(moe_product_stream_kernel, dim3((unsigned)blocks), dim3(ST_THREADS), smem, st,
+             (const __nv_bfloat16*)a_rows, order, max_tiles, top, (const __nv_bfloat16*)w, out, K, N, mode, limit, alpha);
+  DIB_CHECK_LAUNCH();
+  return DIB_OK;
+}
+
 // mode 0: gate and up; 1: down; 2: up alone.  dtype 0 float32, 1 bfloat16.
 int moe_product(const void* a_rows, int dtype, const int* order, int max_tiles, int tile, int top, const void* w,
                 void* out, int K, int N, int mode, float limit, float alpha, cudaStream_t st) {
   if (max_tiles == 0) return DIB_OK;
   if (K < 1 || N < 1 || tile < 1 || tile % GC_ROWS || top < 1) return DIB_BAD_SIZE;
   if (dtype == 1 && K % 8 == 0 && (tile == 16 || tile == 64)) {
-    if (tile == 16) return launch_product_mma<1, 4>(a_rows, order, max_tiles, tile, top, w, out, K, N, mode, limit, alpha, st);
+    if (tile == 16) return launch_product_stream(a_rows, order, max_tiles, top, w, out, K, N, mode, limit, alpha, st);
     return launch_product_mma<4, 4>(a_rows, order, max_tiles, tile, top, w, out, K, N, mode, limit, alpha, st);
   }
   const dim3 grid(max_tiles, (N + GC_COLS - 1) / GC_COLS, tile / GC_ROWS);

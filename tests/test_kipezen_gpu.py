@@ -123,6 +123,27 @@ def test_the_experts_products_alone(dtype, experts, top, width, ff, rows):
         assert torch.equal(few, got[:3])
 
 
+@pytest.mark.parametrize("width, ff, gated", [(256, 512, True), (264, 24, True), (1032, 40, True), (8, 8, True),
+                                              (520, 260 * 4, False), (24, 56, False)])
+def test_the_experts_streamed_products(width, ff, gated):
+    """Tiles of 16 rows: runs of k and blocks of columns that are not full; the rows' bits are those of the
+    64-row tiles (a step with 64 rows an expert on average)."""
+    from deterministic_inference_b200.kernels import ops
+    experts, top = 3, 2
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    rows = 64 * experts // top + 3
+    x = rnd(rows, width)
+    up, down = rnd(experts, (2 if gated else 1) * ff, width) * 0.1, rnd(experts, width, ff) * 0.1
+    ids = torch.rand(rows, experts, generator=g, device="cuda").argsort(1)[:, :top].int()
+    weights = torch.rand(rows, top, generator=g, device="cuda")
+    run = lambda n: ops.routed_experts(x[:n], ids[:n].contiguous(), weights[:n].contiguous(), up, down, None, None, experts,
+                                       torch.bfloat16, gated=gated)
+    whole = run(rows)
+    for n in (1, 5, 17, 40):
+        assert torch.equal(run(n), whole[:n]), n
+
+
 # ---- whole models ------------------------------------------------------------------------------------------
 
 CASES = {       # configuration -> request lengths, seed
