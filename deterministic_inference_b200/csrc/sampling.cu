@@ -152,34 +152,81 @@ __global__ void gumbel_sample_kernel(const float* __restrict__ logits,
 // maximum; then, with the row's maximum and sum put together from the chunks' in chunk
 // order (a row's normaliser never depends on the batch), the chunk's best score; then
 // the best chunk (argmax_final_kernel).
-__global__ void gumbel_stats_kernel(const float* __restrict__ logits,
-                                    const float* __restrict__ temperatures,
-                                    float* __restrict__ cmax, float* __restrict__ csum,
-                                    unsigned* __restrict__ hist_cnt,
-                                    unsigned long long* __restrict__ hist_mass, int R, int V,
-                                    int chunks) {
+//
+// The chunk lies in registers, 16 ids a thread, loaded before anything else is waited for.
+// These kernels are bound by instructions, not by the logits (39 MB for 64 rows of 151,936
+// stay in L2): a probability costs two divisions and an exponential, a score three more
+// logarithms.  So each of them first looks at a cheap value with a margin (log2 of the
+// probability by one FMA, an upper bound of the score by one logarithm more) and forms the
+// exact one, always by the same expressions, only where that can matter.
+constexpr int SAMPLE_THREADS = 256;
+constexpr int PER_THREAD = ARGMAX_CHUNK / SAMPLE_THREADS;
+
+__device__ __forceinline__ void load_chunk(const float* __restrict__ row, int lo, int hi, float (&x)[PER_THREAD]) {
+#pragma unroll
+  for (int j = 0; j < PER_THREAD; ++j) {
+    const int i = lo + threadIdx.x + j * SAMPLE_THREADS;
+    x[j] = i < hi ? row[i] : -INFINITY;
+  }
+}
+
+// top-k / top-p without a sort.  In the order of a descending sort a token stays when
+// its rank is below k and the probability mass before it is at most top_p (rank 0 always
+// stays).  Rank and mass before are both non-increasing in the token's probability, so
+// the kept set is {p >= t} for one threshold t: found by a radix descent over the 31
+// bits of the probability (it has no sign), 10, 11 and 10 bits a pass, with a histogram of
+// counts and of masses per pass.  Masses are added as 40-bit fixed point, so that the order
+// of the additions (atomics) cannot change a bit.  Tokens that tie with the threshold all
+// stay (a sort would keep some of them).  A pass is one kernel with a block per chunk of a
+// row; the histograms lie in global memory (masses [R][FILTER_BINS], then the rows'
+// states and normalisers, then counts; zeroed by the kernel that computes the normaliser); every block works out
+// the bits of the pass before its own, on top of the state that pass's first block left.
+// (Four passes of 8 bits that formed every probability again, added up a warp's equal bins
+// by matching lanes and chained the chunks' normalisers in every thread: 69 us each, and
+// the pick 68 us; with 64 rows of 151,936, 38 of them filtered, the whole draw 318 us, so 122 us.)
+constexpr float MASS_ONE = 1099511627776.0f;     // 2^40
+constexpr int FILTER_PASSES = 3;
+constexpr int FILTER_BINS = 4096;                // 1024 + 2048 + 1024
+__host__ __device__ __forceinline__ constexpr int pass_bits(int pass) { return pass == 1 ? 11 : 10; }
+__host__ __device__ __forceinline__ constexpr int pass_shift(int pass) { return pass == 0 ? 21 : pass == 1 ? 10 : 0; }
+__host__ __device__ __forceinline__ constexpr int pass_first_bin(int pass) { return pass == 0 ? 0 : pass == 1 ? 1024 : 3072; }
+
+struct FilterState {
+  unsigned long long cnt_above, mass_above;   // tokens (and their mass) above the chosen bins
+  unsigned prefix;                            // the threshold's bits found so far
+  unsigned pad;
+};
+
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+gumbel_stats_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
+                    float* __restrict__ cmax, float* __restrict__ csum, unsigned* __restrict__ hist_cnt,
+                    unsigned long long* __restrict__ hist_mass, int V, int chunks) {
   pdl_prologue(logits, temperatures);
   __shared__ float fscratch[32];
   const int r = blockIdx.y, c = blockIdx.x;
-  // the row's top-k / top-p histograms (4 passes x 256 bins) start from zero: the blocks
-  // of the row share the zeroing
+  // the row's top-k / top-p histograms start from zero: the blocks of the row share the zeroing
   if (hist_cnt != nullptr) {
-    for (int e = c * blockDim.x + threadIdx.x; e < 4 * 256; e += chunks * blockDim.x) {
-      const size_t at = ((size_t)(e >> 8) * R + r) * 256 + (e & 255);
-      hist_cnt[at] = 0u;
-      hist_mass[at] = 0ull;
+    for (int e = c * SAMPLE_THREADS + threadIdx.x; e < FILTER_BINS; e += chunks * SAMPLE_THREADS) {
+      hist_cnt[(size_t)r * FILTER_BINS + e] = 0u;
+      hist_mass[(size_t)r * FILTER_BINS + e] = 0ull;
     }
   }
   const float temp = temperatures[r];
   if (temp <= 0.f) return;     // a greedy row needs no normaliser
-  const float* row = logits + (size_t)r * V;
   const int lo = c * ARGMAX_CHUNK, hi = min(V, lo + ARGMAX_CHUNK);
+  float x[PER_THREAD];
+  load_chunk(logits + (size_t)r * V, lo, hi, x);
   float mx = -INFINITY;
-  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) mx = fmaxf(mx, row[i] / temp);
-  mx = block_max(mx, fscratch);
+#pragma unroll
+  for (int j = 0; j < PER_THREAD; ++j) mx = fmaxf(mx, x[j]);
+  // (rounding keeps order: the largest quotient is the quotient of the largest)
+  mx = block_max(mx, fscratch) / temp;
   float sum = 0.f;
-  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) sum += expf(row[i] / temp - mx);
+#pragma unroll
+  for (int j = 0; j < PER_THREAD; ++j)
+    if (lo + (int)threadIdx.x + j * SAMPLE_THREADS < hi) sum += expf(x[j] / temp - mx);
   sum = block_sum(sum, fscratch);
+  if (mx == -INFINITY) sum = 0.f;      // (a chunk of ids that are all out adds nothing to its row)
   if (threadIdx.x == 0) {
     cmax[(size_t)r * chunks + c] = mx;
     csum[(size_t)r * chunks + c] = sum;
@@ -188,218 +235,358 @@ __global__ void gumbel_stats_kernel(const float* __restrict__ logits,
 
 // The row's maximum and sum of exponentials from its chunks', in chunk order: every
 // kernel that needs a probability forms it from these two, with the same expression, so
-// all of them see the same bits.
-__device__ __forceinline__ void row_normaliser(const float* __restrict__ cmax,
-                                               const float* __restrict__ csum, int r, int chunks,
-                                               float& mx, float& sum) {
+// all of them see the same bits.  The exponentials are taken by the threads side by side.
+struct NormaliserScratch {
+  float f[32], e[SAMPLE_THREADS], s[SAMPLE_THREADS];
+};
+__device__ __forceinline__ void row_normaliser(const float* __restrict__ cmax, const float* __restrict__ csum, int r,
+                                               int chunks, NormaliserScratch& sc, float& mx, float& sum) {
+  const float* cm = cmax + (size_t)r * chunks;
+  const float* cs = csum + (size_t)r * chunks;
   mx = -INFINITY;
-  for (int k = 0; k < chunks; ++k) mx = fmaxf(mx, cmax[(size_t)r * chunks + k]);
+  for (int k = threadIdx.x; k < chunks; k += SAMPLE_THREADS) mx = fmaxf(mx, cm[k]);
+  mx = block_max(mx, sc.f);
   sum = 0.f;
-  for (int k = 0; k < chunks; ++k)
-    sum += csum[(size_t)r * chunks + k] * expf(cmax[(size_t)r * chunks + k] - mx);
+  for (int base = 0; base < chunks; base += SAMPLE_THREADS) {
+    __syncthreads();
+    if (base + (int)threadIdx.x < chunks) {
+      sc.e[threadIdx.x] = expf(cm[base + threadIdx.x] - mx);
+      sc.s[threadIdx.x] = cs[base + threadIdx.x];
+    }
+    __syncthreads();
+    const int n = min(SAMPLE_THREADS, chunks - base);
+#pragma unroll 8
+    for (int k = 0; k < n; ++k) sum = __fmaf_rn(sc.s[k], sc.e[k], sum);
+  }
 }
 __device__ __forceinline__ float row_probability(float logit, float temp, float mx, float sum) {
   return expf(logit / temp - mx) / sum;
 }
 
-// top-k / top-p without a sort.  In the order of a descending sort a token stays when
-// its rank is below k and the probability mass before it is at most top_p (rank 0 always
-// stays).  Rank and mass before are both non-increasing in the token's probability, so
-// the kept set is {p >= t} for one threshold t: found by a radix descent over the 32
-// bits of the probability, 8 bits a pass, with a histogram of counts and of masses per
-// pass.  Masses are added as 40-bit fixed point, so that the order of the additions
-// (atomics) cannot change a bit.  Tokens that tie with the threshold all stay (a sort
-// would keep some of them).  A pass is one kernel with a block per chunk of a row; the
-// histograms of the four passes lie in global memory ([4][R][256] counts and masses,
-// zeroed by the kernel that computes the normaliser), and every block works out the
-// bits fixed so far from the histograms of the passes before its own.
-constexpr float MASS_ONE = 1099511627776.0f;     // 2^40
-
-struct FilterState {
-  unsigned prefix;                      // the threshold's bits found so far
-  unsigned long long cnt_above, mass_above;   // tokens (and their mass) above the chosen bins
+// log2 of a probability up to `margin`, by one FMA; not usable (`ok` false) at temperatures
+// and maxima whose products leave the range of float32.
+struct Estimate {
+  float a, c, margin;
+  bool ok;
+  __device__ __forceinline__ Estimate(float temp, float mx, float sum) {
+    a = 1.4426950408889634f / temp;
+    c = fmaf(mx, 1.4426950408889634f, log2f(sum));
+    ok = fabsf(a) < 1e30f && fabsf(c) < 1e30f;
+    // roundings of the quotient, of a and of the FMA: a few 2^-24 of |c| + 150, wherever the
+    // probability is not zero
+    margin = 1e-3f + 1e-6f * fabsf(c);
+  }
+  __device__ __forceinline__ float log2p(float logit) const { return fmaf(logit, a, -c); }
 };
+// bounds of log2p for probabilities whose bits lie in [first, last]; denormal ones have no
+// relative accuracy and get no tight bound
+__device__ __forceinline__ float lower_bound(unsigned first, const Estimate& e) {
+  return first < 0x01000000u ? -INFINITY : log2f(__uint_as_float(first)) - e.margin;
+}
+__device__ __forceinline__ float upper_bound(unsigned last, const Estimate& e) {
+  return last < 0x01000000u ? -100.f : log2f(__uint_as_float(last)) + e.margin;
+}
 
-// Warp 0 of the block: the state after `passes` passes, from their histograms.
+// The whole block: the state after pass `pass`, from the state before it and its histogram.
+struct DescendScratch {
+  unsigned long long m[8];
+  unsigned c[8];
+  int chosen[8];
+  FilterState st;
+};
+template <int BINS>
 __device__ __forceinline__ FilterState filter_descend(const unsigned* __restrict__ hist_cnt,
                                                       const unsigned long long* __restrict__ hist_mass,
-                                                      int R, int r, int passes, unsigned long long k,
-                                                      unsigned long long P) {
-  const int lane = threadIdx.x & 31;
-  FilterState st{0u, 0ull, 0ull};
-  for (int pass = 0; pass < passes; ++pass) {
-    const unsigned* hc = hist_cnt + ((size_t)pass * R + r) * 256 + lane * 8;
-    const unsigned long long* hm = hist_mass + ((size_t)pass * R + r) * 256 + lane * 8;
-    unsigned c[8];
-    unsigned long long m[8], csum = 0ull, msum = 0ull;
+                                                      FilterState st, int shift, unsigned long long k,
+                                                      unsigned long long P, DescendScratch& sc) {
+  constexpr int B = BINS / SAMPLE_THREADS;       // a thread's bins
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned c[B], csum = 0u;
+  unsigned long long m[B], msum = 0ull;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      c[j] = __ldcg(hc + j);
-      m[j] = __ldcg(hm + j);
-      csum += c[j];
-      msum += m[j];
-    }
-    // counts and masses of the bins of higher lanes (an exclusive suffix sum)
-    unsigned long long ca = 0ull, ma = 0ull;
-    {
-      unsigned long long c_run = csum, m_run = msum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long c_up = __shfl_down_sync(0xffffffffu, c_run, o);
-        const unsigned long long m_up = __shfl_down_sync(0xffffffffu, m_run, o);
-        if (lane + o < 32) {
-          c_run += c_up;
-          m_run += m_up;
-        }
-      }
-      ca = st.cnt_above + c_run - csum;     // inclusive suffix minus own
-      ma = st.mass_above + m_run - msum;
-    }
-    // this lane's bins from the highest down: the lowest non-empty bin that is entered
-    // while fewer than k tokens, weighing at most P, lie above it
-    int best = 256;
-    unsigned long long best_ca = 0ull, best_ma = 0ull;
-#pragma unroll
-    for (int j = 7; j >= 0; --j) {
-      if (c[j] != 0u && ca < k && ma <= P) {
-        best = lane * 8 + j;
-        best_ca = ca;
-        best_ma = ma;
-      }
-      ca += c[j];
-      ma += m[j];
-    }
-    int chosen = best;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) chosen = min(chosen, __shfl_xor_sync(0xffffffffu, chosen, o));
-    if (chosen == 256) chosen = 0;      // an empty histogram (cannot happen for a row that is filtered)
-    const int owner = chosen >> 3;
-    st.cnt_above = __shfl_sync(0xffffffffu, best == chosen ? best_ca : 0ull, owner);
-    st.mass_above = __shfl_sync(0xffffffffu, best == chosen ? best_ma : 0ull, owner);
-    st.prefix |= (unsigned)chosen << (24 - 8 * pass);
+  for (int j = 0; j < B; ++j) {
+    c[j] = __ldcg(hist_cnt + threadIdx.x * B + j);
+    m[j] = __ldcg(hist_mass + threadIdx.x * B + j);
+    csum += c[j];
+    msum += m[j];
   }
-  return st;
+  // counts and masses of the bins of higher threads (an exclusive suffix sum)
+  unsigned c_run = csum;
+  unsigned long long m_run = msum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned c_up = __shfl_down_sync(0xffffffffu, c_run, o);
+    const unsigned long long m_up = __shfl_down_sync(0xffffffffu, m_run, o);
+    if (lane + o < 32) {
+      c_run += c_up;
+      m_run += m_up;
+    }
+  }
+  __syncthreads();
+  if (lane == 0) {
+    sc.c[warp] = c_run;
+    sc.m[warp] = m_run;
+  }
+  __syncthreads();
+  unsigned long long ca = st.cnt_above + c_run - csum, ma = st.mass_above + m_run - msum;
+  for (int w = warp + 1; w < SAMPLE_THREADS / 32; ++w) {
+    ca += sc.c[w];
+    ma += sc.m[w];
+  }
+  // this thread's bins from the highest down: the lowest non-empty bin that is entered
+  // while fewer than k tokens, weighing at most P, lie above it
+  int best = BINS;
+  unsigned long long best_ca = 0ull, best_ma = 0ull;
+#pragma unroll
+  for (int j = B - 1; j >= 0; --j) {
+    if (c[j] != 0u && ca < k && ma <= P) {
+      best = threadIdx.x * B + j;
+      best_ca = ca;
+      best_ma = ma;
+    }
+    ca += c[j];
+    ma += m[j];
+  }
+  const int wbest = __reduce_min_sync(0xffffffffu, best);
+  if (lane == 0) sc.chosen[warp] = wbest;
+  __syncthreads();
+  int chosen = sc.chosen[0];
+#pragma unroll
+  for (int w = 1; w < SAMPLE_THREADS / 32; ++w) chosen = min(chosen, sc.chosen[w]);
+  // (an empty histogram, chosen == BINS, cannot happen for a row that is filtered: bin 0 then)
+  if (best == chosen && best < BINS) sc.st = FilterState{best_ca, best_ma, st.prefix | ((unsigned)best << shift), 0u};
+  if (chosen == BINS && threadIdx.x == 0) sc.st = FilterState{0ull, 0ull, st.prefix, 0u};
+  __syncthreads();
+  return sc.st;
+}
+// after pass `pass` (0 .. 2) of row r; `states` holds what the passes before it found, [FILTER_PASSES][R]
+__device__ __forceinline__ FilterState state_after(int pass, const unsigned* hist_cnt,
+                                                   const unsigned long long* hist_mass, const FilterState* states,
+                                                   int R, int r, unsigned long long k, unsigned long long P,
+                                                   DescendScratch& sc) {
+  FilterState st{0ull, 0ull, 0u, 0u};
+  if (pass > 0) {
+    const FilterState* at = states + (size_t)(pass - 1) * R + r;
+    st.cnt_above = __ldcg(&at->cnt_above);
+    st.mass_above = __ldcg(&at->mass_above);
+    st.prefix = __ldcg(&at->prefix);
+  }
+  const size_t first = (size_t)r * FILTER_BINS + pass_first_bin(pass);
+  return pass == 1 ? filter_descend<2048>(hist_cnt + first, hist_mass + first, st, pass_shift(1), k, P, sc)
+                   : filter_descend<1024>(hist_cnt + first, hist_mass + first, st, pass_shift(pass), k, P, sc);
 }
 
 __device__ __forceinline__ bool row_is_filtered(float temp, long long top_k, float top_p) {
   return temp > 0.f && (top_k > 0 || top_p < 1.0f);
 }
 
-__global__ void __launch_bounds__(256)
+template <int PASS>
+__global__ void __launch_bounds__(SAMPLE_THREADS)
 filter_histogram_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
                         const long long* __restrict__ top_ks, const float* __restrict__ top_ps,
                         const float* __restrict__ cmax, const float* __restrict__ csum,
                         unsigned* __restrict__ hist_cnt, unsigned long long* __restrict__ hist_mass,
-                        int pass, int R, int V, int chunks) {
-  pdl_prologue(logits, temperatures, top_ks, top_ps, cmax, csum);
-  __shared__ unsigned s_cnt[256];
-  __shared__ unsigned long long s_mass[256];
-  __shared__ unsigned s_prefix;
+                        FilterState* __restrict__ states, float2* __restrict__ norms, int R, int V, int chunks) {
+  pdl_prologue(logits, temperatures, top_ks, top_ps, cmax, csum, states, norms);
+  constexpr int BINS = 1 << pass_bits(PASS), SHIFT = pass_shift(PASS);
+  // 40-bit masses in two halves: a chunk's sums of either fit 32 bits, which shared memory adds natively
+  __shared__ unsigned s_cnt[BINS], s_low[BINS], s_high[BINS];
+  __shared__ NormaliserScratch nsc;
+  __shared__ DescendScratch dsc;
+  __shared__ float s_list[PASS == 0 ? 1 : ARGMAX_CHUNK];
+  __shared__ int s_listed;
   const int r = blockIdx.y, c = blockIdx.x;
   const float temp = temperatures[r];
   const long long top_k = top_ks[r];
   const float top_p = top_ps[r];
-  if (!row_is_filtered(temp, top_k, top_p)) return;
+  float mx, sum;
+  if (!row_is_filtered(temp, top_k, top_p)) {
+    if (PASS == 0 && c == 0 && temp > 0.f) {       // (the pick reads every row's normaliser)
+      row_normaliser(cmax, csum, r, chunks, nsc, mx, sum);
+      if (threadIdx.x == 0) norms[r] = make_float2(mx, sum);
+    }
+    return;
+  }
+  const int lo = c * ARGMAX_CHUNK, hi = min(V, lo + ARGMAX_CHUNK);
+  float x[PER_THREAD];
+  load_chunk(logits + (size_t)r * V, lo, hi, x);
   const unsigned long long k = top_k > 0 ? (unsigned long long)top_k : (unsigned long long)V + 1;
   const unsigned long long P = top_p >= 1.0f ? ~0ull : (unsigned long long)(top_p * MASS_ONE);
-  s_cnt[threadIdx.x] = 0u;
-  s_mass[threadIdx.x] = 0ull;
-  if (threadIdx.x < 32) {
-    const FilterState st = filter_descend(hist_cnt, hist_mass, R, r, pass, k, P);
-    if (threadIdx.x == 0) s_prefix = st.prefix;
+  for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS) s_cnt[b] = s_low[b] = s_high[b] = 0u;
+  if (threadIdx.x == 0) s_listed = 0;
+  unsigned prefix = 0u;
+  if constexpr (PASS > 0) {
+    const FilterState st = state_after(PASS - 1, hist_cnt, hist_mass, states, R, r, k, P, dsc);
+    if (c == 0 && threadIdx.x == 0) states[(size_t)(PASS - 1) * R + r] = st;
+    prefix = st.prefix;
+  }
+  if constexpr (PASS == 0) {
+    row_normaliser(cmax, csum, r, chunks, nsc, mx, sum);
+    if (c == 0 && threadIdx.x == 0) norms[r] = make_float2(mx, sum);
+  } else {
+    const float2 n = norms[r];
+    mx = n.x;
+    sum = n.y;
   }
   __syncthreads();
-  const unsigned prefix = s_prefix;
-  const int shift = 24 - 8 * pass;
-  const unsigned mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
-  const float* row = logits + (size_t)r * V;
-  float mx, sum;
-  row_normaliser(cmax, csum, r, chunks, mx, sum);
-  const int lo = c * ARGMAX_CHUNK, hi = min(V, lo + ARGMAX_CHUNK);
-  // In the first pass nearly all of a warp's 32 tokens fall into one or two bins (the top
-  // bits of small probabilities): the lanes of a bin add up among themselves and one of
-  // them updates the histogram, instead of 32 atomics on one address.
-  for (int i0 = lo; i0 < hi; i0 += 256) {
-    const int i = i0 + threadIdx.x;
-    unsigned bin = 0xffffffffu;               // no bin: outside the chunk or the prefix
-    unsigned long long m = 0ull;
-    if (i < hi) {
-      const float p = row_probability(row[i], temp, mx, sum);
-      const unsigned key = __float_as_uint(p);
-      if ((key & mask) == prefix) {
-        bin = (key >> shift) & 255u;
-        m = (unsigned long long)(p * MASS_ONE);
+
+  auto add = [&](float logit, bool in) {     // one token of the prefix; every lane of the warp calls
+    const float p = row_probability(logit, temp, mx, sum);
+    const unsigned key = __float_as_uint(p);
+    if constexpr (PASS > 0) in = in && (key >> (SHIFT + pass_bits(PASS))) == (prefix >> (SHIFT + pass_bits(PASS)));
+    const unsigned bin = (key >> SHIFT) & (BINS - 1);
+    const unsigned long long m = (unsigned long long)(p * MASS_ONE);
+    // 32 tokens of one bin (a flat row, a tail that underflows): one addition for the warp
+    const unsigned first = __shfl_sync(0xffffffffu, bin, 0);
+    if (__all_sync(0xffffffffu, in && bin == first)) {
+      const unsigned low = __reduce_add_sync(0xffffffffu, (unsigned)(m & 0xfffffull));
+      const unsigned high = __reduce_add_sync(0xffffffffu, (unsigned)(m >> 20));
+      if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_cnt[bin], 32u);
+        atomicAdd(&s_low[bin], low);
+        atomicAdd(&s_high[bin], high);
       }
+    } else if (in) {
+      atomicAdd(&s_cnt[bin], 1u);
+      atomicAdd(&s_low[bin], (unsigned)(m & 0xfffffull));
+      atomicAdd(&s_high[bin], (unsigned)(m >> 20));
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, bin);
-    if (bin == 0xffffffffu) continue;
-    // the group's mass: 40-bit values as two halves that 32-bit warp sums can take
-    const unsigned lo20 = __reduce_add_sync(peers, (unsigned)(m & 0xfffffull));
-    const unsigned hi20 = __reduce_add_sync(peers, (unsigned)(m >> 20));
-    if ((threadIdx.x & 31) == __ffs(peers) - 1) {
-      atomicAdd(&s_cnt[bin], (unsigned)__popc(peers));
-      atomicAdd(&s_mass[bin], ((unsigned long long)hi20 << 20) + lo20);
+  };
+  if constexpr (PASS == 0) {
+#pragma unroll
+    for (int j = 0; j < PER_THREAD; ++j) add(x[j], lo + (int)threadIdx.x + j * SAMPLE_THREADS < hi);
+  } else {
+    // the tokens that may have the prefix, side by side
+    const Estimate est(temp, mx, sum);
+    const unsigned rest = (1u << (SHIFT + pass_bits(PASS))) - 1u;
+    const float from = lower_bound(prefix, est), to = upper_bound(prefix | rest, est);
+    const int lane = threadIdx.x & 31;
+    unsigned in[PER_THREAD];                   // the warp's, a bit a lane
+    int found = 0;
+#pragma unroll
+    for (int j = 0; j < PER_THREAD; ++j) {
+      const float y = est.log2p(x[j]);
+      in[j] = __ballot_sync(0xffffffffu, lo + (int)threadIdx.x + j * SAMPLE_THREADS < hi &&
+                                             !(est.ok && (y < from || y > to)));
+      found += __popc(in[j]);
     }
+    int at = 0;
+    if (lane == 0 && found > 0) at = atomicAdd(&s_listed, found);
+    at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+    for (int j = 0; j < PER_THREAD; ++j) {
+      if ((in[j] >> lane) & 1u) s_list[at + __popc(in[j] & ((1u << lane) - 1u))] = x[j];
+      at += __popc(in[j]);
+    }
+    __syncthreads();
+    const int n = s_listed;
+    for (int i = threadIdx.x; i - lane < n; i += SAMPLE_THREADS) add(i < n ? s_list[i] : 0.f, i < n);
   }
   __syncthreads();
-  if (s_cnt[threadIdx.x] != 0u) {
-    const size_t at = ((size_t)pass * R + r) * 256 + threadIdx.x;
-    atomicAdd(&hist_cnt[at], s_cnt[threadIdx.x]);
-    atomicAdd(&hist_mass[at], s_mass[threadIdx.x]);
-  }
+  for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS)
+    if (s_cnt[b] != 0u) {
+      const size_t at = (size_t)r * FILTER_BINS + pass_first_bin(PASS) + b;
+      atomicAdd(&hist_cnt[at], s_cnt[b]);
+      atomicAdd(&hist_mass[at], ((unsigned long long)s_high[b] << 20) + s_low[b]);
+    }
 }
 
-__global__ void gumbel_pick_kernel(const float* __restrict__ logits,
-                                   const float* __restrict__ temperatures,
-                                   const long long* __restrict__ seeds,
-                                   const long long* __restrict__ sample_pos,
-                                   const unsigned char* __restrict__ keep,
-                                   const long long* __restrict__ top_ks,
-                                   const float* __restrict__ top_ps,
-                                   const unsigned* __restrict__ hist_cnt,
-                                   const unsigned long long* __restrict__ hist_mass,
-                                   unsigned* __restrict__ thresh,
-                                   const float* __restrict__ cmax, const float* __restrict__ csum,
-                                   float* __restrict__ pv, int* __restrict__ pi, int R, int V,
-                                   int chunks) {
-  pdl_prologue(logits, temperatures, seeds, sample_pos, keep, top_ks, top_ps, hist_cnt, hist_mass, cmax,
-               csum);
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+gumbel_pick_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
+                   const long long* __restrict__ seeds, const long long* __restrict__ sample_pos,
+                   const unsigned char* __restrict__ keep, const long long* __restrict__ top_ks,
+                   const float* __restrict__ top_ps, const unsigned* __restrict__ hist_cnt,
+                   const unsigned long long* __restrict__ hist_mass, const FilterState* __restrict__ states,
+                   const float2* __restrict__ norms, unsigned* __restrict__ thresh, const float* __restrict__ cmax, const float* __restrict__ csum,
+                   float* __restrict__ pv, int* __restrict__ pi, int R, int V, int chunks) {
+  pdl_prologue(logits, temperatures, seeds, sample_pos, keep, top_ks, top_ps, hist_cnt, hist_mass, states, norms,
+               cmax, csum);
   __shared__ Best bscratch[32];
-  __shared__ unsigned s_thresh;
+  __shared__ NormaliserScratch nsc;
+  __shared__ DescendScratch dsc;
   const int r = blockIdx.y, c = blockIdx.x;
-  // the threshold of top-k / top-p: all four passes' histograms are complete
-  if (threadIdx.x < 32) {
-    unsigned t = 0u;
-    if (thresh != nullptr) {
-      const long long top_k = top_ks[r];
-      const float top_p = top_ps[r];
-      if (row_is_filtered(temperatures[r], top_k, top_p)) {
-        const unsigned long long k = top_k > 0 ? (unsigned long long)top_k : (unsigned long long)V + 1;
-        const unsigned long long P = top_p >= 1.0f ? ~0ull : (unsigned long long)(top_p * MASS_ONE);
-        t = filter_descend(hist_cnt, hist_mass, R, r, 4, k, P).prefix;
-      }
-      if (threadIdx.x == 0 && c == 0) thresh[r] = t;
-    }
-    if (threadIdx.x == 0) s_thresh = t;
-  }
-  __syncthreads();
   const float* row = logits + (size_t)r * V;
   const int lo = c * ARGMAX_CHUNK, hi = min(V, lo + ARGMAX_CHUNK);
+  float x[PER_THREAD];
+  load_chunk(row, lo, hi, x);
   const float temp = temperatures[r];
+  // the threshold of top-k / top-p: all passes' histograms are complete
+  unsigned t = 0u;
+  if (thresh != nullptr) {
+    const long long top_k = top_ks[r];
+    const float top_p = top_ps[r];
+    if (row_is_filtered(temp, top_k, top_p)) {
+      const unsigned long long k = top_k > 0 ? (unsigned long long)top_k : (unsigned long long)V + 1;
+      const unsigned long long P = top_p >= 1.0f ? ~0ull : (unsigned long long)(top_p * MASS_ONE);
+      t = state_after(FILTER_PASSES - 1, hist_cnt, hist_mass, states, R, r, k, P, dsc).prefix;
+    }
+    if (threadIdx.x == 0 && c == 0) thresh[r] = t;
+  }
   Best b{-INFINITY, INT_MAX_};
   if (temp <= 0.f) {
-    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) b = better(b, Best{row[i], i});
+#pragma unroll
+    for (int j = 0; j < PER_THREAD; ++j) {
+      const int i = lo + threadIdx.x + j * SAMPLE_THREADS;
+      if (i < hi) b = better(b, Best{x[j], i});
+    }
   } else {
     float mx, sum;
-    row_normaliser(cmax, csum, r, chunks, mx, sum);
+    if (norms != nullptr) {
+      const float2 n = norms[r];
+      mx = n.x;
+      sum = n.y;
+    } else {
+      row_normaliser(cmax, csum, r, chunks, nsc, mx, sum);
+    }
     const long long seed = seeds[r], pos = sample_pos[r];
     const unsigned char* krow = keep ? keep + (size_t)r * V : nullptr;
-    const unsigned t = s_thresh;
-    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-      if (krow && !krow[i]) continue;
-      const float p = row_probability(row[i], temp, mx, sum);
-      if (__float_as_uint(p) < t) continue;
-      b = better(b, Best{logf(p + 1e-10f) + seeded_gumbel(seed, pos, i), i});
+    const Estimate est(temp, mx, sum);
+    const float from = lower_bound(t, est);
+    // An upper bound of every id's score, in bits.  With v = 1 - u, exact, the noise is at most
+    // -log(v), because -log(1 - v) >= v; log(p + 1e-10) is at most the larger of the two logarithms
+    // plus what the smaller adds: 1e-10 / p below p = 2^-20, at most one bit beyond.
+    float ub[PER_THREAD];
+    unsigned alive = 0u;
+    int top = -1;
+    float top_ub = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < PER_THREAD; ++j) {
+      const int i = lo + threadIdx.x + j * SAMPLE_THREADS;
+      const float y = est.log2p(x[j]);
+      const unsigned long long step =
+          ((unsigned long long)seed * 19349663ull) ^ ((unsigned long long)pos * 73856093ull);
+      const unsigned hashed = (unsigned)((step * 8589934591ull) ^ ((unsigned long long)i * 479001599ull)) & 0xffffffu;
+      const float v = (float)(0x1000000u - hashed) * (1.0f / 16777216.0f);
+      ub[j] = fmaxf(y, -33.2192f) + (y > -20.f ? 2e-4f : 1.0f) - __log2f(v) + est.margin;
+      if (!est.ok) ub[j] = INFINITY;
+      if (i < hi && !(krow && !krow[i]) && !(est.ok && y < from)) {
+        alive |= 1u << j;
+        if (top < 0 || ub[j] > top_ub) {
+          top = j;
+          top_ub = ub[j];
+        }
+      }
+    }
+    // every thread's most promising id first, then whatever may still beat the best of those
+    unsigned todo = top >= 0 ? 1u << top : 0u;
+    alive &= ~todo;
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+      if (round == 1) {
+        const float reached = block_best(b, bscratch).v * 1.4426950408889634f;
+        const float slack = 1e-6f * fabsf(reached);
+        todo = 0u;
+#pragma unroll
+        for (int j = 0; j < PER_THREAD; ++j)
+          if (((alive >> j) & 1u) && !(ub[j] < reached - slack)) todo |= 1u << j;
+      }
+      while (todo != 0u) {
+        const int i = lo + threadIdx.x + (__ffs(todo) - 1) * SAMPLE_THREADS;
+        todo &= todo - 1u;
+        const float p = row_probability(row[i], temp, mx, sum);
+        if (__float_as_uint(p) < t) continue;
+        b = better(b, Best{logf(p + 1e-10f) + seeded_gumbel(seed, pos, i), i});
+      }
     }
   }
   b = block_best(b, bscratch);
@@ -450,8 +637,12 @@ int dib_gumbel_sample(const float* logits, const float* temperatures, const long
 // scratch_i: int [R, chunks], chunks = dib_argmax_chunks(V).
 // top_ks / top_ps (both or neither): per-row top-k (<= 0: off) and top-p (>= 1: off),
 // applied by a threshold found without a sort.  thresh: unsigned [R], receives the bits of
-// each row's smallest kept probability (0 = all kept); hist: scratch of 4 * R * 256 * 12
-// bytes, 8-byte aligned (masses first, then counts).
+// each row's smallest kept probability (0 = all kept); hist: scratch of dib_filter_scratch(R)
+// bytes, 8-byte aligned (masses, the rows' states, the rows' normalisers, counts).
+long long dib_filter_scratch(int R) {
+  return (long long)R * (FILTER_BINS * 12ll + FILTER_PASSES * (long long)sizeof(FilterState) + (long long)sizeof(float2));
+}
+
 int dib_gumbel_sample_chunked(const float* logits, const float* temperatures, const long long* seeds,
                               const long long* sample_pos, const unsigned char* keep,
                               const long long* top_ks, const float* top_ps, unsigned* thresh,
@@ -466,21 +657,29 @@ int dib_gumbel_sample_chunked(const float* logits, const float* temperatures, co
   const bool filtered = top_ks != nullptr && top_ps != nullptr && thresh != nullptr && hist != nullptr;
   if (filtered && reinterpret_cast<uintptr_t>(hist) % 8 != 0) return DIB_BAD_ALIGN;
   unsigned long long* hist_mass = filtered ? reinterpret_cast<unsigned long long*>(hist) : nullptr;
-  unsigned* hist_cnt = filtered ? reinterpret_cast<unsigned*>(hist_mass + (size_t)4 * R * 256) : nullptr;
-  dib_launch(gumbel_stats_kernel, dim3(chunks, R), dim3(256), 0, st, logits, temperatures, cmax, csum,
-             hist_cnt, hist_mass, R, V, chunks);
+  FilterState* states = filtered ? reinterpret_cast<FilterState*>(hist_mass + (size_t)R * FILTER_BINS) : nullptr;
+  float2* norms = filtered ? reinterpret_cast<float2*>(states + (size_t)R * FILTER_PASSES) : nullptr;
+  unsigned* hist_cnt = filtered ? reinterpret_cast<unsigned*>(norms + R) : nullptr;
+  const dim3 grid(chunks, R), block(SAMPLE_THREADS);
+  dib_launch(gumbel_stats_kernel, grid, block, 0, st, logits, temperatures, cmax, csum, hist_cnt, hist_mass, V,
+             chunks);
   DIB_CHECK_LAUNCH();
   if (filtered) {
-    for (int pass = 0; pass < 4; ++pass) {
-      dib_launch(filter_histogram_kernel, dim3(chunks, R), dim3(256), 0, st, logits, temperatures, top_ks,
-                 top_ps, (const float*)cmax, (const float*)csum, hist_cnt, hist_mass, pass, R, V, chunks);
-      DIB_CHECK_LAUNCH();
-    }
+    auto pass = [&](auto* kernel) {
+      dib_launch(kernel, grid, block, 0, st, logits, temperatures, top_ks, top_ps, (const float*)cmax,
+                 (const float*)csum, hist_cnt, hist_mass, states, norms, R, V, chunks);
+    };
+    pass(&filter_histogram_kernel<0>);
+    DIB_CHECK_LAUNCH();
+    pass(&filter_histogram_kernel<1>);
+    DIB_CHECK_LAUNCH();
+    pass(&filter_histogram_kernel<2>);
+    DIB_CHECK_LAUNCH();
   }
-  dib_launch(gumbel_pick_kernel, dim3(chunks, R), dim3(256), 0, st, logits, temperatures, seeds,
-             sample_pos, keep, top_ks, top_ps, (const unsigned*)hist_cnt,
-             (const unsigned long long*)hist_mass, filtered ? thresh : (unsigned*)nullptr,
-             (const float*)cmax, (const float*)csum, pv, scratch_i, R, V, chunks);
+  dib_launch(gumbel_pick_kernel, grid, block, 0, st, logits, temperatures, seeds, sample_pos, keep, top_ks, top_ps,
+             (const unsigned*)hist_cnt, (const unsigned long long*)hist_mass, (const FilterState*)states, (const float2*)norms,
+             filtered ? thresh : (unsigned*)nullptr, (const float*)cmax, (const float*)csum, pv, scratch_i, R, V,
+             chunks);
   DIB_CHECK_LAUNCH();
   dib_launch(argmax_final_kernel, dim3(R), dim3(64), 0, st, (const float*)pv, (const int*)scratch_i, out,
              chunks);

@@ -846,14 +846,14 @@ def gumbel_sample(logits: torch.Tensor, temperatures: torch.Tensor, seeds: torch
             if top_ks.shape[0] != r or top_ps.shape[0] != r:
                 raise KernelError("gumbel_sample: top_ks / top_ps lengths differ from the number of rows")
             thresh = torch.empty(r, dtype=torch.int32, device=logits.device)
-            # histograms of the four radix passes: [4, r, 256] 64-bit masses, then 32-bit counts
-            hist = torch.empty(4 * r * 256 * 3 // 2, dtype=torch.int64, device=logits.device)
+            lib.dib_filter_scratch.restype = c_longlong
+            hist = torch.empty(lib.dib_filter_scratch(c_int(r)) // 8, dtype=torch.int64, device=logits.device)
         st = lib.dib_gumbel_sample_chunked(_ptr(logits), _ptr(temperatures), _ptr(seeds),
                                            _ptr(sample_positions), _ptr(keep), _ptr(top_ks),
                                            _ptr(top_ps), _ptr(thresh),
                                            _ptr(hist) if thresh is not None else c_void_p(0),
                                            _ptr(sf), _ptr(si), _ptr(out), c_int(r), c_int(v), _stream())
-        _check(st, "gumbel_sample", kernels=3 if thresh is None else 7)
+        _check(st, "gumbel_sample", kernels=3 if thresh is None else 6)
         return (out, thresh) if return_thresholds else out
     if filtered:
         raise KernelError("gumbel_sample: top_ks / top_ps with more than 65535 rows")
@@ -1124,7 +1124,10 @@ def sigmoid_attention(q: torch.Tensor, kv_cache: torch.Tensor, meta, scale: floa
         # same bits either way).
         group = hq // hkv
         n_dec = meta.num_decode if group <= 16 else 0
-        rows = 128 if max(meta.q_lens[n_dec:], default=0) * group > 64 else 64
+        # (whether portions run on the tcgen05 kernel depends on the layer's sizes alone: a row's bits
+        # do not depend on the step)
+        on_tc = d == 128 and v_head_dim == 128 and 128 % group == 0 and page_size in (8, 16, 32, 64, 128)
+        rows = 128 if on_tc or max(meta.q_lens[n_dec:], default=0) * group > 64 else 64
         lists = meta.scratch.get(("sigmoid_attention_tiles", group, rows))
         if lists is None:
             lists = []
@@ -1145,6 +1148,15 @@ def sigmoid_attention(q: torch.Tensor, kv_cache: torch.Tensor, meta, scale: floa
                 max_chunks = -(-most // SIGMOID_DECODE_CHUNK_TILES)
                 if max_chunks > 1:
                     partial = torch.empty(n_dec, hq, max_chunks, v_head_dim, dtype=torch.float32, device=q.device)
+            if form == 128 and on_tc:
+                st = _lib("attention_prefill_tc").dib_sigmoid_attention_tc(
+                    _ptr(q), _ptr(out), _ptr(kv_cache), c_longlong(kv_cache.shape[0]), _ptr(meta.block_table),
+                    c_int(meta.block_table.shape[1]), _ptr(meta.positions), _ptr(meta.seq_lens), _ptr(tiles),
+                    c_int(tiles.shape[0]), _ptr(head_bias), c_int(hq), c_int(hkv), c_int(d), c_int(v_head_dim),
+                    c_int(page_size), c_float(scale), c_int(win), c_int(int(keep_first)), _stream())
+                if st != -2:
+                    _check(st, "sigmoid_attention(tcgen05)", f"heads {hq}/{hkv}")
+                    continue
             st = _lib("sigmoid_attention").dib_sigmoid_attention_mma(
                 _ptr(q), _ptr(out), _ptr(kv_cache), _ptr(meta.block_table), c_int(meta.block_table.shape[1]),
                 _ptr(meta.positions), _ptr(meta.seq_lens), _ptr(tiles), c_int(tiles.shape[0]), _ptr(head_bias),

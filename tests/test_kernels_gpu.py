@@ -806,6 +806,41 @@ def test_top_k_top_p_threshold_is_what_the_sort_rule_keeps(v):
     assert all(toks[i] == with_mask[i] for i in range(r) if agree[i]) and sum(map(bool, agree)) >= r - 3
 
 
+@pytest.mark.parametrize("v", [4096, 8193, 12288, 12289])
+def test_draws_from_extreme_rows(v):
+    """Rows where the cheap bounds of the sampling kernels say little: flat ones (one bin for all tokens), rows of
+    minus infinity but for a few ids, probabilities below the smallest normal number, temperatures far from 1."""
+    torch.manual_seed(29)
+    base = torch.randn(v, device="cuda")
+    few = torch.full((v,), float("-inf"), device="cuda")
+    few[[0, 5, v - 1]] = torch.tensor([1.0, 2.0, 1.5], device="cuda")
+    rows = [torch.zeros(v, device="cuda"), few, 1e4 * base, base, base, 60 * base, base - 5e4, torch.zeros(v, device="cuda")]
+    logits = torch.stack(rows)
+    r = len(rows)
+    temps = torch.tensor([0.7, 0.9, 1.0, 1e-3, 40.0, 1.0, 0.6, 1.0], device="cuda")
+    seeds = torch.arange(r, device="cuda", dtype=torch.int64) + 5
+    pos = torch.arange(7, 7 + r, device="cuda", dtype=torch.int64)
+    plain = ops().gumbel_sample(logits, temps, seeds, pos)
+    scores = ref.gumbel_scores(logits.double(), temps.double(), seeds, pos)
+    picked = scores.gather(1, plain.long().unsqueeze(1))[:, 0]
+    # 32-bit logits of size 1e4 .. 5e4 over the temperature: their rounding is the score's
+    slack = 1e-4 + 4 * 2.0 ** -24 * (logits.nan_to_num(neginf=0).abs().amax(1) / temps)
+    assert (picked >= scores.amax(1) - slack).all()
+    off = torch.full((r,), -1, device="cuda", dtype=torch.int64)
+    one = torch.ones(r, device="cuda")
+    # equal tokens tie with the threshold and all stay: the draw is the unfiltered one
+    k3 = torch.full((r,), 3, device="cuda", dtype=torch.int64)
+    got, thr = ops().gumbel_sample(logits, temps, seeds, pos, top_ks=k3, top_ps=one, return_thresholds=True)
+    assert got[0] == plain[0] and got[7] == plain[7] and int(got[1]) in (0, 5, v - 1)
+    assert got[2] == logits[2].argmax() and got[3] == logits[3].argmax()
+    best3 = logits.topk(3, dim=1).indices
+    assert all(int(got[i]) in best3[i].tolist() for i in (1, 2, 3, 4, 5, 6))
+    # and with nothing dropped but a tail that weighs nothing
+    got = ops().gumbel_sample(logits, temps, seeds, pos, top_ks=off, top_ps=one * (1 - 2.0 ** -20))
+    p = torch.softmax(logits.double() / temps.double().unsqueeze(1), 1)
+    assert (p.gather(1, got.long().unsqueeze(1)) > 0).all() and got[0] == plain[0] and got[7] == plain[7]
+
+
 def test_top_k_top_p_respected():
     from deterministic_inference_b200.config import SamplingParams
     from deterministic_inference_b200.sampling import sample
