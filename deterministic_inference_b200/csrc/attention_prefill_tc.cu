@@ -1063,6 +1063,247 @@ extend_attention_merge_kernel(const float* __restrict__ part_o, const float* __r
   }
 }
 
+// ------------------------------------------------------------------------------
+// Attention without a softmax: a row's weight for a key is sigmoid(q . k * scale + bias[head]), and the
+// weighted values are added up as they are.  The form of the first kernel above (one query tile of 128
+// rows a CTA, two threads a row), without a maximum, a sum or a rescaling: O only accumulates in tensor
+// memory.  P has two buffers, so that the threads' next tile does not wait for the product with the
+// values.  A window mask may keep the sequence's first `keep` keys visible too: the key tiles that hold
+// them and lie before the window's first tile are walked first.  Key tiles are anchored at position 0
+// and a tile in which a row sees nothing adds exact zeros, so a row's sum depends on its position alone.
+// tiles: int32 [n][3] = (sequence of the step, first token of the tile in the step, tokens).
+// Bound: the special-function unit, two results a weight (an exponential and a reciprocal; 128 x 128
+// weights are 1.05 us of an SM at 16 results a clock), above the tensor core's 0.3 us a tile and the two
+// stages' copies.  (2,048 tokens, window 1,024, 16 heads of 128 over 8: 51 us; the mma.sync form, 64
+// keys a tile, whose warps load, multiply and weigh in turn: 206 us.)
+__device__ __forceinline__ float sigmoid_fast(float x) {      // (as the mma.sync form: relative error about 1e-6)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + fast_exp2(x * -LOG2E)));
+  return r;
+}
+constexpr int SIG_SMEM = 7 * TILE_BYTES + 16 * 8 + 1024;      // Q, two P, two stages of K and V, barriers
+
+__global__ void __launch_bounds__(TC_THREADS, 1)
+sigmoid_attention_tc_kernel(const __grid_constant__ CUtensorMap map, const __nv_bfloat16* __restrict__ q,
+                            __nv_bfloat16* __restrict__ out, const int* __restrict__ block_table, int max_blocks,
+                            const int* __restrict__ positions, const int* __restrict__ seq_lens,
+                            const int* __restrict__ tiles, const float* __restrict__ head_bias, int Hq, int Hkv,
+                            int page_size, float scale, int window, int keep) {
+  if (threadIdx.x == 0) prefetch_tensormap(&map);
+  pdl_prologue(q);
+  extern __shared__ unsigned char smem_dyn[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+  unsigned char* sQ = smem;
+  unsigned char* sP = smem + TILE_BYTES;          // [2]
+  unsigned char* sKV = smem + 3 * TILE_BYTES;     // 2 stages x (K 32 KB + V 32 KB)
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + 7 * TILE_BYTES);
+  unsigned long long* kv_full = bars;             // [2] K and V of a tile are in shared memory
+  unsigned long long* kv_empty = bars + 2;        // [2] both products of the tile have read them
+  unsigned long long* s_full = bars + 4;          // [2] S_i is in tensor memory (buffer i & 1)
+  unsigned long long* s_free = bars + 6;          // [2] the threads of the rows have read it (256)
+  unsigned long long* p_full = bars + 8;          // [2] P_i is in shared memory (256)
+  unsigned long long* p_free = bars + 10;         // [2] O += P_i V_i has completed
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 12);
+
+  // blocks are handed out in x-then-y order: y counts the tiles from the last, the longest under a causal mask
+  const int tile = gridDim.y - 1 - blockIdx.y, kvh = blockIdx.x;
+  const int G = Hq / Hkv;
+  const int seq = tiles[3 * tile], t0 = tiles[3 * tile + 1], ntok = tiles[3 * tile + 2];
+  const int kv_len = seq_lens[seq];
+  const int first_pos = positions[t0], last_pos = first_pos + ntok - 1;
+  const int* bt = block_table + (size_t)seq * max_blocks;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  const int j0 = (window > 0 ? max(first_pos - window + 1, 0) : 0) / TC_N, j1 = last_pos / TC_N;
+  const int kept = window > 0 ? min((keep + TC_N - 1) / TC_N, j0) : 0;
+  const int ntiles = kept + j1 - j0 + 1;
+  auto tile_key = [&](int i) { return (i < kept ? i : j0 + i - kept) * TC_N; };   // the i-th tile's first key
+
+  if (warp == MMA_WARP && lane == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&kv_full[i], 1);
+      mbar_init(&kv_empty[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_free[i], 256);
+      mbar_init(&p_full[i], 256);
+      mbar_init(&p_free[i], 1);
+    }
+    mbar_fence_init();
+  }
+  if (warp == TMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  for (int c = threadIdx.x; c < TC_M * 16; c += TC_THREADS) {      // rows beyond the tile's tokens are zero
+    const int r = c >> 4, ch = c & 15;
+    const int tl = r / G, g = r % G;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (tl < ntok)
+      v = *reinterpret_cast<const uint4*>(q + ((size_t)(t0 + tl) * Hq + (size_t)kvh * G + g) * TC_D + ch * 8);
+    *reinterpret_cast<uint4*>(sQ + sw_chunk_off(r, ch)) = v;
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // Q is read by the MMA unit
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem = *tmem_slot;
+  const unsigned tmem_o = tmem + 256;   // columns 0..127: S (even tiles), 128..255: S (odd), 256..383: O
+  bool ok = true;
+
+  if (warp == TMA_WARP) {
+    const int pages = TC_N / page_size, ops = pages * 4;
+    for (int i = 0; i < ntiles && ok; ++i) {
+      const int st = i & 1;
+      if (i >= 2) ok = mbar_wait(&kv_empty[st], ((i >> 1) - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      if (lane == 0) mbar_expect_tx(&kv_full[st], 2 * TILE_BYTES);
+      __syncwarp();
+      const int k0 = tile_key(i);
+      for (int op = lane; op < ops; op += 32) {
+        const int pi = op >> 2, kv = (op >> 1) & 1, half = op & 1;
+        const int idx = k0 / page_size + pi;
+        const int page = idx < max_blocks ? bt[idx] : 0;
+        const int row0 = (((page * 2 + kv) * Hkv) + kvh) * page_size;
+        tma_load_2d(sKV + st * 2 * TILE_BYTES + kv * TILE_BYTES + half * HALF_BYTES + pi * page_size * 128, &map,
+                    half * 64, row0, &kv_full[st]);
+      }
+    }
+  } else if (warp == MMA_WARP) {
+    if (lane == 0) {
+      constexpr unsigned idesc_s = idesc_f16(TC_M, TC_N, 0);
+      constexpr unsigned idesc_o = idesc_f16(TC_M, TC_D, 1);
+      const unsigned q_addr = smem_u32(sQ);
+      auto issue_s = [&](int i) {
+        const unsigned k_addr = smem_u32(sKV + (i & 1) * 2 * TILE_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < TC_D / 16; ++ks) {
+          const unsigned off = (ks >> 2) * HALF_BYTES + (ks & 3) * 32;
+          tc_mma(tmem + (i & 1) * 128, desc_k_major(q_addr + off), desc_k_major(k_addr + off), idesc_s,
+                 ks > 0 ? 1u : 0u);
+        }
+        tc_commit(&s_full[i & 1]);
+      };
+      ok = mbar_wait(&kv_full[0], 0);
+      if (ok) {
+        tc_fence_after();
+        issue_s(0);
+      }
+      for (int i = 0; i < ntiles && ok; ++i) {
+        if (i + 1 < ntiles) {       // the next tile's scores, while the rows' threads work on this one's
+          ok = mbar_wait(&kv_full[(i + 1) & 1], ((i + 1) >> 1) & 1);
+          if (ok && i + 1 >= 2) ok = mbar_wait(&s_free[(i + 1) & 1], (((i + 1) >> 1) - 1) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          issue_s(i + 1);
+        }
+        ok = mbar_wait(&p_full[i & 1], (i >> 1) & 1);
+        if (!ok) break;
+        tc_fence_after();
+        const unsigned p_addr = smem_u32(sP + (i & 1) * TILE_BYTES);
+        const unsigned v_addr = smem_u32(sKV + (i & 1) * 2 * TILE_BYTES + TILE_BYTES);
+#pragma unroll
+        for (int ks = 0; ks < TC_N / 16; ++ks) {
+          const unsigned a_off = (ks >> 2) * HALF_BYTES + (ks & 3) * 32;   // 16 keys of P
+          const unsigned b_off = ks * 16 * 128;                            // 16 key rows of V
+          tc_mma(tmem_o, desc_k_major(p_addr + a_off), desc_mn_major(v_addr + b_off, HALF_BYTES), idesc_o,
+                 (i > 0 || ks > 0) ? 1u : 0u);
+        }
+        tc_commit(&p_free[i & 1]);
+        tc_commit(&kv_empty[i & 1]);
+      }
+    }
+  } else {
+    const int r = threadIdx.x & 127;
+    const int hf = threadIdx.x >> 7;                 // 0: keys/dims 0..63 of a tile, 1: 64..127
+    const int tl = r / G, g = r % G;
+    const bool valid = tl < ntok;
+    const int hi = valid ? first_pos + tl : -1;
+    const int lo = valid && window > 0 ? max(hi - window + 1, 0) : 0;
+    const float bias = valid && head_bias != nullptr ? head_bias[kvh * G + g] : 0.f;
+    const unsigned lane_base = (unsigned)((warp & 3) * 32) << 16;
+    for (int i = 0; i < ntiles && ok; ++i) {
+      const int b = i & 1, kbase = tile_key(i);
+      ok = mbar_wait(&s_full[b], (i >> 1) & 1);
+      if (ok && i >= 2) ok = mbar_wait(&p_free[b], ((i >> 1) - 1) & 1);     // P_{i-2} has been read
+      if (ok && kbase + TC_N > kv_len) {
+        // rows of V past the sequence's end hold whatever their page held: a weight of 0 must meet a number
+        ok = mbar_wait(&kv_full[b], (i >> 1) & 1);
+        if (ok) {
+          unsigned char* v = sKV + b * 2 * TILE_BYTES + TILE_BYTES;
+          const int from = kv_len - kbase;
+          for (int c = threadIdx.x; c < (TC_N - from) * 16; c += 256)
+            *reinterpret_cast<uint4*>(v + (c & 1) * HALF_BYTES + (from + (c >> 4)) * 128 + ((c >> 1) & 7) * 16) =
+                make_uint4(0, 0, 0, 0);
+        }
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const bool full = kbase >= lo && kbase + TC_N - 1 <= hi;   // no key of the tile is masked
+      unsigned char* p_row = sP + b * TILE_BYTES;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        unsigned v[32], pk[16];
+        tc_ld32(tmem + b * 128 + lane_base + hf * 64 + c * 32, v);
+        tc_wait_ld();
+        const int first = kbase + hf * 64 + c * 32;
+#pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+          float w0 = sigmoid_fast(__fmaf_rn(__uint_as_float(v[k]), scale, bias));
+          float w1 = sigmoid_fast(__fmaf_rn(__uint_as_float(v[k + 1]), scale, bias));
+          if (!full) {
+            const int key = first + k;
+            if (!(key <= hi && (key >= lo || key < keep))) w0 = 0.f;
+            if (!(key + 1 <= hi && (key + 1 >= lo || key + 1 < keep))) w1 = 0.f;
+          }
+          pk[k >> 1] = pack_bf16(w0, w1);
+        }
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch)
+          *reinterpret_cast<uint4*>(p_row + sw_chunk_off(r, hf * 8 + c * 4 + ch)) =
+              make_uint4(pk[ch * 4], pk[ch * 4 + 1], pk[ch * 4 + 2], pk[ch * 4 + 3]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tc_fence_before();
+      mbar_arrive(&s_free[b]);
+      mbar_arrive(&p_full[b]);
+    }
+    if (ok) ok = mbar_wait(&p_free[(ntiles - 1) & 1], ((ntiles - 1) >> 1) & 1);
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after();
+    if (ok) {
+      __nv_bfloat16* dst = out + ((size_t)(t0 + (valid ? tl : 0)) * Hq + (size_t)kvh * G + g) * TC_D + hf * 64;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        unsigned v[32];
+        tc_ld32(tmem_o + lane_base + hf * 64 + c * 32, v);
+        tc_wait_ld();
+        if (valid) {
+#pragma unroll
+          for (int ch = 0; ch < 4; ++ch) {
+            uint4 o4;
+            o4.x = pack_bf16(__uint_as_float(v[ch * 8 + 0]), __uint_as_float(v[ch * 8 + 1]));
+            o4.y = pack_bf16(__uint_as_float(v[ch * 8 + 2]), __uint_as_float(v[ch * 8 + 3]));
+            o4.z = pack_bf16(__uint_as_float(v[ch * 8 + 4]), __uint_as_float(v[ch * 8 + 5]));
+            o4.w = pack_bf16(__uint_as_float(v[ch * 8 + 6]), __uint_as_float(v[ch * 8 + 7]));
+            *reinterpret_cast<uint4*>(dst + c * 32 + ch * 8) = o4;
+          }
+        }
+      }
+    }
+  }
+  if (!ok) atomicExch(&dib_attention_error_word, 1);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == TMA_WARP) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -1230,6 +1471,36 @@ int dib_extend_attention_tc_pair_sink(const void* q, void* out, const void* cach
                token_seq, t_first, num_tokens, Hq, Hkv, max_chunks, chunk_tiles, window, sink);
     DIB_CHECK_LAUNCH();
   }
+  return DIB_OK;
+}
+
+// Attention without a softmax (sigmoid weights) for prompt portions: keys and values of 128, a cache
+// page of [keys: Hkv x page_size x 128 | values].  Tiles of 128 / (Hq / Hkv) tokens of a sequence.
+// Returns DIB_BAD_SIZE for shapes the kernel does not take (the caller then uses the mma.sync form).
+int dib_sigmoid_attention_tc(const void* q, void* out, const void* cache, long long num_pages, const int* block_table,
+                             int max_blocks, const int* positions, const int* seq_lens, const int* tiles,
+                             int num_tiles, const float* head_bias, int Hq, int Hkv, int D, int VD, int page_size,
+                             float scale, int window, int keep, cudaStream_t st) {
+  if (num_tiles == 0) return DIB_OK;
+  if (D != TC_D || VD != TC_D || Hkv < 1 || Hq % Hkv != 0 || TC_M % (Hq / Hkv) != 0 || page_size < 8 ||
+      page_size > TC_N || TC_N % page_size != 0 || num_tiles > 65535 || window < 0 || keep < 0 ||
+      (long long)num_pages * 2 * Hkv * page_size >= (1ll << 31) ||
+      reinterpret_cast<uintptr_t>(cache) % 16 != 0 || reinterpret_cast<uintptr_t>(q) % 16 != 0 ||
+      reinterpret_cast<uintptr_t>(out) % 16 != 0)
+    return DIB_BAD_SIZE;
+  const CUtensorMap* map = cache_map(cache, num_pages, Hkv, page_size, D);
+  if (map == nullptr) return DIB_LAUNCH_FAILED;
+  static DeviceOnce attr_set;
+  if (!attr_set.done()) {
+    if (cudaFuncSetAttribute(sigmoid_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SIG_SMEM) !=
+        cudaSuccess)
+      return DIB_LAUNCH_FAILED;
+    attr_set.mark();
+  }
+  dib_launch(sigmoid_attention_tc_kernel, dim3(Hkv, num_tiles), dim3(TC_THREADS), (size_t)SIG_SMEM, st, *map,
+             (const __nv_bfloat16*)q, (__nv_bfloat16*)out, block_table, max_blocks, positions, seq_lens, tiles,
+             head_bias, Hq, Hkv, page_size, scale, window, keep);
+  DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
 

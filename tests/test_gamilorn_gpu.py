@@ -177,6 +177,57 @@ def test_sigmoid_attention_alone(dtype, heads, kv_heads, dim, vdim, page, window
     assert float(want[0][last].abs().max()) > 50
 
 
+@pytest.mark.parametrize("heads, kv_heads, page, window, keep, lens", [
+    (4, 2, 16, 100, 5, (300, 129)),        # a window within a tile of 128 keys, kept keys in the first
+    (2, 2, 128, None, 0, (257, 64)),       # one head a group, a page a tile
+    (8, 1, 8, 130, 140, (500, 2)),         # a window beyond a tile, kept keys beyond one; groups of 8
+    (4, 1, 32, 256, 0, (640, 33)),
+])
+def test_sigmoid_attention_of_128(heads, kv_heads, page, window, keep, lens):
+    """Keys and values of 128 (the tcgen05 form for prompt portions): against 64 bits at whole and ragged tiles; a row's
+    bits do not depend on the portion it comes in; what a page holds past a sequence's end, not a number here, does
+    not reach a row."""
+    from deterministic_inference_b200.kernels import ops
+    dim, dev = 128, "cuda"
+    g = torch.Generator().manual_seed(heads + page)
+    scale = 0.9 / math.sqrt(dim)
+    rnd = lambda *s: pg.as_stored_bf16(torch.randn(*s, generator=g))
+    seqs = [(rnd(n, heads, dim), rnd(n, kv_heads, dim), rnd(n, kv_heads, dim)) for n in lens]
+    head_bias = torch.randn(heads, generator=g) - 1.0
+    bt, pages = paged(list(lens), page, g)
+    cache = torch.full((pages, 2, kv_heads, page, dim), float("nan"), dtype=torch.bfloat16)
+    for b, (_, k, v) in enumerate(seqs):
+        for p in range(lens[b]):
+            cache[int(bt[b, p // page]), 0, :, p % page] = k[p].bfloat16()
+            cache[int(bt[b, p // page]), 1, :, p % page] = v[p].bfloat16()
+    cache = cache.view(pages, -1).to(dev)
+
+    def run(entries):
+        rows, seq_of, pos_of = [], [], []
+        for i, (b, start, count) in enumerate(entries):
+            rows.append(seqs[b][0][start:start + count])
+            seq_of += [i] * count
+            pos_of += range(start, start + count)
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+        meta = SimpleNamespace(block_table=bt[[b for b, _, _ in entries]].contiguous().to(dev), token_seq=i32(seq_of),
+                               positions=i32(pos_of), seq_lens=i32([s + c for _, s, c in entries]),
+                               q_lens=[c for _, _, c in entries], kv_lens=[s + c for _, s, c in entries], scratch={},
+                               num_decode=0)
+        out = ops.sigmoid_attention(torch.cat(rows).bfloat16().to(dev), cache, meta, scale, head_bias.to(dev), dim, page,
+                                    window, keep).cpu()
+        return list(out.split([c for _, _, c in entries]))
+
+    whole = run([(0, 0, lens[0]), (1, 0, lens[1])])
+    for b, (q, k, v) in enumerate(seqs):
+        want = pg.sigmoid_window_attention(q.double(), k.double(), v.double(), scale, head_bias.double(),
+                                           window or 10 ** 9, keep)
+        close(whole[b].double(), want, "bfloat16", f"attention of sequence {b}", bf16=8e-3)
+    cut = lens[0] // 2 + 3
+    assert torch.equal(run([(1, 0, lens[1]), (0, cut, lens[0] - cut)])[1], whole[0][cut:])
+    assert torch.equal(run([(0, 0, 2)])[0], whole[0][:2])
+    ops.check_kernel_status()
+
+
 # ---- the delta-rule recurrence -----------------------------------------------------------------------
 
 @pytest.mark.parametrize("dtype", list(DTYPES))
