@@ -20,39 +20,89 @@
 // proj row: [r | k | v | g | a_pre | lora hidden] = 5 * H * D + R columns; w2t [R][H * D] (the
 // decay map's second matrix, transposed: the threads of a block read consecutive elements).
 // packed [T][H][6][D] float32: w, a * u, u, k, r, v.
-__global__ void delta_prepare_kernel(Source proj, const void* w2t, int w_dtype, const float* w0,
-                                     const float* a_bias, float* packed, int H, int D, int R,
+// A block takes PREP_TOKENS tokens of a head: an element of w2t is read once for all of them, and
+// all their projected elements are asked for before the first is used.  PROJ 0 / 1: proj is a stored
+// float32 / bfloat16 matrix (a prompt portion's), 2: any source; W: w2t's type; no load of the first two
+// has a branch.  Bound: the 48 bytes
+// written for a channel and token.  (A block a token, which read the head's R x D weights again for
+// each in one chain of R loads a thread, 2,048 tokens of 16 heads of 64: 129 us, so 47.)
+constexpr int PREP_TOKENS = 8, PREP_RANKS = 512;      // tokens of a block; entries of the hidden vector at a time
+template <int PROJ, int W>
+__global__ void delta_prepare_kernel(Source proj, const void* w2t, const float* w0,
+                                     const float* a_bias, float* packed, int T, int H, int D, int R,
                                      float decay_scale, float key_eps) {
-  extern __shared__ float dp_smem[];     // [R] tanh of the lora hidden, then 32 floats of scratch
-  float* th = dp_smem;
-  float* scratch = dp_smem + R;
+  __shared__ __align__(16) float th[PREP_RANKS * PREP_TOKENS];       // tanh of the lora hidden
+  __shared__ float sums[PREP_TOKENS * 32];                           // the warps' sums of squares
   pdl_prologue();
-  const int t = blockIdx.x, h = blockIdx.y, c = threadIdx.x;
+  const int t0 = blockIdx.x * PREP_TOKENS, h = blockIdx.y, c = threadIdx.x;
+  const int tokens = min(PREP_TOKENS, T - t0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int HD = H * D;
-  const long long row = (long long)t * (5 * HD + R);
-  for (int j = threadIdx.x; j < R; j += blockDim.x) th[j] = tanhf(source_load(proj, row + 5 * HD + j));
-  float k = 0.f, r = 0.f, v = 0.f, a = 0.f, w = 0.f;
+  const long long width = 5 * HD + R;
+  auto element = [&](long long at) {
+    if constexpr (PROJ == 0) return reinterpret_cast<const float*>(proj.p)[at];
+    else if constexpr (PROJ == 1) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(proj.p)[at]);
+    else return source_load(proj, at);
+  };
   const int ch = h * D + c;
-  if (c < D) {
-    r = source_load(proj, row + ch);
-    k = source_load(proj, row + HD + ch);
-    v = source_load(proj, row + 2 * HD + ch);
-    a = sigmoid_f32(__fadd_rn(source_load(proj, row + 4 * HD + ch), a_bias != nullptr ? a_bias[ch] : 0.f));
+  float r[PREP_TOKENS], k[PREP_TOKENS], v[PREP_TOKENS], a[PREP_TOKENS], z[PREP_TOKENS];
+#pragma unroll
+  for (int i = 0; i < PREP_TOKENS; ++i) {
+    const bool in = c < D && i < tokens;
+    const long long row = (t0 + i) * width + ch;
+    r[i] = in ? element(row) : 0.f;
+    k[i] = in ? element(row + HD) : 0.f;
+    v[i] = in ? element(row + 2 * HD) : 0.f;
+    a[i] = in ? element(row + 4 * HD) : 0.f;
+    z[i] = 0.f;
   }
-  const float ss = block_sum(k * k, scratch);      // (also orders the writes of th before their reads)
-  if (c < D) {
-    float z = 0.f;
-    for (int j = 0; j < R; ++j) z = __fmaf_rn(load_as(w2t, w_dtype, (long long)j * HD + ch), th[j], z);
-    z = __fadd_rn(z, w0[ch]);
-    w = expf(-decay_scale * sigmoid_f32(z));
-    const float u = k / sqrtf(ss + key_eps);
-    float* out = packed + ((long long)t * H + h) * 6 * D + c;
-    out[0] = w;
-    out[D] = a * u;
+#pragma unroll
+  for (int i = 0; i < PREP_TOKENS; ++i) {
+    const float part = warp_sum(k[i] * k[i]);
+    if (lane == 0) sums[i * 32 + warp] = part;
+  }
+  for (int j0 = 0; j0 < R; j0 += PREP_RANKS) {
+    const int n = min(PREP_RANKS, R - j0);
+    if (j0 > 0) __syncthreads();
+    for (int e = threadIdx.x; e < n * PREP_TOKENS; e += blockDim.x) {
+      const int i = e / n, j = e - i * n;
+      th[j * PREP_TOKENS + i] = i < tokens ? tanhf(element((t0 + i) * width + 5 * HD + j0 + j)) : 0.f;
+    }
+    __syncthreads();
+    if (c < D) {
+#pragma unroll 16
+      for (int j = 0; j < n; ++j) {
+        const long long at = (long long)(j0 + j) * HD + ch;
+        const float w = load_as(w2t, W, at);
+        const float4* x = reinterpret_cast<const float4*>(th + j * PREP_TOKENS);
+#pragma unroll
+        for (int q = 0; q < PREP_TOKENS / 4; ++q) {
+          const float4 y = x[q];
+          z[4 * q] = __fmaf_rn(w, y.x, z[4 * q]);
+          z[4 * q + 1] = __fmaf_rn(w, y.y, z[4 * q + 1]);
+          z[4 * q + 2] = __fmaf_rn(w, y.z, z[4 * q + 2]);
+          z[4 * q + 3] = __fmaf_rn(w, y.w, z[4 * q + 3]);
+        }
+      }
+    }
+  }
+  __syncthreads();                 // (R may be 0)
+  if (c >= D) return;
+  const float bias_w = w0[ch], bias_a = a_bias != nullptr ? a_bias[ch] : 0.f;
+#pragma unroll
+  for (int i = 0; i < PREP_TOKENS; ++i) {
+    if (i >= tokens) break;
+    float ss = 0.f;
+    for (int x = 0; x < warps; ++x) ss += sums[i * 32 + x];
+    const float rate = sigmoid_f32(__fadd_rn(a[i], bias_a));
+    const float u = k[i] / sqrtf(ss + key_eps);
+    float* out = packed + ((long long)(t0 + i) * H + h) * 6 * D + c;
+    out[0] = expf(-decay_scale * sigmoid_f32(__fadd_rn(z[i], bias_w)));
+    out[D] = rate * u;
     out[2 * D] = u;
-    out[3 * D] = k;
-    out[4 * D] = r;
-    out[5 * D] = v;
+    out[3 * D] = k[i];
+    out[4 * D] = r[i];
+    out[5 * D] = v[i];
   }
 }
 
@@ -183,160 +233,259 @@ delta_recurrence_kernel(const float* packed, float* state, long long slot_stride
   }
 }
 
-// The same recurrence with a column's rows over 16 lanes (row i = 64 q + 4 s + e for lane s): a
-// block of four warps per (sequence, head, 8 value columns), two columns a warp, the token's
-// vectors staged once per block, DR_STAGES tokens deep, one barrier a token, the block's slab of
-// the state through shared memory in rows of 32 bytes.  Fewer instructions per token and warp
-// (4 rows a lane at D = 64) and four times the CTAs: the form for steps with few sequences and
-// many tokens (prompt portions).  Its sums are ordered differently from the form above (four
-// chains by e, then a butterfly over 16 lanes), again by D alone.
-template <int MAXR, int DR_STAGES>
-__global__ void __launch_bounds__(128)
+// The same recurrence with a column's rows over LANES = 16 lanes (row i = 64 q + 4 s + e for lane s),
+// CPT columns a thread, WARPS warps a block per (sequence, head, 32 / LANES * CPT * WARPS value
+// columns).  The form for steps with few sequences and many tokens (prompt portions): few warps a
+// scheduler, so a token takes what its instructions and the chain from its state to the next one's
+// take (the row sum's FMA, four exchanges between lanes, one FMA).  Nothing else stands in that
+// chain: a token's vectors are in registers before (the next token's are read while this one is
+// worked on), w S + k v is ready when the sum arrives, and the output's exchanges run one token
+// behind, side by side with the sum's.  One more warp brings the vectors into shared memory,
+// DR_TOKENS tokens at a time, one group ahead, with one barrier a group; strides are constants of
+// the instance (D and E padded with zeros to LANES * MAXR).  Its sums are ordered differently from
+// the form above (four chains by e, then a butterfly over 16 lanes), again by D alone.
+// (2,048 tokens, 16 heads of 64: 245 us, rows over 8 lanes 344, over 4 649 us; 16 heads of 128: 450 us;
+// 512 tokens, 8 heads of 256: 271 us.  Copies by the warps that compute, a barrier a token and both
+// exchanges in the chain: 878, 1,013 and 356 us.)
+template <int Q, int CPT> struct DeltaToken {      // a lane's part of a token's vectors
+  float4 w[Q], b[Q], u[Q], k[Q], r[Q];
+  float v[CPT];
+};
+template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES>
+__global__ void __launch_bounds__(32 * WARPS + 32)
 delta_recurrence_wide_kernel(const float* packed, float* state, long long slot_stride, float* o_out,
                              const int* cu_q_lens, const int* state_slots, int H, int D, int E) {
-  extern __shared__ __align__(16) float dr_smem[];           // [DR_STAGES][5 Dp + Ep]; first also [D][8] of state
-  const int Dp = (D + 63) / 64 * 64, Ep = (E + 63) / 64 * 64;
-  const int SV = 5 * Dp + Ep;                  // a stage: w, b, u, k, r of Dp floats each, then v of Ep
-  const int NR = Dp / 16;                      // rows per lane (<= MAXR)
+  extern __shared__ __align__(16) float dr_smem[];           // [DR_STAGES][DR_TOKENS][6 Dp]
+  constexpr int Q = MAXR / 4;
+  constexpr int Dp = LANES * MAXR;             // D and E, padded with zeros
+  constexpr int COLS = 32 / LANES;             // a warp's columns side by side; CPT times as many in all
+  constexpr int SV = 6 * Dp;                   // a token: w, b, u, k, r, v
   const int b = blockIdx.x, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int s = lane & 15;
-  const int cl = warp * 2 + (lane >> 4);       // this lane's column among the block's 8
-  const int c0 = blockIdx.z * 8, c = c0 + cl;
-  const bool active = c < E;
   pdl_wait();                        // (launched in stream order; nothing is launched ahead of its end either)
   const int t0 = cu_q_lens[b], t1 = cu_q_lens[b + 1];
   if (t1 <= t0) return;
+  const int groups = (t1 - t0 + DR_TOKENS - 1) / DR_TOKENS;
+  if (Dp != D || Dp != E) {
+    for (int i = threadIdx.x; i < DR_STAGES * DR_TOKENS * SV; i += blockDim.x) dr_smem[i] = 0.f;   // the padding stays 0
+    __syncthreads();
+  }
+  if (warp == WARPS) {               // the copies
+    const int PV = 5 * D + E;                  // a token's vectors of one head, as they are stored
+    const bool wide = ((D | E) & 3) == 0;      // every vector starts on 16 bytes
+    const long long token_step = (long long)H * PV;
+    const float* base = packed + ((long long)t0 * H + h) * PV;
+    auto fetch = [&](int g) {
+      if (g < groups) {
+        float* dst = dr_smem + (g % DR_STAGES) * DR_TOKENS * SV;
+        const int n = min(DR_TOKENS, t1 - t0 - g * DR_TOKENS);
+        const float* src = base + (long long)g * DR_TOKENS * token_step;
+        for (int at = wide ? 4 * lane : lane; at < PV; at += wide ? 128 : 32) {
+          const int vsel = at < 5 * D ? at / D : 5;
+          float* to = dst + vsel * Dp + (at - vsel * D);
+          const float* from = src + at;
+          if (wide) {
+            for (int i = 0; i < n; ++i, to += SV, from += token_step) __pipeline_memcpy_async(to, from, 16);
+          } else {
+            for (int i = 0; i < n; ++i, to += SV, from += token_step) __pipeline_memcpy_async(to, from, 4);
+          }
+        }
+      }
+      __pipeline_commit();                     // (an empty group past the end keeps the count)
+    };
+#pragma unroll
+    for (int k = 0; k < DR_STAGES - 1; ++k) fetch(k);
+    for (int g = 0; g < groups; ++g) {
+      __pipeline_wait_prior(DR_STAGES - 2);    // group g has landed
+      __syncthreads();                         // ... for everybody; everybody is done with group g - 1
+      fetch(g + DR_STAGES - 1);                // into the stage of group g - 1
+    }
+    __pipeline_wait_prior(0);
+    return;
+  }
+  const int s = lane % LANES;
+  const int c = (blockIdx.z * WARPS + warp) * COLS * CPT + lane / LANES;       // this lane's columns: c, c + COLS, ...
   const long long slot = state_slots[b];
   const bool kept = slot != 0;       // slot 0 belongs to padding sequences: zero state, nothing stored
   float* S = state + slot * slot_stride + (long long)h * D * E;
-  float* slab = dr_smem;                        // [D][8]
-  for (int i = threadIdx.x; i < D * 8; i += blockDim.x) {
-    const int row = i >> 3, col = i & 7;
-    slab[i] = (kept && c0 + col < E) ? S[(long long)row * E + c0 + col] : 0.f;
-  }
-  __syncthreads();
-  float st[MAXR];
+  float st[CPT][MAXR];
 #pragma unroll
-  for (int ii = 0; ii < MAXR; ++ii) {
-    const int i = (ii >> 2) * 64 + s * 4 + (ii & 3);
-    st[ii] = (ii < NR && i < D) ? slab[i * 8 + cl] : 0.f;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < DR_STAGES * SV; i += blockDim.x) dr_smem[i] = 0.f;   // the padding stays 0
-  __syncthreads();
-  const int PV = 5 * D + E;                    // a token's vectors of one head, as they are stored
-  const bool wide = ((D | E) & 3) == 0;        // every vector starts on 16 bytes
-  // this thread's 16-byte pieces of a token's vectors ((5 D + E) / 4 pieces over 128 threads: at most 3)
-  int src_at[3], dst_at[3];
+  for (int j = 0; j < CPT; ++j)
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const int at = (threadIdx.x + 128 * k) * 4;
-    const int vsel = at < 5 * D ? at / D : 5, d = at - vsel * D;
-    src_at[k] = (wide && at < PV) ? at : -1;
-    dst_at[k] = vsel * Dp + d;
-  }
-  auto prefetch = [&](int t, int stage) {
-    if (t < t1) {
-      const float* src = packed + ((long long)t * H + h) * PV;
-      float* dst = dr_smem + stage * SV;
-      if (wide) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          if (src_at[k] >= 0) __pipeline_memcpy_async(dst + dst_at[k], src + src_at[k], 16);
-      } else {
-        for (int i = threadIdx.x; i < PV; i += blockDim.x) {
-          const int vsel = i < 5 * D ? i / D : 5, d = i - vsel * D;
-          __pipeline_memcpy_async(dst + vsel * Dp + d, src + i, 4);
-        }
-      }
+    for (int ii = 0; ii < MAXR; ++ii) {
+      const int i = (ii >> 2) * (4 * LANES) + s * 4 + (ii & 3);
+      st[j][ii] = (kept && c + j * COLS < E && i < D) ? S[(long long)i * E + c + j * COLS] : 0.f;
     }
-    __pipeline_commit();                       // (an empty group past the end keeps the count)
+  // (volatile: the compiler would move the next token's loads behind the current one's work)
+  auto load4 = [](unsigned at, float4& x) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "r"(at));
   };
+  const unsigned lane_at = (unsigned)__cvta_generic_to_shared(dr_smem) + s * 16;
+  const unsigned v_at = (unsigned)__cvta_generic_to_shared(dr_smem) + (5 * Dp + c) * 4;
+  auto read = [&](int at, DeltaToken<Q, CPT>& x) {
 #pragma unroll
-  for (int k = 0; k < DR_STAGES - 1; ++k) prefetch(t0 + k, k);
-  float* o_at = o_out + ((long long)t0 * H + h) * E + c;
+    for (int q = 0; q < Q; ++q) load4(lane_at + 4 * (at + q * 4 * LANES + 2 * Dp), x.u[q]);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      load4(lane_at + 4 * (at + q * 4 * LANES), x.w[q]);
+      load4(lane_at + 4 * (at + q * 4 * LANES + 3 * Dp), x.k[q]);
+    }
+#pragma unroll
+    for (int j = 0; j < CPT; ++j)
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x.v[j]) : "r"(v_at + 4 * (at + j * COLS)));
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      load4(lane_at + 4 * (at + q * 4 * LANES + Dp), x.b[q]);
+      load4(lane_at + 4 * (at + q * 4 * LANES + 4 * Dp), x.r[q]);
+    }
+  };
+  float* o_at = o_out + ((long long)(t0 - 1) * H + h) * E + c;    // where the token before the current one's output goes
   const long long o_step = (long long)H * E;
-  for (int t = t0; t < t1; ++t) {
-    const int stage = (t - t0) % DR_STAGES;
-    __pipeline_wait_prior(DR_STAGES - 2);      // this thread's copies of token t have landed
-    __syncthreads();                           // ... and everybody's; everybody is done with token t - 1
-    prefetch(t + DR_STAGES - 1, (stage + DR_STAGES - 1) % DR_STAGES);     // into the stage of token t - 1
-    const float* vw = dr_smem + stage * SV;
-    const float* vb = vw + Dp;
-    const float* vu = vb + Dp;
-    const float* vk = vu + Dp;
-    const float* vr = vk + Dp;
-    const float v = active ? vr[Dp + c] : 0.f;
-    float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+  float o_part[CPT] = {};                                    // this lane's part of it
+  bool stores = false;                                       // there is a token before, and this lane stores its output
+  auto store = [&](const float (&o)[CPT]) {
 #pragma unroll
-    for (int q = 0; q < MAXR / 4; ++q) {
-      if (q * 4 < NR) {
-        const float4 u4 = *reinterpret_cast<const float4*>(vu + q * 64 + s * 4);
-        d0 = __fmaf_rn(u4.x, st[q * 4 + 0], d0);
-        d1 = __fmaf_rn(u4.y, st[q * 4 + 1], d1);
-        d2 = __fmaf_rn(u4.z, st[q * 4 + 2], d2);
-        d3 = __fmaf_rn(u4.w, st[q * 4 + 3], d3);
+    for (int j = 0; j < CPT; ++j)
+      if (stores && c + j * COLS < E) o_at[j * COLS] = o[j];
+  };
+  auto work = [&](const DeltaToken<Q, CPT>& x) {
+    float dot[CPT], o[CPT];
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) {
+      float d0 = 0.f, d1 = 0.f, d2 = 0.f, d3 = 0.f;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        d0 = __fmaf_rn(x.u[q].x, st[j][q * 4 + 0], d0);
+        d1 = __fmaf_rn(x.u[q].y, st[j][q * 4 + 1], d1);
+        d2 = __fmaf_rn(x.u[q].z, st[j][q * 4 + 2], d2);
+        d3 = __fmaf_rn(x.u[q].w, st[j][q * 4 + 3], d3);
+      }
+      dot[j] = __fadd_rn(__fadd_rn(d0, d1), __fadd_rn(d2, d3));
+      o[j] = o_part[j];
+    }
+#pragma unroll
+    for (int m = 1; m < LANES; m <<= 1) {
+      float dx[CPT], ox[CPT];
+#pragma unroll
+      for (int j = 0; j < CPT; ++j) {
+        dx[j] = __shfl_xor_sync(0xffffffffu, dot[j], m);
+        ox[j] = __shfl_xor_sync(0xffffffffu, o[j], m);
+      }
+#pragma unroll
+      for (int j = 0; j < CPT; ++j) {
+        dot[j] = __fadd_rn(dot[j], dx[j]);
+        o[j] = __fadd_rn(o[j], ox[j]);
       }
     }
-    float dot = __fadd_rn(__fadd_rn(d0, d1), __fadd_rn(d2, d3));
 #pragma unroll
-    for (int m = 1; m < 16; m <<= 1) dot = __fadd_rn(dot, __shfl_xor_sync(0xffffffffu, dot, m));
-    float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+    for (int j = 0; j < CPT; ++j)
 #pragma unroll
-    for (int q = 0; q < MAXR / 4; ++q) {
-      if (q * 4 < NR) {
-        const int at = q * 64 + s * 4;
-        const float4 w4 = *reinterpret_cast<const float4*>(vw + at);
-        const float4 b4 = *reinterpret_cast<const float4*>(vb + at);
-        const float4 k4 = *reinterpret_cast<const float4*>(vk + at);
-        const float4 r4 = *reinterpret_cast<const float4*>(vr + at);
-        float n0 = __fmaf_rn(k4.x, v, __fmaf_rn(-b4.x, dot, __fmul_rn(w4.x, st[q * 4 + 0])));
-        float n1 = __fmaf_rn(k4.y, v, __fmaf_rn(-b4.y, dot, __fmul_rn(w4.y, st[q * 4 + 1])));
-        float n2 = __fmaf_rn(k4.z, v, __fmaf_rn(-b4.z, dot, __fmul_rn(w4.z, st[q * 4 + 2])));
-        float n3 = __fmaf_rn(k4.w, v, __fmaf_rn(-b4.w, dot, __fmul_rn(w4.w, st[q * 4 + 3])));
-        st[q * 4 + 0] = n0; st[q * 4 + 1] = n1; st[q * 4 + 2] = n2; st[q * 4 + 3] = n3;
-        o0 = __fmaf_rn(r4.x, n0, o0);
-        o1 = __fmaf_rn(r4.y, n1, o1);
-        o2 = __fmaf_rn(r4.z, n2, o2);
-        o3 = __fmaf_rn(r4.w, n3, o3);
+      for (int q = 0; q < Q; ++q) {
+        st[j][q * 4 + 0] = __fmaf_rn(x.k[q].x, x.v[j], __fmul_rn(x.w[q].x, st[j][q * 4 + 0]));
+        st[j][q * 4 + 1] = __fmaf_rn(x.k[q].y, x.v[j], __fmul_rn(x.w[q].y, st[j][q * 4 + 1]));
+        st[j][q * 4 + 2] = __fmaf_rn(x.k[q].z, x.v[j], __fmul_rn(x.w[q].z, st[j][q * 4 + 2]));
+        st[j][q * 4 + 3] = __fmaf_rn(x.k[q].w, x.v[j], __fmul_rn(x.w[q].w, st[j][q * 4 + 3]));
       }
-    }
-    float o = __fadd_rn(__fadd_rn(o0, o1), __fadd_rn(o2, o3));
-#pragma unroll
-    for (int m = 1; m < 16; m <<= 1) o = __fadd_rn(o, __shfl_xor_sync(0xffffffffu, o, m));
-    if (active && s == 0) *o_at = o;
+    store(o);
     o_at += o_step;
-  }
-  __pipeline_wait_prior(0);
-  __syncthreads();                   // the ring is free: the slab goes out through it
+    stores = s == 0;
 #pragma unroll
-  for (int ii = 0; ii < MAXR; ++ii) {
-    const int i = (ii >> 2) * 64 + s * 4 + (ii & 3);
-    if (ii < NR && i < D) slab[i * 8 + cl] = st[ii];
+    for (int j = 0; j < CPT; ++j) {
+      float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        st[j][q * 4 + 0] = __fmaf_rn(-x.b[q].x, dot[j], st[j][q * 4 + 0]);
+        st[j][q * 4 + 1] = __fmaf_rn(-x.b[q].y, dot[j], st[j][q * 4 + 1]);
+        st[j][q * 4 + 2] = __fmaf_rn(-x.b[q].z, dot[j], st[j][q * 4 + 2]);
+        st[j][q * 4 + 3] = __fmaf_rn(-x.b[q].w, dot[j], st[j][q * 4 + 3]);
+        o0 = __fmaf_rn(x.r[q].x, st[j][q * 4 + 0], o0);
+        o1 = __fmaf_rn(x.r[q].y, st[j][q * 4 + 1], o1);
+        o2 = __fmaf_rn(x.r[q].z, st[j][q * 4 + 2], o2);
+        o3 = __fmaf_rn(x.r[q].w, st[j][q * 4 + 3], o3);
+      }
+      o_part[j] = __fadd_rn(__fadd_rn(o0, o1), __fadd_rn(o2, o3));
+    }
+  };
+
+  for (int g = 0; g < groups; ++g) {
+    __syncthreads();
+    const int at = (g % DR_STAGES) * DR_TOKENS * SV;
+    const int n = t1 - t0 - g * DR_TOKENS;
+    DeltaToken<Q, CPT> x, y;
+    if (n < DR_TOKENS) {
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        read(at + i * SV, x);
+        work(x);
+      }
+    } else {
+      read(at, x);
+#pragma unroll
+      for (int i = 0; i < DR_TOKENS; i += 2) {
+        read(at + (i + 1) * SV, y);
+        work(x);
+        if (i + 2 < DR_TOKENS) read(at + (i + 2) * SV, x);
+        work(y);
+      }
+    }
   }
-  __syncthreads();
-  if (kept)
-    for (int i = threadIdx.x; i < D * 8; i += blockDim.x) {
-      const int row = i >> 3, col = i & 7;
-      if (c0 + col < E) S[(long long)row * E + c0 + col] = slab[i];
+#pragma unroll
+  for (int m = 1; m < LANES; m <<= 1)
+#pragma unroll
+    for (int j = 0; j < CPT; ++j) o_part[j] = __fadd_rn(o_part[j], __shfl_xor_sync(0xffffffffu, o_part[j], m));
+  store(o_part);
+#pragma unroll
+  for (int j = 0; j < CPT; ++j)
+#pragma unroll
+    for (int ii = 0; ii < MAXR; ++ii) {
+      const int i = (ii >> 2) * (4 * LANES) + s * 4 + (ii & 3);
+      if (kept && c + j * COLS < E && i < D) S[(long long)i * E + c + j * COLS] = st[j][ii];
     }
 }
 
 // y[t, h, :] = o / sqrt(mean(o^2) + eps) * norm_w[h, :] * sigmoid(g[t, h, :])
-__global__ void delta_output_kernel(const float* o, Source proj, const float* norm_w, void* out, int out_dtype,
-                                    int H, int D, int R, float eps) {
-  __shared__ float scratch[32];
+// A warp per (token, head), 32 elements at a time: the sum of squares is the butterflies' over 32
+// consecutive elements, added in index order.  CHUNKS: how many of them a row has at most (0: any
+// number, read again behind the sum); the gate and the weight are asked for before the sum is made.
+// (2,048 tokens, 16 heads of 64: 10 us; blocks of D threads with a row each: 35 us.)
+constexpr int OUT_WARPS = 8;
+template <int CHUNKS>
+__global__ void __launch_bounds__(OUT_WARPS * 32)
+delta_output_kernel(const float* o, Source proj, const float* norm_w, void* out, int out_dtype, long long rows,
+                    int H, int D, int R, float eps) {
   pdl_prologue();
-  const int t = blockIdx.x, h = blockIdx.y, c = threadIdx.x;
-  const int HD = H * D;
-  const long long at = ((long long)t * H + h) * D + c;
-  const float x = c < D ? o[at] : 0.f;
-  const float ss = block_sum(x * x, scratch);
-  if (c < D) {
+  const long long row = (long long)blockIdx.x * OUT_WARPS + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  const int lane = threadIdx.x & 31;
+  const long long t = row / H;
+  const int h = (int)(row - t * H), HD = H * D;
+  const long long gate = t * (5 * HD + R) + 3 * HD + h * D;
+  float ss = 0.f;
+  if constexpr (CHUNKS > 0) {
+    float x[CHUNKS], g[CHUNKS], w[CHUNKS];
+#pragma unroll
+    for (int j = 0; j < CHUNKS; ++j) {
+      const int c = 32 * j + lane;
+      x[j] = c < D ? o[row * D + c] : 0.f;
+      g[j] = c < D ? source_load(proj, gate + c) : 0.f;
+      w[j] = c < D ? norm_w[h * D + c] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < CHUNKS; ++j)
+      if (32 * j < D) ss += warp_sum(x[j] * x[j]);
     const float rstd = 1.0f / sqrtf(ss / (float)D + eps);
-    const float g = source_load(proj, (long long)t * (5 * HD + R) + 3 * HD + h * D + c);
-    store_as(out, out_dtype, at, x * rstd * norm_w[h * D + c] * sigmoid_f32(g));
+#pragma unroll
+    for (int j = 0; j < CHUNKS; ++j)
+      if (32 * j + lane < D) store_as(out, out_dtype, row * D + 32 * j + lane, x[j] * rstd * w[j] * sigmoid_f32(g[j]));
+  } else {
+    for (int c0 = 0; c0 < D; c0 += 32) {
+      const float x = c0 + lane < D ? o[row * D + c0 + lane] : 0.f;
+      ss += warp_sum(x * x);
+    }
+    const float rstd = 1.0f / sqrtf(ss / (float)D + eps);
+    for (int c = lane; c < D; c += 32)
+      store_as(out, out_dtype, row * D + c,
+               o[row * D + c] * rstd * norm_w[h * D + c] * sigmoid_f32(source_load(proj, gate + c)));
   }
 }
 
@@ -433,24 +582,29 @@ static int launch_recurrence(const float* packed, float* state, long long slot_s
   return DIB_OK;
 }
 
-template <int MAXR, int DR_STAGES>
+template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES>
 static int launch_recurrence_wide(const float* packed, float* state, long long slot_stride, float* o_out,
                                   const int* cu_q_lens, const int* state_slots, int B, int H, int D, int E,
                                   cudaStream_t st) {
-  const int Dp = (D + 63) / 64 * 64, Ep = (E + 63) / 64 * 64;
-  size_t smem = sizeof(float) * DR_STAGES * (5 * Dp + Ep);       // 12 KB at D = E = 64, 24 at 256
-  if (smem < sizeof(float) * 8 * D) smem = sizeof(float) * 8 * D;
+  constexpr int COLUMNS = 32 / LANES * CPT * WARPS;        // a block's
+  constexpr size_t smem = sizeof(float) * DR_STAGES * DR_TOKENS * 6 * LANES * MAXR;    // 48 KB for 64, 96 for 128 and 256
+  auto* kernel = &delta_recurrence_wide_kernel<MAXR, LANES, CPT, WARPS, DR_TOKENS, DR_STAGES>;
+  static DeviceOnce once;
+  if (!once.done()) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return DIB_LAUNCH_FAILED;
+    once.mark();
+  }
   // Launched in plain stream order, not ahead of its predecessor's end: blocks that are placed
   // while the kernel before still fills the GPU land several to an SM on the SMs that happen to
   // be free, and a long chain of dependent instructions then shares its scheduler for the whole
-  // kernel (2,048 tokens, 16 heads of 64: 2.0 ms against 1.0 ms).
+  // kernel.
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(B, H, (E + 7) / 8);
-  cfg.blockDim = dim3(128);
+  cfg.gridDim = dim3(B, H, (E + COLUMNS - 1) / COLUMNS);
+  cfg.blockDim = dim3(32 * WARPS + 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchKernelEx(&cfg, delta_recurrence_wide_kernel<MAXR, DR_STAGES>, packed, state, slot_stride, o_out,
-                     cu_q_lens, state_slots, H, D, E);
+  cudaLaunchKernelEx(&cfg, kernel, packed, state, slot_stride, o_out, cu_q_lens, state_slots, H, D, E);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
@@ -463,8 +617,12 @@ int dib_delta_prepare(const void* proj, int kind, int splits, long long stride, 
   if (T_ == 0) return DIB_OK;
   if (H < 1 || H > 65535 || D < 1 || D > 1024 || R < 0 || R > 8192) return DIB_BAD_SIZE;
   if (w_dtype != 0 && w_dtype != 1) return DIB_BAD_DTYPE;
-  dib_launch(delta_prepare_kernel, dim3(T_, H), dim3((D + 31) / 32 * 32), sizeof(float) * (R + 32), st,
-             make_source(proj, kind, splits, stride), w2t, w_dtype, w0, a_bias, packed, H, D, R, decay_scale,
+  const int form = kind == 1 ? 1 : splits <= 1 ? 0 : 2;
+  auto* kernel = form == 0   ? (w_dtype == 1 ? &delta_prepare_kernel<0, 1> : &delta_prepare_kernel<0, 0>)
+                 : form == 1 ? (w_dtype == 1 ? &delta_prepare_kernel<1, 1> : &delta_prepare_kernel<1, 0>)
+                             : (w_dtype == 1 ? &delta_prepare_kernel<2, 1> : &delta_prepare_kernel<2, 0>);
+  dib_launch(kernel, dim3(ceil_div_host(T_, PREP_TOKENS), H), dim3((D + 31) / 32 * 32), 0, st,
+             make_source(proj, kind, splits, stride), w2t, w0, a_bias, packed, T_, H, D, R, decay_scale,
              key_eps);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
@@ -481,11 +639,11 @@ int dib_delta_recurrence(const float* packed, float* state, long long slot_strid
   if (B == 0) return DIB_OK;
   if (H < 1 || H > 65535 || D < 1 || D > 256 || E < 1 || E > 256) return DIB_BAD_SIZE;
   const int big = D > E ? D : E;       // (the staging's pieces are counted for the larger of the two)
-#define DIB_DR(F, MAXR, STAGES) return F<MAXR, STAGES>(packed, state, slot_stride, o_out, cu_q_lens, state_slots, B, H, D, E, st)
+#define DIB_DR(F, ...) return F<__VA_ARGS__>(packed, state, slot_stride, o_out, cu_q_lens, state_slots, B, H, D, E, st)
   if (form == 1) {
-    if (big <= 64) DIB_DR(launch_recurrence_wide, 4, 8);
-    if (big <= 128) DIB_DR(launch_recurrence_wide, 8, 6);
-    DIB_DR(launch_recurrence_wide, 16, 4);
+    if (big <= 64) DIB_DR(launch_recurrence_wide, 4, 16, 1, 4, 16, 2);
+    if (big <= 128) DIB_DR(launch_recurrence_wide, 8, 16, 2, 4, 16, 2);
+    DIB_DR(launch_recurrence_wide, 16, 16, 2, 4, 8, 2);
   }
   if (big <= 64) DIB_DR(launch_recurrence, 16, 8);
   if (big <= 128) DIB_DR(launch_recurrence, 32, 6);
@@ -499,8 +657,10 @@ int dib_delta_output(const float* o, const void* proj, int kind, int splits, lon
   if (T_ == 0) return DIB_OK;
   if (H < 1 || H > 65535 || D < 1 || D > 1024) return DIB_BAD_SIZE;
   if (out_dtype != 0 && out_dtype != 1) return DIB_BAD_DTYPE;
-  dib_launch(delta_output_kernel, dim3(T_, H), dim3((D + 31) / 32 * 32), 0, st, o,
-             make_source(proj, kind, splits, stride), norm_w, out, out_dtype, H, D, R, eps);
+  const long long rows = (long long)T_ * H;
+  auto* kernel = D <= 64 ? &delta_output_kernel<2> : D <= 128 ? &delta_output_kernel<4> : &delta_output_kernel<0>;
+  dib_launch(kernel, dim3(ceil_div_host(rows, OUT_WARPS)), dim3(OUT_WARPS * 32), 0, st, o,
+             make_source(proj, kind, splits, stride), norm_w, out, out_dtype, rows, H, D, R, eps);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
