@@ -6,12 +6,15 @@
 // its own position alone.
 //
 // Page layout: the keys of a page [Hkv, page_size, D], then its values [Hkv, page_size, Dv].
+#include <type_traits>
+
 #include "sigmoid_attention_mma.cuh"
-#include "source.cuh"
+#include "source_vec.cuh"
 
 // Projection rows [q heads | k heads | v heads] plus a bias: q to q_out [T, Hq, D], k and v
-// into the token's cache slot (slot = page * page_size + offset; negative: skip).
-template <typename T>
+// into the token's cache slot (slot = page * page_size + offset; negative: skip).  VEC: four elements a
+// thread and step, where heads, rows and pointers allow it.
+template <typename T, bool VEC>
 __global__ void qkv_bias_cache_kernel(Source qkv, const float* bias, T* q_out, T* cache,
                                       const int* slot_mapping, int Hq, int Hkv, int D, int VD,
                                       int page_size, long long num_pages, int write_cache) {
@@ -24,20 +27,32 @@ __global__ void qkv_bias_cache_kernel(Source qkv, const float* bias, T* q_out, T
   const long long page = slot >= 0 ? slot / page_size : -1;
   const int off = slot >= 0 ? slot % page_size : 0;
   const bool ok = page >= 0 && page < num_pages;
-  for (int c = threadIdx.x; c < width; c += blockDim.x) {
-    float v = source_load(qkv, (long long)t * width + c);
-    if (bias != nullptr) v = __fadd_rn(v, bias[c]);
-    if (c < nq) {
-      Elem<T>::store(q_out + (long long)t * nq + c, v);
-    } else if (ok) {
-      if (c < nq + nk) {
-        const int g = (c - nq) / D, d = (c - nq) % D;
-        Elem<T>::store(cache + page * page_elems + ((long long)g * page_size + off) * D + d, v);
-      } else {
-        const int g = (c - nq - nk) / VD, d = (c - nq - nk) % VD;
-        Elem<T>::store(cache + page * page_elems + (long long)Hkv * page_size * D +
-                           ((long long)g * page_size + off) * VD + d, v);
+  auto place = [&](int c) -> T* {          // where column c goes (null: nowhere)
+    if (c < nq) return q_out + (long long)t * nq + c;
+    if (!ok) return nullptr;
+    if (c < nq + nk) {
+      const int g = (c - nq) / D, d = (c - nq) % D;
+      return cache + page * page_elems + ((long long)g * page_size + off) * D + d;
+    }
+    const int g = (c - nq - nk) / VD, d = (c - nq - nk) % VD;
+    return cache + page * page_elems + (long long)Hkv * page_size * D + ((long long)g * page_size + off) * VD + d;
+  };
+  if constexpr (VEC) {
+    for (int c = 4 * threadIdx.x; c < width; c += 4 * blockDim.x) {
+      float4 v = source_load4(qkv, (long long)t * width + c);
+      if (bias != nullptr) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + c);
+        v = make_float4(__fadd_rn(v.x, b.x), __fadd_rn(v.y, b.y), __fadd_rn(v.z, b.z), __fadd_rn(v.w, b.w));
       }
+      T* to = place(c);
+      if (to != nullptr) store4(to, v);
+    }
+  } else {
+    for (int c = threadIdx.x; c < width; c += blockDim.x) {
+      float v = source_load(qkv, (long long)t * width + c);
+      if (bias != nullptr) v = __fadd_rn(v, bias[c]);
+      T* to = place(c);
+      if (to != nullptr) Elem<T>::store(to, v);
     }
   }
 }
@@ -144,13 +159,18 @@ int dib_qkv_bias_cache(const void* qkv, int kind, int splits, long long stride, 
   if (Hq < 1 || Hkv < 1 || D < 1 || VD < 1 || page_size < 1) return DIB_BAD_SIZE;
   const Source s = make_source(qkv, kind, splits, stride);
   const int wc = cache != nullptr ? 1 : 0;
-  if (dtype == 0)
-    dib_launch(qkv_bias_cache_kernel<float>, dim3(T_), dim3(256), 0, st, s, bias, (float*)q_out, (float*)cache,
-               slot_mapping, Hq, Hkv, D, VD, page_size, num_pages, wc);
-  else if (dtype == 1)
-    dib_launch(qkv_bias_cache_kernel<__nv_bfloat16>, dim3(T_), dim3(256), 0, st, s, bias,
-               (__nv_bfloat16*)q_out, (__nv_bfloat16*)cache, slot_mapping, Hq, Hkv, D, VD, page_size,
+  const bool vec = D % 4 == 0 && VD % 4 == 0 && source_takes_vectors(s) && (uintptr_t)bias % 16 == 0 &&
+                   vectors_start_at(q_out, dtype) && vectors_start_at(cache, dtype);
+  auto go = [&](auto* kernel, auto* tag) {
+    using E = std::remove_pointer_t<decltype(tag)>;
+    dib_launch(kernel, dim3(T_), dim3(256), 0, st, s, bias, (E*)q_out, (E*)cache, slot_mapping, Hq, Hkv, D, VD, page_size,
                num_pages, wc);
+  };
+  if (dtype == 0)
+    go(vec ? &qkv_bias_cache_kernel<float, true> : &qkv_bias_cache_kernel<float, false>, (float*)nullptr);
+  else if (dtype == 1)
+    go(vec ? &qkv_bias_cache_kernel<__nv_bfloat16, true> : &qkv_bias_cache_kernel<__nv_bfloat16, false>,
+       (__nv_bfloat16*)nullptr);
   else return DIB_BAD_DTYPE;
   DIB_CHECK_LAUNCH();
   return DIB_OK;

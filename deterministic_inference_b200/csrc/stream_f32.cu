@@ -3,7 +3,7 @@
 // (alone, or after adding up to three scaled outputs to it), the scaled sum as a
 // tensor, the xIELU activation and the soft cap of the logits.  All arithmetic is float32;
 // inputs that come from a matrix product may be its split-k partial products.
-#include "source.cuh"
+#include "source_vec.cuh"
 
 // out[t] = table[ids[t]] + pos_table[positions[t]], float32
 __global__ void embed_pos_kernel(const void* table, const void* pos_table, int dtype, const int* ids,
@@ -436,42 +436,51 @@ __global__ void weighted_sum_kernel(Source x0, float a0, Source x1, float a1, in
   }
 }
 
-// xIELU: z > 0: ap z^2 + z / 2;  z <= 0: an (exp(z) - 1 - z) + z / 2
-__global__ void xielu_kernel(Source z, float ap, float an, void* out, int out_dtype, long long n) {
-  pdl_prologue();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const float x = source_load(z, i);
-    const float y = x > 0.f ? __fmaf_rn(__fmul_rn(ap, x), x, 0.5f * x)
-                            : __fmaf_rn(an, expm1f(x) - x, 0.5f * x);
-    store_as(out, out_dtype, i, y);
+// out = f(z), element by element; VEC: four at a time (n a multiple of 4, see source_takes_vectors)
+template <bool VEC, typename F>
+__device__ __forceinline__ void each_element(const Source& z, void* out, int out_dtype, long long n, F f) {
+  const long long step = (long long)gridDim.x * blockDim.x;
+  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if constexpr (VEC) {
+    for (; i < n / 4; i += step) {
+      const float4 x = source_load4(z, 4 * i);
+      store4_as(out, out_dtype, 4 * i, make_float4(f(x.x), f(x.y), f(x.z), f(x.w)));
+    }
+  } else {
+    for (; i < n; i += step) store_as(out, out_dtype, i, f(source_load(z, i)));
   }
+}
+// xIELU: z > 0: ap z^2 + z / 2;  z <= 0: an (exp(z) - 1 - z) + z / 2
+template <bool VEC>
+__global__ void xielu_kernel(Source z, float ap, float an, void* out, int out_dtype, long long n) {
+  pdl_prologue(z.p);
+  each_element<VEC>(z, out, out_dtype, n, [&](float x) {
+    return x > 0.f ? __fmaf_rn(__fmul_rn(ap, x), x, 0.5f * x) : __fmaf_rn(an, expm1f(x) - x, 0.5f * x);
+  });
 }
 
 // out = max(z, 0)^2
+template <bool VEC>
 __global__ void squared_relu_kernel(Source z, void* out, int out_dtype, long long n) {
   pdl_prologue(z.p);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const float x = fmaxf(source_load(z, i), 0.f);
-    store_as(out, out_dtype, i, x * x);
-  }
+  each_element<VEC>(z, out, out_dtype, n, [](float x) {
+    x = fmaxf(x, 0.f);
+    return x * x;
+  });
 }
 
 // x = cap * tanh(x / cap), in place
-__global__ void softcap_kernel(float* x, float cap, long long n) {
-  pdl_prologue();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    x[i] = cap * tanhf(x[i] / cap);
+template <bool VEC>
+__global__ void softcap_kernel(Source x, float* out, float cap, long long n) {
+  pdl_prologue(x.p);
+  each_element<VEC>(x, out, 0, n, [&](float v) { return cap * tanhf(v / cap); });
 }
 
 // x = x * a, in place
-__global__ void scale_kernel(float* x, float a, long long n) {
-  pdl_prologue();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    x[i] = __fmul_rn(x[i], a);
+template <bool VEC>
+__global__ void scale_kernel(Source x, float* out, float a, long long n) {
+  pdl_prologue(x.p);
+  each_element<VEC>(x, out, 0, n, [&](float v) { return __fmul_rn(v, a); });
 }
 
 static inline int flat_grid(long long n, int block) {
@@ -629,8 +638,11 @@ int dib_xielu(const void* z, int kind, int splits, long long stride, float ap, f
               int out_dtype, long long n, cudaStream_t st) {
   if (n == 0) return DIB_OK;
   if (out_dtype != 0 && out_dtype != 1) return DIB_BAD_DTYPE;
-  dib_launch(xielu_kernel, dim3(flat_grid(n, 256)), dim3(256), 0, st, make_source(z, kind, splits, stride), ap,
-             an, out, out_dtype, n);
+  const Source src = make_source(z, kind, splits, stride);
+  if (n % 4 == 0 && source_takes_vectors(src) && vectors_start_at(out, out_dtype))
+    dib_launch(xielu_kernel<true>, dim3(flat_grid(n / 4, 256)), dim3(256), 0, st, src, ap, an, out, out_dtype, n);
+  else
+    dib_launch(xielu_kernel<false>, dim3(flat_grid(n, 256)), dim3(256), 0, st, src, ap, an, out, out_dtype, n);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
@@ -639,22 +651,34 @@ int dib_squared_relu(const void* z, int kind, int splits, long long stride, void
                      cudaStream_t st) {
   if (n == 0) return DIB_OK;
   if (out_dtype != 0 && out_dtype != 1) return DIB_BAD_DTYPE;
-  dib_launch(squared_relu_kernel, dim3(flat_grid(n, 256)), dim3(256), 0, st, make_source(z, kind, splits, stride), out,
-             out_dtype, n);
+  const Source src = make_source(z, kind, splits, stride);
+  // (a few rows of split sums: one element a thread keeps more loads in flight)
+  if (n >= 148 * 2048 * 4 && n % 4 == 0 && source_takes_vectors(src) && vectors_start_at(out, out_dtype))
+    dib_launch(squared_relu_kernel<true>, dim3(flat_grid(n / 4, 256)), dim3(256), 0, st, src, out, out_dtype, n);
+  else
+    dib_launch(squared_relu_kernel<false>, dim3(flat_grid(n, 256)), dim3(256), 0, st, src, out, out_dtype, n);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
 
 int dib_scale(float* x, float a, long long n, cudaStream_t st) {
   if (n == 0) return DIB_OK;
-  dib_launch(scale_kernel, dim3(flat_grid(n, 256)), dim3(256), 0, st, x, a, n);
+  const Source src = make_source(x, 0, 1, 0);
+  if (n % 4 == 0 && source_takes_vectors(src))
+    dib_launch(scale_kernel<true>, dim3(flat_grid(n / 4, 256)), dim3(256), 0, st, src, x, a, n);
+  else
+    dib_launch(scale_kernel<false>, dim3(flat_grid(n, 256)), dim3(256), 0, st, src, x, a, n);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
 
 int dib_softcap(float* x, float cap, long long n, cudaStream_t st) {
   if (n == 0) return DIB_OK;
-  dib_launch(softcap_kernel, dim3(flat_grid(n, 256)), dim3(256), 0, st, x, cap, n);
+  const Source src = make_source(x, 0, 1, 0);
+  if (n % 4 == 0 && source_takes_vectors(src))
+    dib_launch(softcap_kernel<true>, dim3(flat_grid(n / 4, 256)), dim3(256), 0, st, src, x, cap, n);
+  else
+    dib_launch(softcap_kernel<false>, dim3(flat_grid(n, 256)), dim3(256), 0, st, src, x, cap, n);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }

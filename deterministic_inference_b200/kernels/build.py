@@ -56,8 +56,8 @@ EXTRA_HEADERS = {
     "attention_bf16": ("attention_bf16_kernels.cuh",),
     "decode_attention_noalloc": ("attention_bf16_kernels.cuh", "decode_attention_noalloc.h"),
     "attention_prefill_tc": ("attention_bf16_kernels.cuh",),
-    "stream_f32": ("source.cuh",),
-    "sigmoid_attention": ("source.cuh", "sigmoid_attention_mma.cuh"),
+    "stream_f32": ("source.cuh", "source_vec.cuh"),
+    "sigmoid_attention": ("source.cuh", "source_vec.cuh", "sigmoid_attention_mma.cuh"),
     "delta_rule": ("source.cuh", "conv_tail.cuh"),
     "masked_attention": ("source.cuh", "masked_attention_mma.cuh", "sigmoid_attention_mma.cuh", "conv_tail.cuh"),
     "state_space": ("source.cuh", "conv_tail.cuh"),

@@ -72,6 +72,40 @@ def test_stream_kernels_alone(dtype):
     close(ops.softcap_(logits.clone().to(dev), 11.0), pg.softcap(logits.double(), 11.0), "float32", "soft cap")
 
 
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("rows, width, splits", [(3, 4, 1), (5, 132, 3), (2048, 12, 1), (700, 2052, 1)])
+def test_elements_by_fours_are_those_one_by_one(dtype, rows, width, splits):
+    """The element-wise kernels on memory that allows vectors of four and on the same values one element further on,
+    which does not: the same bits."""
+    from deterministic_inference_b200.kernels import ops
+    dt, dev = DTYPES[dtype], "cuda"
+    g = torch.Generator(device=dev).manual_seed(width)
+
+    def both(f, kind=torch.float32):
+        x = (3 * torch.randn(splits, rows, width, generator=g, device=dev)).to(kind)
+        there = torch.empty(x.numel() + 1, dtype=kind, device=dev)[1:].view(x.shape).copy_(x)
+        source = lambda t: ops.SplitSum(t, torch.float32) if splits > 1 else t[0]
+        assert torch.equal(f(source(x)), f(source(there)))
+
+    both(lambda z: ops.xielu(z, 0.7, 1.3, dt))
+    both(lambda z: ops.squared_relu(z, dt))
+    if splits == 1:
+        both(lambda z: ops.softcap_(z, 11.0))
+        both(lambda z: ops.scale_(z, 0.3))
+        both(lambda z: ops.xielu(z, 0.7, 1.3, dt), torch.bfloat16)
+    dim = width // 4
+    bias = torch.randn(width, generator=g, device=dev)
+    slots = torch.randperm(rows, device=dev).int()
+    caches = []
+
+    def split_heads(qkv):
+        caches.append(torch.zeros(-(-rows // 16), 16 * 3 * dim, dtype=dt, device=dev))
+        return ops.qkv_bias_cache(qkv, bias, 1, 1, dim, 2 * dim, caches[-1], slots, 16, dt)
+
+    both(split_heads)
+    assert torch.equal(caches[0], caches[1])
+
+
 # ---- attention without a softmax ---------------------------------------------------------------------
 
 def paged(n_tokens_per_seq, page, generator):
