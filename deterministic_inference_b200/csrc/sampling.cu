@@ -177,30 +177,34 @@ __device__ __forceinline__ void load_chunk(const float* __restrict__ row, int lo
 // bits of the probability (it has no sign), 10, 11 and 10 bits a pass, with a histogram of
 // counts and of masses per pass.  Masses are added as 40-bit fixed point, so that the order
 // of the additions (atomics) cannot change a bit.  Tokens that tie with the threshold all
-// stay (a sort would keep some of them).  A pass is one kernel with a block per chunk of a
-// row; the histograms lie in global memory (masses [R][FILTER_BINS], then the rows'
-// states and normalisers, then counts; zeroed by the kernel that computes the normaliser); every block works out
-// the bits of the pass before its own, on top of the state that pass's first block left.
+// stay (a sort would keep some of them).  The first two passes have a block per chunk of a
+// row; the block that is last to add its histogram to the row's works out the row's bits and
+// leaves them for the next pass.  The first forms every probability; the second only those
+// whose log2 may lie in the first's bin, and lists the bin's probabilities; the third is a
+// block a row over that list (over the row again, where the list is too short).
 // (Four passes of 8 bits that formed every probability again, added up a warp's equal bins
 // by matching lanes and chained the chunks' normalisers in every thread: 69 us each, and
-// the pick 68 us; with 64 rows of 151,936, 38 of them filtered, the whole draw 318 us, so 122 us.)
+// the pick 68 us; with 64 rows of 151,936, 38 of them filtered, the whole draw 318 us.  Three
+// passes over the chunks, each of whose blocks works out the pass before: 122 us; so
+// 104 us.)
 constexpr float MASS_ONE = 1099511627776.0f;     // 2^40
-constexpr int FILTER_PASSES = 3;
-constexpr int FILTER_BINS = 4096;                // 1024 + 2048 + 1024
-__host__ __device__ __forceinline__ constexpr int pass_bits(int pass) { return pass == 1 ? 11 : 10; }
-__host__ __device__ __forceinline__ constexpr int pass_shift(int pass) { return pass == 0 ? 21 : pass == 1 ? 10 : 0; }
-__host__ __device__ __forceinline__ constexpr int pass_first_bin(int pass) { return pass == 0 ? 0 : pass == 1 ? 1024 : 3072; }
+constexpr int FILTER_BINS0 = 1024, FILTER_BINS1 = 2048, FILTER_BINS2 = 1024;      // of the passes
+constexpr int FILTER_SHIFT0 = 21, FILTER_SHIFT1 = 10;
+constexpr int FILTER_BINS = FILTER_BINS0 + FILTER_BINS1;       // a row's in global memory
+constexpr int FILTER_LIST = 16384;                             // probabilities a row's list holds
 
 struct FilterState {
   unsigned long long cnt_above, mass_above;   // tokens (and their mass) above the chosen bins
   unsigned prefix;                            // the threshold's bits found so far
   unsigned pad;
 };
+// a row's counters: blocks that have added to the first and to the second histogram, listed probabilities
+enum { MARK_FIRST = 0, MARK_SECOND = 1, MARK_LISTED = 2, ROW_MARKS = 4 };
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 gumbel_stats_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
                     float* __restrict__ cmax, float* __restrict__ csum, unsigned* __restrict__ hist_cnt,
-                    unsigned long long* __restrict__ hist_mass, int V, int chunks) {
+                    unsigned long long* __restrict__ hist_mass, unsigned* __restrict__ marks, int V, int chunks) {
   pdl_prologue(logits, temperatures);
   __shared__ float fscratch[32];
   const int r = blockIdx.y, c = blockIdx.x;
@@ -210,6 +214,7 @@ gumbel_stats_kernel(const float* __restrict__ logits, const float* __restrict__ 
       hist_cnt[(size_t)r * FILTER_BINS + e] = 0u;
       hist_mass[(size_t)r * FILTER_BINS + e] = 0ull;
     }
+    if (c == 0 && threadIdx.x < ROW_MARKS) marks[(size_t)r * ROW_MARKS + threadIdx.x] = 0u;
   }
   const float temp = temperatures[r];
   if (temp <= 0.f) return;     // a greedy row needs no normaliser
@@ -294,9 +299,9 @@ struct DescendScratch {
   int chosen[8];
   FilterState st;
 };
-template <int BINS>
-__device__ __forceinline__ FilterState filter_descend(const unsigned* __restrict__ hist_cnt,
-                                                      const unsigned long long* __restrict__ hist_mass,
+// (SHARED: the histograms lie in shared memory)
+template <int BINS, bool SHARED = false>
+__device__ __forceinline__ FilterState filter_descend(const unsigned* hist_cnt, const unsigned long long* hist_mass,
                                                       FilterState st, int shift, unsigned long long k,
                                                       unsigned long long P, DescendScratch& sc) {
   constexpr int B = BINS / SAMPLE_THREADS;       // a thread's bins
@@ -305,8 +310,8 @@ __device__ __forceinline__ FilterState filter_descend(const unsigned* __restrict
   unsigned long long m[B], msum = 0ull;
 #pragma unroll
   for (int j = 0; j < B; ++j) {
-    c[j] = __ldcg(hist_cnt + threadIdx.x * B + j);
-    m[j] = __ldcg(hist_mass + threadIdx.x * B + j);
+    c[j] = SHARED ? hist_cnt[threadIdx.x * B + j] : __ldcg(hist_cnt + threadIdx.x * B + j);
+    m[j] = SHARED ? hist_mass[threadIdx.x * B + j] : __ldcg(hist_mass + threadIdx.x * B + j);
     csum += c[j];
     msum += m[j];
   }
@@ -359,49 +364,76 @@ __device__ __forceinline__ FilterState filter_descend(const unsigned* __restrict
   __syncthreads();
   return sc.st;
 }
-// after pass `pass` (0 .. 2) of row r; `states` holds what the passes before it found, [FILTER_PASSES][R]
-__device__ __forceinline__ FilterState state_after(int pass, const unsigned* hist_cnt,
-                                                   const unsigned long long* hist_mass, const FilterState* states,
-                                                   int R, int r, unsigned long long k, unsigned long long P,
-                                                   DescendScratch& sc) {
-  FilterState st{0ull, 0ull, 0u, 0u};
-  if (pass > 0) {
-    const FilterState* at = states + (size_t)(pass - 1) * R + r;
-    st.cnt_above = __ldcg(&at->cnt_above);
-    st.mass_above = __ldcg(&at->mass_above);
-    st.prefix = __ldcg(&at->prefix);
-  }
-  const size_t first = (size_t)r * FILTER_BINS + pass_first_bin(pass);
-  return pass == 1 ? filter_descend<2048>(hist_cnt + first, hist_mass + first, st, pass_shift(1), k, P, sc)
-                   : filter_descend<1024>(hist_cnt + first, hist_mass + first, st, pass_shift(pass), k, P, sc);
+// Has every block of the row added to its histogram (this one just has)?  The same answer in all threads.
+__device__ __forceinline__ bool last_of_row(unsigned* mark, int chunks, bool* flag) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) *flag = atomicAdd(mark, 1u) == (unsigned)chunks - 1u;
+  __syncthreads();
+  if (*flag) __threadfence();
+  return *flag;
 }
+// One token's probability into histograms of `bins` counts and masses in halves of 20 bits, whose sums over a
+// chunk fit 32 bits; every lane of the warp calls.  32 tokens of one bin (a flat row, a tail that underflows) are
+// one addition.
+__device__ __forceinline__ void count_token(float p, unsigned bin, bool in, unsigned* cnt, unsigned* low, unsigned* high) {
+  const unsigned long long m = (unsigned long long)(p * MASS_ONE);
+  const unsigned first = __shfl_sync(0xffffffffu, bin, 0);
+  if (__all_sync(0xffffffffu, in && bin == first)) {
+    const unsigned l = __reduce_add_sync(0xffffffffu, (unsigned)(m & 0xfffffull));
+    const unsigned h = __reduce_add_sync(0xffffffffu, (unsigned)(m >> 20));
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&cnt[bin], 32u);
+      atomicAdd(&low[bin], l);
+      atomicAdd(&high[bin], h);
+    }
+  } else if (in) {
+    atomicAdd(&cnt[bin], 1u);
+    atomicAdd(&low[bin], (unsigned)(m & 0xfffffull));
+    atomicAdd(&high[bin], (unsigned)(m >> 20));
+  }
+}
+template <int BINS>
+__device__ __forceinline__ void add_histogram(const unsigned* cnt, const unsigned* low, const unsigned* high,
+                                              unsigned* __restrict__ hist_cnt,
+                                              unsigned long long* __restrict__ hist_mass) {
+  for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS)
+    if (cnt[b] != 0u) {
+      atomicAdd(&hist_cnt[b], cnt[b]);
+      atomicAdd(&hist_mass[b], ((unsigned long long)high[b] << 20) + low[b]);
+    }
+}
+// what a row asks for: fewer than k tokens above a kept one, weighing at most P
+struct FilterLimits {
+  unsigned long long k, P;
+  __device__ __forceinline__ FilterLimits(long long top_k, float top_p, int V)
+      : k(top_k > 0 ? (unsigned long long)top_k : (unsigned long long)V + 1),
+        P(top_p >= 1.0f ? ~0ull : (unsigned long long)(top_p * MASS_ONE)) {}
+};
 
 __device__ __forceinline__ bool row_is_filtered(float temp, long long top_k, float top_p) {
   return temp > 0.f && (top_k > 0 || top_p < 1.0f);
 }
 
-template <int PASS>
+// states: [2][R], what the first and the second pass find
 __global__ void __launch_bounds__(SAMPLE_THREADS)
-filter_histogram_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
-                        const long long* __restrict__ top_ks, const float* __restrict__ top_ps,
-                        const float* __restrict__ cmax, const float* __restrict__ csum,
-                        unsigned* __restrict__ hist_cnt, unsigned long long* __restrict__ hist_mass,
-                        FilterState* __restrict__ states, float2* __restrict__ norms, int R, int V, int chunks) {
-  pdl_prologue(logits, temperatures, top_ks, top_ps, cmax, csum, states, norms);
-  constexpr int BINS = 1 << pass_bits(PASS), SHIFT = pass_shift(PASS);
-  // 40-bit masses in two halves: a chunk's sums of either fit 32 bits, which shared memory adds natively
-  __shared__ unsigned s_cnt[BINS], s_low[BINS], s_high[BINS];
+filter_first_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
+                    const long long* __restrict__ top_ks, const float* __restrict__ top_ps,
+                    const float* __restrict__ cmax, const float* __restrict__ csum, unsigned* hist_cnt,
+                    unsigned long long* hist_mass, FilterState* __restrict__ states, float2* __restrict__ norms,
+                    unsigned* marks, int V, int chunks) {
+  pdl_prologue(logits, temperatures, top_ks, top_ps, cmax, csum);
+  __shared__ unsigned s_cnt[FILTER_BINS0], s_low[FILTER_BINS0], s_high[FILTER_BINS0];
   __shared__ NormaliserScratch nsc;
   __shared__ DescendScratch dsc;
-  __shared__ float s_list[PASS == 0 ? 1 : ARGMAX_CHUNK];
-  __shared__ int s_listed;
+  __shared__ bool s_last;
   const int r = blockIdx.y, c = blockIdx.x;
   const float temp = temperatures[r];
   const long long top_k = top_ks[r];
   const float top_p = top_ps[r];
   float mx, sum;
   if (!row_is_filtered(temp, top_k, top_p)) {
-    if (PASS == 0 && c == 0 && temp > 0.f) {       // (the pick reads every row's normaliser)
+    if (c == 0 && temp > 0.f) {                    // (the pick reads every row's normaliser)
       row_normaliser(cmax, csum, r, chunks, nsc, mx, sum);
       if (threadIdx.x == 0) norms[r] = make_float2(mx, sum);
     }
@@ -410,118 +442,171 @@ filter_histogram_kernel(const float* __restrict__ logits, const float* __restric
   const int lo = c * ARGMAX_CHUNK, hi = min(V, lo + ARGMAX_CHUNK);
   float x[PER_THREAD];
   load_chunk(logits + (size_t)r * V, lo, hi, x);
-  const unsigned long long k = top_k > 0 ? (unsigned long long)top_k : (unsigned long long)V + 1;
-  const unsigned long long P = top_p >= 1.0f ? ~0ull : (unsigned long long)(top_p * MASS_ONE);
-  for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS) s_cnt[b] = s_low[b] = s_high[b] = 0u;
-  if (threadIdx.x == 0) s_listed = 0;
-  unsigned prefix = 0u;
-  if constexpr (PASS > 0) {
-    const FilterState st = state_after(PASS - 1, hist_cnt, hist_mass, states, R, r, k, P, dsc);
-    if (c == 0 && threadIdx.x == 0) states[(size_t)(PASS - 1) * R + r] = st;
-    prefix = st.prefix;
-  }
-  if constexpr (PASS == 0) {
-    row_normaliser(cmax, csum, r, chunks, nsc, mx, sum);
-    if (c == 0 && threadIdx.x == 0) norms[r] = make_float2(mx, sum);
-  } else {
-    const float2 n = norms[r];
-    mx = n.x;
-    sum = n.y;
+  for (int b = threadIdx.x; b < FILTER_BINS0; b += SAMPLE_THREADS) s_cnt[b] = s_low[b] = s_high[b] = 0u;
+  row_normaliser(cmax, csum, r, chunks, nsc, mx, sum);
+  if (c == 0 && threadIdx.x == 0) norms[r] = make_float2(mx, sum);
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < PER_THREAD; ++j) {
+    const float p = row_probability(x[j], temp, mx, sum);
+    count_token(p, (__float_as_uint(p) >> FILTER_SHIFT0) & (FILTER_BINS0 - 1),
+                lo + (int)threadIdx.x + j * SAMPLE_THREADS < hi, s_cnt, s_low, s_high);
   }
   __syncthreads();
+  hist_cnt += (size_t)r * FILTER_BINS;
+  hist_mass += (size_t)r * FILTER_BINS;
+  add_histogram<FILTER_BINS0>(s_cnt, s_low, s_high, hist_cnt, hist_mass);
+  if (last_of_row(&marks[(size_t)r * ROW_MARKS + MARK_FIRST], chunks, &s_last)) {
+    const FilterLimits lim(top_k, top_p, V);
+    const FilterState st = filter_descend<FILTER_BINS0>(hist_cnt, hist_mass, FilterState{0ull, 0ull, 0u, 0u}, FILTER_SHIFT0,
+                                                        lim.k, lim.P, dsc);
+    if (threadIdx.x == 0) states[r] = st;
+  }
+}
 
-  auto add = [&](float logit, bool in) {     // one token of the prefix; every lane of the warp calls
-    const float p = row_probability(logit, temp, mx, sum);
-    const unsigned key = __float_as_uint(p);
-    if constexpr (PASS > 0) in = in && (key >> (SHIFT + pass_bits(PASS))) == (prefix >> (SHIFT + pass_bits(PASS)));
-    const unsigned bin = (key >> SHIFT) & (BINS - 1);
-    const unsigned long long m = (unsigned long long)(p * MASS_ONE);
-    // 32 tokens of one bin (a flat row, a tail that underflows): one addition for the warp
-    const unsigned first = __shfl_sync(0xffffffffu, bin, 0);
-    if (__all_sync(0xffffffffu, in && bin == first)) {
-      const unsigned low = __reduce_add_sync(0xffffffffu, (unsigned)(m & 0xfffffull));
-      const unsigned high = __reduce_add_sync(0xffffffffu, (unsigned)(m >> 20));
-      if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&s_cnt[bin], 32u);
-        atomicAdd(&s_low[bin], low);
-        atomicAdd(&s_high[bin], high);
-      }
-    } else if (in) {
-      atomicAdd(&s_cnt[bin], 1u);
-      atomicAdd(&s_low[bin], (unsigned)(m & 0xfffffull));
-      atomicAdd(&s_high[bin], (unsigned)(m >> 20));
-    }
-  };
-  if constexpr (PASS == 0) {
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+filter_second_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
+                     const long long* __restrict__ top_ks, const float* __restrict__ top_ps, unsigned* hist_cnt,
+                     unsigned long long* hist_mass, FilterState* __restrict__ states, const float2* __restrict__ norms,
+                     unsigned* marks, float* __restrict__ list, int R, int V, int chunks) {
+  pdl_prologue(logits, temperatures, top_ks, top_ps, norms);
+  __shared__ unsigned s_cnt[FILTER_BINS1], s_low[FILTER_BINS1], s_high[FILTER_BINS1];
+  __shared__ DescendScratch dsc;
+  __shared__ float s_list[ARGMAX_CHUNK];
+  __shared__ int s_listed;
+  __shared__ bool s_last;
+  const int r = blockIdx.y, c = blockIdx.x, lane = threadIdx.x & 31;
+  const float temp = temperatures[r];
+  const long long top_k = top_ks[r];
+  const float top_p = top_ps[r];
+  if (!row_is_filtered(temp, top_k, top_p)) return;
+  const int lo = c * ARGMAX_CHUNK, hi = min(V, lo + ARGMAX_CHUNK);
+  float x[PER_THREAD];
+  load_chunk(logits + (size_t)r * V, lo, hi, x);
+  FilterState st{__ldcg(&states[r].cnt_above), __ldcg(&states[r].mass_above), __ldcg(&states[r].prefix), 0u};
+  const float2 norm = norms[r];
+  for (int b = threadIdx.x; b < FILTER_BINS1; b += SAMPLE_THREADS) s_cnt[b] = s_low[b] = s_high[b] = 0u;
+  if (threadIdx.x == 0) s_listed = 0;
+  // the tokens that may have the prefix, side by side
+  const Estimate est(temp, norm.x, norm.y);
+  const float from = lower_bound(st.prefix, est), to = upper_bound(st.prefix | ((1u << FILTER_SHIFT0) - 1u), est);
+  unsigned in[PER_THREAD];                   // the warp's, a bit a lane
+  int found = 0;
 #pragma unroll
-    for (int j = 0; j < PER_THREAD; ++j) add(x[j], lo + (int)threadIdx.x + j * SAMPLE_THREADS < hi);
-  } else {
-    // the tokens that may have the prefix, side by side
-    const Estimate est(temp, mx, sum);
-    const unsigned rest = (1u << (SHIFT + pass_bits(PASS))) - 1u;
-    const float from = lower_bound(prefix, est), to = upper_bound(prefix | rest, est);
-    const int lane = threadIdx.x & 31;
-    unsigned in[PER_THREAD];                   // the warp's, a bit a lane
-    int found = 0;
+  for (int j = 0; j < PER_THREAD; ++j) {
+    const float y = est.log2p(x[j]);
+    in[j] = __ballot_sync(0xffffffffu, lo + (int)threadIdx.x + j * SAMPLE_THREADS < hi && !(est.ok && (y < from || y > to)));
+    found += __popc(in[j]);
+  }
+  __syncthreads();
+  int at = 0;
+  if (lane == 0 && found > 0) at = atomicAdd(&s_listed, found);
+  at = __shfl_sync(0xffffffffu, at, 0);
 #pragma unroll
-    for (int j = 0; j < PER_THREAD; ++j) {
-      const float y = est.log2p(x[j]);
-      in[j] = __ballot_sync(0xffffffffu, lo + (int)threadIdx.x + j * SAMPLE_THREADS < hi &&
-                                             !(est.ok && (y < from || y > to)));
-      found += __popc(in[j]);
-    }
-    int at = 0;
-    if (lane == 0 && found > 0) at = atomicAdd(&s_listed, found);
-    at = __shfl_sync(0xffffffffu, at, 0);
-#pragma unroll
-    for (int j = 0; j < PER_THREAD; ++j) {
-      if ((in[j] >> lane) & 1u) s_list[at + __popc(in[j] & ((1u << lane) - 1u))] = x[j];
-      at += __popc(in[j]);
+  for (int j = 0; j < PER_THREAD; ++j) {
+    if ((in[j] >> lane) & 1u) s_list[at + __popc(in[j] & ((1u << lane) - 1u))] = x[j];
+    at += __popc(in[j]);
+  }
+  __syncthreads();
+  hist_cnt += (size_t)r * FILTER_BINS + FILTER_BINS0;
+  hist_mass += (size_t)r * FILTER_BINS + FILTER_BINS0;
+  const int n = s_listed;
+  if (n > 0) {
+    unsigned* listed = &marks[(size_t)r * ROW_MARKS + MARK_LISTED];
+    for (int i = threadIdx.x; i - lane < n; i += SAMPLE_THREADS) {
+      const float p = row_probability(i < n ? s_list[i] : 0.f, temp, norm.x, norm.y);
+      const unsigned key = __float_as_uint(p);
+      const bool mine = i < n && (key >> FILTER_SHIFT0) == (st.prefix >> FILTER_SHIFT0);
+      count_token(p, (key >> FILTER_SHIFT1) & (FILTER_BINS1 - 1), mine, s_cnt, s_low, s_high);
+      const unsigned ballot = __ballot_sync(0xffffffffu, mine);
+      unsigned where = 0u;
+      if (lane == 0 && ballot != 0u) where = atomicAdd(listed, (unsigned)__popc(ballot));
+      where = __shfl_sync(0xffffffffu, where, 0) + __popc(ballot & ((1u << lane) - 1u));
+      if (mine && where < (unsigned)FILTER_LIST) list[(size_t)r * FILTER_LIST + where] = p;
     }
     __syncthreads();
-    const int n = s_listed;
-    for (int i = threadIdx.x; i - lane < n; i += SAMPLE_THREADS) add(i < n ? s_list[i] : 0.f, i < n);
+    add_histogram<FILTER_BINS1>(s_cnt, s_low, s_high, hist_cnt, hist_mass);
+  }
+  if (last_of_row(&marks[(size_t)r * ROW_MARKS + MARK_SECOND], chunks, &s_last)) {
+    const FilterLimits lim(top_k, top_p, V);
+    st = filter_descend<FILTER_BINS1>(hist_cnt, hist_mass, st, FILTER_SHIFT1, lim.k, lim.P, dsc);
+    if (threadIdx.x == 0) states[R + r] = st;
+  }
+}
+
+// One block a row: the last 10 bits, from the listed probabilities that have the first 21.
+__global__ void __launch_bounds__(SAMPLE_THREADS)
+filter_third_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
+                    const long long* __restrict__ top_ks, const float* __restrict__ top_ps,
+                    const FilterState* __restrict__ states, const float2* __restrict__ norms,
+                    const unsigned* __restrict__ marks, const float* __restrict__ list, unsigned* __restrict__ thresh,
+                    int R, int V) {
+  pdl_prologue(logits, temperatures, top_ks, top_ps, states, norms, marks, list);
+  __shared__ unsigned s_cnt[FILTER_BINS2];
+  __shared__ unsigned long long s_mass[FILTER_BINS2];
+  __shared__ DescendScratch dsc;
+  const int r = blockIdx.x, lane = threadIdx.x & 31;
+  const float temp = temperatures[r];
+  const long long top_k = top_ks[r];
+  const float top_p = top_ps[r];
+  if (!row_is_filtered(temp, top_k, top_p)) {
+    if (threadIdx.x == 0) thresh[r] = 0u;
+    return;
+  }
+  const FilterState st = states[R + r];
+  const unsigned listed = marks[(size_t)r * ROW_MARKS + MARK_LISTED];
+  const float2 norm = norms[r];
+  for (int b = threadIdx.x; b < FILTER_BINS2; b += SAMPLE_THREADS) {
+    s_cnt[b] = 0u;
+    s_mass[b] = 0ull;
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < BINS; b += SAMPLE_THREADS)
-    if (s_cnt[b] != 0u) {
-      const size_t at = (size_t)r * FILTER_BINS + pass_first_bin(PASS) + b;
-      atomicAdd(&hist_cnt[at], s_cnt[b]);
-      atomicAdd(&hist_mass[at], ((unsigned long long)s_high[b] << 20) + s_low[b]);
+  const bool whole = listed <= (unsigned)FILTER_LIST;          // the list has them all
+  const int n = whole ? (int)listed : V;
+  const float* from = whole ? list + (size_t)r * FILTER_LIST : logits + (size_t)r * V;
+#pragma unroll 4
+  for (int i = threadIdx.x; i - lane < n; i += SAMPLE_THREADS) {
+    float p = i < n ? from[i] : 0.f;
+    if (!whole) p = row_probability(p, temp, norm.x, norm.y);
+    const unsigned key = __float_as_uint(p);
+    const bool mine = i < n && (key >> FILTER_SHIFT1) == (st.prefix >> FILTER_SHIFT1);
+    const unsigned bin = key & (FILTER_BINS2 - 1);
+    const unsigned long long m = (unsigned long long)(p * MASS_ONE);
+    const unsigned first = __shfl_sync(0xffffffffu, bin, 0);
+    if (__all_sync(0xffffffffu, mine && bin == first)) {
+      const unsigned long long sum = ((unsigned long long)__reduce_add_sync(0xffffffffu, (unsigned)(m >> 20)) << 20) +
+                                     __reduce_add_sync(0xffffffffu, (unsigned)(m & 0xfffffull));
+      if (lane == 0) {
+        atomicAdd(&s_cnt[bin], 32u);
+        atomicAdd(&s_mass[bin], sum);
+      }
+    } else if (mine) {
+      atomicAdd(&s_cnt[bin], 1u);
+      atomicAdd(&s_mass[bin], m);
     }
+  }
+  __syncthreads();
+  const FilterLimits lim(top_k, top_p, V);
+  const FilterState last = filter_descend<FILTER_BINS2, true>(s_cnt, s_mass, st, 0, lim.k, lim.P, dsc);
+  if (threadIdx.x == 0) thresh[r] = last.prefix;
 }
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 gumbel_pick_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
                    const long long* __restrict__ seeds, const long long* __restrict__ sample_pos,
-                   const unsigned char* __restrict__ keep, const long long* __restrict__ top_ks,
-                   const float* __restrict__ top_ps, const unsigned* __restrict__ hist_cnt,
-                   const unsigned long long* __restrict__ hist_mass, const FilterState* __restrict__ states,
-                   const float2* __restrict__ norms, unsigned* __restrict__ thresh, const float* __restrict__ cmax, const float* __restrict__ csum,
-                   float* __restrict__ pv, int* __restrict__ pi, int R, int V, int chunks) {
-  pdl_prologue(logits, temperatures, seeds, sample_pos, keep, top_ks, top_ps, hist_cnt, hist_mass, states, norms,
-               cmax, csum);
+                   const unsigned char* __restrict__ keep, const unsigned* __restrict__ thresh,
+                   const float2* __restrict__ norms, const float* __restrict__ cmax, const float* __restrict__ csum,
+                   float* __restrict__ pv, int* __restrict__ pi, int V, int chunks) {
+  pdl_prologue(logits, temperatures, seeds, sample_pos, keep, thresh, norms, cmax, csum);
   __shared__ Best bscratch[32];
   __shared__ NormaliserScratch nsc;
-  __shared__ DescendScratch dsc;
   const int r = blockIdx.y, c = blockIdx.x;
   const float* row = logits + (size_t)r * V;
   const int lo = c * ARGMAX_CHUNK, hi = min(V, lo + ARGMAX_CHUNK);
   float x[PER_THREAD];
   load_chunk(row, lo, hi, x);
   const float temp = temperatures[r];
-  // the threshold of top-k / top-p: all passes' histograms are complete
-  unsigned t = 0u;
-  if (thresh != nullptr) {
-    const long long top_k = top_ks[r];
-    const float top_p = top_ps[r];
-    if (row_is_filtered(temp, top_k, top_p)) {
-      const unsigned long long k = top_k > 0 ? (unsigned long long)top_k : (unsigned long long)V + 1;
-      const unsigned long long P = top_p >= 1.0f ? ~0ull : (unsigned long long)(top_p * MASS_ONE);
-      t = state_after(FILTER_PASSES - 1, hist_cnt, hist_mass, states, R, r, k, P, dsc).prefix;
-    }
-    if (threadIdx.x == 0 && c == 0) thresh[r] = t;
-  }
+  const unsigned t = thresh != nullptr ? thresh[r] : 0u;       // of top-k / top-p
   Best b{-INFINITY, INT_MAX_};
   if (temp <= 0.f) {
 #pragma unroll
@@ -638,9 +723,10 @@ int dib_gumbel_sample(const float* logits, const float* temperatures, const long
 // top_ks / top_ps (both or neither): per-row top-k (<= 0: off) and top-p (>= 1: off),
 // applied by a threshold found without a sort.  thresh: unsigned [R], receives the bits of
 // each row's smallest kept probability (0 = all kept); hist: scratch of dib_filter_scratch(R)
-// bytes, 8-byte aligned (masses, the rows' states, the rows' normalisers, counts).
+// bytes, 8-byte aligned.
 long long dib_filter_scratch(int R) {
-  return (long long)R * (FILTER_BINS * 12ll + FILTER_PASSES * (long long)sizeof(FilterState) + (long long)sizeof(float2));
+  return (long long)R * (FILTER_BINS * 12ll + 2 * (long long)sizeof(FilterState) + (long long)sizeof(float2) +
+                         4ll * ROW_MARKS + 4ll * FILTER_LIST);
 }
 
 int dib_gumbel_sample_chunked(const float* logits, const float* temperatures, const long long* seeds,
@@ -656,30 +742,31 @@ int dib_gumbel_sample_chunked(const float* logits, const float* temperatures, co
   float* pv = scratch_f + 2 * (size_t)R * chunks;
   const bool filtered = top_ks != nullptr && top_ps != nullptr && thresh != nullptr && hist != nullptr;
   if (filtered && reinterpret_cast<uintptr_t>(hist) % 8 != 0) return DIB_BAD_ALIGN;
+  // masses, the rows' states and normalisers, then what needs 4 bytes only
   unsigned long long* hist_mass = filtered ? reinterpret_cast<unsigned long long*>(hist) : nullptr;
   FilterState* states = filtered ? reinterpret_cast<FilterState*>(hist_mass + (size_t)R * FILTER_BINS) : nullptr;
-  float2* norms = filtered ? reinterpret_cast<float2*>(states + (size_t)R * FILTER_PASSES) : nullptr;
+  float2* norms = filtered ? reinterpret_cast<float2*>(states + (size_t)2 * R) : nullptr;
   unsigned* hist_cnt = filtered ? reinterpret_cast<unsigned*>(norms + R) : nullptr;
+  unsigned* marks = filtered ? hist_cnt + (size_t)R * FILTER_BINS : nullptr;
+  float* list = filtered ? reinterpret_cast<float*>(marks + (size_t)R * ROW_MARKS) : nullptr;
   const dim3 grid(chunks, R), block(SAMPLE_THREADS);
-  dib_launch(gumbel_stats_kernel, grid, block, 0, st, logits, temperatures, cmax, csum, hist_cnt, hist_mass, V,
+  dib_launch(gumbel_stats_kernel, grid, block, 0, st, logits, temperatures, cmax, csum, hist_cnt, hist_mass, marks, V,
              chunks);
   DIB_CHECK_LAUNCH();
   if (filtered) {
-    auto pass = [&](auto* kernel) {
-      dib_launch(kernel, grid, block, 0, st, logits, temperatures, top_ks, top_ps, (const float*)cmax,
-                 (const float*)csum, hist_cnt, hist_mass, states, norms, R, V, chunks);
-    };
-    pass(&filter_histogram_kernel<0>);
+    dib_launch(filter_first_kernel, grid, block, 0, st, logits, temperatures, top_ks, top_ps, (const float*)cmax,
+               (const float*)csum, hist_cnt, hist_mass, states, norms, marks, V, chunks);
     DIB_CHECK_LAUNCH();
-    pass(&filter_histogram_kernel<1>);
+    dib_launch(filter_second_kernel, grid, block, 0, st, logits, temperatures, top_ks, top_ps, hist_cnt, hist_mass,
+               states, (const float2*)norms, marks, list, R, V, chunks);
     DIB_CHECK_LAUNCH();
-    pass(&filter_histogram_kernel<2>);
+    dib_launch(filter_third_kernel, dim3(R), block, 0, st, logits, temperatures, top_ks, top_ps,
+               (const FilterState*)states, (const float2*)norms, (const unsigned*)marks, (const float*)list, thresh, R, V);
     DIB_CHECK_LAUNCH();
   }
-  dib_launch(gumbel_pick_kernel, grid, block, 0, st, logits, temperatures, seeds, sample_pos, keep, top_ks, top_ps,
-             (const unsigned*)hist_cnt, (const unsigned long long*)hist_mass, (const FilterState*)states, (const float2*)norms,
-             filtered ? thresh : (unsigned*)nullptr, (const float*)cmax, (const float*)csum, pv, scratch_i, R, V,
-             chunks);
+  dib_launch(gumbel_pick_kernel, grid, block, 0, st, logits, temperatures, seeds, sample_pos, keep,
+             filtered ? (const unsigned*)thresh : (const unsigned*)nullptr, (const float2*)norms, (const float*)cmax,
+             (const float*)csum, pv, scratch_i, V, chunks);
   DIB_CHECK_LAUNCH();
   dib_launch(argmax_final_kernel, dim3(R), dim3(64), 0, st, (const float*)pv, (const int*)scratch_i, out,
              chunks);
