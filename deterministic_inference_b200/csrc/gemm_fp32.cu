@@ -1,8 +1,8 @@
 // True float32 matrix product on the CUDA cores: C[M,N] = A[M,K] * W[N,K]^T.
 //
 // This is the matrix product of the 32-bit path: plain FMA, no tensor cores and
-// no reduced-precision mode.  An output element is eight partial sums: k belongs to
-// partial (k / 4) % 8, each partial adds its k in index order, and the partials are
+// no reduced-precision mode.  An output element is eight partial sums (from K = 512 on; one
+// chain over k in index order below, see gemm_fp32_short_kernel): k belongs to partial (k / 4) % 8, each partial adds its k in index order, and the partials are
 // added one after the other.  That order is a function of K alone, whatever the tile,
 // so a row's result does not depend on M: the same token gives the same bits in any
 // batch.  (Distance from 64-bit sums at K = 1024 .. 3072: 2.1e-7 .. 3.6e-7 of the norm.
@@ -130,6 +130,72 @@ gemm_fp32_kernel(const float* __restrict__ A, const float* __restrict__ W, float
   }
 }
 
+// Short sums (K below SHORT_K): one chain over all k in index order, as there is little to divide; the
+// eight warps of a block take 16 x 32 outputs each of a tile of 64 x 64, from stages copied the same way.
+// (204 rows: 768 x 192 9.7 us, 1,024 x 500 23 us; divided 5.9 and 12 us, but then the logits of a small
+// model's ill-conditioned rows move by as much as they are off; 64 x 64 x 16 in order, as before: 21, 54 us.)
+constexpr int SHORT_K = 512, SH_B = 64, SH_BK = 32, SH_STAGES = 3, SH_LD = SH_BK + 4;
+template <bool VEC>
+__global__ void __launch_bounds__(THREADS)
+gemm_fp32_short_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out,
+                       int M, int N, int K) {
+  extern __shared__ __align__(16) float smem[];
+  pdl_prologue(A, W);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r0 = (warp >> 1) * 16 + (lane >> 3), c0 = (warp & 1) * 32 + (lane & 7);      // + 4 i, + 8 j
+  const int row_tiles = (M + SH_B - 1) / SH_B;
+  const int m0 = (int)(blockIdx.x % row_tiles) * SH_B, n0 = (int)(blockIdx.x / row_tiles) * SH_B;
+  const int steps = (K + SH_BK - 1) / SH_BK;
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  auto fetch = [&](int s) {
+    if (s < steps) {
+      float* st = smem + (s % SH_STAGES) * 2 * SH_B * SH_LD;
+      copy_rows<SH_B, SH_BK, SH_LD, VEC>(st, A, m0, M, s * SH_BK, K);
+      copy_rows<SH_B, SH_BK, SH_LD, VEC>(st + SH_B * SH_LD, W, n0, N, s * SH_BK, K);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < SH_STAGES - 1; ++s) fetch(s);
+  for (int s = 0; s < steps; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(SH_STAGES - 2) : "memory");
+    __syncthreads();                 // stage s is there for all; stage s - 1 has been read by all
+    fetch(s + SH_STAGES - 1);
+    const float* sa = smem + (s % SH_STAGES) * 2 * SH_B * SH_LD + r0 * SH_LD;
+    const float* sw = smem + (s % SH_STAGES) * 2 * SH_B * SH_LD + (SH_B + c0) * SH_LD;
+#pragma unroll
+    for (int k = 0; k < SH_BK; k += 4) {
+      float4 a[4], b[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[i] = *reinterpret_cast<const float4*>(sa + 4 * i * SH_LD + k);
+        b[i] = *reinterpret_cast<const float4*>(sw + 8 * i * SH_LD + k);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+          acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+          acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+          acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+        }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int r = m0 + r0 + 4 * i, c = n0 + c0 + 8 * j;
+      if (r < M && c < N) out[(size_t)r * N + c] = acc[i][j];
+    }
+}
+
 template <typename C, bool VEC>
 int launch_vec(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
   static DeviceOnce once;
@@ -146,11 +212,28 @@ int launch_vec(const float* A, const float* W, float* out, int M, int N, int K, 
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
+template <bool VEC>
+int launch_short(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
+  constexpr int smem = 4 * SH_STAGES * 2 * SH_B * SH_LD;           // 55 KB
+  static DeviceOnce once;
+  if (!once.done()) {
+    if (cudaFuncSetAttribute(gemm_fp32_short_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return DIB_LAUNCH_FAILED;
+    }
+    once.mark();
+  }
+  const long long blocks = (long long)ceil_div_host(M, SH_B) * ceil_div_host(N, SH_B);
+  if (blocks > 0x7fffffffll) return DIB_BAD_SIZE;
+  dib_launch(gemm_fp32_short_kernel<VEC>, dim3((unsigned)blocks), dim3(THREADS), smem, st, A, W, out, M, N, K);
+  DIB_CHECK_LAUNCH();
+  return DIB_OK;
+}
+// 16-byte copies want rows that start on 16 bytes
+bool takes_vectors(const float* A, const float* W, int K) { return K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0; }
 template <typename C>
 int launch(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
-  // 16-byte copies want rows that start on 16 bytes
-  const bool vec = K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-  return vec ? launch_vec<C, true>(A, W, out, M, N, K, st) : launch_vec<C, false>(A, W, out, M, N, K, st);
+  return takes_vectors(A, W, K) ? launch_vec<C, true>(A, W, out, M, N, K, st) : launch_vec<C, false>(A, W, out, M, N, K, st);
 }
 
 // The tiles, by rows and columns.  The choice: the tile whose fullest SM is done first.  With
@@ -178,6 +261,8 @@ extern "C" int dib_gemm_fp32(const float* A, const float* W, float* out, int M, 
   if (M == 0 || N == 0) return DIB_OK;
   if (K <= 0) return DIB_BAD_SIZE;
   if (ceil_div_host(M, 64) > 65535) return DIB_BAD_SIZE;
+  if (K < SHORT_K)
+    return takes_vectors(A, W, K) ? launch_short<true>(A, W, out, M, N, K, st) : launch_short<false>(A, W, out, M, N, K, st);
   const float cost[5] = {estimate<T8>(M, N, 7.f, 4.3f), estimate<T8w>(M, N, 10.f, 7.2f), estimate<T16>(M, N, 8.f, 6.3f),
                          estimate<T32>(M, N, 13.f, 11.f), estimate<T64>(M, N, 22.f, 18.7f)};
   int best = 0;

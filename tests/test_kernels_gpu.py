@@ -176,10 +176,12 @@ def test_linear_fp32_is_true_fp32(m, n, k):
     torch.testing.assert_close(got.double(), want, atol=2e-5 * (k ** 0.5), rtol=1e-5)
 
 
-@pytest.mark.parametrize("n,k", [(31, 33), (33, 64), (65, 130), (4096, 260), (1024, 1028)])
+@pytest.mark.parametrize("n,k", [(31, 33), (33, 64), (65, 130), (4096, 260), (100, 511), (100, 512),
+                                 (4096, 513), (65, 578), (1024, 1028)])
 def test_linear_fp32_tiles_give_the_same_bits(n, k):
     """Every tile the row count and the width may choose adds in one order: the row's bits are those of the
-    row alone, at the edges of the tiles; against 64 bits the error is that of eight chains of k / 8."""
+    row alone, at the edges of the tiles; against 64 bits the error is that of eight chains of k / 8, or of one
+    below 512."""
     torch.manual_seed(16)
     x = torch.randn(400, k, device="cuda")
     w = torch.randn(n, k, device="cuda")
@@ -190,7 +192,7 @@ def test_linear_fp32_tiles_give_the_same_bits(n, k):
             if r < m:
                 assert torch.equal(got[r], one[0]), (m, r)
         # a chain of c terms: at most c * 2^-24 of the sum of the terms' sizes, and 8 partials more
-        bound = (k / 8 + 16) * 2.0 ** -24 * (x[:m].abs().double() @ w.abs().double().T)
+        bound = ((k / 8 if k >= 512 else k) + 16) * 2.0 ** -24 * (x[:m].abs().double() @ w.abs().double().T)
         assert ((got.double() - x[:m].double() @ w.double().T).abs() <= bound).all(), m
 
 
