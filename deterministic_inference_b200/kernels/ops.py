@@ -1549,10 +1549,14 @@ def gated_linear_recurrence(proj, bias: torch.Tensor, conv_weight: torch.Tensor,
 # A row's bits do not depend on the tile it is computed in.
 EXPERT_TILE_ROWS = 16
 EXPERT_TILE_ROWS_LARGE = 64
-# bfloat16 steps that bring an expert EXPERT_TILE_ROWS_TC rows on average: the sorted rows become a
-# matrix of their own and both products run on the tcgen05 kernel of ``gemm_bf16_large`` (a tile of 128
-# rows times its expert's matrix).  DIB200_EXPERTS_TC=0 (read once) leaves that form out.
+# bfloat16 steps that bring an expert EXPERTS_TC_FROM rows on average: the sorted rows become a
+# matrix of their own and both products run on the tcgen05 kernel of ``gemm_bf16_large`` (a tile of
+# EXPERT_TILE_ROWS_TC rows times its expert's matrix).  Whole feed-forward on B200, mma.sync / tcgen05 in us
+# at 8, 16, 32, 64, 127 rows an expert: 16 experts of 1,024 x 1,536 63 / 72, 79 / 72, 117 / 72, 182 / 74,
+# 243 / 84; 64 of 1,024 x 512 84 / 82, 108 / 84, 173 / 86, 188 / 92, 275 / 113; 8 of 2,048 x 2,048 70 / 78,
+# 83 / 78, 127 / 80, 229 / 80, 328 / 92.  DIB200_EXPERTS_TC=0 (read once) leaves that form out.
 EXPERT_TILE_ROWS_TC = 128
+EXPERTS_TC_FROM = 16
 EXPERTS_TC = __import__("os").environ.get("DIB200_EXPERTS_TC", "1") != "0"
 
 
@@ -1611,7 +1615,7 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
     then its up rows), ``w_down`` [E, W, F], both of x's type.  The (token, expert) pairs are sorted by
     expert on the device into tiles of EXPERT_TILE_ROWS (or EXPERT_TILE_ROWS_LARGE) rows of one expert; a
     row's sums run over k in an order that its tile does not change, so a token's result does not depend
-    on what else is in the step."""
+    on what else is in the step (but for the step's form: see EXPERTS_TC_FROM)."""
     _need(x, "x", None, 2)
     table, weight = None, 0.0
     if isinstance(ids, TableChoice):
@@ -1642,7 +1646,7 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
     lib = _lib("routed_experts")
     dev = x.device
     pairs = t * top
-    on_tc = EXPERTS_TC and x.dtype == torch.bfloat16 and pairs >= EXPERT_TILE_ROWS_TC * n_exp \
+    on_tc = EXPERTS_TC and x.dtype == torch.bfloat16 and pairs >= EXPERTS_TC_FROM * n_exp \
         and f % (128 if gated else 256) == 0 and w % 256 == 0 and x.is_contiguous()
     tile = EXPERT_TILE_ROWS_TC if on_tc \
         else EXPERT_TILE_ROWS_LARGE if pairs >= EXPERT_TILE_ROWS_LARGE * n_exp else EXPERT_TILE_ROWS

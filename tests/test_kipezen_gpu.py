@@ -125,10 +125,11 @@ def test_the_experts_products_alone(dtype, experts, top, width, ff, rows):
 
 @pytest.mark.parametrize("width, ff, gated", [(256, 512, True), (264, 24, True), (1032, 40, True), (8, 8, True),
                                               (520, 260 * 4, False), (24, 56, False)])
-def test_the_experts_streamed_products(width, ff, gated):
+def test_the_experts_streamed_products(width, ff, gated, monkeypatch):
     """Tiles of 16 rows: runs of k and blocks of columns that are not full; the rows' bits are those of the
     64-row tiles (a step with 64 rows an expert on average)."""
     from deterministic_inference_b200.kernels import ops
+    monkeypatch.setattr(ops, "EXPERTS_TC", False)
     experts, top = 3, 2
     g = torch.Generator(device="cuda").manual_seed(width)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
