@@ -677,7 +677,7 @@ int dib_sigmoid_gate_(void* x, const void* gate, int kind, int splits, long long
 
 // The tensor-core form (bfloat16; Dk and Dv multiples of 16, Dv at most 256): tiles [num_tiles][3] =
 // (sequence, first token among the sequence's new tokens, tokens) of at most rows / (Hq / Hkv) tokens
-// each; rows 64 or 128.
+// each; rows 64 or 128, or 16: tiles of ONE token (decoded), whose keys the CTA's four warps share.
 // partial_o / partial_ml given (tiles of ONE token only): a token's key tiles are cut into chunks of
 // chunk_tiles, a CTA each, merged by a second kernel over the step's first num_tokens tokens.
 int dib_masked_attention_mma(const void* q, void* out, const void* cache, const int* block_table, int max_blocks,
@@ -689,7 +689,7 @@ int dib_masked_attention_mma(const void* q, void* out, const void* cache, const 
                              int num_tokens, float softcap, cudaStream_t st) {
   if (num_tiles == 0) return DIB_OK;
   if (Dk < 16 || Dk % 16 || Dv < 16 || Dv % 16 || Dv > 256 || Hkv < 1 || Hq % Hkv != 0 || Hq / Hkv > rows ||
-      (rows != 64 && rows != 128) || page_size < 1 || mask_kind < 0 || mask_kind > 2 ||
+      (rows != 16 && rows != 64 && rows != 128) || page_size < 1 || mask_kind < 0 || mask_kind > 2 ||
       (mask_kind > 0 && mask_size < 1) || keep < 0 || (keep > 0 && mask_kind != 1) ||
       (Dv_stored != 0 && Dv_stored != Dv) || (Dv_stored == 0 && Dv > Dk) ||
       num_tiles > 1 << 30 || Hkv > 65535 || max_chunks > 65535 || (partial_o != nullptr && chunk_tiles < 1))
@@ -700,6 +700,12 @@ int dib_masked_attention_mma(const void* q, void* out, const void* cache, const 
                                   sink, Hq, Hkv, Dk, Dv, Dv_stored, page_size, scale, mask_kind, mask_size, keep, g, \
                                   gate_row, gate_col, gate_heads, partial_o, partial_ml, chunk_tiles, max_chunks, num_tokens, softcap, st)
   const int nv = (Dv + 63) / 64;
+  if (rows == 16) {
+    if (nv == 1) DIB_MAM(4, 16);
+    if (nv == 2) DIB_MAM(8, 16);
+    if (nv == 3) DIB_MAM(12, 16);
+    DIB_MAM(16, 16);
+  }
   if (rows == 64) {
     if (nv == 1) DIB_MAM(4, 64);
     if (nv == 2) DIB_MAM(8, 64);

@@ -323,6 +323,236 @@ masked_attention_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, const __
   }
 }
 
+// The same for decoded tokens whose head groups have at most 16 heads: one token's rows fill 16 of an
+// mma.sync tile, which ONE of the warps above would work on alone.  Here the four warps share the rows
+// and take 16 of a tile's 64 keys each, every warp with a softmax of its own; at the end the warps'
+// sums meet in shared memory and are put together in warp order, against the largest of their maxima.
+// Chunks of key tiles and their merge as above.  (8 tokens, 16 heads over one latent row of 256, some 200
+// keys: 15 us; one warp of the four: 19 us.)
+constexpr int DEC_ROWS = 16, DEC_WARPS = 4;
+template <int NV16>
+__global__ void __launch_bounds__(DEC_WARPS * 32)
+masked_attention_decode_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, const __nv_bfloat16* cache,
+                                   const int* block_table, int bt_width, const int* positions, const int* seq_lens,
+                                   const int* cu_q_lens, const int* tiles, const float* sink, int Hq, int Hkv, int D,
+                                   int VD, int VD_stored, int page_size, float scale, int mask_kind, int mask_size,
+                                   int keep, Source gate, long long gate_row, long long gate_col, int gate_heads,
+                                   float* partial_o, float* partial_ml, int chunk_tiles, int max_chunks, float softcap) {
+  extern __shared__ __align__(16) unsigned char mam_smem[];
+  const int R = Hq / Hkv;
+  const bool in_keys = VD_stored == 0;
+  const int qs = D + PAD, vs = in_keys ? qs : VD + PAD;   // row strides in elements
+  __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(mam_smem);            // [DEC_ROWS][qs]
+  __nv_bfloat16* Ks = Qs + DEC_ROWS * qs;                                     // [2][KT][qs]
+  __nv_bfloat16* Vs = in_keys ? Ks : Ks + 2 * KT * qs;                        // [2][KT][vs]
+  __shared__ long long k_off[2][KT], v_off[2][KT];
+  __shared__ float sm[DEC_WARPS][DEC_ROWS], sl[DEC_WARPS][DEC_ROWS];
+  pdl_prologue(q, cache, gate.p);
+  const int g = blockIdx.y, b = tiles[3 * blockIdx.x], start = tiles[3 * blockIdx.x + 1];
+  const int q_begin = cu_q_lens[b], q_len = cu_q_lens[b + 1] - q_begin;
+  if (start >= q_len) return;               // (the whole CTA: the sequence brings no such token)
+  const int t = q_begin + start;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gid = lane >> 2, tig = lane & 3;
+  const int kv_len = seq_lens[b], pos = positions[t];
+  const int* bt = block_table + (long long)b * bt_width;
+  const long long page_elems = (long long)Hkv * page_size * (D + VD_stored);
+
+  const int lo = first_seen(pos, mask_kind, mask_size), t_first = lo / KT;
+  const int n_kept = kept_tiles(keep, t_first);
+  const int n_tiles = n_kept + pos / KT - t_first + 1;
+  auto tile_at = [&](int it) { return it < n_kept ? it : t_first + it - n_kept; };   // walk step -> key tile
+  const bool chunked = partial_o != nullptr;
+  const int chunk = chunked ? blockIdx.z : 0;
+  const int it_begin = chunked ? chunk * chunk_tiles : 0;
+  const int it_end = (chunked && it_begin + chunk_tiles < n_tiles) ? it_begin + chunk_tiles : n_tiles;
+  if (it_begin >= n_tiles) return;          // (the whole CTA: no such chunk at this position)
+
+  const int dchunks = D / 8, vchunks = VD / 8;
+  for (int idx = threadIdx.x; idx < DEC_ROWS * dchunks; idx += blockDim.x) {
+    const int r = idx / dchunks, ch = idx - r * dchunks;
+    copy16(Qs + r * qs + ch * 8, q + ((long long)t * Hq + g * R + (r < R ? r : 0)) * D + ch * 8, r < R);
+  }
+  auto find_rows = [&](int it) {          // by the first KT threads, for tile `it` (if there is one)
+    if (threadIdx.x < KT && it < it_end) {
+      const int j = tile_at(it) * KT + threadIdx.x;
+      long long ko = -1, vo = -1;
+      if (j < kv_len) {
+        // (a key beyond the table's width, a padding sequence's, reads page 0)
+        const long long base = (long long)(j / page_size < bt_width ? bt[j / page_size] : 0) * page_elems;
+        const long long r = (long long)g * page_size + j % page_size;
+        ko = base + r * D;
+        vo = base + (long long)Hkv * page_size * D + r * VD;
+      }
+      k_off[it & 1][threadIdx.x] = ko;
+      v_off[it & 1][threadIdx.x] = vo;
+    }
+  };
+  auto load_tile = [&](int stage) {
+    __nv_bfloat16* kd = Ks + stage * KT * qs;
+    for (int idx = threadIdx.x; idx < KT * dchunks; idx += blockDim.x) {
+      const int jj = idx / dchunks, ch = idx - jj * dchunks;
+      const long long off = k_off[stage][jj];
+      copy16(kd + jj * qs + ch * 8, cache + (off < 0 ? 0 : off) + ch * 8, off >= 0);
+    }
+    if (!in_keys) {
+      __nv_bfloat16* vd = Vs + stage * KT * vs;
+      for (int idx = threadIdx.x; idx < KT * vchunks; idx += blockDim.x) {
+        const int jj = idx / vchunks, ch = idx - jj * vchunks;
+        const long long off = v_off[stage][jj];
+        copy16(vd + jj * vs + ch * 8, cache + (off < 0 ? 0 : off) + ch * 8, off >= 0);
+      }
+    }
+    __pipeline_commit();
+  };
+  const float scale_log2 = scale * MA_LOG2E;
+  const SoftCap cap(softcap, scale);
+  float o[NV16 * 2][4];
+#pragma unroll
+  for (int n = 0; n < NV16 * 2; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+  float m_row[2] = {MA_NEG_BIG, MA_NEG_BIG}, l_row[2] = {0.f, 0.f};
+
+  find_rows(it_begin);
+  find_rows(it_begin + 1);
+  __syncthreads();
+  load_tile(it_begin & 1);
+  for (int it = it_begin; it < it_end; ++it) {
+    const int stage = it & 1;
+    if (it + 1 < it_end) {
+      load_tile(stage ^ 1);
+      find_rows(it + 2);        // into this tile's entries: its copies were issued a round ago
+      __pipeline_wait_prior(1);
+    } else {
+      __pipeline_wait_prior(0);
+    }
+    __syncthreads();
+    const int k0 = tile_at(it) * KT + warp * 16;                 // this warp's keys
+    if (k0 <= pos && (k0 + 15 >= lo || k0 < keep)) {
+      const __nv_bfloat16* kd = Ks + (stage * KT + warp * 16) * qs;
+      const __nv_bfloat16* vd = Vs + (stage * KT + warp * 16) * vs;
+      float s[2][4], s2[2][4];               // (even and odd steps of 16 dimensions: shorter chains)
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] = s2[n][e] = 0.f;
+      auto score = [&](int kk, float (&to)[2][4]) {
+        unsigned a0, a1, a2, a3, b0, b1, b2, b3;
+        ldsm_x4(a0, a1, a2, a3, Qs + (lane & 15) * qs + kk * 16 + (lane >> 4) * 8);
+        ldsm_x4(b0, b1, b2, b3, kd + ((lane & 7) + ((lane >> 4) << 3)) * qs + kk * 16 + ((lane >> 3) & 1) * 8);
+        mma_bf16(to[0], a0, a1, a2, a3, b0, b1);
+        mma_bf16(to[1], a0, a1, a2, a3, b2, b3);
+      };
+      const int steps = D / 16;
+#pragma unroll 4
+      for (int kk = 0; kk + 1 < steps; kk += 2) {
+        score(kk, s);
+        score(kk + 1, s2);
+      }
+      if (steps & 1) score(steps - 1, s);
+      float mx[2] = {MA_NEG_BIG, MA_NEG_BIG};
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int j = k0 + n * 8 + tig * 2 + (e & 1);
+          const bool sees = j <= pos && (j >= lo || j < keep);
+          const float raw = __fadd_rn(s[n][e], s2[n][e]);
+          s[n][e] = sees ? (softcap > 0.f ? cap(raw) : raw * scale_log2) : MA_NEG_BIG;
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
+        }
+      float alpha[2], ref[2], sum[2] = {0.f, 0.f};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+        const float m_new = fmaxf(m_row[h], mx[h]);
+        ref[h] = m_new <= -1e29f ? 0.f : m_new;       // nothing seen yet: every weight becomes 0
+        alpha[h] = ex2(m_row[h] - ref[h]);
+        m_row[h] = m_new;
+      }
+      unsigned p[2][2];
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float w0 = ex2(s[n][2 * h] - ref[h]), w1 = ex2(s[n][2 * h + 1] - ref[h]);
+          sum[h] += w0 + w1;
+          p[n][h] = pack_bf16(w0, w1);
+        }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 1);
+        sum[h] += __shfl_xor_sync(0xffffffffu, sum[h], 2);
+        l_row[h] = l_row[h] * alpha[h] + sum[h];
+      }
+#pragma unroll
+      for (int np = 0; np < NV16; ++np) {
+        if (np * 16 < VD) {
+          unsigned b0, b1, b2, b3;
+          ldsm_x4_trans(b0, b1, b2, b3, vd + ((lane & 7) + ((lane >> 3) & 1) * 8) * vs + np * 16 + (lane >> 4) * 8);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            float(&c)[4] = o[2 * np + u];
+            c[0] *= alpha[0];
+            c[1] *= alpha[0];
+            c[2] *= alpha[1];
+            c[3] *= alpha[1];
+          }
+          mma_bf16(o[2 * np], p[0][0], p[0][1], p[1][0], p[1][1], b0, b1);
+          mma_bf16(o[2 * np + 1], p[0][0], p[0][1], p[1][0], p[1][1], b2, b3);
+        }
+      }
+    }
+    __syncthreads();       // the stage is written again two tiles on
+  }
+
+  // the warps' sums of the same rows meet in the tiles' buffers (the loop ended with a barrier)
+  float* part = reinterpret_cast<float*>(Ks);          // [DEC_WARPS][DEC_ROWS][VD]
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = gid + 8 * h;
+    if (tig == 0) {
+      sm[warp][r] = m_row[h];
+      sl[warp][r] = l_row[h];
+    }
+#pragma unroll
+    for (int n = 0; n < NV16 * 2; ++n) {
+      const int col = n * 8 + tig * 2;
+      if (col < VD)
+        *reinterpret_cast<float2*>(part + (warp * DEC_ROWS + r) * VD + col) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
+    }
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < R * VD; idx += blockDim.x) {
+    const int r = idx / VD, col = idx - r * VD, head = g * R + r;
+    const long long row = (long long)t * Hq + head;
+    float M = sm[0][r];
+#pragma unroll
+    for (int w = 1; w < DEC_WARPS; ++w) M = fmaxf(M, sm[w][r]);
+    const float sink_l = sink != nullptr && !chunked ? sink[head] * MA_LOG2E : MA_NEG_BIG;
+    M = fmaxf(M, sink_l);
+    const float ref = M <= -1e29f ? 0.f : M;
+    float v = 0.f, l = sink != nullptr && !chunked ? ex2(sink_l - ref) : 0.f;
+#pragma unroll
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      const float a = ex2(sm[w][r] - ref);
+      l = __fmaf_rn(sl[w][r], a, l);
+      v = __fmaf_rn(part[(w * DEC_ROWS + r) * VD + col], a, v);
+    }
+    if (chunked) {
+      partial_o[(row * max_chunks + chunk) * VD + col] = v;
+      if (col == 0) *reinterpret_cast<float2*>(partial_ml + (row * max_chunks + chunk) * 2) = make_float2(M, l);
+      continue;
+    }
+    v *= 1.0f / l;
+    if (gate.p != nullptr) {
+      const long long at = (long long)t * gate_row + gate_col + (gate_heads ? head : (long long)head * VD + col);
+      v = round_to<__nv_bfloat16>(v) * sigmoid_f32(round_to<__nv_bfloat16>(source_load(gate, at)));
+    }
+    out[row * VD + col] = __float2bfloat16_rn(v);
+  }
+}
+
 // out[t, h, :] from the row's chunks, in chunk order: with M the largest of the chunks' maxima (and
 // of the sink), out = sum_c o_c 2^(m_c - M) / (sum_c l_c 2^(m_c - M) + 2^(sink - M)), then the gate.
 // A token at position p has ceil(tiles(p) / chunk_tiles) chunks, tiles(p) as the kernel above counts.
@@ -364,9 +594,11 @@ __global__ void masked_attention_merge_kernel(const float* partial_o, const floa
 constexpr int MAX_DYNAMIC_SMEM = 224 * 1024;
 
 static inline size_t smem_bytes(int D, int VD, int VD_stored, int rows) {
-  size_t n = (size_t)rows * (D + PAD) + 2 * (size_t)KT * (D + PAD);
-  if (VD_stored > 0) n += 2 * (size_t)KT * (VD + PAD);
-  return sizeof(__nv_bfloat16) * n;
+  size_t tiles = 2 * (size_t)KT * (D + PAD);
+  if (VD_stored > 0) tiles += 2 * (size_t)KT * (VD + PAD);
+  // (16 rows: the warps' float32 sums take the tiles' place at the end)
+  if (rows == DEC_ROWS && tiles < 2 * (size_t)DEC_WARPS * DEC_ROWS * VD) tiles = 2 * (size_t)DEC_WARPS * DEC_ROWS * VD;
+  return sizeof(__nv_bfloat16) * ((size_t)rows * (D + PAD) + tiles);
 }
 
 template <int NV16, int ROWS>
@@ -378,14 +610,18 @@ static int launch(const void* q, void* out, const void* cache, const int* block_
   const size_t smem = smem_bytes(D, VD, VD_stored, ROWS);
   if (smem > MAX_DYNAMIC_SMEM) return DIB_BAD_SIZE;
   const bool chunked = partial_o != nullptr && max_chunks > 1;
+  // ROWS 16: decoded tokens, the warps sharing the rows
+  auto* kernel = [] {
+    if constexpr (ROWS == DEC_ROWS) return &masked_attention_decode_mma_kernel<NV16>;
+    else return &masked_attention_mma_kernel<NV16, ROWS>;
+  }();
   static DeviceOnce once;
   if (!once.done()) {
-    if (cudaFuncSetAttribute(masked_attention_mma_kernel<NV16, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             MAX_DYNAMIC_SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_DYNAMIC_SMEM) != cudaSuccess)
       return DIB_LAUNCH_FAILED;
     once.mark();
   }
-  dib_launch(masked_attention_mma_kernel<NV16, ROWS>, dim3(num_tiles, Hkv, chunked ? max_chunks : 1), dim3(ROWS * 2),
+  dib_launch(kernel, dim3(num_tiles, Hkv, chunked ? max_chunks : 1), dim3(ROWS == DEC_ROWS ? DEC_WARPS * 32 : ROWS * 2),
              smem, st, (const __nv_bfloat16*)q, (__nv_bfloat16*)out, (const __nv_bfloat16*)cache, block_table,
              bt_width, positions, seq_lens, cu_q_lens, tiles, sink, Hq, Hkv, D, VD, VD_stored, page_size, scale, mask_kind,
              mask_size, keep, gate, gate_row, gate_col, gate_heads, chunked ? partial_o : (float*)nullptr,

@@ -2019,7 +2019,8 @@ def masked_attention(q: torch.Tensor, kv_cache: torch.Tensor, meta, scale: float
         rows = 128 if (group > 64 or max(meta.q_lens[n_dec:], default=0) * group > 64) else 64
         if smem_of(rows) > 224 * 1024 and group <= 64:
             rows = 64
-        dec_rows = 64 if group <= 64 else 128
+        # (decoded tokens of up to 16 heads a group: a CTA's warps share the token's keys)
+        dec_rows = 16 if group <= 16 else 64 if group <= 64 else 128
         if smem_of(rows) <= 224 * 1024 and smem_of(dec_rows) <= 224 * 1024:
             key = ("masked_attention_tiles", group, rows)
             lists = meta.scratch.get(key)

@@ -437,3 +437,72 @@ def test_greedy_generation_through_the_entry_point(name, dtype, model_dirs):
                 gap = float(logits[best] - logits[t])
                 assert dtype == "bfloat16" and gap < 0.25, f"token {t} instead of {best}, logits {gap:.3g} apart"
             ids.append(t)
+
+
+@pytest.mark.parametrize("hq, hkv, dk, dv, in_keys, mask, size, keep, with_sink, cap", [
+    (16, 1, 256, 192, True, "causal", None, 0, False, None),
+    (1, 1, 48, 16, True, "causal", None, 0, True, None),          # an odd number of steps of 16 dimensions
+    (6, 2, 80, 64, False, "window", 70, 5, True, None),           # kept keys, a window across tiles
+    (32, 2, 64, 256, False, "chunk", 100, 0, False, 9.0),
+])
+def test_decoded_tokens_on_four_warps(hq, hkv, dk, dv, in_keys, mask, size, keep, with_sink, cap):
+    """One decoded token a sequence, up to 16 heads a group: keys at and beside a tile of 64 and a chunk of two tiles,
+    against 64 bits; a token's bits alone are those among the others."""
+    from types import SimpleNamespace
+
+    from deterministic_inference_b200.kernels import ops
+    dev, page = "cuda", 16
+    g = torch.Generator(device=dev).manual_seed(dk)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=dev).bfloat16()
+    lens = [1, 16, 63, 64, 65, 129, 300]
+    stored = 0 if in_keys else dv
+    pages = [-(-n // page) for n in lens]
+    table = torch.zeros(len(lens), max(pages), dtype=torch.int32)
+    perm = (torch.randperm(sum(pages)) + 1).tolist()
+    cache = torch.full((sum(pages) + 1, hkv * page * (dk + stored)), float("nan"), dtype=torch.bfloat16, device=dev)
+    keys, values = [], []
+    for b, n in enumerate(lens):
+        k = rnd(n, hkv, dk)
+        v = k[..., :dv] if in_keys else rnd(n, hkv, dv)
+        for i in range(pages[b]):
+            table[b, i] = at = perm.pop()
+            rows = slice(i * page, min(n, (i + 1) * page))
+            m = rows.stop - rows.start
+            cache[at, :hkv * page * dk].view(hkv, page, dk)[:, :m] = k[rows].transpose(0, 1)
+            if stored:
+                cache[at, hkv * page * dk:].view(hkv, page, dv)[:, :m] = v[rows].transpose(0, 1)
+        keys.append(k)
+        values.append(v)
+    q = rnd(len(lens), hq, dk)
+    sink = torch.randn(hq, generator=g, device=dev) if with_sink else None
+    scale = dk ** -0.5
+
+    def run(which):
+        i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+        n = len(which)
+        meta = SimpleNamespace(block_table=table[which].contiguous().to(dev), token_seq=i32(range(n)),
+                               positions=i32([lens[b] - 1 for b in which]), seq_lens=i32([lens[b] for b in which]),
+                               cu_q_lens=i32(range(n + 1)), q_lens=[1] * n, kv_lens=[lens[b] for b in which], scratch={},
+                               num_decode=n)
+        return ops.masked_attention(q[which].contiguous(), cache, meta, scale, hkv, dv, page, mask, size, sink,
+                                    values_in_keys=in_keys, keep_first=keep, softcap=cap)
+
+    got = run(list(range(len(lens))))
+    for b, n in enumerate(lens):
+        j = torch.arange(n, device=dev)
+        p = n - 1
+        first = {"causal": 0, "window": p - (size or 0) + 1, "chunk": p // (size or 1) * (size or 1)}[mask]
+        sees = (j >= first) | (j < keep)
+        group = lambda x: x.double().repeat_interleave(hq // hkv, dim=1)
+        s = torch.einsum("hd,jhd->hj", q[b].double(), group(keys[b])) * scale
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        w = torch.exp(s.masked_fill(~sees, float("-inf")))
+        den = w.sum(1) + (torch.exp(sink.double()) if with_sink else 0)
+        want = torch.einsum("hj,jhd->hd", w, group(values[b])) / den[:, None]
+        # weights and the result are rounded to bfloat16 (2^-9 each), a weight against its warp's maximum
+        err = float((got[b].double() - want).abs().max())
+        assert err <= 2.0 ** -7 * float(group(values[b]).abs().max()), (n, err)
+        # (alone, a token of one chunk is finished in the kernel, among longer ones by the merge)
+        alone = run([b])[0]
+        assert torch.equal(alone, got[b]) if n > 128 else float((alone - got[b]).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
