@@ -51,6 +51,15 @@ def test_retention_alone(tmp_path, dtype, dim, vdim, decay, rot):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim, vdim, decay, rot", [
+    (24, 144, (0.99, 0.9), 8),                # a head's columns over four blocks, 36 each
+    (128, 256, (0.995,), 128),                # every thread's rows in one run of loads
+])
+def test_retention_over_a_cluster(tmp_path, dtype, dim, vdim, decay, rot):
+    nm.retention_case(tmp_path, dtype, "cuda", dim, vdim, decay, rot)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("experts, top, ff, limit", [(12, 3, 20, 0.5), (5, 1, 24, 1.0), (4, 4, 8, 0.7), (1, 1, 16, 0.3),
                                                      (64, 6, 32, 0.6)])
 def test_experts_of_a_table_alone(tmp_path, dtype, experts, top, ff, limit):
