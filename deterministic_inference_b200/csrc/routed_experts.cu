@@ -159,9 +159,9 @@ constexpr int SORT_THREADS = 1024;
 __global__ void __launch_bounds__(SORT_THREADS)
 moe_sort_kernel(const int* ids, const int* __restrict__ table, int top, int V, int pairs, int E, int tile, int max_tiles,
                 int* __restrict__ order) {
-  __shared__ int count[SORT_THREADS], first_tile[SORT_THREADS + 1], scan[SORT_THREADS];
+  __shared__ int count[SORT_THREADS], first_tile[SORT_THREADS + 1], warp_tiles[32];
   pdl_prologue(ids);
-  const int e = threadIdx.x;
+  const int e = threadIdx.x, threads = blockDim.x, lane = threadIdx.x & 31;
   auto expert_of = [&](int i) {
     if (table == nullptr) return ids[i];
     const int t = i / top, id = ids[t] < 0 ? 0 : (ids[t] >= V ? V - 1 : ids[t]);
@@ -169,32 +169,33 @@ moe_sort_kernel(const int* ids, const int* __restrict__ table, int top, int V, i
   };
   count[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += SORT_THREADS) {
+  for (int i = threadIdx.x; i < pairs; i += threads) {
     const int x = expert_of(i);
     if (x >= 0 && x < E) atomicAdd(&count[x], 1);
   }
   __syncthreads();
   const int my_tiles = e < E ? (count[e] + tile - 1) / tile : 0;
-  scan[e] = my_tiles;
-  __syncthreads();
-  for (int o = 1; o < SORT_THREADS; o <<= 1) {        // inclusive scan
-    const int v = e >= o ? scan[e - o] : 0;
-    __syncthreads();
-    scan[e] += v;
-    __syncthreads();
+  int upto = my_tiles;                                // an inclusive scan over the warp, then over the warps
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += v;
   }
-  first_tile[e + 1] = scan[e];
+  if (lane == 31) warp_tiles[e >> 5] = upto;
+  __syncthreads();
+  for (int w = 0; w < e >> 5; ++w) upto += warp_tiles[w];
+  first_tile[e + 1] = upto;
   if (e == 0) first_tile[0] = 0;
   count[e] = 0;                                       // now the expert's cursor
   __syncthreads();
   int* tile_expert = order + (long long)max_tiles * tile;
-  for (int i = threadIdx.x; i < max_tiles * tile; i += SORT_THREADS) order[i] = -1;
-  for (int i = threadIdx.x; i < max_tiles; i += SORT_THREADS) tile_expert[i] = -1;
+  for (int i = threadIdx.x; i < max_tiles * tile; i += threads) order[i] = -1;
+  for (int i = threadIdx.x; i < max_tiles; i += threads) tile_expert[i] = -1;
   __syncthreads();
   if (e < E)
     for (int k = first_tile[e]; k < first_tile[e + 1] && k < max_tiles; ++k) tile_expert[k] = e;
   if (e == 0) tile_expert[max_tiles] = first_tile[E] < max_tiles ? first_tile[E] : max_tiles;   // tiles in use: the first ones
-  for (int i = threadIdx.x; i < pairs; i += SORT_THREADS) {
+  for (int i = threadIdx.x; i < pairs; i += threads) {
     const int x = expert_of(i);
     if (x < 0 || x >= E) continue;
     const long long at = (long long)first_tile[x] * tile + atomicAdd(&count[x], 1);
@@ -695,7 +696,9 @@ int dib_moe_sort(const int* ids, const int* table, int top, int V, int pairs, in
                  cudaStream_t st) {
   if (pairs == 0) return DIB_OK;
   if (E < 1 || E > SORT_THREADS || tile < 1 || max_tiles < 1 || (table != nullptr && (top < 1 || V < 1))) return DIB_BAD_SIZE;
-  dib_launch(moe_sort_kernel, dim3(1), dim3(SORT_THREADS), 0, st, ids, table, top, V, pairs, E, tile, max_tiles, order);
+  // (a thread an expert at least; a decode step's few pairs do with fewer threads, whose barriers are cheaper)
+  const int threads = E <= 256 && pairs <= 1024 ? 256 : SORT_THREADS;
+  dib_launch(moe_sort_kernel, dim3(1), dim3(threads), 0, st, ids, table, top, V, pairs, E, tile, max_tiles, order);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
