@@ -1554,7 +1554,9 @@ EXPERT_TILE_ROWS_LARGE = 64
 # EXPERT_TILE_ROWS_TC rows times its expert's matrix).  Whole feed-forward on B200, mma.sync / tcgen05 in us
 # at 8, 16, 32, 64, 127 rows an expert: 16 experts of 1,024 x 1,536 63 / 72, 79 / 72, 117 / 72, 182 / 74,
 # 243 / 84; 64 of 1,024 x 512 84 / 82, 108 / 84, 173 / 86, 188 / 92, 275 / 113; 8 of 2,048 x 2,048 70 / 78,
-# 83 / 78, 127 / 80, 229 / 80, 328 / 92.  DIB200_EXPERTS_TC=0 (read once) leaves that form out.
+# 83 / 78, 127 / 80, 229 / 80, 328 / 92.  Steps of at most OWN_KERNEL_ROWS tokens never run there: up to that
+# size the dense products keep to one kernel too, and a decoded token's bits do not depend on the batch.
+# DIB200_EXPERTS_TC=0 (read once) leaves that form out.
 EXPERT_TILE_ROWS_TC = 128
 EXPERTS_TC_FROM = 16
 EXPERTS_TC = __import__("os").environ.get("DIB200_EXPERTS_TC", "1") != "0"
@@ -1646,8 +1648,9 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
     lib = _lib("routed_experts")
     dev = x.device
     pairs = t * top
+    from .gemm_bf16 import OWN_KERNEL_ROWS, _sms
     on_tc = EXPERTS_TC and x.dtype == torch.bfloat16 and pairs >= EXPERTS_TC_FROM * n_exp \
-        and f % (128 if gated else 256) == 0 and w % 256 == 0 and x.is_contiguous()
+        and t > OWN_KERNEL_ROWS and f % (128 if gated else 256) == 0 and w % 256 == 0 and x.is_contiguous()
     tile = EXPERT_TILE_ROWS_TC if on_tc \
         else EXPERT_TILE_ROWS_LARGE if pairs >= EXPERT_TILE_ROWS_LARGE * n_exp else EXPERT_TILE_ROWS
     max_tiles = pairs // tile + min(n_exp, pairs) + 1
@@ -1656,7 +1659,6 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
     _check(st, "routed_experts(sort)", f"{n_exp} experts (at most 1024)")
     per_pair = torch.empty(pairs, w, dtype=torch.float32, device=dev)
     if on_tc:
-        from .gemm_bf16 import _sms
         large = _lib("gemm_bf16_large")
         rows = max_tiles * tile
         tile_expert = c_void_p(order.data_ptr() + 4 * rows)

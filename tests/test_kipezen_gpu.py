@@ -145,6 +145,22 @@ def test_the_experts_streamed_products(width, ff, gated, monkeypatch):
         assert torch.equal(run(n), whole[:n]), n
 
 
+def test_the_experts_of_a_decode_step_do_not_depend_on_the_batch():
+    """A step of 64 tokens that brings an expert 32 rows has a single token's bits; one of 65 is another form."""
+    from deterministic_inference_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(7)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, up, down = rnd(65, 256), rnd(4, 512, 256) * 0.1, rnd(4, 256, 256) * 0.1
+    ids = torch.rand(65, 4, generator=g, device="cuda").argsort(1)[:, :2].int()
+    weights = torch.rand(65, 2, generator=g, device="cuda")
+    run = lambda n: ops.routed_experts(x[:n], ids[:n].contiguous(), weights[:n].contiguous(), up, down, None, None, 4,
+                                       torch.bfloat16)
+    one, batch, more = run(1), run(64), run(65)
+    assert torch.equal(batch[:1], one)
+    # hidden values round to bfloat16 (2^-8 each way) where the order of summation tips them
+    assert float((more[:64] - batch).abs().max()) <= 1e-2 * float(batch.abs().max())
+
+
 # ---- whole models ------------------------------------------------------------------------------------------
 
 CASES = {       # configuration -> request lengths, seed
