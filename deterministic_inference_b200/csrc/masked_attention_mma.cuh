@@ -178,11 +178,12 @@ masked_attention_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, const __
   find_rows(it_begin + 1);
   __syncthreads();
   load_tile(it_begin, it_begin & 1);
+  __syncthreads();              // the loop's first turn writes the entries that these copies read
   for (int it = it_begin; it < it_end; ++it) {
     const int stage = it & 1;
     if (it + 1 < it_end) {
       load_tile(it + 1, stage ^ 1);
-      find_rows(it + 2);        // into this tile's entries: its copies were issued a round ago
+      find_rows(it + 2);        // into this tile's entries: its copies were issued before the last barrier
       __pipeline_wait_prior(1);
     } else {
       __pipeline_wait_prior(0);
@@ -416,11 +417,12 @@ masked_attention_decode_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, c
   find_rows(it_begin + 1);
   __syncthreads();
   load_tile(it_begin & 1);
+  __syncthreads();              // the loop's first turn writes the entries that these copies read
   for (int it = it_begin; it < it_end; ++it) {
     const int stage = it & 1;
     if (it + 1 < it_end) {
       load_tile(stage ^ 1);
-      find_rows(it + 2);        // into this tile's entries: its copies were issued a round ago
+      find_rows(it + 2);        // into this tile's entries: its copies were issued before the last barrier
       __pipeline_wait_prior(1);
     } else {
       __pipeline_wait_prior(0);
