@@ -373,7 +373,7 @@ moe_product_stream_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* _
                           float alpha) {
   extern __shared__ __align__(16) unsigned char gp_smem[];
   __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(gp_smem);
-  __shared__ float up_sums[2][32][4];
+  __shared__ __align__(16) float up_sums[2][32][4];
   pdl_prologue(a_rows, order);
   const int tl = blockIdx.x % max_tiles;
   const int expert = order[(long long)max_tiles * ST_A + tl];

@@ -75,3 +75,27 @@ def test_row_offsets_of_key_tiles_are_not_written_while_they_are_read(where, ahe
 
 def test_the_walks_are_there():
     assert len(_walks()) == 3
+
+
+WIDTH = {"float2": 8, "uint2": 8, "int2": 8, "float4": 16, "uint4": 16, "int4": 16, "__nv_bfloat162": 4, "half2": 4}
+TYPE = {"float": 4, "int": 4, "unsigned": 4, "double": 8, "long long": 8, "unsigned long long": 8, "__nv_bfloat16": 2}
+
+
+def test_arrays_in_shared_memory_that_are_read_as_vectors_start_on_them():
+    """An array in static shared memory is aligned to its elements; one whose elements are read or written several at a
+    time says so."""
+    declared = re.compile(r"__shared__ ((?:__align__\((\d+)\) )?)((?:unsigned |long )*\w+) ([^;]+);")
+    seen = 0
+    for path in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]):
+        text = re.sub(r"extern __shared__[^;]+;", "", path.read_text())
+        for m in declared.finditer(text):
+            kind = m.group(3).strip()
+            align = int(m.group(2) or TYPE.get(kind, 0))
+            if not align:
+                continue                      # (a struct of its own)
+            for name in re.findall(r"(\w+)\s*\[[^,]*", m.group(4)):
+                for use in re.finditer(rf"reinterpret_cast<(?:const )?(\w+)\s*\*>\(&?{name}\b", text):
+                    seen += 1
+                    need = WIDTH.get(use.group(1), 16)
+                    assert align % need == 0, f"{path.name}: {name} is read as {use.group(1)}, aligned to {align}"
+    assert seen >= 2
