@@ -49,6 +49,18 @@ struct SoftCap {
     return __fmaf_rn(-2.0f * size, r, size);
   }
 };
+// exp(sink) joins the denominator of a row whose scores' maximum is m (units of log 2); a sink above every score becomes
+// the reference.  The operations are the merge kernel's for one chunk, so a token's bits are the same where it is
+// finished at once and where it is merged.
+struct SinkJoin {
+  float own, scale;      // the sink's share; what the row's sums are multiplied by
+  __device__ __forceinline__ SinkJoin(float sink, float m) {
+    const float sl = sink * MA_LOG2E, ref = fmaxf(m, sl);
+    own = ex2(sl - ref);
+    scale = ex2(m - ref);
+  }
+  __device__ __forceinline__ float denominator(float l) const { return __fmaf_rn(l, scale, own); }
+};
 __device__ __forceinline__ int first_seen(int pos, int mask_kind, int mask_size) {
   if (mask_kind == 1) return pos - mask_size + 1 > 0 ? pos - mask_size + 1 : 0;
   if (mask_kind == 2) return pos > 0 ? pos / mask_size * mask_size : 0;
@@ -294,15 +306,12 @@ masked_attention_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, const __
     }
     float l = l_row[h];
     if (sink != nullptr) {
-      // exp(sink) joins the denominator; a sink above every score becomes the reference
-      const float sl = sink[head] * MA_LOG2E;
-      const float ref = fmaxf(m_row[h], sl);
-      const float a = ex2(m_row[h] - ref);
-      l = l * a + ex2(sl - ref);
+      const SinkJoin j(sink[head], m_row[h]);
+      l = j.denominator(l);
 #pragma unroll
       for (int n = 0; n < NV16 * 2; ++n) {
-        o[n][2 * h] *= a;
-        o[n][2 * h + 1] *= a;
+        o[n][2 * h] *= j.scale;
+        o[n][2 * h + 1] *= j.scale;
       }
     }
     const float inv = 1.0f / l;
@@ -531,10 +540,8 @@ masked_attention_decode_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, c
     float M = sm[0][r];
 #pragma unroll
     for (int w = 1; w < DEC_WARPS; ++w) M = fmaxf(M, sm[w][r]);
-    const float sink_l = sink != nullptr && !chunked ? sink[head] * MA_LOG2E : MA_NEG_BIG;
-    M = fmaxf(M, sink_l);
     const float ref = M <= -1e29f ? 0.f : M;
-    float v = 0.f, l = sink != nullptr && !chunked ? ex2(sink_l - ref) : 0.f;
+    float v = 0.f, l = 0.f;
 #pragma unroll
     for (int w = 0; w < DEC_WARPS; ++w) {
       const float a = ex2(sm[w][r] - ref);
@@ -545,6 +552,11 @@ masked_attention_decode_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, c
       partial_o[(row * max_chunks + chunk) * VD + col] = v;
       if (col == 0) *reinterpret_cast<float2*>(partial_ml + (row * max_chunks + chunk) * 2) = make_float2(M, l);
       continue;
+    }
+    if (sink != nullptr) {       // behind the warps' sums, as the merge adds it to a single chunk's: the same bits
+      const SinkJoin j(sink[head], M);
+      l = j.denominator(l);
+      v *= j.scale;
     }
     v *= 1.0f / l;
     if (gate.p != nullptr) {
@@ -577,7 +589,7 @@ __global__ void masked_attention_merge_kernel(const float* partial_o, const floa
   float L = sink != nullptr ? ex2(sl - M) : 0.f;
   for (int c = 0; c < chunks; ++c) {
     const float2 ml = *reinterpret_cast<const float2*>(partial_ml + (row * max_chunks + c) * 2);
-    L += ml.y * ex2(ml.x - M);
+    L = __fmaf_rn(ml.y, ex2(ml.x - M), L);
   }
   const float inv = 1.0f / L;
   for (int col = threadIdx.x; col < VD; col += blockDim.x) {

@@ -444,10 +444,12 @@ def test_greedy_generation_through_the_entry_point(name, dtype, model_dirs):
     (1, 1, 48, 16, True, "causal", None, 0, True, None),          # an odd number of steps of 16 dimensions
     (6, 2, 80, 64, False, "window", 70, 5, True, None),           # kept keys, a window across tiles
     (32, 2, 64, 256, False, "chunk", 100, 0, False, 9.0),
+    (12, 3, 64, 64, False, "causal", None, 0, True, 9.0),         # a sink beside a cap: scores and sinks of one size
 ])
 def test_decoded_tokens_on_four_warps(hq, hkv, dk, dv, in_keys, mask, size, keep, with_sink, cap):
     """One decoded token a sequence, up to 16 heads a group: keys at and beside a tile of 64 and a chunk of two tiles,
-    against 64 bits; a token's bits alone are those among the others."""
+    against 64 bits; a token's bits alone are those among the others, and those of a captured step, whose lengths are
+    upper bounds."""
     from types import SimpleNamespace
 
     from deterministic_inference_b200.kernels import ops
@@ -477,13 +479,13 @@ def test_decoded_tokens_on_four_warps(hq, hkv, dk, dv, in_keys, mask, size, keep
     sink = torch.randn(hq, generator=g, device=dev) if with_sink else None
     scale = dk ** -0.5
 
-    def run(which):
+    def run(which, bound=0):
         i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
         n = len(which)
         meta = SimpleNamespace(block_table=table[which].contiguous().to(dev), token_seq=i32(range(n)),
                                positions=i32([lens[b] - 1 for b in which]), seq_lens=i32([lens[b] for b in which]),
-                               cu_q_lens=i32(range(n + 1)), q_lens=[1] * n, kv_lens=[lens[b] for b in which], scratch={},
-                               num_decode=n)
+                               cu_q_lens=i32(range(n + 1)), q_lens=[1] * n,
+                               kv_lens=[max(bound, lens[b]) for b in which], scratch={}, num_decode=n)
         return ops.masked_attention(q[which].contiguous(), cache, meta, scale, hkv, dv, page, mask, size, sink,
                                     values_in_keys=in_keys, keep_first=keep, softcap=cap)
 
@@ -503,6 +505,32 @@ def test_decoded_tokens_on_four_warps(hq, hkv, dk, dv, in_keys, mask, size, keep
         # weights and the result are rounded to bfloat16 (2^-9 each), a weight against its warp's maximum
         err = float((got[b].double() - want).abs().max())
         assert err <= 2.0 ** -7 * float(group(values[b]).abs().max()), (n, err)
-        # (alone, a token of one chunk is finished in the kernel, among longer ones by the merge)
-        alone = run([b])[0]
-        assert torch.equal(alone, got[b]) if n > 128 else float((alone - got[b]).abs().max()) <= 2.0 ** -7 * float(want.abs().max())
+        # (alone, a token of one chunk is finished in the kernel, among longer ones and in a captured step by the merge)
+        assert torch.equal(run([b])[0], got[b]), n
+        assert torch.equal(run([b], bound=1000)[0], got[b]), n
+
+
+@pytest.mark.parametrize("hq, hkv, dk, dv, cap", [(16, 1, 80, 64, None), (16, 16, 64, 64, 9.0), (20, 1, 64, 48, None)])
+def test_a_sink_joins_a_decoded_tokens_sums_in_one_order(hq, hkv, dk, dv, cap):
+    """512 tokens of one chunk of keys each, with a sink: finished in the kernel or, where the step's lengths are upper
+    bounds (a captured step) or another sequence is longer, by the merge.  Equal in every bit; rounded to bfloat16, one
+    result in some ten thousands shows another order of the float32 operations, so there are many of them."""
+    from types import SimpleNamespace
+
+    from deterministic_inference_b200.kernels import ops
+    dev, page, n = "cuda", 128, 512
+    g = torch.Generator(device=dev).manual_seed(dk + hq)
+    lens = [1 + (37 * b) % 127 for b in range(n)]
+    cache = torch.randn(n + 1, hkv * page * (dk + dv), generator=g, device=dev).bfloat16()
+    q = torch.randn(n, hq, dk, generator=g, device=dev).bfloat16()
+    sink = 2.0 * torch.randn(hq, generator=g, device=dev)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+
+    def run(bound):
+        meta = SimpleNamespace(block_table=i32([[b + 1] for b in range(n)]), token_seq=i32(range(n)),
+                               positions=i32([m - 1 for m in lens]), seq_lens=i32(lens), cu_q_lens=i32(range(n + 1)),
+                               q_lens=[1] * n, kv_lens=[max(bound, m) for m in lens], scratch={}, num_decode=n)
+        return ops.masked_attention(q, cache, meta, dk ** -0.5, hkv, dv, page, "causal", None, sink, softcap=cap)
+
+    alone, merged = run(0), run(129)
+    assert int((alone != merged).sum()) == 0
