@@ -1554,8 +1554,9 @@ EXPERT_TILE_ROWS_LARGE = 64
 # EXPERT_TILE_ROWS_TC rows times its expert's matrix).  Whole feed-forward on B200, mma.sync / tcgen05 in us
 # at 8, 16, 32, 64, 127 rows an expert: 16 experts of 1,024 x 1,536 63 / 72, 79 / 72, 117 / 72, 182 / 74,
 # 243 / 84; 64 of 1,024 x 512 84 / 82, 108 / 84, 173 / 86, 188 / 92, 275 / 113; 8 of 2,048 x 2,048 70 / 78,
-# 83 / 78, 127 / 80, 229 / 80, 328 / 92.  Steps of at most OWN_KERNEL_ROWS tokens never run there: up to that
-# size the dense products keep to one kernel too, and a decoded token's bits do not depend on the batch.
+# 83 / 78, 127 / 80, 229 / 80, 328 / 92.  Steps of at most ``gemm_bf16.MAX_ROWS`` tokens never run there: up to
+# that size the dense products keep to one kernel too, and a decoded token's bits do not depend on the batch.  (With
+# ``library_products`` off that is every step: a token's bits then do not depend on its portion.)
 # DIB200_EXPERTS_TC=0 (read once) leaves that form out.
 EXPERT_TILE_ROWS_TC = 128
 EXPERTS_TC_FROM = 16
@@ -1648,9 +1649,9 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
     lib = _lib("routed_experts")
     dev = x.device
     pairs = t * top
-    from .gemm_bf16 import OWN_KERNEL_ROWS, _sms
+    from . import gemm_bf16
     on_tc = EXPERTS_TC and x.dtype == torch.bfloat16 and pairs >= EXPERTS_TC_FROM * n_exp \
-        and t > OWN_KERNEL_ROWS and f % (128 if gated else 256) == 0 and w % 256 == 0 and x.is_contiguous()
+        and t > gemm_bf16.MAX_ROWS and f % (128 if gated else 256) == 0 and w % 256 == 0 and x.is_contiguous()
     tile = EXPERT_TILE_ROWS_TC if on_tc \
         else EXPERT_TILE_ROWS_LARGE if pairs >= EXPERT_TILE_ROWS_LARGE * n_exp else EXPERT_TILE_ROWS
     max_tiles = pairs // tile + min(n_exp, pairs) + 1
@@ -1669,12 +1670,12 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
         hidden = torch.empty(rows, f, dtype=x.dtype, device=dev)
         st = large.dib_gemm_bf16_large_grouped(_ptr(sorted_x), _ptr(w_gate_up), _ptr(hidden), c_int(rows), c_int(f),
                                                c_int(w), c_int(1 if gated else 2), c_int(0), tile_expert, c_int(n_exp),
-                                               c_float(limit), c_float(alpha), c_int(_sms(dev)), _stream())
+                                               c_float(limit), c_float(alpha), c_int(gemm_bf16._sms(dev)), _stream())
         _check(st, "routed_experts(gate and up, tcgen05)", f"rows {rows}, F {f}, W {w}")
         sorted_y = torch.empty(rows, w, dtype=torch.float32, device=dev)
         st = large.dib_gemm_bf16_large_grouped(_ptr(hidden), _ptr(w_down), _ptr(sorted_y), c_int(rows), c_int(w),
                                                c_int(f), c_int(0), c_int(1), tile_expert, c_int(n_exp),
-                                               c_float(0.0), c_float(0.0), c_int(_sms(dev)), _stream())
+                                               c_float(0.0), c_float(0.0), c_int(gemm_bf16._sms(dev)), _stream())
         _check(st, "routed_experts(down, tcgen05)", f"rows {rows}, F {f}, W {w}")
         st = lib.dib_moe_scatter_rows(_ptr(sorted_y), _ptr(order), c_longlong(rows), c_int(w), _ptr(per_pair), _stream())
         _check(st, "routed_experts(rows back to their pairs)")

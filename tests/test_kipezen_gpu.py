@@ -161,6 +161,54 @@ def test_the_experts_of_a_decode_step_do_not_depend_on_the_batch():
     assert float((more[:64] - batch).abs().max()) <= 1e-2 * float(batch.abs().max())
 
 
+def test_the_experts_keep_to_one_form_without_the_library():
+    """``library_products=False``: a token's bits are the same in a step of 1, 100, 128 (16 rows an expert) or 512."""
+    from deterministic_inference_b200.kernels import gemm_bf16, ops
+    g = torch.Generator(device="cuda").manual_seed(8)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, up, down = rnd(512, 256), rnd(16, 256, 256) * 0.1, rnd(16, 256, 128) * 0.1
+    ids = torch.rand(512, 16, generator=g, device="cuda").argsort(1)[:, :2].int()
+    weights = torch.rand(512, 2, generator=g, device="cuda")
+    run = lambda n: ops.routed_experts(x[:n], ids[:n].contiguous(), weights[:n].contiguous(), up, down, None, None, 16,
+                                       torch.bfloat16)
+    gemm_bf16.set_library_products(False)
+    try:
+        whole = run(512)
+        for n in (1, 64, 65, 100, 127, 128):
+            assert torch.equal(run(n), whole[:n]), n
+    finally:
+        gemm_bf16.set_library_products(True)
+
+
+def test_bits_of_a_token_do_not_depend_on_its_portion_without_the_library(tmp_path):
+    """A model with routed experts under ``library_products=False``: the logits of a request in portions of 512 and of
+    100 are equal bit for bit (100 tokens bring an expert 12.5 rows, 512 bring it 64)."""
+    from deterministic_inference_b200 import EngineConfig
+    from deterministic_inference_b200.config import KipezenConfig
+    from deterministic_inference_b200.engine.batch import SequenceInput
+    from deterministic_inference_b200.engine.runner import ModelRunner
+    from deterministic_inference_b200.kernels import gemm_bf16
+    from deterministic_inference_b200.weights import write_random_model
+    layer = ku.parallel(2, 1, 64, 64, 150, 3, 32, 10000.0, 64, 2, 2, mlp=ku.moe(16, 2, 128, 2.0, groups=(2, 2), shared=128))
+    write_random_model(KipezenConfig.from_dict({"architecture": "Kipezen", "vocab": 160, "width": 256,
+                                                "norm": {"eps": 1e-5}, "layers": [layer, layer]}), 57, tmp_path)
+    ku.sharpen(tmp_path)
+    tokens = ku.requests(160, [612], 58)[0]
+    rows = {}
+    try:
+        for portion in (512, 100):
+            r = ModelRunner(EngineConfig(model_path=str(tmp_path), dtype="bfloat16", kv_pool_tokens=2048, page_size=16,
+                                         max_reqs=4, max_seq_len=1024, cuda_graphs=False, library_products=False))
+            slot, got = r.cache.allocate_slot(), []
+            for c in range(0, len(tokens), portion):
+                n = min(portion, len(tokens) - c)
+                got.append(r.step([SequenceInput(slot, tokens[c:c + n], c, list(range(n)))])[0].clone())
+            rows[portion] = torch.cat(got)
+    finally:
+        gemm_bf16.set_library_products(True)
+    assert int((rows[512] != rows[100]).any(1).sum()) == 0
+
+
 # ---- whole models ------------------------------------------------------------------------------------------
 
 CASES = {       # configuration -> request lengths, seed
