@@ -1556,7 +1556,8 @@ EXPERT_TILE_ROWS_LARGE = 64
 # 243 / 84; 64 of 1,024 x 512 84 / 82, 108 / 84, 173 / 86, 188 / 92, 275 / 113; 8 of 2,048 x 2,048 70 / 78,
 # 83 / 78, 127 / 80, 229 / 80, 328 / 92.  Steps of at most ``gemm_bf16.MAX_ROWS`` tokens never run there: up to
 # that size the dense products keep to one kernel too, and a decoded token's bits do not depend on the batch.  (With
-# ``library_products`` off that is every step: a token's bits then do not depend on its portion.)
+# ``library_products`` off that is every step: a token's bits then do not depend on its portion.)  Under
+# ``large_products`` "own", where a row's bits change at that line only, all larger steps run there.
 # DIB200_EXPERTS_TC=0 (read once) leaves that form out.
 EXPERT_TILE_ROWS_TC = 128
 EXPERTS_TC_FROM = 16
@@ -1650,8 +1651,9 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
     dev = x.device
     pairs = t * top
     from . import gemm_bf16
-    on_tc = EXPERTS_TC and x.dtype == torch.bfloat16 and pairs >= EXPERTS_TC_FROM * n_exp \
-        and t > gemm_bf16.MAX_ROWS and f % (128 if gated else 256) == 0 and w % 256 == 0 and x.is_contiguous()
+    on_tc = EXPERTS_TC and x.dtype == torch.bfloat16 and t > gemm_bf16.MAX_ROWS \
+        and (pairs >= EXPERTS_TC_FROM * n_exp or gemm_bf16.LARGE_PRODUCTS == "own") \
+        and f % (128 if gated else 256) == 0 and w % 256 == 0 and x.is_contiguous()
     tile = EXPERT_TILE_ROWS_TC if on_tc \
         else EXPERT_TILE_ROWS_LARGE if pairs >= EXPERT_TILE_ROWS_LARGE * n_exp else EXPERT_TILE_ROWS
     max_tiles = pairs // tile + min(n_exp, pairs) + 1

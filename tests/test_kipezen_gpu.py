@@ -180,6 +180,27 @@ def test_the_experts_keep_to_one_form_without_the_library():
         gemm_bf16.set_library_products(True)
 
 
+@pytest.mark.parametrize("products", ["own", "auto"])
+def test_the_experts_change_form_at_stated_lines(products, monkeypatch):
+    """``large_products="own"``: a row's bits change at the 64-row line only, not with the rows an expert gets (65 tokens
+    bring it 8 rows, 128 bring 16, 512 bring 64).  By default they change at 16 rows an expert."""
+    from deterministic_inference_b200.kernels import gemm_bf16, ops
+    monkeypatch.setattr(gemm_bf16, "LARGE_PRODUCTS", products)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    line = 64 if products == "own" else 127
+    for gated, ff in ((True, 128), (False, 256)):
+        x, up, down = rnd(512, 256), rnd(16, ff * (2 if gated else 1), 256) * 0.1, rnd(16, 256, ff) * 0.1
+        ids = torch.rand(512, 16, generator=g, device="cuda").argsort(1)[:, :2].int()
+        weights = torch.rand(512, 2, generator=g, device="cuda")
+        run = lambda n: ops.routed_experts(x[:n], ids[:n].contiguous(), weights[:n].contiguous(), up, down, None, None, 16,
+                                           torch.bfloat16, gated=gated)
+        whole, few = run(512), run(line)
+        for n in (1, 64, 65, 127, 128, 300):
+            assert torch.equal(run(n), (few if n <= line else whole)[:n]), (gated, n)
+    ops.check_kernel_status()
+
+
 def test_bits_of_a_token_do_not_depend_on_its_portion_without_the_library(tmp_path):
     """A model with routed experts under ``library_products=False``: the logits of a request in portions of 512 and of
     100 are equal bit for bit (100 tokens bring an expert 12.5 rows, 512 bring it 64)."""
