@@ -14,6 +14,8 @@
 // (RMS norm over a head, weight, silu gate) have kernels of their own below.
 #include <cuda_pipeline.h>
 
+#include <type_traits>
+
 #include "source.cuh"
 #include "conv_tail.cuh"
 
@@ -27,15 +29,15 @@
 // written for a channel and token.  (A block a token, which read the head's R x D weights again for
 // each in one chain of R loads a thread, 2,048 tokens of 16 heads of 64: 129 us, so 47.)
 constexpr int PREP_TOKENS = 8, PREP_RANKS = 512;      // tokens of a block; entries of the hidden vector at a time
-template <int PROJ, int W>
-__global__ void delta_prepare_kernel(Source proj, const void* w2t, const float* w0,
-                                     const float* a_bias, float* packed, int T, int H, int D, int R,
-                                     float decay_scale, float key_eps) {
-  __shared__ __align__(16) float th[PREP_RANKS * PREP_TOKENS];       // tanh of the lora hidden
-  __shared__ float sums[PREP_TOKENS * 32];                           // the warps' sums of squares
+template <int TOKENS, int PROJ, int W>
+__global__ void __launch_bounds__(TOKENS == 1 ? 1024 : 256)
+delta_prepare_kernel(Source proj, const void* w2t, const float* w0, const float* a_bias, float* packed, int T, int H,
+                     int D, int R, float decay_scale, float key_eps) {
+  __shared__ __align__(16) float th[PREP_RANKS * TOKENS];            // tanh of the lora hidden
+  __shared__ float sums[TOKENS * 32];                                // the warps' sums of squares
   pdl_prologue();
-  const int t0 = blockIdx.x * PREP_TOKENS, h = blockIdx.y, c = threadIdx.x;
-  const int tokens = min(PREP_TOKENS, T - t0);
+  const int t0 = blockIdx.x * TOKENS, h = blockIdx.y, c = threadIdx.x;
+  const int tokens = min(TOKENS, T - t0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int HD = H * D;
   const long long width = 5 * HD + R;
@@ -45,9 +47,9 @@ __global__ void delta_prepare_kernel(Source proj, const void* w2t, const float* 
     else return source_load(proj, at);
   };
   const int ch = h * D + c;
-  float r[PREP_TOKENS], k[PREP_TOKENS], v[PREP_TOKENS], a[PREP_TOKENS], z[PREP_TOKENS];
+  float r[TOKENS], k[TOKENS], v[TOKENS], a[TOKENS], z[TOKENS];
 #pragma unroll
-  for (int i = 0; i < PREP_TOKENS; ++i) {
+  for (int i = 0; i < TOKENS; ++i) {
     const bool in = c < D && i < tokens;
     const long long row = (t0 + i) * width + ch;
     r[i] = in ? element(row) : 0.f;
@@ -57,16 +59,16 @@ __global__ void delta_prepare_kernel(Source proj, const void* w2t, const float* 
     z[i] = 0.f;
   }
 #pragma unroll
-  for (int i = 0; i < PREP_TOKENS; ++i) {
+  for (int i = 0; i < TOKENS; ++i) {
     const float part = warp_sum(k[i] * k[i]);
     if (lane == 0) sums[i * 32 + warp] = part;
   }
   for (int j0 = 0; j0 < R; j0 += PREP_RANKS) {
     const int n = min(PREP_RANKS, R - j0);
     if (j0 > 0) __syncthreads();
-    for (int e = threadIdx.x; e < n * PREP_TOKENS; e += blockDim.x) {
+    for (int e = threadIdx.x; e < n * TOKENS; e += blockDim.x) {
       const int i = e / n, j = e - i * n;
-      th[j * PREP_TOKENS + i] = i < tokens ? tanhf(element((t0 + i) * width + 5 * HD + j0 + j)) : 0.f;
+      th[j * TOKENS + i] = i < tokens ? tanhf(element((t0 + i) * width + 5 * HD + j0 + j)) : 0.f;
     }
     __syncthreads();
     if (c < D) {
@@ -74,14 +76,18 @@ __global__ void delta_prepare_kernel(Source proj, const void* w2t, const float* 
       for (int j = 0; j < n; ++j) {
         const long long at = (long long)(j0 + j) * HD + ch;
         const float w = load_as(w2t, W, at);
-        const float4* x = reinterpret_cast<const float4*>(th + j * PREP_TOKENS);
+        if constexpr (TOKENS == 1) {
+          z[0] = __fmaf_rn(w, th[j], z[0]);
+        } else {
+          const float4* x = reinterpret_cast<const float4*>(th + j * TOKENS);
 #pragma unroll
-        for (int q = 0; q < PREP_TOKENS / 4; ++q) {
-          const float4 y = x[q];
-          z[4 * q] = __fmaf_rn(w, y.x, z[4 * q]);
-          z[4 * q + 1] = __fmaf_rn(w, y.y, z[4 * q + 1]);
-          z[4 * q + 2] = __fmaf_rn(w, y.z, z[4 * q + 2]);
-          z[4 * q + 3] = __fmaf_rn(w, y.w, z[4 * q + 3]);
+          for (int q = 0; q < TOKENS / 4; ++q) {
+            const float4 y = x[q];
+            z[4 * q] = __fmaf_rn(w, y.x, z[4 * q]);
+            z[4 * q + 1] = __fmaf_rn(w, y.y, z[4 * q + 1]);
+            z[4 * q + 2] = __fmaf_rn(w, y.z, z[4 * q + 2]);
+            z[4 * q + 3] = __fmaf_rn(w, y.w, z[4 * q + 3]);
+          }
         }
       }
     }
@@ -90,7 +96,7 @@ __global__ void delta_prepare_kernel(Source proj, const void* w2t, const float* 
   if (c >= D) return;
   const float bias_w = w0[ch], bias_a = a_bias != nullptr ? a_bias[ch] : 0.f;
 #pragma unroll
-  for (int i = 0; i < PREP_TOKENS; ++i) {
+  for (int i = 0; i < TOKENS; ++i) {
     if (i >= tokens) break;
     float ss = 0.f;
     for (int x = 0; x < warps; ++x) ss += sums[i * 32 + x];
@@ -617,13 +623,18 @@ int dib_delta_prepare(const void* proj, int kind, int splits, long long stride, 
   if (T_ == 0) return DIB_OK;
   if (H < 1 || H > 65535 || D < 1 || D > 1024 || R < 0 || R > 8192) return DIB_BAD_SIZE;
   if (w_dtype != 0 && w_dtype != 1) return DIB_BAD_DTYPE;
-  const int form = kind == 1 ? 1 : splits <= 1 ? 0 : 2;
-  auto* kernel = form == 0   ? (w_dtype == 1 ? &delta_prepare_kernel<0, 1> : &delta_prepare_kernel<0, 0>)
-                 : form == 1 ? (w_dtype == 1 ? &delta_prepare_kernel<1, 1> : &delta_prepare_kernel<1, 0>)
-                             : (w_dtype == 1 ? &delta_prepare_kernel<2, 1> : &delta_prepare_kernel<2, 0>);
-  dib_launch(kernel, dim3(ceil_div_host(T_, PREP_TOKENS), H), dim3((D + 31) / 32 * 32), 0, st,
-             make_source(proj, kind, splits, stride), w2t, w0, a_bias, packed, T_, H, D, R, decay_scale,
-             key_eps);
+  const Source src = make_source(proj, kind, splits, stride);
+  auto go = [&](auto tokens) {
+    constexpr int N = decltype(tokens)::value;
+    auto* kernel = kind == 1     ? (w_dtype == 1 ? &delta_prepare_kernel<N, 1, 1> : &delta_prepare_kernel<N, 1, 0>)
+                   : splits <= 1 ? (w_dtype == 1 ? &delta_prepare_kernel<N, 0, 1> : &delta_prepare_kernel<N, 0, 0>)
+                                 : (w_dtype == 1 ? &delta_prepare_kernel<N, 2, 1> : &delta_prepare_kernel<N, 2, 0>);
+    dib_launch(kernel, dim3(ceil_div_host(T_, N), H), dim3((D + 31) / 32 * 32), 0, st, src, w2t, w0, a_bias, packed, T_,
+               H, D, R, decay_scale, key_eps);
+  };
+  // (heads of more than 256: a block's registers do not reach for the values of several tokens)
+  if (D <= 256) go(std::integral_constant<int, PREP_TOKENS>{});
+  else go(std::integral_constant<int, 1>{});
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }

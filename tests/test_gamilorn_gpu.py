@@ -319,6 +319,46 @@ def test_delta_rule_alone(dtype, heads, dim, rank):
     assert not torch.isnan(state[1:]).any()
 
 
+def prepared(proj, heads, dim, rank, w2_t, w0, a_bias):
+    """The delta rule's vectors [tokens, heads, 6, dim] by the kernel; ``proj`` float32 or bfloat16 [tokens, width], or
+    float32 split sums [splits, tokens, width]."""
+    from ctypes import c_float, c_int, c_longlong
+
+    from deterministic_inference_b200.kernels import ops
+    splits, n = (1, proj.shape[0]) if proj.dim() == 2 else proj.shape[:2]
+    out = torch.full((n, heads, 6, dim), float("nan"), device=proj.device)
+    st = ops._lib("delta_rule").dib_delta_prepare(
+        ops._ptr(proj), c_int(1 if proj.dtype == torch.bfloat16 else 0), c_int(splits), c_longlong(proj.stride(0) if splits > 1 else 0),
+        ops._ptr(w2_t), c_int(1 if w2_t.dtype == torch.bfloat16 else 0), ops._ptr(w0), ops._ptr(a_bias), ops._ptr(out),
+        c_int(n), c_int(heads), c_int(dim), c_int(rank), c_float(math.exp(-0.5)), c_float(1e-6), ops._stream())
+    assert st == 0, st
+    return out
+
+
+def prepared_in_64_bits(proj, heads, dim, rank, w2_t, w0, a_bias):
+    p, hd = proj.double(), heads * dim
+    r, k, v = (p[:, i * hd:(i + 1) * hd].view(-1, heads, dim) for i in range(3))
+    rate = torch.sigmoid(p[:, 4 * hd:5 * hd] + a_bias.double()).view(-1, heads, dim)
+    w = torch.exp(-math.exp(-0.5) * torch.sigmoid(torch.tanh(p[:, 5 * hd:]) @ w2_t.double() + w0.double()))
+    u = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+    return torch.stack([w.view(-1, heads, dim), rate * u, u, k, r, v], dim=2)
+
+
+@pytest.mark.parametrize("dtype", list(DTYPES))
+@pytest.mark.parametrize("dim", [256, 257, 1000, 1024])
+def test_the_delta_rules_vectors_of_wide_heads(dim, dtype):
+    """Every head size the call accepts: a block of up to 1,024 threads has the registers it needs."""
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    rank, heads, n = 12, 2, 11
+    proj = torch.randn(n, 5 * heads * dim + rank, generator=g, device="cuda").to(DTYPES[dtype])
+    w2_t = torch.randn(rank, heads * dim, generator=g, device="cuda").to(DTYPES[dtype])
+    w0, a_bias = torch.randn(heads * dim, generator=g, device="cuda") - 2, torch.randn(heads * dim, generator=g, device="cuda")
+    got = prepared(proj, heads, dim, rank, w2_t, w0, a_bias)
+    want = prepared_in_64_bits(proj, heads, dim, rank, w2_t, w0, a_bias)
+    # a chain of `rank` terms of size |w2| <= 5 into the decay; a few roundings elsewhere
+    assert float((got.double() - want).abs().max()) <= (5 * rank + 32) * 2.0 ** -24 * float(want.abs().max())
+
+
 # ---- whole models through the trace runner -----------------------------------------------------------
 
 CASES = {
