@@ -22,15 +22,20 @@
 // proj row: [r | k | v | g | a_pre | lora hidden] = 5 * H * D + R columns; w2t [R][H * D] (the
 // decay map's second matrix, transposed: the threads of a block read consecutive elements).
 // packed [T][H][6][D] float32: w, a * u, u, k, r, v.
-// A block takes PREP_TOKENS tokens of a head: an element of w2t is read once for all of them, and
-// all their projected elements are asked for before the first is used.  PROJ 0 / 1: proj is a stored
-// float32 / bfloat16 matrix (a prompt portion's), 2: any source; W: w2t's type; no load of the first two
-// has a branch.  Bound: the 48 bytes
-// written for a channel and token.  (A block a token, which read the head's R x D weights again for
-// each in one chain of R loads a thread, 2,048 tokens of 16 heads of 64: 129 us, so 47.)
-constexpr int PREP_TOKENS = 8, PREP_RANKS = 512;      // tokens of a block; entries of the hidden vector at a time
+// A block takes TOKENS tokens of a head: an element of w2t is read once for all of them, and all their
+// projected elements are asked for before the first is used, of split sums (PROJ 2) a split of all of
+// them at a time.  PROJ 0 / 1: proj is a stored float32 / bfloat16 matrix; W: w2t's type.  A token's
+// vectors are the same in every form, which the launcher picks by what is quickest.  Bound: by latency
+// below some hundred tokens (the chain over R), then by the 48 bytes written for a channel and token.
+// (16 heads of 64, R = 64, us: split sums, one token a block, 1 / 8 / 64 tokens of eight splits 4.0 / 4.2 / 8.2;
+// eight tokens a block and the splits an element at a time 10.3 / 51 / 47.  Stored, two / four tokens a
+// block: 8 tokens 3.9 / 5.7, 128 tokens 7.4 / 9.9, 256 tokens 8.3 / 10.3, 512 tokens 13.3 / 11.8, 2,048
+// tokens 46 / 34; eight 10.2, 11.2, 14.9, 16, 38.)
+constexpr int PREP_RANKS = 512;                       // entries of the hidden vector at a time
+constexpr int PREP_FOUR_FROM = 384;                   // tokens from which on a block takes four
+// (The second bound of the launch leaves the compiler the registers that sixteen weights in flight need.)
 template <int TOKENS, int PROJ, int W>
-__global__ void __launch_bounds__(TOKENS == 1 ? 1024 : 256)
+__global__ void __launch_bounds__(TOKENS == 1 ? 1024 : 256, TOKENS == 1 ? 1 : 4)
 delta_prepare_kernel(Source proj, const void* w2t, const float* w0, const float* a_bias, float* packed, int T, int H,
                      int D, int R, float decay_scale, float key_eps) {
   __shared__ __align__(16) float th[PREP_RANKS * TOKENS];            // tanh of the lora hidden
@@ -48,18 +53,33 @@ delta_prepare_kernel(Source proj, const void* w2t, const float* w0, const float*
   };
   const int ch = h * D + c;
   float r[TOKENS], k[TOKENS], v[TOKENS], a[TOKENS], z[TOKENS];
+  if constexpr (PROJ == 2) {
+    static_assert(TOKENS == 1, "split sums are a few tokens'");
+    r[0] = k[0] = v[0] = a[0] = -0.f;                  // (-0 plus the first split is that split)
+    if (c < D) {
+      const float* f = reinterpret_cast<const float*>(proj.p) + t0 * width + ch;
+#pragma unroll 4
+      for (int sp = 0; sp < proj.splits; ++sp, f += proj.stride) {
+        r[0] = __fadd_rn(r[0], f[0]);
+        k[0] = __fadd_rn(k[0], f[HD]);
+        v[0] = __fadd_rn(v[0], f[2 * HD]);
+        a[0] = __fadd_rn(a[0], f[4 * HD]);
+      }
+    }
+  } else {
 #pragma unroll
-  for (int i = 0; i < TOKENS; ++i) {
-    const bool in = c < D && i < tokens;
-    const long long row = (t0 + i) * width + ch;
-    r[i] = in ? element(row) : 0.f;
-    k[i] = in ? element(row + HD) : 0.f;
-    v[i] = in ? element(row + 2 * HD) : 0.f;
-    a[i] = in ? element(row + 4 * HD) : 0.f;
-    z[i] = 0.f;
+    for (int i = 0; i < TOKENS; ++i) {
+      const bool in = c < D && i < tokens;
+      const long long row = (t0 + i) * width + ch;
+      r[i] = in ? element(row) : 0.f;
+      k[i] = in ? element(row + HD) : 0.f;
+      v[i] = in ? element(row + 2 * HD) : 0.f;
+      a[i] = in ? element(row + 4 * HD) : 0.f;
+    }
   }
 #pragma unroll
   for (int i = 0; i < TOKENS; ++i) {
+    z[i] = 0.f;
     const float part = warp_sum(k[i] * k[i]);
     if (lane == 0) sums[i * 32 + warp] = part;
   }
@@ -74,20 +94,19 @@ delta_prepare_kernel(Source proj, const void* w2t, const float* w0, const float*
     if (c < D) {
 #pragma unroll 16
       for (int j = 0; j < n; ++j) {
-        const long long at = (long long)(j0 + j) * HD + ch;
-        const float w = load_as(w2t, W, at);
+        const float w = load_as(w2t, W, (long long)(j0 + j) * HD + ch);
         if constexpr (TOKENS == 1) {
           z[0] = __fmaf_rn(w, th[j], z[0]);
+        } else if constexpr (TOKENS == 2) {
+          const float2 y = *reinterpret_cast<const float2*>(th + j * 2);
+          z[0] = __fmaf_rn(w, y.x, z[0]);
+          z[1] = __fmaf_rn(w, y.y, z[1]);
         } else {
-          const float4* x = reinterpret_cast<const float4*>(th + j * TOKENS);
-#pragma unroll
-          for (int q = 0; q < TOKENS / 4; ++q) {
-            const float4 y = x[q];
-            z[4 * q] = __fmaf_rn(w, y.x, z[4 * q]);
-            z[4 * q + 1] = __fmaf_rn(w, y.y, z[4 * q + 1]);
-            z[4 * q + 2] = __fmaf_rn(w, y.z, z[4 * q + 2]);
-            z[4 * q + 3] = __fmaf_rn(w, y.w, z[4 * q + 3]);
-          }
+          const float4 y = *reinterpret_cast<const float4*>(th + j * 4);
+          z[0] = __fmaf_rn(w, y.x, z[0]);
+          z[1] = __fmaf_rn(w, y.y, z[1]);
+          z[2] = __fmaf_rn(w, y.z, z[2]);
+          z[3] = __fmaf_rn(w, y.w, z[3]);
         }
       }
     }
@@ -624,17 +643,22 @@ int dib_delta_prepare(const void* proj, int kind, int splits, long long stride, 
   if (H < 1 || H > 65535 || D < 1 || D > 1024 || R < 0 || R > 8192) return DIB_BAD_SIZE;
   if (w_dtype != 0 && w_dtype != 1) return DIB_BAD_DTYPE;
   const Source src = make_source(proj, kind, splits, stride);
-  auto go = [&](auto tokens) {
+  auto go = [&](auto tokens, auto* kernel) {
     constexpr int N = decltype(tokens)::value;
-    auto* kernel = kind == 1     ? (w_dtype == 1 ? &delta_prepare_kernel<N, 1, 1> : &delta_prepare_kernel<N, 1, 0>)
-                   : splits <= 1 ? (w_dtype == 1 ? &delta_prepare_kernel<N, 0, 1> : &delta_prepare_kernel<N, 0, 0>)
-                                 : (w_dtype == 1 ? &delta_prepare_kernel<N, 2, 1> : &delta_prepare_kernel<N, 2, 0>);
     dib_launch(kernel, dim3(ceil_div_host(T_, N), H), dim3((D + 31) / 32 * 32), 0, st, src, w2t, w0, a_bias, packed, T_,
                H, D, R, decay_scale, key_eps);
   };
+  auto stored = [&](auto tokens) {
+    constexpr int N = decltype(tokens)::value;
+    go(tokens, kind == 1 ? (w_dtype == 1 ? &delta_prepare_kernel<N, 1, 1> : &delta_prepare_kernel<N, 1, 0>)
+                         : (w_dtype == 1 ? &delta_prepare_kernel<N, 0, 1> : &delta_prepare_kernel<N, 0, 0>));
+  };
+  const std::integral_constant<int, 1> one;
+  if (kind != 1 && splits > 1) go(one, w_dtype == 1 ? &delta_prepare_kernel<1, 2, 1> : &delta_prepare_kernel<1, 2, 0>);
   // (heads of more than 256: a block's registers do not reach for the values of several tokens)
-  if (D <= 256) go(std::integral_constant<int, PREP_TOKENS>{});
-  else go(std::integral_constant<int, 1>{});
+  else if (D > 256) stored(one);
+  else if (T_ < PREP_FOUR_FROM) stored(std::integral_constant<int, 2>{});
+  else stored(std::integral_constant<int, 4>{});
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }

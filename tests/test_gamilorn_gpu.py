@@ -359,6 +359,33 @@ def test_the_delta_rules_vectors_of_wide_heads(dim, dtype):
     assert float((got.double() - want).abs().max()) <= (5 * rank + 32) * 2.0 ** -24 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("heads, dim, rank", [(3, 64, 64), (2, 40, 513), (1, 256, 0), (2, 20, 7)])
+def test_the_delta_rules_vectors_in_every_form(heads, dim, rank):
+    """One, two or four tokens a block, by the step's tokens, stored projections of both types and split sums: a token's
+    vectors are those of the token alone, at the edges of the blocks and of the hidden vector's runs; split sums give
+    what their sum in split order gives, and all are 64 bits' up to rounding."""
+    g = torch.Generator(device="cuda").manual_seed(dim + rank)
+    hd, width, n = heads * dim, 5 * heads * dim + rank, 387
+    parts = torch.randn(3, n, width, generator=g, device="cuda")
+    total = (parts[0] + parts[1]) + parts[2]
+    w2_t = torch.randn(rank, hd, generator=g, device="cuda").bfloat16()
+    w0, a_bias = torch.randn(hd, generator=g, device="cuda") - 2, torch.randn(hd, generator=g, device="cuda")
+    run = lambda x: prepared(x, heads, dim, rank, w2_t, w0, a_bias)
+    whole = run(total)
+    want = prepared_in_64_bits(total, heads, dim, rank, w2_t, w0, a_bias)
+    # a chain of `rank` terms of size |w2| <= 5 into the decay; a few roundings elsewhere
+    assert float((whole.double() - want).abs().max()) <= (5 * rank + 32) * 2.0 ** -24 * float(want.abs().max())
+    assert torch.equal(run(parts), whole)
+    for m in (1, 2, 3, 8, 65, 383, 384, 385, 386):
+        assert torch.equal(run(total[:m]), whole[:m]), m
+        assert torch.equal(run(parts[:, :m].contiguous()), whole[:m]), m
+    stored = total.bfloat16()
+    rounded = run(stored)
+    assert torch.equal(rounded, run(stored.float()))
+    for m in (1, 383):
+        assert torch.equal(run(stored[:m]), rounded[:m]), m
+
+
 # ---- whole models through the trace runner -----------------------------------------------------------
 
 CASES = {
