@@ -472,9 +472,11 @@ delta_recurrence_wide_kernel(const float* packed, float* state, long long slot_s
 // A warp per (token, head), 32 elements at a time: the sum of squares is the butterflies' over 32
 // consecutive elements, added in index order.  CHUNKS: how many of them a row has at most (0: any
 // number, read again behind the sum); the gate and the weight are asked for before the sum is made.
-// (2,048 tokens, 16 heads of 64: 10 us; blocks of D threads with a row each: 35 us.)
+// SPLIT: the gate is split sums (decoded tokens), loaded four splits of all its elements at a time.
+// (16 heads of 64, us: 2,048 tokens 8.5, blocks of D threads with a row each 34; 8 tokens of eight splits
+// 2.2, an element's splits at a time 3.0, blocks of D threads 2.3.)
 constexpr int OUT_WARPS = 8;
-template <int CHUNKS>
+template <int CHUNKS, bool SPLIT>
 __global__ void __launch_bounds__(OUT_WARPS * 32)
 delta_output_kernel(const float* o, Source proj, const float* norm_w, void* out, int out_dtype, long long rows,
                     int H, int D, int R, float eps) {
@@ -492,8 +494,13 @@ delta_output_kernel(const float* o, Source proj, const float* norm_w, void* out,
     for (int j = 0; j < CHUNKS; ++j) {
       const int c = 32 * j + lane;
       x[j] = c < D ? o[row * D + c] : 0.f;
-      g[j] = c < D ? source_load(proj, gate + c) : 0.f;
       w[j] = c < D ? norm_w[h * D + c] : 0.f;
+    }
+    if (SPLIT) {
+      source_load_strided<CHUNKS, 4>(proj, gate, lane, 32, D, g);
+    } else {
+#pragma unroll
+      for (int j = 0; j < CHUNKS; ++j) g[j] = 32 * j + lane < D ? source_load(proj, gate + 32 * j + lane) : 0.f;
     }
 #pragma unroll
     for (int j = 0; j < CHUNKS; ++j)
@@ -693,7 +700,9 @@ int dib_delta_output(const float* o, const void* proj, int kind, int splits, lon
   if (H < 1 || H > 65535 || D < 1 || D > 1024) return DIB_BAD_SIZE;
   if (out_dtype != 0 && out_dtype != 1) return DIB_BAD_DTYPE;
   const long long rows = (long long)T_ * H;
-  auto* kernel = D <= 64 ? &delta_output_kernel<2> : D <= 128 ? &delta_output_kernel<4> : &delta_output_kernel<0>;
+  auto* kernel = kind != 1 && splits > 1
+                     ? (D <= 64 ? &delta_output_kernel<2, true> : D <= 128 ? &delta_output_kernel<4, true> : &delta_output_kernel<0, true>)
+                     : (D <= 64 ? &delta_output_kernel<2, false> : D <= 128 ? &delta_output_kernel<4, false> : &delta_output_kernel<0, false>);
   dib_launch(kernel, dim3(ceil_div_host(rows, OUT_WARPS)), dim3(OUT_WARPS * 32), 0, st, o,
              make_source(proj, kind, splits, stride), norm_w, out, out_dtype, rows, H, D, R, eps);
   DIB_CHECK_LAUNCH();

@@ -386,6 +386,38 @@ def test_the_delta_rules_vectors_in_every_form(heads, dim, rank):
         assert torch.equal(run(stored[:m]), rounded[:m]), m
 
 
+@pytest.mark.parametrize("heads, dim", [(16, 64), (3, 20), (2, 128), (1, 100), (2, 200)])
+@pytest.mark.parametrize("splits", [2, 4, 5, 8, 11])
+def test_the_delta_rules_output_from_split_sums(heads, dim, splits):
+    """The gate as split sums gives the bits of their sum in split order, for any number of splits."""
+    from ctypes import c_float, c_int, c_longlong
+
+    from deterministic_inference_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(dim + splits)
+    n, rank, hd = 5, 3, heads * dim
+    parts = torch.randn(splits, n, 5 * hd + rank, generator=g, device="cuda")
+    total = parts[0].clone()
+    for x in parts[1:]:
+        total += x
+    o, norm_w = torch.randn(n, hd, generator=g, device="cuda"), torch.rand(hd, generator=g, device="cuda")
+
+    def run(proj, k):
+        out = torch.full((n, hd), float("nan"), device="cuda")
+        st = ops._lib("delta_rule").dib_delta_output(
+            ops._ptr(o), ops._ptr(proj), c_int(0), c_int(k), c_longlong(total.numel()), ops._ptr(norm_w), ops._ptr(out),
+            c_int(0), c_int(n), c_int(heads), c_int(dim), c_int(rank), c_float(1e-6), ops._stream())
+        assert st == 0, st
+        return out
+
+    got = run(total, 1)
+    assert torch.equal(run(parts, splits), got)
+    x = o.double().view(n, heads, dim)
+    want = (x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6)).reshape(n, hd) * norm_w.double() * \
+        torch.sigmoid(total[:, 3 * hd:4 * hd].double())
+    # a norm over up to 200 elements and a few roundings
+    assert float((got.double() - want).abs().max()) <= (dim / 2 + 16) * 2.0 ** -24 * float(want.abs().max())
+
+
 # ---- whole models through the trace runner -----------------------------------------------------------
 
 CASES = {
