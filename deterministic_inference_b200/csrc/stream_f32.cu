@@ -639,7 +639,11 @@ int dib_xielu(const void* z, int kind, int splits, long long stride, float ap, f
   if (n == 0) return DIB_OK;
   if (out_dtype != 0 && out_dtype != 1) return DIB_BAD_DTYPE;
   const Source src = make_source(z, kind, splits, stride);
-  if (n % 4 == 0 && source_takes_vectors(src) && vectors_start_at(out, out_dtype))
+  // (a few rows: one element a thread keeps more loads in flight.  Rows of 3,072, one / four elements a thread in us:
+  // split sums of eight, 8 rows 1.7 / 2.1, 32 rows 2.3 / 2.3, 64 rows 2.8 / 3.0; stored, 8 rows 1.33 / 1.43, 16 rows
+  // 1.54 / 1.43, 64 rows 2.2 / 1.9, 2,048 rows 14.2 / 11.6)
+  const bool many = n >= (kind != 1 && splits > 1 ? 148 * 2048 * 4 : 148 * 256);
+  if (many && n % 4 == 0 && source_takes_vectors(src) && vectors_start_at(out, out_dtype))
     dib_launch(xielu_kernel<true>, dim3(flat_grid(n / 4, 256)), dim3(256), 0, st, src, ap, an, out, out_dtype, n);
   else
     dib_launch(xielu_kernel<false>, dim3(flat_grid(n, 256)), dim3(256), 0, st, src, ap, an, out, out_dtype, n);

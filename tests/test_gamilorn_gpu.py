@@ -73,7 +73,8 @@ def test_stream_kernels_alone(dtype):
 
 
 @pytest.mark.parametrize("dtype", list(DTYPES))
-@pytest.mark.parametrize("rows, width, splits", [(3, 4, 1), (5, 132, 3), (2048, 12, 1), (700, 2052, 1)])
+@pytest.mark.parametrize("rows, width, splits", [(3, 4, 1), (5, 132, 3), (2048, 12, 1), (700, 2052, 1), (148, 256, 1),
+                                                 (400, 3072, 2)])
 def test_elements_by_fours_are_those_one_by_one(dtype, rows, width, splits):
     """The element-wise kernels on memory that allows vectors of four and on the same values one element further on,
     which does not: the same bits."""
