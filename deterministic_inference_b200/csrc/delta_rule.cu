@@ -263,20 +263,23 @@ delta_recurrence_kernel(const float* packed, float* state, long long slot_stride
 // columns).  The form for steps with few sequences and many tokens (prompt portions): few warps a
 // scheduler, so a token takes what its instructions and the chain from its state to the next one's
 // take (the row sum's FMA, four exchanges between lanes, one FMA).  Nothing else stands in that
-// chain: a token's vectors are in registers before (the next token's are read while this one is
-// worked on), w S + k v is ready when the sum arrives, and the output's exchanges run one token
+// chain: a token's vectors are in registers before, w S + k v is ready when the sum arrives, and the output's exchanges run one token
 // behind, side by side with the sum's.  One more warp brings the vectors into shared memory,
 // DR_TOKENS tokens at a time, one group ahead, with one barrier a group; strides are constants of
 // the instance (D and E padded with zeros to LANES * MAXR).  Its sums are ordered differently from
 // the form above (four chains by e, then a butterfly over 16 lanes), again by D alone.
-// (2,048 tokens, 16 heads of 64: 245 us, rows over 8 lanes 344, over 4 649 us; 16 heads of 128: 450 us;
-// 512 tokens, 8 heads of 256: 271 us.  Copies by the warps that compute, a barrier a token and both
-// exchanges in the chain: 878, 1,013 and 356 us.)
+// NEXT: the next token's vectors are read while one is worked on; not with D or E above 128, where two
+// tokens' take all registers there are and half as many warps fit an SM (4 heads of 256, 8 x 64 tokens:
+// 140 us, read in their turn 103; 16 heads of 200, 16 x 64 tokens: 783 and 554; one sequence of 256
+// tokens, 4 heads of 256: 132 and 125).
+// (2,048 tokens, 16 heads of 64: 230 us, rows over 8 lanes 344, over 4 649 us; 8 heads of 128: 412 us;
+// 4 heads of 256: 968 us.  Copies by the warps that compute, a barrier a token and both exchanges in the
+// chain: 864, 907 and 1,102 us; 16 x 64 tokens, 16 heads of 200: 646 us.)
 template <int Q, int CPT> struct DeltaToken {      // a lane's part of a token's vectors
   float4 w[Q], b[Q], u[Q], k[Q], r[Q];
   float v[CPT];
 };
-template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES>
+template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES, bool NEXT>
 __global__ void __launch_bounds__(32 * WARPS + 32)
 delta_recurrence_wide_kernel(const float* packed, float* state, long long slot_stride, float* o_out,
                              const int* cu_q_lens, const int* state_slots, int H, int D, int E) {
@@ -435,9 +438,9 @@ delta_recurrence_wide_kernel(const float* packed, float* state, long long slot_s
   for (int g = 0; g < groups; ++g) {
     __syncthreads();
     const int at = (g % DR_STAGES) * DR_TOKENS * SV;
-    const int n = t1 - t0 - g * DR_TOKENS;
+    const int n = min(t1 - t0 - g * DR_TOKENS, DR_TOKENS);
     DeltaToken<Q, CPT> x, y;
-    if (n < DR_TOKENS) {
+    if (!NEXT || n < DR_TOKENS) {
 #pragma unroll 1
       for (int i = 0; i < n; ++i) {
         read(at + i * SV, x);
@@ -614,13 +617,13 @@ static int launch_recurrence(const float* packed, float* state, long long slot_s
   return DIB_OK;
 }
 
-template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES>
+template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES, bool NEXT>
 static int launch_recurrence_wide(const float* packed, float* state, long long slot_stride, float* o_out,
                                   const int* cu_q_lens, const int* state_slots, int B, int H, int D, int E,
                                   cudaStream_t st) {
   constexpr int COLUMNS = 32 / LANES * CPT * WARPS;        // a block's
   constexpr size_t smem = sizeof(float) * DR_STAGES * DR_TOKENS * 6 * LANES * MAXR;    // 48 KB for 64, 96 for 128 and 256
-  auto* kernel = &delta_recurrence_wide_kernel<MAXR, LANES, CPT, WARPS, DR_TOKENS, DR_STAGES>;
+  auto* kernel = &delta_recurrence_wide_kernel<MAXR, LANES, CPT, WARPS, DR_TOKENS, DR_STAGES, NEXT>;
   static DeviceOnce once;
   if (!once.done()) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -683,9 +686,9 @@ int dib_delta_recurrence(const float* packed, float* state, long long slot_strid
   const int big = D > E ? D : E;       // (the staging's pieces are counted for the larger of the two)
 #define DIB_DR(F, ...) return F<__VA_ARGS__>(packed, state, slot_stride, o_out, cu_q_lens, state_slots, B, H, D, E, st)
   if (form == 1) {
-    if (big <= 64) DIB_DR(launch_recurrence_wide, 4, 16, 1, 4, 16, 2);
-    if (big <= 128) DIB_DR(launch_recurrence_wide, 8, 16, 2, 4, 16, 2);
-    DIB_DR(launch_recurrence_wide, 16, 16, 2, 4, 8, 2);
+    if (big <= 64) DIB_DR(launch_recurrence_wide, 4, 16, 1, 4, 16, 2, true);
+    if (big <= 128) DIB_DR(launch_recurrence_wide, 8, 16, 2, 4, 16, 2, true);
+    DIB_DR(launch_recurrence_wide, 16, 16, 2, 4, 8, 2, false);
   }
   if (big <= 64) DIB_DR(launch_recurrence, 16, 8);
   if (big <= 128) DIB_DR(launch_recurrence, 32, 6);
