@@ -56,14 +56,132 @@ __device__ __forceinline__ float turned(Get get, int d, int rot, float pos, cons
 // ---- token by token --------------------------------------------------------------------------------
 // VEC columns a thread (4 where P is a multiple of 4).  Thread (rg, cg) has the rows rg, rg + RG, ...
 // of column group cg; a column's read-out adds a thread's rows in ascending order and then the RG
-// shares in order: the order depends on N and P alone.  in_smem: the state lives in shared memory
+// shares in order, the norm's sum of squares 32 consecutive columns by a butterfly and then those in
+// order: the orders depend on N and P alone.  in_smem: the state lives in shared memory
 // while the sequence's tokens are walked (else in the slot; a sequence on slot 0 then forgets
 // each token).
-// The columns are cut over the blocks of a cluster (gridDim.z of them, by P alone), which exchange only
-// their shares of the norm's sum of squares: a state of 128 x 256 moves through four SMs instead of one.
-// (8 sequences, 8 heads of 128 x 256, a token each: 10.3 us; a block a head: 12.6 us.)
-constexpr int ST = 256;
-__host__ __device__ __forceinline__ int step_blocks(int P) { return P >= 128 && P % 16 == 0 ? 4 : 1; }
+constexpr int ST = 256, MOST_COLUMNS = 4096;
+constexpr int PARTS = 4;               // blocks of a cluster, each with a part of a head's columns
+__host__ __device__ __forceinline__ bool in_parts(int P) { return P >= 256 && P % (32 * PARTS) == 0; }
+// column groups side by side (CG): a part's where heads may be cut into parts, else as many as there are
+template <int VEC> __host__ __device__ __forceinline__ int column_groups(int P) {
+  if (VEC == 4 && in_parts(P)) return P / (4 * PARTS);
+  return P / VEC < ST ? P / VEC : ST;
+}
+// o[c], the RG shares of column c in order, for this block's columns, and their squares' sums by 32
+__device__ __forceinline__ void read_out(const float* part, int pp, int RG, int columns, float* os, float* squares) {
+  for (int c0 = 0; c0 < columns; c0 += ST) {
+    const int c = c0 + threadIdx.x;
+    float o = 0.f;
+    if (c < columns) {
+      o = part[c];
+      for (int r = 1; r < RG; ++r) o = __fadd_rn(o, part[r * pp + c]);
+      os[c] = o;
+    }
+    const float ss = warp_sum(o * o);
+    if ((threadIdx.x & 31) == 0 && c < columns) squares[c >> 5] = ss;
+  }
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(ST)
+retention_step_kernel(Source proj, long long row_width, const float* __restrict__ decay, const float* __restrict__ freq,
+                      int rot, const int* __restrict__ positions, float* state, long long slot_stride,
+                      const int* __restrict__ cu_q_lens, const int* __restrict__ state_slots, void* out, int out_dtype,
+                      int H, int N, int P, float k_scale, float eps, int in_smem) {
+  using V = typename Cols<VEC>::T;
+  extern __shared__ __align__(16) float rs_smem[];   // q [N], k [N], v [P], o [P], shares [RG][P], state [N][P] (in_smem)
+  __shared__ float squares[MOST_COLUMNS / 32];
+  pdl_prologue(proj.p, state);
+  const int b = blockIdx.x, h = blockIdx.y;
+  const int t0 = cu_q_lens[b], n_tok = cu_q_lens[b + 1] - t0;
+  if (n_tok <= 0) return;
+  const long long slot = state_slots[b];
+  const int np = (N + 3) / 4 * 4, pp = (P + 3) / 4 * 4;
+  float* qs = rs_smem;
+  float* ks = qs + np;
+  float* vs = ks + np;
+  float* os = vs + pp;
+  float* part = os + pp;
+  const int cols = P / VEC;
+  const int CG = column_groups<VEC>(P), RG = ST / CG;
+  const int cg = threadIdx.x % CG, rg = threadIdx.x / CG;
+  float* sm_state = part + RG * pp;
+  float* srow = state + slot * slot_stride + (long long)h * N * P;
+  const float d = decay[h];
+  const bool bf = out_dtype == 1;
+  const long long qc = (long long)h * N, kc = (long long)(H + h) * N, vc = 2ll * H * N + (long long)h * P,
+                  gc = vc + (long long)H * P;
+  auto load = [&](long long at) {
+    const float x = source_load(proj, at);
+    return bf ? round_to<__nv_bfloat16>(x) : x;
+  };
+  if (in_smem) {
+    for (int i = threadIdx.x; i < N * P; i += ST) sm_state[i] = slot != 0 ? srow[i] : 0.f;
+    __syncthreads();
+  }
+  V* S = reinterpret_cast<V*>(in_smem ? sm_state : srow);
+  const bool keeps = in_smem || slot != 0;
+  for (int k = 0; k < n_tok; ++k) {
+    const int t = t0 + k;
+    const long long row = (long long)t * row_width;
+    const float pos = (float)positions[t];
+    for (int i = threadIdx.x; i < 2 * N; i += ST) {
+      const bool is_k = i >= N;
+      const int e = is_k ? i - N : i;
+      const long long at = row + (is_k ? kc : qc);
+      const float x = turned([&](int j) { return load(at + j); }, e, rot, pos, freq);
+      if (is_k) ks[e] = __fmul_rn(x, k_scale);
+      else qs[e] = x;
+    }
+    for (int i = threadIdx.x; i < P; i += ST) vs[i] = load(row + vc + i);
+    __syncthreads();
+    if (rg < RG)
+      for (int c = cg; c < cols; c += CG) {
+        const V v = reinterpret_cast<const V*>(vs)[c];
+        V acc = {};
+        constexpr int AHEAD = 8;         // rows whose loads are issued before the first is used
+        for (int r0 = rg; r0 < N; r0 += AHEAD * RG) {
+          V s[AHEAD];
+#pragma unroll
+          for (int u = 0; u < AHEAD; ++u) {
+            const int r = r0 + u * RG;
+            if (r < N && keeps) s[u] = S[(long long)r * cols + c];
+            else s[u] = V{};
+          }
+#pragma unroll
+          for (int u = 0; u < AHEAD; ++u) {
+            const int r = r0 + u * RG;
+            if (r < N) {
+              col_step(s[u], acc, d, ks[r], qs[r], v);
+              if (keeps) S[(long long)r * cols + c] = s[u];
+            }
+          }
+        }
+        reinterpret_cast<V*>(part + rg * pp)[c] = acc;
+      }
+    __syncthreads();
+    read_out(part, pp, RG, P, os, squares);
+    __syncthreads();
+    float total = 0.f;
+    for (int g = 0; g < (P + 31) / 32; ++g) total = __fadd_rn(total, squares[g]);
+    const float rstd = 1.0f / sqrtf(total / (float)P + eps);
+    for (int c = threadIdx.x; c < P; c += ST) {
+      const float g = load(row + gc + c);
+      store_as(out, out_dtype, (long long)t * H * P + (long long)h * P + c, os[c] * rstd * (g * sigmoid_f32(g)));
+    }
+    __syncthreads();
+  }
+  if (in_smem && slot != 0)
+    for (int i = threadIdx.x; i < N * P; i += ST) srow[i] = sm_state[i];
+}
+
+// The same for few (sequence, head) pairs, with a head's columns over the four blocks of a cluster, which
+// exchange their sums of squares: a state of 128 x 256 moves through four SMs instead of one, and a
+// thread's first rows are asked for before q and k are made.  Every order is that of the kernel above.
+// (Heads of 128 x 256, a token each, cluster / block in us: 8 heads 6.0 / 7.7, 64 heads 7.1 / 9.2, 96 heads,
+// whose 384 blocks run two after the other, 13.2 / 9.4, 512 heads 51 / 20; 2 heads of 256 x 512 9.3 / 18.8.)
+constexpr int CLUSTER_HEADS = 64;      // pairs up to which a step takes this form: all their blocks run at once
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -76,34 +194,30 @@ __device__ __forceinline__ float of_block(const float* p, int rank) {      // *p
   return v;
 }
 
-template <int VEC>
 __global__ void __launch_bounds__(ST)
-retention_step_kernel(Source proj, long long row_width, const float* __restrict__ decay, const float* __restrict__ freq,
-                      int rot, const int* __restrict__ positions, float* state, long long slot_stride,
-                      const int* __restrict__ cu_q_lens, const int* __restrict__ state_slots, void* out, int out_dtype,
-                      int H, int N, int P, float k_scale, float eps, int in_smem) {
-  using V = typename Cols<VEC>::T;
-  extern __shared__ __align__(16) float rs_smem[];   // q [N], k [N], v [P], o [P], shares [RG][P], state [N][P] (in_smem)
-  __shared__ float scratch[32];
-  __shared__ float squares[2];                       // of even and of odd tokens, this block's columns
+retention_step_cluster_kernel(Source proj, long long row_width, const float* __restrict__ decay,
+                              const float* __restrict__ freq, int rot, const int* __restrict__ positions, float* state,
+                              long long slot_stride, const int* __restrict__ cu_q_lens,
+                              const int* __restrict__ state_slots, void* out, int out_dtype, int H, int N, int P,
+                              float k_scale, float eps, int in_smem) {
+  extern __shared__ __align__(16) float rs_smem[];   // q [N], k [N], v [PB], o [PB], shares [RG][PB], state [N][PB] (in_smem)
+  __shared__ float squares[2][MOST_COLUMNS / PARTS / 32];      // of even and of odd tokens, this block's columns
   pdl_prologue(proj.p, state);
-  const int blocks = gridDim.z, rank = blockIdx.z;   // (the cluster's shape is 1, 1, blocks)
-  const int PB = P / blocks, c0 = rank * PB;         // this block's columns
+  const int rank = blockIdx.z, PB = P / PARTS, c0 = rank * PB;         // this block's columns (a multiple of 32)
   const int b = blockIdx.x, h = blockIdx.y;
   const int t0 = cu_q_lens[b], n_tok = cu_q_lens[b + 1] - t0;
-  if (n_tok <= 0) return;
+  if (n_tok <= 0) return;                            // (the whole cluster)
   const long long slot = state_slots[b];
-  const int np = (N + 3) / 4 * 4, pp = (PB + 3) / 4 * 4;
+  const int np = (N + 3) / 4 * 4;
   float* qs = rs_smem;
   float* ks = qs + np;
   float* vs = ks + np;
-  float* os = vs + pp;
-  float* part = os + pp;
-  const int cols = PB / VEC, row_cols = (in_smem ? PB : P) / VEC;       // in units of V: a block's, a state row's
-  const int CG = cols < ST ? cols : ST, RG = ST / CG;
+  float* os = vs + PB;
+  float* part = os + PB;
+  const int CG = column_groups<4>(P), RG = ST / CG;
   const int cg = threadIdx.x % CG, rg = threadIdx.x / CG;
-  float* sm_state = part + RG * pp;
-  float* srow = state + slot * slot_stride + (long long)h * N * P;
+  float* sm_state = part + RG * PB;
+  float* srow = state + slot * slot_stride + (long long)h * N * P + c0;
   const float d = decay[h];
   const bool bf = out_dtype == 1;
   const long long qc = (long long)h * N, kc = (long long)(H + h) * N, vc = 2ll * H * N + (long long)h * P + c0,
@@ -113,23 +227,26 @@ retention_step_kernel(Source proj, long long row_width, const float* __restrict_
     return bf ? round_to<__nv_bfloat16>(x) : x;
   };
   if (in_smem) {
-    for (int i = threadIdx.x; i < N * PB; i += ST) sm_state[i] = slot != 0 ? srow[(long long)(i / PB) * P + c0 + i % PB] : 0.f;
+    for (int i = threadIdx.x; i < N * PB; i += ST) sm_state[i] = slot != 0 ? srow[(long long)(i / PB) * P + i % PB] : 0.f;
     __syncthreads();
   }
-  V* S = reinterpret_cast<V*>(in_smem ? sm_state : srow + c0);
+  float4* S = reinterpret_cast<float4*>(in_smem ? sm_state : srow);
+  const long long row_step = (in_smem ? PB : P) / 4;
   const bool keeps = in_smem || slot != 0;
   for (int k = 0; k < n_tok; ++k) {
     const int t = t0 + k;
     const long long row = (long long)t * row_width;
     const float pos = (float)positions[t];
     constexpr int AHEAD = 8;         // rows whose loads are issued before the first is used
-    V first[AHEAD];                  // (the first ones before q and k are made)
+    float4 s[AHEAD];
+    auto rows = [&](int r0) {
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      const int r = rg + u * RG;
-      if (rg < RG && cg < cols && r < N && keeps) first[u] = S[(long long)r * row_cols + cg];
-      else first[u] = V{};
-    }
+      for (int u = 0; u < AHEAD; ++u) {
+        const int r = r0 + u * RG;
+        s[u] = r < N && keeps ? S[r * row_step + cg] : float4{};
+      }
+    };
+    if (rg < RG) rows(rg);           // (the first ones before q and k are made)
     for (int i = threadIdx.x; i < 2 * N; i += ST) {
       const bool is_k = i >= N;
       const int e = is_k ? i - N : i;
@@ -140,45 +257,28 @@ retention_step_kernel(Source proj, long long row_width, const float* __restrict_
     }
     for (int i = threadIdx.x; i < PB; i += ST) vs[i] = load(row + vc + i);
     __syncthreads();
-    if (rg < RG)
-      for (int c = cg; c < cols; c += CG) {
-        const V v = reinterpret_cast<const V*>(vs)[c];
-        V acc = {};
-        for (int r0 = rg; r0 < N; r0 += AHEAD * RG) {
-          V s[AHEAD];
+    if (rg < RG) {
+      const float4 v = reinterpret_cast<const float4*>(vs)[cg];
+      float4 acc = {};
+      for (int r0 = rg; r0 < N; r0 += AHEAD * RG) {
+        if (r0 != rg) rows(r0);
 #pragma unroll
-          for (int u = 0; u < AHEAD; ++u) {
-            const int r = r0 + u * RG;
-            if (r0 == rg && c == cg) s[u] = first[u];
-            else if (r < N && keeps) s[u] = S[(long long)r * row_cols + c];
-            else s[u] = V{};
-          }
-#pragma unroll
-          for (int u = 0; u < AHEAD; ++u) {
-            const int r = r0 + u * RG;
-            if (r < N) {
-              col_step(s[u], acc, d, ks[r], qs[r], v);
-              if (keeps) S[(long long)r * row_cols + c] = s[u];
-            }
+        for (int u = 0; u < AHEAD; ++u) {
+          const int r = r0 + u * RG;
+          if (r < N) {
+            col_step(s[u], acc, d, ks[r], qs[r], v);
+            if (keeps) S[r * row_step + cg] = s[u];
           }
         }
-        reinterpret_cast<V*>(part + rg * pp)[c] = acc;
       }
+      reinterpret_cast<float4*>(part + rg * PB)[cg] = acc;
+    }
     __syncthreads();
-    float ss = 0.f;
-    for (int c = threadIdx.x; c < PB; c += ST) {
-      float o = part[c];
-      for (int r = 1; r < RG; ++r) o = __fadd_rn(o, part[r * pp + c]);
-      os[c] = o;
-      ss = __fmaf_rn(o, o, ss);
-    }
-    float total = block_sum(ss, scratch);
-    if (blocks > 1) {                      // the blocks' shares in their order
-      if (threadIdx.x == 0) squares[k & 1] = total;
-      cluster_barrier();
-      total = of_block(&squares[k & 1], 0);
-      for (int z = 1; z < blocks; ++z) total = __fadd_rn(total, of_block(&squares[k & 1], z));
-    }
+    read_out(part, PB, RG, PB, os, squares[k & 1]);
+    cluster_barrier();
+    float total = 0.f;
+    for (int z = 0; z < PARTS; ++z)
+      for (int g = 0; g < PB / 32; ++g) total = __fadd_rn(total, of_block(&squares[k & 1][g], z));
     const float rstd = 1.0f / sqrtf(total / (float)P + eps);
     for (int c = threadIdx.x; c < PB; c += ST) {
       const float g = load(row + gc + c);
@@ -187,8 +287,8 @@ retention_step_kernel(Source proj, long long row_width, const float* __restrict_
     __syncthreads();
   }
   if (in_smem && slot != 0)
-    for (int i = threadIdx.x; i < N * PB; i += ST) srow[(long long)(i / PB) * P + c0 + i % PB] = sm_state[i];
-  if (blocks > 1) cluster_barrier();       // nobody reads this block's shares any more
+    for (int i = threadIdx.x; i < N * PB; i += ST) srow[(long long)(i / PB) * P + i % PB] = sm_state[i];
+  cluster_barrier();                 // nobody reads this block's sums any more
 }
 
 // ---- chunks ----------------------------------------------------------------------------------------
@@ -617,30 +717,38 @@ int dib_retention_step(const void* proj, int kind, int splits, long long stride,
                        const int* cu_q_lens, const int* state_slots, void* out, int out_dtype, int B, int H, int N, int P,
                        float k_scale, float eps, int in_smem, cudaStream_t st) {
   if (B == 0) return DIB_OK;
-  if (H < 1 || H > 65535 || N < 1 || N > 2048 || P < 1 || P > 4096 || rot < 0 || rot > N || rot % 2 ||
+  if (H < 1 || H > 65535 || N < 1 || N > 2048 || P < 1 || P > MOST_COLUMNS || rot < 0 || rot > N || rot % 2 ||
       (rot > 0 && freq == nullptr) || row_width < 2ll * H * (N + P) || slot_stride < (long long)H * N * P)
     return DIB_BAD_SIZE;
   if (out_dtype != 0 && out_dtype != 1) return DIB_BAD_DTYPE;
   const bool v4 = P % 4 == 0 && slot_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(state) & 15) == 0;
-  const int blocks = v4 ? step_blocks(P) : 1, PB = P / blocks;
-  auto smem_of = [&](int columns) {
-    const int cols = v4 ? columns / 4 : columns, CG = cols < ST ? cols : ST, RG = ST / CG;
-    const size_t np = (N + 3) / 4 * 4, pp = (columns + 3) / 4 * 4;
-    return sizeof(float) * (2 * np + 2 * pp + (size_t)RG * pp + (in_smem ? (size_t)N * columns : 0));
+  const int np = (N + 3) / 4 * 4, pp = (P + 3) / 4 * 4;
+  auto smem_of = [&](int CG, int columns) {
+    return sizeof(float) * (2 * (size_t)np + 2 * (size_t)columns + (size_t)(ST / CG) * columns + (in_smem ? (size_t)N * columns : 0));
   };
-  const size_t smem = smem_of(PB);
-  if (smem_of(P) > MOST_SMEM) return DIB_BAD_SIZE;         // (the limit is that of a whole head in one block)
+  const int cols = v4 ? P / 4 : P;
+  if (smem_of(cols < ST ? cols : ST, pp) > MOST_SMEM) return DIB_BAD_SIZE;
+  const int CG = v4 ? column_groups<4>(P) : column_groups<1>(P);
   const Source src = make_source(proj, kind, splits, stride);
-  static DeviceOnce once4, once1;
-  DeviceOnce& once = v4 ? once4 : once1;
-  auto kern = v4 ? retention_step_kernel<4> : retention_step_kernel<1>;
+  // (a whole head in parts needs more memory for its shares; where it does not fit a cluster's quarter does)
+  const bool cluster = v4 && in_parts(P) && ((long long)B * H <= CLUSTER_HEADS || smem_of(CG, pp) > MOST_SMEM);
+  const size_t smem = smem_of(CG, cluster ? P / PARTS : pp);
+  static DeviceOnce once4, once1, once_cluster;
+  DeviceOnce& once = cluster ? once_cluster : v4 ? once4 : once1;
+  auto kern = cluster ? retention_step_cluster_kernel : v4 ? retention_step_kernel<4> : retention_step_kernel<1>;
   if (!once.done()) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM) != cudaSuccess)
       return DIB_LAUNCH_FAILED;
     once.mark();
   }
+  if (!cluster) {
+    dib_launch(kern, dim3(B, H), dim3(ST), smem, st, src, row_width, decay, freq, rot, positions, state, slot_stride,
+               cu_q_lens, state_slots, out, out_dtype, H, N, P, k_scale, eps, in_smem);
+    DIB_CHECK_LAUNCH();
+    return DIB_OK;
+  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(B, H, blocks);
+  cfg.gridDim = dim3(B, H, PARTS);
   cfg.blockDim = dim3(ST);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -648,7 +756,7 @@ int dib_retention_step(const void* proj, int kind, int splits, long long stride,
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 1;
   attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = blocks;
+  attr[0].val.clusterDim.z = PARTS;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;

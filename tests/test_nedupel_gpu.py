@@ -52,11 +52,63 @@ def test_retention_alone(tmp_path, dtype, dim, vdim, decay, rot):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("dim, vdim, decay, rot", [
-    (24, 144, (0.99, 0.9), 8),                # a head's columns over four blocks, 36 each
-    (128, 256, (0.995,), 128),                # every thread's rows in one run of loads
+    (24, 144, (0.99, 0.9), 8),                # a block of its own
+    (128, 256, (0.995,), 128),                # four blocks; every thread's rows in one run of loads
+    (24, 272, (0.99, 0.9), 8),                # many columns, no multiple of 128: a block
+    (24, 384, (0.99, 0.9), 8),                # a head's columns over four blocks, 96 each
 ])
 def test_retention_over_a_cluster(tmp_path, dtype, dim, vdim, decay, rot):
     nm.retention_case(tmp_path, dtype, "cuda", dim, vdim, decay, rot)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads, dim, vdim", [(2, 24, 384), (8, 128, 256), (1, 40, 512), (2, 16, 1024), (2, 24, 272),
+                                              (4, 64, 128)])
+def test_retention_of_many_decoded_tokens_has_one_tokens_bits(dtype, heads, dim, vdim):
+    """A head's columns over a cluster (few sequences) or in one block (many): outputs and states of the first sequences
+    are equal in every bit."""
+    from types import SimpleNamespace
+
+    from deterministic_inference_b200.kernels import ops
+    dt = {"float32": torch.float32, "bfloat16": torch.bfloat16}[dtype]
+    g = torch.Generator(device="cuda").manual_seed(vdim)
+    n = 150 // heads + 3
+    i32 = lambda x: torch.tensor(list(x), dtype=torch.int32, device="cuda")
+    proj = torch.randn(n, 2 * heads * (dim + vdim), generator=g, device="cuda").to(dt)
+    decay, freq = torch.rand(heads, generator=g, device="cuda"), torch.rand(4, generator=g, device="cuda")
+    before = torch.randn(n + 1, heads * dim * vdim, generator=g, device="cuda")
+    runs = []
+    for count in (n, 3):
+        state = before.clone()
+        step = SimpleNamespace(num_seqs=count, num_decode=count, positions=i32(range(7, 7 + count)),
+                               cu_q_lens=i32(range(count + 1)), state_slots=i32(range(1, count + 1)))
+        out = ops.retention(proj[:count], decay, freq, state, step, heads, dim, vdim, 1e-6, dt)
+        runs.append((out[:3], state[:4]))
+    assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
+
+
+@pytest.mark.parametrize("dim", [120, 206])         # the shares of four parts fit a block beside the state, or do not
+def test_retention_of_many_portions_has_one_portions_bits(dim):
+    """float32 portions, walked with the state in shared memory, of one sequence and of nine (72 heads)."""
+    from types import SimpleNamespace
+
+    from deterministic_inference_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    heads, vdim, n = 8, 256, 3
+    i32 = lambda x: torch.tensor(list(x), dtype=torch.int32, device="cuda")
+    assert ops._lib("retention").dib_retention_state_fits(dim, vdim) == 1
+    proj = torch.randn(9 * n, 2 * heads * (dim + vdim), generator=g, device="cuda")
+    decay, freq = torch.rand(heads, generator=g, device="cuda"), torch.rand(4, generator=g, device="cuda")
+    before = torch.randn(10, heads * dim * vdim, generator=g, device="cuda")
+    runs = []
+    for count in (9, 1):
+        state = before.clone()
+        step = SimpleNamespace(num_seqs=count, num_decode=0, positions=i32(list(range(n)) * count),
+                               cu_q_lens=i32(range(0, n * count + 1, n)), state_slots=i32(range(1, count + 1)))
+        out = ops.retention(proj[:n * count], decay, freq, state, step, heads, dim, vdim, 1e-6, torch.float32)
+        runs.append((out[:n], state[:2]))
+    assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
+
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
