@@ -287,9 +287,10 @@ moe_product_mma_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __re
       *reinterpret_cast<uint4*>(As + r * as + c8 * 8) = v;
     }
     __syncthreads();
-    // The weight loads of AHEAD steps are issued before the first step's products.  No load has a
-    // condition: past the run's end it reads the row's first elements, which meet the zeros staged there.
-    constexpr int AHEAD = 2;
+    // The weight loads of AHEAD steps are issued before the first step's products (tiles of 16 rows are
+    // bound by the loads in flight).  No load has a condition: past the run's end it reads the row's
+    // first elements, which meet the zeros staged there.
+    constexpr int AHEAD = MT == 1 ? 16 / NJ : 2;
     for (int k0 = 0; k0 < kpad; k0 += 32 * AHEAD) {
       uint4 b[AHEAD][NJ];
 #pragma unroll
@@ -355,15 +356,13 @@ moe_product_mma_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __re
     }
 }
 
-// The same for tiles of 16 rows (decoded tokens), where an expert's weights are read for a few rows
+// The same for few tiles of 16 rows (decoded tokens), where an expert's weights are read for a few rows
 // and the time is that of their bytes.  A CTA takes 32 rows of B (mode 0: 16 of the gate and the same
 // 16 of up), a warp 8 of them, and brings them and the tile's A rows into shared memory in runs of
 // ST_K k, ST_STAGES - 1 runs ahead by asynchronous copies of whole 512-byte pieces of a row: at
 // K = 1024 all of a CTA's 64 KB are asked for at once, by two CTAs an SM, while others multiply.  A
-// row's sum is the same as above: steps of 32 k, ascending, in the same permutation.
-// (8 tokens, 2 of 16 experts each, 1024 x 1536, 66 MB and 33 MB of weights: gate and up 22 .. 27 us, down
-// 13 .. 15 us; weights loaded into registers 16 loads ahead, four warps of 32 columns a CTA: 50 and
-// 59 .. 75 us.)
+// row's sum is the same as above: steps of 32 k, ascending, in the same permutation.  (Which of the two
+// runs, and what both take: product_times.)
 constexpr int ST_THREADS = 128, ST_B = 32, ST_A = 16, ST_K = 256, ST_STAGES = 4;
 constexpr int ST_LD = ST_K + GP_PAD;
 constexpr int ST_STAGE = (ST_B + ST_A) * ST_LD;                    // elements
@@ -562,9 +561,9 @@ __global__ void moe_combine_kernel(const float* __restrict__ per_pair, const flo
 template <int MT, int NJ>
 int launch_product_mma(const void* a_rows, const int* order, int max_tiles, int tile, int top, const void* w, void* out,
                        int K, int N, int mode, float limit, float alpha, cudaStream_t st) {
-  // the A rows' k are staged in runs of KC (a multiple of 64) that fit 64 KB.  The runs do not change the
-  // order of a sum.
-  int KC = (64 * 1024 / (MT * 16 * 2) - GP_PAD) / 64 * 64;
+  // the A rows' k are staged in runs of KC (a multiple of 64) that fit 64 KB; tiles of 16 rows in runs that
+  // fit 16 KB, so that an SM holds many CTAs.  The runs do not change the order of a sum.
+  int KC = ((MT == 1 ? 16 : 64) * 1024 / (MT * 16 * 2) - GP_PAD) / 64 * 64;
   if (KC > (K + 63) / 64 * 64) KC = (K + 63) / 64 * 64;
   const size_t smem = (size_t)MT * 16 * (KC + GP_PAD) * 2;
   static DeviceOnce once;
@@ -599,13 +598,33 @@ int launch_product_stream(const void* a_rows, const int* order, int max_tiles, i
   return DIB_OK;
 }
 
-// mode 0: gate and up; 1: down; 2: up alone.  dtype 0 float32, 1 bfloat16.
-int moe_product(const void* a_rows, int dtype, const int* order, int max_tiles, int tile, int top, const void* w,
-                void* out, int K, int N, int mode, float limit, float alpha, cudaStream_t st) {
+// Tiles of 16 rows: streamed weights for few tiles, whose other form has too few CTAs to fill the GPU and walks all
+// of K in one chain; that form for many, where its CTAs (four times as many an SM) hide one another's start and
+// end.  Both give the same bits.  The times are fits to single products, in us with weights from memory (registers /
+// streamed): 16 experts of 1,024 x 1,536, 8 tokens, up 20 / 19, down 24 / 10, 33 tokens 25 / 31 and 28 / 15; 64 of
+// 2,048 x 512, 4 tokens 37 / 31 and 14 / 22, 64 tokens 57 / 63 and 31 / 49; 8 of 4,096 x 4,096, 8 tokens 87 / 84 and
+// 71 / 43; 128 of 2,048 x 768, 64 tokens 145 / 182 and 78 / 107; 512 of 512 x 256, 64 tokens 40 / 80 and 19 / 55.  A
+// layer's two products take the same form: one behind the other they are slower in two forms than in either (sort
+// to combine, 16 experts of 1,024 x 1,536, 33 tokens: registers 58, streamed 50, up streamed 98, down streamed 68;
+// 64 of 2,048 x 512, 64 tokens: 94, 119, 122, 152).
+void product_times(int tiles, int K, int rows_b, float& registers, float& streamed) {
+  const float megabytes = 2e-6f * tiles * (float)K * (float)rows_b;
+  const float waves = (float)tiles * ((rows_b + ST_B - 1) / ST_B) / (2 * 148);
+  const float chain = 1.0f + 0.0137f * K + megabytes / 10.5f, bytes = 3.0f + megabytes / 5.0f;
+  streamed += (waves > 1.f ? waves : 1.f) * (2.0f + 0.0038f * K);
+  registers += chain > bytes ? chain : bytes;
+}
+
+// mode 0: gate and up; 1: down; 2: up alone.  dtype 0 float32, 1 bfloat16.  streams: tiles of 16 rows stream
+// their weights (see dib_moe_streams).
+int moe_product(const void* a_rows, int dtype, const int* order, int max_tiles, int tile, int streams, int top,
+                const void* w, void* out, int K, int N, int mode, float limit, float alpha, cudaStream_t st) {
   if (max_tiles == 0) return DIB_OK;
   if (K < 1 || N < 1 || tile < 1 || tile % GC_ROWS || top < 1) return DIB_BAD_SIZE;
   if (dtype == 1 && K % 8 == 0 && (tile == 16 || tile == 64)) {
-    if (tile == 16) return launch_product_stream(a_rows, order, max_tiles, top, w, out, K, N, mode, limit, alpha, st);
+    if (tile == 16 && streams)
+      return launch_product_stream(a_rows, order, max_tiles, top, w, out, K, N, mode, limit, alpha, st);
+    if (tile == 16) return launch_product_mma<1, 4>(a_rows, order, max_tiles, tile, top, w, out, K, N, mode, limit, alpha, st);
     return launch_product_mma<4, 4>(a_rows, order, max_tiles, tile, top, w, out, K, N, mode, limit, alpha, st);
   }
   const dim3 grid(max_tiles, (N + GC_COLS - 1) / GC_COLS, tile / GC_ROWS);
@@ -703,21 +722,29 @@ int dib_moe_sort(const int* ids, const int* table, int top, int V, int pairs, in
   return DIB_OK;
 }
 
+// Do tiles of 16 rows, about `tiles` of them in use, stream their weights (both products of a layer)?
+int dib_moe_streams(int tiles, int F, int W, int gated) {
+  float registers = 0.f, streamed = 0.f;
+  product_times(tiles, W, gated ? 2 * F : F, registers, streamed);
+  product_times(tiles, F, W, registers, streamed);
+  return streamed <= registers ? 1 : 0;
+}
+
 // limit > 0: the limited gate (limit, alpha); else silu
-int dib_moe_gate_up(const void* x, int dtype, const int* order, int max_tiles, int tile, int top, const void* w_gate_up,
-                    void* hidden, int F, int W, float limit, float alpha, cudaStream_t st) {
-  return moe_product(x, dtype, order, max_tiles, tile, top, w_gate_up, hidden, W, F, 0, limit, alpha, st);
+int dib_moe_gate_up(const void* x, int dtype, const int* order, int max_tiles, int tile, int streams, int top,
+                    const void* w_gate_up, void* hidden, int F, int W, float limit, float alpha, cudaStream_t st) {
+  return moe_product(x, dtype, order, max_tiles, tile, streams, top, w_gate_up, hidden, W, F, 0, limit, alpha, st);
 }
 
 // experts without a gate: w_up [experts][F][W], hidden = the erf gelu of the product
-int dib_moe_up(const void* x, int dtype, const int* order, int max_tiles, int tile, int top, const void* w_up, void* hidden,
-               int F, int W, cudaStream_t st) {
-  return moe_product(x, dtype, order, max_tiles, tile, top, w_up, hidden, W, F, 2, 0.f, 0.f, st);
+int dib_moe_up(const void* x, int dtype, const int* order, int max_tiles, int tile, int streams, int top,
+               const void* w_up, void* hidden, int F, int W, cudaStream_t st) {
+  return moe_product(x, dtype, order, max_tiles, tile, streams, top, w_up, hidden, W, F, 2, 0.f, 0.f, st);
 }
 
-int dib_moe_down(const void* hidden, int dtype, const int* order, int max_tiles, int tile, const void* w_down,
-                 float* per_pair, int F, int W, cudaStream_t st) {
-  return moe_product(hidden, dtype, order, max_tiles, tile, 1, w_down, per_pair, F, W, 1, 0.f, 0.f, st);
+int dib_moe_down(const void* hidden, int dtype, const int* order, int max_tiles, int tile, int streams,
+                 const void* w_down, float* per_pair, int F, int W, cudaStream_t st) {
+  return moe_product(hidden, dtype, order, max_tiles, tile, streams, 1, w_down, per_pair, F, W, 1, 0.f, 0.f, st);
 }
 
 // shared null: no shared expert.  weights null: every weight is `weight`.

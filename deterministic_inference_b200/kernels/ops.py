@@ -1683,16 +1683,20 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
         _check(st, "routed_experts(rows back to their pairs)")
     else:
         hidden = torch.empty(max_tiles * tile, f, dtype=x.dtype, device=dev)
+        # the experts that tokens' choices at random name, and tiles that are not full
+        named = n_exp * (1.0 - (1.0 - min(top, n_exp) / n_exp) ** t)
+        streams = lib.dib_moe_streams(c_int(int(max(named, pairs / tile + named / 2))), c_int(f), c_int(w),
+                                      c_int(1 if gated else 0))
         if gated:
-            st = lib.dib_moe_gate_up(_ptr(x), c_int(_dt(x, "x")), _ptr(order), c_int(max_tiles), c_int(tile), c_int(top),
-                                     _ptr(w_gate_up), _ptr(hidden), c_int(f), c_int(w), c_float(limit), c_float(alpha),
-                                     _stream())
+            st = lib.dib_moe_gate_up(_ptr(x), c_int(_dt(x, "x")), _ptr(order), c_int(max_tiles), c_int(tile),
+                                     c_int(streams), c_int(top), _ptr(w_gate_up), _ptr(hidden), c_int(f), c_int(w),
+                                     c_float(limit), c_float(alpha), _stream())
         else:
-            st = lib.dib_moe_up(_ptr(x), c_int(_dt(x, "x")), _ptr(order), c_int(max_tiles), c_int(tile), c_int(top),
-                                _ptr(w_gate_up), _ptr(hidden), c_int(f), c_int(w), _stream())
+            st = lib.dib_moe_up(_ptr(x), c_int(_dt(x, "x")), _ptr(order), c_int(max_tiles), c_int(tile),
+                                c_int(streams), c_int(top), _ptr(w_gate_up), _ptr(hidden), c_int(f), c_int(w), _stream())
         _check(st, "routed_experts(gate and up)")
-        st = lib.dib_moe_down(_ptr(hidden), c_int(_dt(x, "x")), _ptr(order), c_int(max_tiles), c_int(tile), _ptr(w_down),
-                              _ptr(per_pair), c_int(f), c_int(w), _stream())
+        st = lib.dib_moe_down(_ptr(hidden), c_int(_dt(x, "x")), _ptr(order), c_int(max_tiles), c_int(tile),
+                              c_int(streams), _ptr(w_down), _ptr(per_pair), c_int(f), c_int(w), _stream())
         _check(st, "routed_experts(down)")
     out = torch.empty(t, w, dtype=torch.float32, device=dev)
     if shared is not None:

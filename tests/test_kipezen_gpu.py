@@ -145,6 +145,35 @@ def test_the_experts_streamed_products(width, ff, gated, monkeypatch):
         assert torch.equal(run(n), whole[:n]), n
 
 
+@pytest.mark.parametrize("width, ff, gated", [(512, 264, True), (264, 520, False), (1032, 200, True)])
+def test_the_experts_products_in_few_and_many_tiles(width, ff, gated, monkeypatch):
+    """Tiles of 16 rows of 256 experts: streamed weights for one token's few tiles, weights in registers for the many of
+    64 and of 300 tokens (some experts with two tiles), columns that are not full; a token's bits are the same, and
+    those of the plain product up to rounding."""
+    from deterministic_inference_b200.kernels import ops
+    monkeypatch.setattr(ops, "EXPERTS_TC", False)
+    experts, top, rows = 256, 8, 300
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x = rnd(rows, width)
+    up, down = rnd(experts, (2 if gated else 1) * ff, width) * 0.1, rnd(experts, width, ff) * 0.1
+    ids = torch.rand(rows, experts, generator=g, device="cuda").argsort(1)[:, :top].int()
+    weights = torch.rand(rows, top, generator=g, device="cuda")
+    run = lambda a, b: ops.routed_experts(x[a:b], ids[a:b].contiguous(), weights[a:b].contiguous(), up, down, None, None,
+                                          experts, torch.bfloat16, gated=gated)
+    whole = run(0, rows)
+    assert torch.equal(run(0, 64), whole[:64])
+    for r in (0, 7, 299):
+        assert torch.equal(run(r, r + 1)[0], whole[r]), r
+        want = torch.zeros(width, dtype=torch.float64, device="cuda")
+        for j in range(top):
+            e = int(ids[r, j])
+            z = x[r].double() @ up[e].double().T
+            h = torch.nn.functional.silu(z[:ff]) * z[ff:] if gated else torch.nn.functional.gelu(z)
+            want += float(weights[r, j]) * (h.bfloat16().double() @ down[e].double().T)
+        assert float((whole[r].double() - want).abs().max()) <= 1e-2 * float(want.abs().max())
+
+
 def test_the_experts_of_a_decode_step_do_not_depend_on_the_batch():
     """A step of 64 tokens that brings an expert 32 rows has a single token's bits; one of 65 is another form."""
     from deterministic_inference_b200.kernels import ops
