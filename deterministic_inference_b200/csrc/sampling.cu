@@ -181,7 +181,9 @@ __device__ __forceinline__ void load_chunk(const float* __restrict__ row, int lo
 // row; the block that is last to add its histogram to the row's works out the row's bits and
 // leaves them for the next pass.  The first forms every probability; the second only those
 // whose log2 may lie in the first's bin, and lists the bin's probabilities; the third is a
-// block a row over that list (over the row again, where the list is too short).
+// block a row over that list.  A flat row has more tokens in one bin than the list holds:
+// THIRD_BLOCKS blocks go over the row again then and add to a histogram as the others do (8 such
+// rows of 151,936: the whole draw 91 us; by one block a row 398 us).
 // (Four passes of 8 bits that formed every probability again, added up a warp's equal bins
 // by matching lanes and chained the chunks' normalisers in every thread: 69 us each, and
 // the pick 68 us; with 64 rows of 151,936, 38 of them filtered, the whole draw 318 us.  Three
@@ -191,15 +193,17 @@ constexpr float MASS_ONE = 1099511627776.0f;     // 2^40
 constexpr int FILTER_BINS0 = 1024, FILTER_BINS1 = 2048, FILTER_BINS2 = 1024;      // of the passes
 constexpr int FILTER_SHIFT0 = 21, FILTER_SHIFT1 = 10;
 constexpr int FILTER_BINS = FILTER_BINS0 + FILTER_BINS1;       // a row's in global memory
+static_assert(FILTER_BINS2 <= FILTER_BINS0, "the third pass may use the first one's histogram");
 constexpr int FILTER_LIST = 16384;                             // probabilities a row's list holds
+constexpr int THIRD_BLOCKS = 8;                                // blocks a row of the third pass
 
 struct FilterState {
   unsigned long long cnt_above, mass_above;   // tokens (and their mass) above the chosen bins
   unsigned prefix;                            // the threshold's bits found so far
   unsigned pad;
 };
-// a row's counters: blocks that have added to the first and to the second histogram, listed probabilities
-enum { MARK_FIRST = 0, MARK_SECOND = 1, MARK_LISTED = 2, ROW_MARKS = 4 };
+// a row's counters: blocks that have added to the first, the second and the third histogram, listed probabilities
+enum { MARK_FIRST = 0, MARK_SECOND = 1, MARK_LISTED = 2, MARK_THIRD = 3, ROW_MARKS = 4 };
 
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 gumbel_stats_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
@@ -531,49 +535,60 @@ filter_second_kernel(const float* __restrict__ logits, const float* __restrict__
     const FilterLimits lim(top_k, top_p, V);
     st = filter_descend<FILTER_BINS1>(hist_cnt, hist_mass, st, FILTER_SHIFT1, lim.k, lim.P, dsc);
     if (threadIdx.x == 0) states[R + r] = st;
+    // a list that overflowed: the third pass counts into the first one's histogram
+    if (__ldcg(&marks[(size_t)r * ROW_MARKS + MARK_LISTED]) > (unsigned)FILTER_LIST)
+      for (int b = threadIdx.x; b < FILTER_BINS2; b += SAMPLE_THREADS) {
+        hist_cnt[b - FILTER_BINS0] = 0u;
+        hist_mass[b - FILTER_BINS0] = 0ull;
+      }
   }
 }
 
-// One block a row: the last 10 bits, from the listed probabilities that have the first 21.
+// The last 10 bits, from the listed probabilities that have the first 21: a row's first block; where the list is
+// too short all of them, from the row.
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 filter_third_kernel(const float* __restrict__ logits, const float* __restrict__ temperatures,
                     const long long* __restrict__ top_ks, const float* __restrict__ top_ps,
                     const FilterState* __restrict__ states, const float2* __restrict__ norms,
-                    const unsigned* __restrict__ marks, const float* __restrict__ list, unsigned* __restrict__ thresh,
-                    int R, int V) {
+                    unsigned* marks, const float* __restrict__ list, unsigned* hist_cnt, unsigned long long* hist_mass,
+                    unsigned* __restrict__ thresh, int R, int V) {
   pdl_prologue(logits, temperatures, top_ks, top_ps, states, norms, marks, list);
   __shared__ unsigned s_cnt[FILTER_BINS2];
   __shared__ unsigned long long s_mass[FILTER_BINS2];
   __shared__ DescendScratch dsc;
-  const int r = blockIdx.x, lane = threadIdx.x & 31;
+  __shared__ bool s_last;
+  const int r = blockIdx.y, part = blockIdx.x, lane = threadIdx.x & 31;
   const float temp = temperatures[r];
   const long long top_k = top_ks[r];
   const float top_p = top_ps[r];
   if (!row_is_filtered(temp, top_k, top_p)) {
-    if (threadIdx.x == 0) thresh[r] = 0u;
+    if (part == 0 && threadIdx.x == 0) thresh[r] = 0u;
     return;
   }
   const FilterState st = states[R + r];
-  const unsigned listed = marks[(size_t)r * ROW_MARKS + MARK_LISTED];
+  const unsigned listed = __ldcg(&marks[(size_t)r * ROW_MARKS + MARK_LISTED]);
+  const bool whole = listed <= (unsigned)FILTER_LIST;          // the list has them all
+  if (whole && part > 0) return;
   const float2 norm = norms[r];
   for (int b = threadIdx.x; b < FILTER_BINS2; b += SAMPLE_THREADS) {
     s_cnt[b] = 0u;
     s_mass[b] = 0ull;
   }
   __syncthreads();
-  const bool whole = listed <= (unsigned)FILTER_LIST;          // the list has them all
   const int n = whole ? (int)listed : V;
   const float* from = whole ? list + (size_t)r * FILTER_LIST : logits + (size_t)r * V;
+  const int first = whole ? threadIdx.x : part * SAMPLE_THREADS + threadIdx.x;
+  const int step = whole ? SAMPLE_THREADS : THIRD_BLOCKS * SAMPLE_THREADS;
 #pragma unroll 4
-  for (int i = threadIdx.x; i - lane < n; i += SAMPLE_THREADS) {
+  for (int i = first; i - lane < n; i += step) {
     float p = i < n ? from[i] : 0.f;
     if (!whole) p = row_probability(p, temp, norm.x, norm.y);
     const unsigned key = __float_as_uint(p);
     const bool mine = i < n && (key >> FILTER_SHIFT1) == (st.prefix >> FILTER_SHIFT1);
     const unsigned bin = key & (FILTER_BINS2 - 1);
     const unsigned long long m = (unsigned long long)(p * MASS_ONE);
-    const unsigned first = __shfl_sync(0xffffffffu, bin, 0);
-    if (__all_sync(0xffffffffu, mine && bin == first)) {
+    const unsigned bin0 = __shfl_sync(0xffffffffu, bin, 0);
+    if (__all_sync(0xffffffffu, mine && bin == bin0)) {
       const unsigned long long sum = ((unsigned long long)__reduce_add_sync(0xffffffffu, (unsigned)(m >> 20)) << 20) +
                                      __reduce_add_sync(0xffffffffu, (unsigned)(m & 0xfffffull));
       if (lane == 0) {
@@ -587,7 +602,20 @@ filter_third_kernel(const float* __restrict__ logits, const float* __restrict__ 
   }
   __syncthreads();
   const FilterLimits lim(top_k, top_p, V);
-  const FilterState last = filter_descend<FILTER_BINS2, true>(s_cnt, s_mass, st, 0, lim.k, lim.P, dsc);
+  FilterState last;
+  if (whole) {
+    last = filter_descend<FILTER_BINS2, true>(s_cnt, s_mass, st, 0, lim.k, lim.P, dsc);
+  } else {
+    hist_cnt += (size_t)r * FILTER_BINS;
+    hist_mass += (size_t)r * FILTER_BINS;
+    for (int b = threadIdx.x; b < FILTER_BINS2; b += SAMPLE_THREADS)
+      if (s_cnt[b] != 0u) {
+        atomicAdd(&hist_cnt[b], s_cnt[b]);
+        atomicAdd(&hist_mass[b], s_mass[b]);
+      }
+    if (!last_of_row(&marks[(size_t)r * ROW_MARKS + MARK_THIRD], THIRD_BLOCKS, &s_last)) return;
+    last = filter_descend<FILTER_BINS2>(hist_cnt, hist_mass, st, 0, lim.k, lim.P, dsc);
+  }
   if (threadIdx.x == 0) thresh[r] = last.prefix;
 }
 
@@ -760,8 +788,9 @@ int dib_gumbel_sample_chunked(const float* logits, const float* temperatures, co
     dib_launch(filter_second_kernel, grid, block, 0, st, logits, temperatures, top_ks, top_ps, hist_cnt, hist_mass,
                states, (const float2*)norms, marks, list, R, V, chunks);
     DIB_CHECK_LAUNCH();
-    dib_launch(filter_third_kernel, dim3(R), block, 0, st, logits, temperatures, top_ks, top_ps,
-               (const FilterState*)states, (const float2*)norms, (const unsigned*)marks, (const float*)list, thresh, R, V);
+    dib_launch(filter_third_kernel, dim3(THIRD_BLOCKS, R), block, 0, st, logits, temperatures, top_ks, top_ps,
+               (const FilterState*)states, (const float2*)norms, marks, (const float*)list, hist_cnt, hist_mass, thresh, R,
+               V);
     DIB_CHECK_LAUNCH();
   }
   dib_launch(gumbel_pick_kernel, grid, block, 0, st, logits, temperatures, seeds, sample_pos, keep,

@@ -843,6 +843,35 @@ def test_draws_from_extreme_rows(v):
     assert (p.gather(1, got.long().unsqueeze(1)) > 0).all() and got[0] == plain[0] and got[7] == plain[7]
 
 
+@pytest.mark.parametrize("v", [151936, 40001])
+def test_thresholds_of_flat_rows(v):
+    """Rows whose tokens nearly all lie in one bin of the first pass, more than a row's list holds, beside one that does
+    not: fewer than top_k tokens above the threshold and at least as many from it on, at most top_p of the mass above
+    it and more from it on (up to probabilities that two computations round differently)."""
+    torch.manual_seed(31)
+    r = 9
+    logits = torch.randn(r, v, device="cuda") * torch.tensor([0.03, 0.02, 0.05, 3.0, 0.03, 0.01, 0.04, 0.03, 0.02],
+                                                             device="cuda").unsqueeze(1)
+    temps = torch.tensor([1.0, 0.7, 1.0, 1.0, 2.0, 1.0, 0.0, 1.0, 1.0], device="cuda")
+    top_ks = torch.tensor([30000, -1, 5, 50, 1, v - 1, 7, -1, 20000], device="cuda", dtype=torch.int64)
+    top_ps = torch.tensor([1.0, 0.6, 1.0, 0.9, 1.0, 1.0, 0.5, 1.0, 0.1], device="cuda")
+    seeds, pos = torch.arange(r, device="cuda") + 3, torch.arange(r, device="cuda") + 90
+    toks, thr = ops().gumbel_sample(logits, temps, seeds, pos, top_ks=top_ks, top_ps=top_ps, return_thresholds=True)
+    again = ops().gumbel_sample(logits, temps, seeds, pos, top_ks=top_ks, top_ps=top_ps, return_thresholds=True)
+    assert torch.equal(again[0], toks) and torch.equal(again[1], thr)
+    plain = ops().gumbel_sample(logits, temps, seeds, pos)
+    assert thr[6] == 0 and toks[6] == logits[6].argmax() and thr[7] == 0 and toks[7] == plain[7]
+    p = torch.softmax(logits.double() / torch.where(temps > 0, temps, torch.ones_like(temps)).double().unsqueeze(1), 1)
+    edge = thr.view(torch.float32).double().unsqueeze(1)
+    # two exponentials, the division and the normaliser's sum: some 2^-20 of a probability
+    above, upto = p > edge * (1 + 2.0 ** -19), p >= edge * (1 - 2.0 ** -19)
+    for i in (0, 1, 2, 3, 4, 5, 8):
+        k, mass = int(top_ks[i]) if top_ks[i] > 0 else v + 1, float(top_ps[i])
+        assert int(above[i].sum()) < k and float(p[i][above[i]].sum()) <= mass + 1e-6, i
+        assert int(upto[i].sum()) >= k or float(p[i][upto[i]].sum()) > mass - 1e-6, i
+        assert upto[i, toks[i]], i
+
+
 def test_top_k_top_p_respected():
     from deterministic_inference_b200.config import SamplingParams
     from deterministic_inference_b200.sampling import sample
