@@ -195,6 +195,7 @@ constexpr int FILTER_SHIFT0 = 21, FILTER_SHIFT1 = 10;
 constexpr int FILTER_BINS = FILTER_BINS0 + FILTER_BINS1;       // a row's in global memory
 static_assert(FILTER_BINS2 <= FILTER_BINS0, "the third pass may use the first one's histogram");
 constexpr int FILTER_LIST = 16384;                             // probabilities a row's list holds
+constexpr int FILTER_ROWS = 512;                               // filtered rows at a time: 52 MB of scratch
 constexpr int THIRD_BLOCKS = 8;                                // blocks a row of the third pass
 
 struct FilterState {
@@ -751,10 +752,11 @@ int dib_gumbel_sample(const float* logits, const float* temperatures, const long
 // top_ks / top_ps (both or neither): per-row top-k (<= 0: off) and top-p (>= 1: off),
 // applied by a threshold found without a sort.  thresh: unsigned [R], receives the bits of
 // each row's smallest kept probability (0 = all kept); hist: scratch of dib_filter_scratch(R)
-// bytes, 8-byte aligned.
+// bytes, 8-byte aligned (more than FILTER_ROWS rows go through it in turn, in stream order).
 long long dib_filter_scratch(int R) {
-  return (long long)R * (FILTER_BINS * 12ll + 2 * (long long)sizeof(FilterState) + (long long)sizeof(float2) +
-                         4ll * ROW_MARKS + 4ll * FILTER_LIST);
+  return (R < FILTER_ROWS ? R : FILTER_ROWS) *
+         (FILTER_BINS * 12ll + 2 * (long long)sizeof(FilterState) + (long long)sizeof(float2) + 4ll * ROW_MARKS +
+          4ll * FILTER_LIST);
 }
 
 int dib_gumbel_sample_chunked(const float* logits, const float* temperatures, const long long* seeds,
@@ -765,11 +767,21 @@ int dib_gumbel_sample_chunked(const float* logits, const float* temperatures, co
   if (R == 0) return DIB_OK;
   if (V < 1 || R > 65535) return DIB_BAD_SIZE;
   const int chunks = (V + ARGMAX_CHUNK - 1) / ARGMAX_CHUNK;
+  const bool filtered = top_ks != nullptr && top_ps != nullptr && thresh != nullptr && hist != nullptr;
+  if (filtered && reinterpret_cast<uintptr_t>(hist) % 8 != 0) return DIB_BAD_ALIGN;
+  if (filtered && R > FILTER_ROWS) {       // rows in turn through the same scratch (it is 100 KB a row)
+    for (int r = 0; r < R; r += FILTER_ROWS) {
+      const int n = R - r < FILTER_ROWS ? R - r : FILTER_ROWS;
+      const int status = dib_gumbel_sample_chunked(
+          logits + (size_t)r * V, temperatures + r, seeds + r, sample_pos + r, keep != nullptr ? keep + (size_t)r * V : keep,
+          top_ks + r, top_ps + r, thresh + r, hist, scratch_f, scratch_i, out + r, n, V, st);
+      if (status != DIB_OK) return status;
+    }
+    return DIB_OK;
+  }
   float* cmax = scratch_f;
   float* csum = scratch_f + (size_t)R * chunks;
   float* pv = scratch_f + 2 * (size_t)R * chunks;
-  const bool filtered = top_ks != nullptr && top_ps != nullptr && thresh != nullptr && hist != nullptr;
-  if (filtered && reinterpret_cast<uintptr_t>(hist) % 8 != 0) return DIB_BAD_ALIGN;
   // masses, the rows' states and normalisers, then what needs 4 bytes only
   unsigned long long* hist_mass = filtered ? reinterpret_cast<unsigned long long*>(hist) : nullptr;
   FilterState* states = filtered ? reinterpret_cast<FilterState*>(hist_mass + (size_t)R * FILTER_BINS) : nullptr;

@@ -853,7 +853,8 @@ def gumbel_sample(logits: torch.Tensor, temperatures: torch.Tensor, seeds: torch
                                            _ptr(top_ps), _ptr(thresh),
                                            _ptr(hist) if thresh is not None else c_void_p(0),
                                            _ptr(sf), _ptr(si), _ptr(out), c_int(r), c_int(v), _stream())
-        _check(st, "gumbel_sample", kernels=3 if thresh is None else 6)
+        # (filtered rows go through the scratch 512 at a time)
+        _check(st, "gumbel_sample", kernels=3 if thresh is None else 6 * -(-r // 512))
         return (out, thresh) if return_thresholds else out
     if filtered:
         raise KernelError("gumbel_sample: top_ks / top_ps with more than 65535 rows")

@@ -872,6 +872,35 @@ def test_thresholds_of_flat_rows(v):
         assert upto[i, toks[i]], i
 
 
+@pytest.mark.parametrize("rows", [512, 513, 1100])
+def test_many_filtered_rows_share_one_scratch(rows):
+    """The scratch of top-k / top-p is that of 512 rows, whatever the call's; the draws and thresholds of rows at and
+    beyond that line are those of the rows alone."""
+    from ctypes import c_int, c_longlong
+    lib = ops()._lib("sampling")
+    lib.dib_filter_scratch.restype = c_longlong
+    assert lib.dib_filter_scratch(c_int(65535)) == lib.dib_filter_scratch(c_int(512)) <= 64 << 20
+    torch.manual_seed(37)
+    v = 9001
+    logits = 3 * torch.randn(rows, v, device="cuda")
+    logits[511:] *= 0.02                                       # (some flat ones)
+    temps = torch.full((rows,), 0.8, device="cuda")
+    top_ks = torch.randint(-5, 60, (rows,), device="cuda")
+    top_ps = torch.rand(rows, device="cuda") * 0.5 + 0.6
+    keep = (torch.rand(rows, v, device="cuda") < 0.9).to(torch.uint8)
+    seeds, pos = torch.arange(rows, device="cuda") + 3, torch.arange(rows, device="cuda") + 90
+    for mask in (None, keep):
+        got, thr = ops().gumbel_sample(logits, temps, seeds, pos, mask, top_ks=top_ks, top_ps=top_ps, return_thresholds=True)
+        for a in (0, 500, 511, 512, rows - 5):
+            b = min(rows, a + 5)
+            if a >= rows:
+                continue
+            one, one_thr = ops().gumbel_sample(logits[a:b], temps[a:b], seeds[a:b], pos[a:b],
+                                               None if mask is None else mask[a:b], top_ks=top_ks[a:b], top_ps=top_ps[a:b],
+                                               return_thresholds=True)
+            assert torch.equal(got[a:b], one) and torch.equal(thr[a:b], one_thr), (a, mask is None)
+
+
 def test_top_k_top_p_respected():
     from deterministic_inference_b200.config import SamplingParams
     from deterministic_inference_b200.sampling import sample
