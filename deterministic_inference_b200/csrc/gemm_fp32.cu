@@ -1,13 +1,13 @@
 // True float32 matrix product on the CUDA cores: C[M,N] = A[M,K] * W[N,K]^T.
 //
 // This is the matrix product of the 32-bit path: plain FMA, no tensor cores and
-// no reduced-precision mode.  An output element is eight partial sums (from K = 512 on; one
-// chain over k in index order below, see gemm_fp32_short_kernel): k belongs to partial (k / 4) % 8, each partial adds its k in index order, and the partials are
-// added one after the other.  That order is a function of K alone, whatever the tile,
-// so a row's result does not depend on M: the same token gives the same bits in any
-// batch.  (Distance from 64-bit sums at K = 1024 .. 3072: 2.1e-7 .. 3.6e-7 of the norm.
-// The logits of 204 rows through 28 layers came to 9.1e-7, against 2.1e-6 with one chain
-// over all k.)
+// no reduced-precision mode.  From K = 512 on an output element is eight partial sums: k
+// belongs to partial (k / 4) % 8, each partial adds its k in index order, and the partials
+// are added one after the other.  Below, it is one chain over k in index order
+// (gemm_fp32_short_kernel).  The order is a function of K alone, whatever the tile, so a
+// row's result does not depend on M: the same token gives the same bits in any batch.
+// (Distance from 64-bit sums at K = 1024 .. 3072: 2.1e-7 .. 3.6e-7 of the norm.  The logits
+// of 204 rows through 28 layers came to 9.1e-7, against 2.1e-6 with one chain over all k.)
 //
 // Both operands lie k-contiguous, and stay so in shared memory (copied 16 bytes at a
 // time, two or three stages ahead).  The eight warps of a block share one output tile
@@ -133,7 +133,9 @@ gemm_fp32_kernel(const float* __restrict__ A, const float* __restrict__ W, float
 // Short sums (K below SHORT_K): one chain over all k in index order, as there is little to divide; the
 // eight warps of a block take 16 x 32 outputs each of a tile of 64 x 64, from stages copied the same way.
 // (204 rows: 768 x 192 9.7 us, 1,024 x 500 23 us; divided 5.9 and 12 us, but then the logits of a small
-// model's ill-conditioned rows move by as much as they are off; 64 x 64 x 16 in order, as before: 21, 54 us.)
+// model's ill-conditioned rows move by as much as they are off; 64 x 64 x 16 in order, as before: 21, 54 us.
+// 512 lies between the sizes of such small models, whose bits stay as they were, and of real ones; it is no
+// crossover: the divided form would be quicker, and nearer to 64 bits on average, below it too.)
 constexpr int SHORT_K = 512, SH_B = 64, SH_BK = 32, SH_STAGES = 3, SH_LD = SH_BK + 4;
 template <bool VEC>
 __global__ void __launch_bounds__(THREADS)
@@ -241,7 +243,8 @@ int launch(const float* A, const float* W, float* out, int M, int N, int K, cuda
 // what a tile adds on an SM that has several; measured per 1024 k, in us.  (M = 64, N = 4096:
 // 8 x 32 38.9, 16 x 32 32.8, 32 x 32 28.7, 64 x 32 30.7 us a call; M = 212, N = 1024, K = 2048:
 // 16 x 32 57, 32 x 32 49, 64 x 32 51; a step of
-// 204 rows of a 28-layer model: 38.8 ms, against 67.1 ms with tiles of 64 x 64 x 16, one in flight.)
+// 204 rows of a 28-layer model: 38.8 ms, against 67.1 ms with tiles of 64 x 64 x 16, one in flight.)  The rule
+// counts a B200's 148 SMs; every tile gives the same bits.
 using T64 = Tile<64, 32, 8, 8, 32, 3, 2>;
 using T32 = Tile<32, 32, 8, 4, 64, 3, 2>;
 using T16 = Tile<16, 32, 4, 4, 64, 3, 3>;

@@ -610,8 +610,9 @@ constexpr int MAX_DYNAMIC_SMEM = 224 * 1024;
 static inline size_t smem_bytes(int D, int VD, int VD_stored, int rows) {
   size_t tiles = 2 * (size_t)KT * (D + PAD);
   if (VD_stored > 0) tiles += 2 * (size_t)KT * (VD + PAD);
-  // (16 rows: the warps' float32 sums take the tiles' place at the end)
-  if (rows == DEC_ROWS && tiles < 2 * (size_t)DEC_WARPS * DEC_ROWS * VD) tiles = 2 * (size_t)DEC_WARPS * DEC_ROWS * VD;
+  // (16 rows: the warps' float32 sums, 2 x 64 x VD elements, take the tiles' place at the end; they fit, as values are
+  // stored, in tiles of their own, or are the first VD <= D elements of the keys)
+  static_assert(DEC_WARPS * DEC_ROWS <= KT, "the warps' sums fit the place of two tiles");
   return sizeof(__nv_bfloat16) * ((size_t)rows * (D + PAD) + tiles);
 }
 

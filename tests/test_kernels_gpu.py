@@ -177,16 +177,18 @@ def test_linear_fp32_is_true_fp32(m, n, k):
 
 
 @pytest.mark.parametrize("n,k", [(31, 33), (33, 64), (65, 130), (4096, 260), (100, 511), (100, 512),
-                                 (4096, 513), (65, 578), (1024, 1028)])
+                                 (4096, 513), (65, 578), (1024, 1028), (40003, 516), (4099, 1028), (40003, 517),
+                                 (4099, 1030)])
 def test_linear_fp32_tiles_give_the_same_bits(n, k):
     """Every tile the row count and the width may choose adds in one order: the row's bits are those of the
     row alone, at the edges of the tiles; against 64 bits the error is that of eight chains of k / 8, or of one
-    below 512."""
+    below 512.  (The last four widths, no multiple of a tile's, reach all five tiles from K = 512 on, each with
+    copies of 16 and of 4 bytes.)"""
     torch.manual_seed(16)
     x = torch.randn(400, k, device="cuda")
     w = torch.randn(n, k, device="cuda")
     rows = [ops().linear(x[r:r + 1], w) for r in (0, 7, 8, 16, 33)]
-    for m in (7, 8, 9, 16, 17, 32, 33, 63, 64, 65, 129, 400):
+    for m in (7, 8, 9, 16, 17, 32, 33, 63, 64, 65, 129, 204, 400):
         got = ops().linear(x[:m], w)
         for r, one in zip((0, 7, 8, 16, 33), rows):
             if r < m:
