@@ -5,6 +5,7 @@
 #include <map>
 #include <tuple>
 
+#define DIB_LENGTHS_EARLY 1
 #include "attention_bf16_kernels.cuh"
 
 // ------------------------------------------------------------------------------

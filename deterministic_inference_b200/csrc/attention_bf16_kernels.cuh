@@ -506,54 +506,75 @@ decode_attention_stage1_kernel(const __nv_bfloat16* __restrict__ q,
 // chunk order.  Two kernels do this: the first with one thread per output dimension,
 // for steps whose longest sequence has few chunks; the second with a group of threads per
 // chunk, for long sequences.  Both give the same bits for a sequence, whatever else is in
-// the batch.  The partial results of the first chunk are requested before the
-// sequence's length is known (what lies beyond its last split is read but not used), so
-// a sequence of one chunk waits for memory once.
+// the batch.
+// DIB_LENGTHS_EARLY 1: the lengths are the step's own metadata, which no kernel of the step writes, and are read
+// ahead of the wait; 0 (an entry point for other hosts): behind it.
+#ifndef DIB_LENGTHS_EARLY
+#define DIB_LENGTHS_EARLY 0
+#endif
 __global__ void decode_attention_stage2_kernel(const float* __restrict__ part_o,
                                                const float* __restrict__ part_lse,
                                                const int* __restrict__ seq_lens,
                                                __nv_bfloat16* __restrict__ out, int max_splits,
                                                int Hq, int D, int window,
                                                const float* __restrict__ sink) {
-  pdl_prologue(part_o, part_lse);
+  pdl_trigger();
   constexpr int CH = MERGE_CH;
   const int b = blockIdx.x, h = blockIdx.y;
   const size_t row = ((size_t)b * Hq + h) * max_splits;
-  const int kv_len = seq_lens[b];
-  float lse_r[CH], o_r[CH][1];
-#pragma unroll
-  for (int j = 0; j < CH; ++j) lse_r[j] = j < max_splits ? part_lse[row + j] : NEG_BIG;
-#pragma unroll
-  for (int j = 0; j < CH; ++j)
-    o_r[j][0] = (j < max_splits && (int)threadIdx.x < D) ? part_o[(row + j) * D + threadIdx.x] : 0.f;
+  if (!DIB_LENGTHS_EARLY) pdl_wait(part_o, part_lse, seq_lens);
   // (a caller that passes fewer splits than the sequence has keys for gets a result over
   // the splits there are, never a read beyond the row)
   int s0, s1;
-  merge_range(kv_len, window, max_splits, s0, s1);
+  merge_range(seq_lens[b], window, max_splits, s0, s1);
   const int c0 = s0 / CH, c1 = s1 / CH;
+  if (DIB_LENGTHS_EARLY) pdl_wait(part_o, part_lse);
+  // the first two chunks' partial results together (up to 32 splits, 4,096 keys, in one trip to memory)
+  float lse_r[2][CH], o_r[2][CH][1];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int j = 0; j < CH; ++j) {
+      const int s = (c0 + u) * CH + j;
+      const bool in = s >= s0 && s <= s1;
+      lse_r[u][j] = in ? part_lse[row + s] : NEG_BIG;
+      o_r[u][j][0] = in && (int)threadIdx.x < D ? part_o[(row + s) * D + threadIdx.x] : 0.f;
+    }
   float M = NEG_BIG;
 #pragma unroll
-  for (int j = 0; j < CH; ++j)
-    if (j >= s0 && j <= s1) M = fmaxf(M, lse_r[j]);
-  for (int s = max(s0, CH); s <= s1; ++s) M = fmaxf(M, part_lse[row + s]);
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int j = 0; j < CH; ++j) M = fmaxf(M, lse_r[u][j]);
+  for (int s = (c0 + 2) * CH; s <= s1; ++s) M = fmaxf(M, part_lse[row + s]);
   // a sink: exp(sink[head]) joins the denominator; without one the sum is left as it is (x + 0 = x)
   const float sink_w = sink != nullptr ? merge_weight(sink[h], M) : 0.f;
   bool first = true;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float total[1] = {0.f}, total_den = 0.f;
-    for (int c = c0; c <= c1; ++c) {
-      if (c > 0 || !first) {
+    float total[1] = {0.f}, total_den = 0.f, acc[1], den;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (c0 + u > c1) break;
+      if (!first) {
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-          const int s = c * CH + j;
-          const bool in = s >= s0 && s <= s1;
-          lse_r[j] = in ? part_lse[row + s] : NEG_BIG;
-          o_r[j][0] = in ? part_o[(row + s) * D + d] : 0.f;
+          const int s = (c0 + u) * CH + j;
+          o_r[u][j][0] = s >= s0 && s <= s1 ? part_o[(row + s) * D + d] : 0.f;
         }
       }
-      float acc[1], den;
-      merge_chunk<1>(lse_r, o_r, c, s0, s1, M, acc, den);
-      merge_add<1>(c == c0, acc, den, total, total_den);
+      merge_chunk<1>(lse_r[u], o_r[u], c0 + u, s0, s1, M, acc, den);
+      merge_add<1>(u == 0, acc, den, total, total_den);
+    }
+    for (int c = c0 + 2; c <= c1; ++c) {
+      float lse_c[CH], o_c[CH][1];
+#pragma unroll
+      for (int j = 0; j < CH; ++j) {
+        const int s = c * CH + j;
+        const bool in = s >= s0 && s <= s1;
+        lse_c[j] = in ? part_lse[row + s] : NEG_BIG;
+        o_c[j][0] = in ? part_o[(row + s) * D + d] : 0.f;
+      }
+      merge_chunk<1>(lse_c, o_c, c, s0, s1, M, acc, den);
+      merge_add<1>(false, acc, den, total, total_den);
     }
     out[((size_t)b * Hq + h) * D + d] = __float2bfloat16_rn(merge_finish(total[0], __fadd_rn(total_den, sink_w)));
     first = false;
@@ -571,7 +592,7 @@ decode_attention_stage2_wide_kernel(const float* __restrict__ part_o,
                                     const int* __restrict__ seq_lens,
                                     __nv_bfloat16* __restrict__ out, int max_splits, int Hq, int D,
                                     int window, const float* __restrict__ sink) {
-  pdl_prologue(part_o, part_lse);
+  pdl_trigger();
   constexpr int CH = MERGE_CH;
   __shared__ float s_acc[MERGE_MAX_CHUNKS][128];
   __shared__ float s_den[MERGE_MAX_CHUNKS];
@@ -580,7 +601,9 @@ decode_attention_stage2_wide_kernel(const float* __restrict__ part_o,
   const int d = threadIdx.x, g = threadIdx.y;
   const int groups = blockDim.y;
   const size_t row = ((size_t)b * Hq + h) * max_splits;
+  if (!DIB_LENGTHS_EARLY) pdl_wait(part_o, part_lse, seq_lens);
   const int kv_len = seq_lens[b];
+  if (DIB_LENGTHS_EARLY) pdl_wait(part_o, part_lse);
   // chunk g is requested before the sequence's length is known: it is this group's
   // first chunk unless a window has moved the range past it
   float lse_r[CH], o_r[CH][1];

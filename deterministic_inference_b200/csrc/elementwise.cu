@@ -255,20 +255,27 @@ __global__ void qk_norm_rope_cache_vec_kernel(
     const float* __restrict__ cos_sin, int max_pos, const int* __restrict__ positions,
     const int* __restrict__ slot_mapping, int T_tokens, int Hq, int Hkv, int page_size,
     long long num_pages) {
-  pdl_prologue(qkv, parts, positions, slot_mapping);
+  pdl_trigger();
   constexpr int D = EPL * 32;
   const int warps_per_block = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int heads = Hq + 2 * Hkv;
   const long long total = (long long)T_tokens * heads;
   const long long item0 = ((long long)blockIdx.x * warps_per_block + warp) * ITEMS;
-  if (item0 >= total) return;
+  if (item0 >= total) {
+    pdl_wait();
+    return;
+  }
 
   // A warp takes ITEMS consecutive (token, head) items and issues the loads of all of
-  // them before it works on any, so their memory round-trips overlap.
+  // them before it works on any, so their memory round-trips overlap.  The step's positions and cache slots do
+  // not change while its kernels run, and the rotation table and the norms' weights never: with one item a
+  // warp (decoded tokens) all of them are there before the projection is, whose trip to memory is the only one then.
   float v[ITEMS][EPL];
   int tok[ITEMS], head[ITEMS], pos[ITEMS], slot[ITEMS];
   bool act[ITEMS];
+  constexpr bool EARLY = ITEMS == 1;
+  float cc[EPL], sn[EPL], wn[EPL];
 #pragma unroll
   for (int it = 0; it < ITEMS; ++it) {
     const long long item = item0 + it;
@@ -277,6 +284,26 @@ __global__ void qk_norm_rope_cache_vec_kernel(
     head[it] = act[it] ? (int)(item % heads) : 0;
     pos[it] = 0;
     slot[it] = -1;
+    if (!act[it]) continue;
+    if (cos_sin != nullptr && head[it] < Hq + Hkv) {
+      const int p = positions[tok[it]];
+      pos[it] = p < 0 ? 0 : (p >= max_pos ? max_pos - 1 : p);
+    }
+    if (head[it] >= Hq && kv_cache != nullptr) slot[it] = slot_mapping[tok[it]];
+  }
+  if (EARLY && head[0] < Hq + Hkv) {
+    const float* nw = head[0] < Hq ? q_norm_w : k_norm_w;
+    const float* tab = cos_sin + (size_t)pos[0] * D + (lane & 15) * EPL;
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) {
+      wn[k] = nw != nullptr ? nw[lane * EPL + k] : 0.f;
+      cc[k] = cos_sin != nullptr ? tab[k] : 0.f;
+      sn[k] = cos_sin != nullptr ? tab[D / 2 + k] : 0.f;
+    }
+  }
+  pdl_wait(qkv, parts);
+#pragma unroll
+  for (int it = 0; it < ITEMS; ++it) {
     if (!act[it]) continue;
     if (parts == nullptr) {
       const T* src = qkv + ((size_t)tok[it] * heads + head[it]) * D + lane * EPL;
@@ -307,11 +334,6 @@ __global__ void qk_norm_rope_cache_vec_kernel(
 #pragma unroll
       for (int k = 0; k < EPL; ++k) v[it][k] = round_to<T>(v[it][k]);
     }
-    if (cos_sin != nullptr && head[it] < Hq + Hkv) {
-      const int p = positions[tok[it]];
-      pos[it] = p < 0 ? 0 : (p >= max_pos ? max_pos - 1 : p);
-    }
-    if (head[it] >= Hq && kv_cache != nullptr) slot[it] = slot_mapping[tok[it]];
   }
 
 #pragma unroll
@@ -342,7 +364,7 @@ __global__ void qk_norm_rope_cache_vec_kernel(
       ss = sumsq_group<1>(one);
       const float rstd = rms_rstd(ss, D, eps);
 #pragma unroll
-      for (int k = 0; k < EPL; ++k) v[it][k] = norm_scale(v[it][k], rstd, nw[lane * EPL + k]);
+      for (int k = 0; k < EPL; ++k) v[it][k] = norm_scale(v[it][k], rstd, EARLY ? wn[k] : nw[lane * EPL + k]);
     }
     if (cos_sin != nullptr && (is_q || is_k)) {
       const float* tab = cos_sin + (size_t)pos[it] * D;
@@ -351,8 +373,8 @@ __global__ void qk_norm_rope_cache_vec_kernel(
 #pragma unroll
       for (int k = 0; k < EPL; ++k) {
         const float partner = __shfl_xor_sync(0xffffffffu, v[it][k], 16);
-        const float c = tab[j0 + k], sn = tab[D / 2 + j0 + k];
-        v[it][k] = upper ? rope_second(partner, v[it][k], c, sn) : rope_first(v[it][k], partner, c, sn);
+        const float c = EARLY ? cc[k] : tab[j0 + k], s = EARLY ? sn[k] : tab[D / 2 + j0 + k];
+        v[it][k] = upper ? rope_second(partner, v[it][k], c, s) : rope_first(v[it][k], partner, c, s);
       }
     }
     Pack<T, EPL> o;
@@ -540,8 +562,15 @@ add_rms_norm_split_kernel(const float* __restrict__ parts, int S,
                                           long long split_stride, T* __restrict__ residual,
                                           const float* __restrict__ w, T* __restrict__ out, int H,
                                           float eps) {
-  pdl_prologue(parts, residual);
+  pdl_trigger();
   __shared__ float scratch[128];
+  float4 ww[ITERS];     // (a constant: its trip to memory is over before the partials are there)
+#pragma unroll
+  for (int it = 0; it < ITERS; ++it) {
+    const int i = (it * blockDim.x + threadIdx.x) * 4;
+    ww[it] = i < H ? *reinterpret_cast<const float4*>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  pdl_wait(parts, residual);
   const size_t base = (size_t)blockIdx.x * H;
   float v[ITERS][4];
   float ss[ITERS][1];
@@ -575,12 +604,6 @@ add_rms_norm_split_kernel(const float* __restrict__ parts, int S,
       ss[it][0] = sumsq4(v[it][0], v[it][1], v[it][2], v[it][3]);
       *reinterpret_cast<Pack<T, 4>*>(residual + base + i) = o;
     }
-  }
-  float4 ww[ITERS];     // requested before the reduction, used after it
-#pragma unroll
-  for (int it = 0; it < ITERS; ++it) {
-    const int i = (it * blockDim.x + threadIdx.x) * 4;
-    ww[it] = i < H ? *reinterpret_cast<const float4*>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const float total = sumsq_row<ITERS, 1>(ss, H / 4, scratch);
   const float rstd = rms_rstd(total, H, eps);

@@ -141,11 +141,20 @@ template <int TERMS, int VPT, int AHEAD>
 __global__ void stream_norm_kernel(float* residual, Source x0, float a0, Source x1, float a1,
                                    const float* w, void* out, int out_dtype, int W, float eps) {
   __shared__ float scratch[32];
-  pdl_prologue(x0.p, x1.p, residual);
+  constexpr int N = VPT > 0 ? VPT : 1;
+  pdl_trigger();
+  float wv[N];                       // (a constant: its trip to memory is over before the row is there)
+  if (VPT > 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      wv[i] = c < W && out != nullptr ? w[c] : 0.f;
+    }
+  }
+  pdl_wait(x0.p, x1.p, residual);
   const long long base = (long long)blockIdx.x * W;
   float ss = 0.f;
   if (VPT > 0) {
-    constexpr int N = VPT > 0 ? VPT : 1;
     float r[N], v[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -175,7 +184,7 @@ __global__ void stream_norm_kernel(float* residual, Source x0, float a0, Source 
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
-      if (c < W) store_as(out, out_dtype, base + c, r[i] * rstd * w[c]);
+      if (c < W) store_as(out, out_dtype, base + c, r[i] * rstd * wv[i]);
     }
     return;
   }
