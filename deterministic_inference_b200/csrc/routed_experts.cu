@@ -357,14 +357,16 @@ moe_product_mma_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __re
 }
 
 // The same for few tiles of 16 rows (decoded tokens), where an expert's weights are read for a few rows
-// and the time is that of their bytes.  A CTA takes 32 rows of B (mode 0: 16 of the gate and the same
-// 16 of up), a warp 8 of them, and brings them and the tile's A rows into shared memory in runs of
-// ST_K k, ST_STAGES - 1 runs ahead by asynchronous copies of whole 512-byte pieces of a row: at
-// K = 1024 all of a CTA's 64 KB are asked for at once, by two CTAs an SM, while others multiply.  A
-// row's sum is the same as above: steps of 32 k, ascending, in the same permutation.  (Which of the two
-// runs, and what both take: product_times.)
+// and the time is that of their bytes.  An item is 32 rows of B (mode 0: 16 of the gate and the same
+// 16 of up) against a tile; a warp multiplies 8 of the rows and brings them and the tile's A rows into
+// shared memory in runs of ST_K k, ST_STAGES - 1 runs ahead by asynchronous copies of whole 512-byte
+// pieces of a row.  Two CTAs an SM walk the items of the tiles in use, and the copies run on from an item
+// to the next, so that memory is idle at the kernel's start alone.  A row's sum is the same as above:
+// steps of 32 k, ascending, in the same permutation.  (Which of the two runs, and what both take:
+// product_times.)
 constexpr int ST_THREADS = 128, ST_B = 32, ST_A = 16, ST_K = 256, ST_STAGES = 4;
 constexpr int ST_LD = ST_K + GP_PAD;
+constexpr int ST_CTAS = 2 * 148;          // two an SM
 constexpr int ST_STAGE = (ST_B + ST_A) * ST_LD;                    // elements
 __global__ void __launch_bounds__(ST_THREADS, 2)
 moe_product_stream_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __restrict__ order, int max_tiles,
@@ -374,88 +376,102 @@ moe_product_stream_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* _
   __nv_bfloat16* ring = reinterpret_cast<__nv_bfloat16*>(gp_smem);
   __shared__ __align__(16) float up_sums[2][32][4];
   pdl_prologue(a_rows, order);
-  const int tl = blockIdx.x % max_tiles;
-  const int expert = order[(long long)max_tiles * ST_A + tl];
-  if (expert < 0) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+  const int* experts = order + (long long)max_tiles * ST_A;
+  const int tiles = experts[max_tiles];                  // the tiles in use: the first ones
   const int cols = mode == 0 ? ST_B / 2 : ST_B;
-  const int n0 = (int)(blockIdx.x / max_tiles) * cols;
-  const int* pairs = order + (long long)tl * ST_A;
+  const long long items = (long long)tiles * ((N + cols - 1) / cols);
+  if (blockIdx.x >= items) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tig = lane & 3;
+  const int runs = (K + ST_K - 1) / ST_K;                // of an item
+  // neighbouring CTAs take neighbouring tiles: other experts, whose weights lie elsewhere
+  long long next = blockIdx.x;                           // the item whose runs are fetched, and which of them
+  int next_run = 0;
   // this warp copies rows warp, warp + 4, ... of a run: 32 lanes of 16 bytes each
   constexpr int ROWS = (ST_B + ST_A) / 4;
   const __nv_bfloat16* from[ROWS];                       // null: a row of zeros
+  auto fetch = [&](int stage) {
+    if (next < items) {
+      if (next_run == 0) {
+        const int tl = (int)(next % tiles), n0 = (int)(next / tiles) * cols, expert = experts[tl];
 #pragma unroll
-  for (int i = 0; i < ROWS; ++i) {
-    const int r = warp + 4 * i;
-    from[i] = nullptr;
-    if (r < ST_B) {
-      const int n = n0 + (mode == 0 ? r % (ST_B / 2) : r);
-      const long long rb = (mode == 0 && r >= ST_B / 2 ? (long long)N : 0ll) + n;
-      if (n < N) from[i] = w + ((long long)expert * (mode == 0 ? 2 * N : N) + rb) * K + lane * 8;
-    } else {
-      const int pair = pairs[r - ST_B];
-      const long long arow = mode != 1 ? pair / top : (long long)tl * ST_A + r - ST_B;
-      if (pair >= 0) from[i] = a_rows + arow * K + lane * 8;
-    }
-  }
-  const int runs = (K + ST_K - 1) / ST_K;
-  auto fetch = [&](int run) {
-    if (run < runs) {
-      const bool in = run * ST_K + lane * 8 < K;
-      __nv_bfloat16* to = ring + (run % ST_STAGES) * ST_STAGE + warp * ST_LD + lane * 8;
+        for (int i = 0; i < ROWS; ++i) {
+          const int r = warp + 4 * i;
+          from[i] = nullptr;
+          if (r < ST_B) {
+            const int n = n0 + (mode == 0 ? r % (ST_B / 2) : r);
+            const long long rb = (mode == 0 && r >= ST_B / 2 ? (long long)N : 0ll) + n;
+            if (n < N) from[i] = w + ((long long)expert * (mode == 0 ? 2 * N : N) + rb) * K + lane * 8;
+          } else {
+            const long long row = (long long)tl * ST_A + r - ST_B;
+            const int pair = order[row];
+            if (pair >= 0) from[i] = a_rows + (mode != 1 ? (long long)(pair / top) : row) * K + lane * 8;
+          }
+        }
+      }
+      const bool in = next_run * ST_K + lane * 8 < K;
+      __nv_bfloat16* to = ring + stage * ST_STAGE + warp * ST_LD + lane * 8;
 #pragma unroll
       for (int i = 0; i < ROWS; ++i) {
         const bool there = in && from[i] != nullptr;
-        const __nv_bfloat16* src = there ? from[i] + run * ST_K : w;
+        const __nv_bfloat16* src = there ? from[i] + next_run * ST_K : w;
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::
                          "r"((unsigned)__cvta_generic_to_shared(to + 4 * i * ST_LD)), "l"(src), "r"(there ? 16 : 0)
                      : "memory");
       }
+      if (++next_run == runs) {
+        next_run = 0;
+        next += gridDim.x;
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  int stage = 0;                                         // the stage that is multiplied next
 #pragma unroll
   for (int k = 0; k < ST_STAGES - 1; ++k) fetch(k);
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int run = 0; run < runs; ++run) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(ST_STAGES - 2) : "memory");
-    __syncthreads();                 // the run is there for all; the one before has been read by all
-    fetch(run + ST_STAGES - 1);
-    const __nv_bfloat16* b = ring + (run % ST_STAGES) * ST_STAGE + (warp * 8 + g) * ST_LD + tig * 8;
-    const __nv_bfloat16* a = ring + (run % ST_STAGES) * ST_STAGE + (ST_B + g) * ST_LD + tig * 8;
-    const int klen = min(ST_K, K - run * ST_K);
+  for (long long item = blockIdx.x; item < items; item += gridDim.x) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int run = 0; run < runs; ++run) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(ST_STAGES - 2) : "memory");
+      __syncthreads();               // the run is there for all; the one before has been read by all
+      fetch((stage + ST_STAGES - 1) % ST_STAGES);
+      const __nv_bfloat16* b = ring + stage * ST_STAGE + (warp * 8 + g) * ST_LD + tig * 8;
+      const __nv_bfloat16* a = ring + stage * ST_STAGE + (ST_B + g) * ST_LD + tig * 8;
+      const int klen = min(ST_K, K - run * ST_K);
 #pragma unroll 4
-    for (int k = 0; k < klen; k += 32) {
-      const uint4 lo = *reinterpret_cast<const uint4*>(a + k);
-      const uint4 hi = *reinterpret_cast<const uint4*>(a + 8 * ST_LD + k);
-      const uint4 x = *reinterpret_cast<const uint4*>(b + k);
-      mma_bf16_16816(acc, lo.x, hi.x, lo.y, hi.y, x.x, x.y);
-      mma_bf16_16816(acc, lo.z, hi.z, lo.w, hi.w, x.z, x.w);
+      for (int k = 0; k < klen; k += 32) {
+        const uint4 lo = *reinterpret_cast<const uint4*>(a + k);
+        const uint4 hi = *reinterpret_cast<const uint4*>(a + 8 * ST_LD + k);
+        const uint4 x = *reinterpret_cast<const uint4*>(b + k);
+        mma_bf16_16816(acc, lo.x, hi.x, lo.y, hi.y, x.x, x.y);
+        mma_bf16_16816(acc, lo.z, hi.z, lo.w, hi.w, x.z, x.w);
+      }
+      stage = (stage + 1) % ST_STAGES;
+    }
+    if (mode == 0) {                 // the warps of up hand their sums to those of the gate
+      if (warp >= 2) *reinterpret_cast<float4*>(up_sums[warp - 2][lane]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      __syncthreads();
+      if (warp >= 2) continue;       // (read before the next run's barrier, written again after it)
+    }
+    const int tl = (int)(item % tiles), n0 = (int)(item / tiles) * cols;
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int r = g + 8 * hh;
+      const int pair = order[(long long)tl * ST_A + r];
+      if (pair < 0) continue;
+      const long long row = mode == 1 ? pair : (long long)tl * ST_A + r;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int n = n0 + warp * 8 + tig * 2 + e;
+        const float v = acc[2 * hh + e];
+        if (n >= N) continue;
+        if (mode == 1) reinterpret_cast<float*>(out)[row * N + n] = v;
+        else
+          reinterpret_cast<__nv_bfloat16*>(out)[row * N + n] =
+              __float2bfloat16_rn(mode == 0 ? expert_gate(v, up_sums[warp][lane][2 * hh + e], limit, alpha) : gelu_erf(v));
+      }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (mode == 0) {                   // the warps of up hand their sums to those of the gate
-    if (warp >= 2) *reinterpret_cast<float4*>(up_sums[warp - 2][lane]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    __syncthreads();
-    if (warp >= 2) return;
-  }
-#pragma unroll
-  for (int hh = 0; hh < 2; ++hh) {
-    const int r = g + 8 * hh;
-    const int pair = pairs[r];
-    if (pair < 0) continue;
-    const long long row = mode == 1 ? pair : (long long)tl * ST_A + r;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int n = n0 + warp * 8 + tig * 2 + e;
-      const float v = acc[2 * hh + e];
-      if (n >= N) continue;
-      if (mode == 1) reinterpret_cast<float*>(out)[row * N + n] = v;
-      else
-        reinterpret_cast<__nv_bfloat16*>(out)[row * N + n] =
-            __float2bfloat16_rn(mode == 0 ? expert_gate(v, up_sums[warp][lane][2 * hh + e], limit, alpha) : gelu_erf(v));
-    }
-  }
 }
 
 // CUDA-core form: any type, any sizes.  A CTA takes 16 rows of a tile (blockIdx.z picks them) and 128
@@ -592,7 +608,7 @@ int launch_product_stream(const void* a_rows, const int* order, int max_tiles, i
   const int cols = mode == 0 ? ST_B / 2 : ST_B;
   const long long blocks = (long long)max_tiles * ((N + cols - 1) / cols);
   if (blocks > 0x7fffffffll) return DIB_BAD_SIZE;
-  dib_launch(moe_product_stream_kernel, dim3((unsigned)blocks), dim3(ST_THREADS), smem, st,
+  dib_launch(moe_product_stream_kernel, dim3((unsigned)(blocks < ST_CTAS ? blocks : ST_CTAS)), dim3(ST_THREADS), smem, st,
              (const __nv_bfloat16*)a_rows, order, max_tiles, top, (const __nv_bfloat16*)w, out, K, N, mode, limit, alpha);
   DIB_CHECK_LAUNCH();
   return DIB_OK;

@@ -1173,3 +1173,65 @@ def test_qkv_projection_with_the_norms_in_its_epilogue_gives_the_bits_of_the_two
         a, b = qf[..., :d // 2], qf[..., d // 2:]
         qf = torch.cat([a * c - b * s, b * c + a * s], dim=-1)
     torch.testing.assert_close(want_q.float(), qf, atol=3e-2 * float(qf.abs().max()), rtol=3e-2)
+
+
+# ---- routed experts of a few rows: the streamed form ---------------------------------------------------
+
+@pytest.mark.parametrize("experts,f,w,tokens,top", [(1, 16, 8, 1, 1), (3, 40, 264, 5, 2), (16, 1536, 1024, 8, 2),
+                                                    (16, 200, 520, 33, 2), (40, 72, 256, 64, 8), (7, 336, 1032, 60, 3)])
+def test_streamed_experts_give_the_bits_of_the_register_form(experts, f, w, tokens, top):
+    """CTAs that walk many items (and fewer items than CTAs), ragged columns and runs of k, tiles that are not full:
+    every row as by the form with a CTA an item."""
+    from ctypes import c_float, c_int
+    o, lib = ops(), ops()._lib("routed_experts")
+    g = torch.Generator(device="cuda").manual_seed(f + tokens)
+    ids = torch.stack([torch.randperm(experts, generator=g, device="cuda")[:top] for _ in range(tokens)]).int().contiguous()
+    x = torch.randn(tokens, w, generator=g, device="cuda").bfloat16()
+    gate_up = torch.randn(experts, 2 * f, w, generator=g, device="cuda").bfloat16()
+    down = torch.randn(experts, w, f, generator=g, device="cuda").bfloat16()
+    pairs = tokens * top
+    max_tiles = pairs // 16 + min(experts, pairs)
+    order = torch.empty(max_tiles * 17 + 1, dtype=torch.int32, device="cuda")
+    assert lib.dib_moe_sort(o._ptr(ids), o._ptr(None), c_int(top), c_int(0), c_int(pairs), c_int(experts), c_int(16),
+                            c_int(max_tiles), o._ptr(order), o._stream()) == 0
+    got = []
+    for streams in (0, 1):
+        outs = []
+        for gated in (True, False):
+            hidden = torch.zeros(max_tiles * 16, f, dtype=torch.bfloat16, device="cuda")
+            rest = (c_int(max_tiles), c_int(16), c_int(streams), c_int(top))
+            weights = gate_up if gated else gate_up[:, :f].contiguous()
+            if gated:
+                st = lib.dib_moe_gate_up(o._ptr(x), c_int(1), o._ptr(order), *rest, o._ptr(weights), o._ptr(hidden),
+                                         c_int(f), c_int(w), c_float(7.0), c_float(1.702), o._stream())
+            else:
+                st = lib.dib_moe_up(o._ptr(x), c_int(1), o._ptr(order), *rest, o._ptr(weights), o._ptr(hidden), c_int(f),
+                                    c_int(w), o._stream())
+            assert st == 0
+            per_pair = torch.zeros(pairs, w, device="cuda")
+            assert lib.dib_moe_down(o._ptr(hidden), c_int(1), o._ptr(order), c_int(max_tiles), c_int(16), c_int(streams),
+                                    o._ptr(down), o._ptr(per_pair), c_int(f), c_int(w), o._stream()) == 0
+            outs += [hidden, per_pair]
+        got.append(outs)
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    assert bool((got[0][1] != 0).any())
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 40, 512), (5, 64, 1024), (70, 100, 1028)])
+def test_linear_fp32_numbers_that_bfloat16_cannot_hold(m, n, k):
+    """Infinities, not-a-numbers and the largest numbers come out as FMA gives them; numbers of all sizes keep float32's
+    accuracy."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(m, k, generator=g, device="cuda") * 2.0 ** torch.randint(-40, 40, (m, 1), generator=g, device="cuda")
+    w = torch.randn(n, k, generator=g, device="cuda") * 2.0 ** torch.randint(-40, 40, (n, 1), generator=g, device="cuda")
+    want = x.double() @ w.double().T
+    # the eight partials' chains of k / 128 sums and what the parts leave out, as in the test of the tiles
+    bound = (k / 8 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert ((ops().linear(x, w).double() - want).abs() <= bound).all()
+    x[:, 3], w[:, 3], w[0, 3] = 3.4e38, 0.0, 1.0                      # rounds up beyond bfloat16's range
+    w[1, 5], w[2, 7] = float("inf"), float("nan")
+    got, want = ops().linear(x, w), x @ w.T
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    assert torch.equal(got[torch.isinf(got)], want[torch.isinf(want)])
+    assert (got[:, 0].double() - (x.double() @ w.double().T)[:, 0]).abs().max() <= 3.4e38 * 2.0 ** -22
