@@ -287,13 +287,19 @@ class CacheManager:
         return out
 
     def reset_fresh_state(self) -> None:
-        """Zero the state rows of slots handed out since the last call."""
-        fresh = self.take_fresh_slots()
-        if fresh and self.state_groups:
-            idx = torch.tensor(fresh, dtype=torch.long, device=self.device)
-            for g in self.state_groups.values():
-                if g.array is not None:
-                    g.array[:, idx] = 0
+        """Zero the state rows of slots handed out since the last call: a fill for every run of neighbouring
+        slots, which the host issues without waiting for the GPU (slots come from a stack, so a batch that
+        comes together lies in a few runs)."""
+        fresh = sorted(self.take_fresh_slots())
+        if not fresh or not self.state_groups:
+            return
+        first = fresh[0]
+        for i, slot in enumerate(fresh):
+            if i + 1 == len(fresh) or fresh[i + 1] != slot + 1:
+                for g in self.state_groups.values():
+                    if g.array is not None:
+                        g.array[:, first:slot + 1].zero_()
+                first = fresh[i + 1] if i + 1 < len(fresh) else slot
 
     # ---- pages ---------------------------------------------------------------------
 
