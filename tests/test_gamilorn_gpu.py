@@ -320,6 +320,78 @@ def test_delta_rule_alone(dtype, heads, dim, rank):
     assert not torch.isnan(state[1:]).any()
 
 
+@pytest.mark.parametrize("heads, dim, rank", [(3, 64, 16), (2, 64, 65), (2, 128, 5)])
+@pytest.mark.parametrize("fast", [False, True])
+@pytest.mark.parametrize("kind", ["bfloat16", "float32", "split"])
+def test_the_delta_rule_in_chunks(heads, dim, rank, fast, kind, monkeypatch):
+    """Portions in chunks of 16 tokens beside decoded tokens and shorter portions, from states that are not zero: at both
+    sides of a chunk's edge, against 64 bits and against the token-by-token form; a sequence's bits do not depend on the
+    others'.  (Heads of 128 run in chunks from 48 tokens on, heads of 64 from 112.)"""
+    from deterministic_inference_b200.kernels import ops
+    g, dev, hd = torch.Generator().manual_seed(dim + rank), "cuda", heads * dim
+    lens = (1, 1, 2, 47, 48, 49, 111, 112, 113, 129, 160, 150)   # the last one on the padding's slot
+    slots = (7, 1, 2, 3, 4, 5, 6, 8, 9, 10, 11, 0)
+    w2 = pg.as_stored_bf16(torch.randn(hd, rank, generator=g))
+    w0, a_bias = torch.randn(hd, generator=g) + (6.0 if fast else -3.0), torch.randn(hd, generator=g)
+    norm_w = 1.0 + 0.1 * torch.randn(hd, generator=g)
+    projs = [pg.as_stored_bf16(torch.randn(n, 5 * hd + rank, generator=g)) for n in lens]
+    if fast:                                                     # decays at their fastest, e^(-0.6) a token
+        for p in projs:
+            p[:, 5 * hd:] = 0
+    first = torch.randn(12, heads, dim, dim, generator=g)
+    first[0] = float("nan")                                      # nobody's slot
+
+    def run(who):
+        state = first.to(dev)
+        x = torch.cat([projs[i] for i in who]).to(dev)
+        if kind == "bfloat16":
+            x = x.bfloat16()
+        if kind == "split":                                      # two parts whose sum is exact
+            x = ops.SplitSum(torch.stack([0.5 * x, 0.5 * x]), torch.float32)
+        cu = [0]
+        for i in who:
+            cu.append(cu[-1] + lens[i])
+        step = SimpleNamespace(cu_q_lens=torch.tensor(cu, dtype=torch.int32, device=dev), num_seqs=len(who),
+                               state_slots=torch.tensor([slots[i] for i in who], dtype=torch.int32, device=dev),
+                               num_decode=sum(lens[i] == 1 for i in who))
+        if kind == "bfloat16":                                   # (with the lengths unknown on the host both forms are launched)
+            step.q_lens = [lens[i] for i in who]
+        y = ops.delta_rule(x, w2.t().contiguous().to(dev), w0.to(dev), a_bias.to(dev), norm_w.to(dev), state, step, heads,
+                           dim, rank, math.exp(-0.5), 1e-6, 2e-5, torch.float32)
+        return [y[cu[j]:cu[j + 1]].cpu() for j in range(len(who))], state.cpu()
+
+    everyone = list(range(len(lens)))
+    got, state = run(everyone)
+    monkeypatch.setattr(ops, "DELTA_FORM", "1")
+    by_token, state_by_token = run(everyone)
+    monkeypatch.setattr(ops, "DELTA_FORM", "auto")
+    # what one order of the float32 sums differs from another by: a token's three sums of dim terms, over the tokens
+    # that a state still feels, as sums of squares grow; the root mean square divides both alike
+    bound = lambda n: 16 * 2.0 ** -24 * math.sqrt(dim + n)
+    for i, n in enumerate(lens):
+        p, shape = projs[i].double(), (n, heads, dim)
+        r, k, v, gate = (p[:, j * hd:(j + 1) * hd] for j in range(4))
+        rate = torch.sigmoid(p[:, 4 * hd:5 * hd] + a_bias.double()).view(shape)
+        decay = pg.decay_of(p[:, 5 * hd:], torch.eye(rank, dtype=torch.float64), w2.double(), w0.double()).view(shape)
+        start = first[slots[i]].double() if slots[i] else torch.zeros(heads, dim, dim, dtype=torch.float64)
+        r, k, v = r.reshape(shape), k.reshape(shape), v.reshape(shape)
+        unit, o, s = k / torch.sqrt((k ** 2).sum(-1, keepdim=True) + 1e-6), [], start
+        for t in range(n):
+            read = torch.einsum("hd,hde->he", unit[t], s)
+            s = decay[t][..., None] * s - (rate[t] * unit[t])[..., None] * read[:, None] + k[t][..., None] * v[t][:, None]
+            o.append(torch.einsum("hd,hde->he", r[t], s))
+        want = pg.unit_rms(torch.stack(o), 2e-5).reshape(n, hd) * norm_w.double() * torch.sigmoid(gate)
+        scale = float(want.abs().max())
+        assert float((got[i].double() - want).abs().max()) <= bound(n) * scale, (i, n)
+        assert float((by_token[i].double() - want).abs().max()) <= bound(n) * scale, (i, n)
+        if slots[i]:
+            for st in (state, state_by_token):
+                assert float((st[slots[i]].double() - s).abs().max()) <= bound(n) * float(s.abs().max()), (i, n)
+    assert torch.isnan(state[0]).all()
+    for i in (6, 7, 10):
+        assert torch.equal(run([i])[0][0], got[i]), i
+
+
 def prepared(proj, heads, dim, rank, w2_t, w0, a_bias):
     """The delta rule's vectors [tokens, heads, 6, dim] by the kernel; ``proj`` float32 or bfloat16 [tokens, width], or
     float32 split sums [splits, tokens, width]."""
