@@ -359,16 +359,18 @@ moe_product_mma_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __re
 // The same for few tiles of 16 rows (decoded tokens), where an expert's weights are read for a few rows
 // and the time is that of their bytes.  An item is 32 rows of B (mode 0: 16 of the gate and the same
 // 16 of up) against a tile; a warp multiplies 8 of the rows and brings them and the tile's A rows into
-// shared memory in runs of ST_K k, ST_STAGES - 1 runs ahead by asynchronous copies of whole 512-byte
-// pieces of a row.  Two CTAs an SM walk the items of the tiles in use, and the copies run on from an item
-// to the next, so that memory is idle at the kernel's start alone.  A row's sum is the same as above:
+// shared memory in runs of ST_K k, a run ahead by asynchronous copies of whole 512-byte
+// pieces of a row.  Four CTAs an SM walk the items of the tiles in use, and the copies run on from an item
+// to the next, so that memory is idle at the kernel's start alone.  (Four CTAs of two stages keep as much under way
+// as two of four, wait for one another less and share the items out more evenly: sort to combine, 16 experts
+// of 1,024 x 1,536, 8 tokens 30 against 38 us, 64 tokens 40 against 50; 8 of 4,096 x 4,096, 64 tokens 187 against 199.)  A row's sum is the same as above:
 // steps of 32 k, ascending, in the same permutation.  (Which of the two runs, and what both take:
 // product_times.)
-constexpr int ST_THREADS = 128, ST_B = 32, ST_A = 16, ST_K = 256, ST_STAGES = 4;
+constexpr int ST_THREADS = 128, ST_B = 32, ST_A = 16, ST_K = 256, ST_STAGES = 2;
 constexpr int ST_LD = ST_K + GP_PAD;
-constexpr int ST_CTAS = 2 * 148;          // two an SM
+constexpr int ST_CTAS = 4 * 148;          // four an SM
 constexpr int ST_STAGE = (ST_B + ST_A) * ST_LD;                    // elements
-__global__ void __launch_bounds__(ST_THREADS, 2)
+__global__ void __launch_bounds__(ST_THREADS, 4)
 moe_product_stream_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __restrict__ order, int max_tiles,
                           int top, const __nv_bfloat16* __restrict__ w, void* out, int K, int N, int mode, float limit,
                           float alpha) {
@@ -598,7 +600,7 @@ int launch_product_mma(const void* a_rows, const int* order, int max_tiles, int 
 
 int launch_product_stream(const void* a_rows, const int* order, int max_tiles, int top, const void* w, void* out, int K,
                           int N, int mode, float limit, float alpha, cudaStream_t st) {
-  constexpr size_t smem = sizeof(__nv_bfloat16) * ST_STAGES * ST_STAGE;      // 108 KB
+  constexpr size_t smem = sizeof(__nv_bfloat16) * ST_STAGES * ST_STAGE;      // 54 KB
   static DeviceOnce once;
   if (!once.done()) {
     if (cudaFuncSetAttribute(moe_product_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -615,19 +617,17 @@ int launch_product_stream(const void* a_rows, const int* order, int max_tiles, i
 }
 
 // Tiles of 16 rows: streamed weights for few tiles, whose other form has too few CTAs to fill the GPU and walks all
-// of K in one chain; that form for many, where its CTAs (four times as many an SM) hide one another's start and
-// end.  Both give the same bits.  The times are fits to single products, in us with weights from memory (registers /
-// streamed): 16 experts of 1,024 x 1,536, 8 tokens, up 20 / 19, down 24 / 10, 33 tokens 25 / 31 and 28 / 15; 64 of
-// 2,048 x 512, 4 tokens 37 / 31 and 14 / 22, 64 tokens 57 / 63 and 31 / 49; 8 of 4,096 x 4,096, 8 tokens 87 / 84 and
-// 71 / 43; 128 of 2,048 x 768, 64 tokens 145 / 182 and 78 / 107; 512 of 512 x 256, 64 tokens 40 / 80 and 19 / 55.  A
-// layer's two products take the same form: one behind the other they are slower in two forms than in either (sort
-// to combine, 16 experts of 1,024 x 1,536, 33 tokens: registers 58, streamed 50, up streamed 98, down streamed 68;
-// 64 of 2,048 x 512, 64 tokens: 94, 119, 122, 152).
+// of K in one chain; that form for many small ones, where its CTAs hide one another's start and end.  Both give
+// the same bits, and a layer's two products take the same form.  The times are fits, in us with weights from memory;
+// measured from the sort to the combination (registers / streamed): 16 experts of 1,024 x 1,536, 8 tokens 51 / 30, 64 tokens
+// 61 / 40; 64 of 2,048 x 512, 4 tokens 55 / 49, 16 tokens 79 / 87, 64 tokens 92 / 99; 8 of 4,096 x 4,096, 8 tokens
+// 158 / 127, 64 tokens 257 / 187; 128 of 2,048 x 768, 4 tokens 64 / 65, 64 tokens 228 / 253; 512 of 512 x 256, 8 tokens
+// 19 / 21, 64 tokens 64 / 75.
 void product_times(int tiles, int K, int rows_b, float& registers, float& streamed) {
   const float megabytes = 2e-6f * tiles * (float)K * (float)rows_b;
-  const float waves = (float)tiles * ((rows_b + ST_B - 1) / ST_B) / (2 * 148);
+  const float items = (float)tiles * ((rows_b + ST_B - 1) / ST_B);
   const float chain = 1.0f + 0.0137f * K + megabytes / 10.5f, bytes = 3.0f + megabytes / 5.0f;
-  streamed += (waves > 1.f ? waves : 1.f) * (2.0f + 0.0038f * K);
+  streamed += 5.5f + megabytes / 5.9f + 0.0015f * items;
   registers += chain > bytes ? chain : bytes;
 }
 
