@@ -237,30 +237,53 @@ latent_prepare_kernel(Source proj, long long row_width, T* __restrict__ q_out, T
                       const int* __restrict__ positions, const int* __restrict__ slot_mapping,
                       int T_tokens, int H, int Dn, int R, int C, int page_size, long long num_pages, int pairs,
                       float amp) {
-  pdl_prologue(proj.p);
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int slots = H + 1;
   const long long item = (long long)blockIdx.x * WARPS + warp;
-  if (item >= (long long)T_tokens * slots) return;
+  if (item >= (long long)T_tokens * slots) {
+    pdl_wait();
+    return;
+  }
   const int t = (int)(item / slots), s = (int)(item % slots);
   const long long row = (long long)t * row_width;
+  // The step's positions and slots do not change while its kernels run, the frequencies and the weight never: the
+  // angles of a lane's first elements, and where the row goes, are there before the projection is.
   const float pos = (float)positions[t];
   const int half = R / 2;
+  auto angle = [&](int d, float& c, float& sn) {
+    const float a = __fmul_rn(pos, freq[pairs ? d >> 1 : (d < half ? d : d - half)]);
+    c = __fmul_rn(amp, cosf(a));
+    sn = __fmul_rn(amp, sinf(a));
+  };
+  constexpr int EARLY = 2, KEEP = 8;
+  float ce[EARLY], se[EARLY];
+#pragma unroll
+  for (int i = 0; i < EARLY; ++i)
+    if (lane + 32 * i < R) angle(lane + 32 * i, ce[i], se[i]);
+  const int slot = s == 0 && cache != nullptr ? slot_mapping[t] : -1;
+  pdl_wait(proj.p);
   long long src;       // the R elements to rotate
   T* dst;
   if (s == 0) {
-    if (cache == nullptr) return;
-    const int slot = slot_mapping[t];
-    if (slot < 0 || slot >= num_pages * page_size) return;
+    if (cache == nullptr || slot < 0 || slot >= num_pages * page_size) return;
     T* crow = cache + (long long)slot * (C + R);
     const long long lat = row + (long long)H * (Dn + R);
     float ss = 0.f;
-    for (int d = lane; d < C; d += 32) {
-      const float v = round_to<T>(source_load(proj, lat + d));
-      ss = __fmaf_rn(v, v, ss);
+    float v[KEEP];                   // (asked for together; what does not fit is read again)
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) v[i] = lane + 32 * i < C ? round_to<T>(source_load(proj, lat + lane + 32 * i)) : 0.f;
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) ss = __fmaf_rn(v[i], v[i], ss);
+    for (int d = lane + 32 * KEEP; d < C; d += 32) {
+      const float x = round_to<T>(source_load(proj, lat + d));
+      ss = __fmaf_rn(x, x, ss);
     }
     const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)C + eps);
-    for (int d = lane; d < C; d += 32)
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+      if (lane + 32 * i < C) Elem<T>::store(crow + lane + 32 * i, v[i] * rstd * c_w[lane + 32 * i]);
+    for (int d = lane + 32 * KEEP; d < C; d += 32)
       Elem<T>::store(crow + d, round_to<T>(source_load(proj, lat + d)) * rstd * c_w[d]);
     src = lat + C;
     dst = crow + C;
@@ -268,13 +291,19 @@ latent_prepare_kernel(Source proj, long long row_width, T* __restrict__ q_out, T
     src = row + (long long)(s - 1) * (Dn + R) + Dn;
     dst = q_out + ((long long)t * H + (s - 1)) * (C + R) + C;
   }
-  for (int d = lane; d < R; d += 32) {
+  auto turn = [&](int d, float c, float sn) {
     const bool first = pairs ? (d & 1) == 0 : d < half;
-    const float a = __fmul_rn(pos, freq[pairs ? d >> 1 : (first ? d : d - half)]);
-    const float c = __fmul_rn(amp, cosf(a)), sn = __fmul_rn(amp, sinf(a));
     const float u = round_to<T>(source_load(proj, src + d));
     const float o = round_to<T>(source_load(proj, src + (pairs ? (d ^ 1) : (first ? d + half : d - half))));
     Elem<T>::store(dst + d, first ? __fmaf_rn(u, c, -__fmul_rn(o, sn)) : __fmaf_rn(u, c, __fmul_rn(o, sn)));
+  };
+#pragma unroll
+  for (int i = 0; i < EARLY; ++i)
+    if (lane + 32 * i < R) turn(lane + 32 * i, ce[i], se[i]);
+  for (int d = lane + 32 * EARLY; d < R; d += 32) {
+    float c, sn;
+    angle(d, c, sn);
+    turn(d, c, sn);
   }
 }
 

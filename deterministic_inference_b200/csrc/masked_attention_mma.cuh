@@ -357,10 +357,15 @@ masked_attention_decode_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, c
   __nv_bfloat16* Vs = in_keys ? Ks : Ks + 2 * KT * qs;                        // [2][KT][vs]
   __shared__ long long k_off[2][KT], v_off[2][KT];
   __shared__ float sm[DEC_WARPS][DEC_ROWS], sl[DEC_WARPS][DEC_ROWS];
-  pdl_prologue(q, cache, gate.p);
+  pdl_trigger();
+  // The step's lists, lengths, positions and block tables do not change while its kernels run: where the first
+  // two tiles' rows lie is found ahead of the wait (four trips to memory, one behind the other).
   const int g = blockIdx.y, b = tiles[3 * blockIdx.x], start = tiles[3 * blockIdx.x + 1];
   const int q_begin = cu_q_lens[b], q_len = cu_q_lens[b + 1] - q_begin;
-  if (start >= q_len) return;               // (the whole CTA: the sequence brings no such token)
+  if (start >= q_len) {                     // (the whole CTA: the sequence brings no such token)
+    pdl_wait();
+    return;
+  }
   const int t = q_begin + start;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, tig = lane & 3;
@@ -376,13 +381,12 @@ masked_attention_decode_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, c
   const int chunk = chunked ? blockIdx.z : 0;
   const int it_begin = chunked ? chunk * chunk_tiles : 0;
   const int it_end = (chunked && it_begin + chunk_tiles < n_tiles) ? it_begin + chunk_tiles : n_tiles;
-  if (it_begin >= n_tiles) return;          // (the whole CTA: no such chunk at this position)
+  if (it_begin >= n_tiles) {                // (the whole CTA: no such chunk at this position)
+    pdl_wait();
+    return;
+  }
 
   const int dchunks = D / 8, vchunks = VD / 8;
-  for (int idx = threadIdx.x; idx < DEC_ROWS * dchunks; idx += blockDim.x) {
-    const int r = idx / dchunks, ch = idx - r * dchunks;
-    copy16(Qs + r * qs + ch * 8, q + ((long long)t * Hq + g * R + (r < R ? r : 0)) * D + ch * 8, r < R);
-  }
   auto find_rows = [&](int it) {          // by the first KT threads, for tile `it` (if there is one)
     if (threadIdx.x < KT && it < it_end) {
       const int j = tile_at(it) * KT + threadIdx.x;
@@ -424,6 +428,11 @@ masked_attention_decode_mma_kernel(const __nv_bfloat16* q, __nv_bfloat16* out, c
 
   find_rows(it_begin);
   find_rows(it_begin + 1);
+  pdl_wait(q, cache, gate.p);
+  for (int idx = threadIdx.x; idx < DEC_ROWS * dchunks; idx += blockDim.x) {
+    const int r = idx / dchunks, ch = idx - r * dchunks;
+    copy16(Qs + r * qs + ch * 8, q + ((long long)t * Hq + g * R + (r < R ? r : 0)) * D + ch * 8, r < R);
+  }
   __syncthreads();
   load_tile(it_begin & 1);
   __syncthreads();              // the loop's first turn writes the entries that these copies read
@@ -575,13 +584,14 @@ __global__ void masked_attention_merge_kernel(const float* partial_o, const floa
                                               int mask_kind, int mask_size, int keep, Source gate,
                                               long long gate_row, long long gate_col, int gate_heads,
                                               int chunk_tiles, int max_chunks) {
-  pdl_prologue(partial_o, partial_ml, gate.p);
+  pdl_trigger();
   const int t = blockIdx.x, h = blockIdx.y;
-  const int pos = positions[t];
+  const int pos = positions[t];             // (as above: ahead of the wait)
   const int t_first = first_seen(pos, mask_kind, mask_size) / KT;
   const int n_tiles = kept_tiles(keep, t_first) + pos / KT - t_first + 1;
   int chunks = (n_tiles + chunk_tiles - 1) / chunk_tiles;
   if (chunks > max_chunks) chunks = max_chunks;
+  pdl_wait(partial_o, partial_ml, gate.p);
   const long long row = (long long)t * Hq + h;
   const float sl = sink != nullptr ? sink[h] * MA_LOG2E : MA_NEG_BIG;
   float M = sl;
