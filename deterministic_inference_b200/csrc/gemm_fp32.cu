@@ -1,45 +1,29 @@
-// True float32 matrix product on the CUDA cores: C[M,N] = A[M,K] * W[N,K]^T.
+// True float32 matrix product: C[M,N] = A[M,K] * W[N,K]^T.
 //
-// This is the matrix product of the 32-bit path: plain FMA, no tensor cores and
-// no reduced-precision mode.  From K = 512 on an output element is eight partial sums: k
-// belongs to partial (k / 4) % 8, each partial adds its k in index order, and the partials
-// are added one after the other.  Below, it is one chain over k in index order
-// (gemm_fp32_short_kernel).  The order is a function of K alone, whatever the tile, so a
-// row's result does not depend on M: the same token gives the same bits in any batch.
-// (Distance from 64-bit sums at K = 1024 .. 3072: 2.1e-7 .. 3.6e-7 of the norm.  The logits
-// of 204 rows through 28 layers came to 9.1e-7, against 2.1e-6 with one chain over all k.)
-//
-// Both operands lie k-contiguous, and stay so in shared memory (copied 16 bytes at a
-// time, two or three stages ahead).  The eight warps of a block share one output tile
-// and divide k, warp w taking the partial w, so that even a tile of few outputs keeps
-// an SM's four schedulers busy with large thread tiles.  A thread reads four k of a row
-// with one 16-byte load: 16 loads for 256 FMA at 8 x 8 outputs a thread.
-// Bound: shared-memory reads and FMA issue about equally (8 x 8 outputs a thread, two
-// blocks an SM: 1000 x 4096 x 1024 in 262 us, 52% of the FMA rate; paired FMA with
-// even and odd k in one instruction needs twice the accumulators, one block an SM:
-// 299 us); the weights' bytes for a few rows (8 x 151936 x 1024: 136 us, 4.6 TB/s).
+// This is the matrix product of the 32-bit path; no reduced-precision mode.  From K = 512 on the products run
+// on the tensor cores without giving up a bit of an operand: every float32 number is the exact sum of three
+// bfloat16 numbers (8 bits each; rounded to nearest, what is left, what is left of that), and of the nine
+// products of two such sums the six that matter are formed, the smallest first; the three left out are below
+// 2^-25 of the product.  k is cut into blocks of 64 and these into `parts(K)` runs.  The tensor core sums a
+// block from zero, in float32; a run adds its blocks up in index order with float32 additions outside the tensor
+// core, and the runs are added in order.  Below K = 512 an element is one chain of FMA over k in index order
+// (gemm_fp32_short_kernel).  The order is a function of K alone, whatever the tile, so a row's result does not
+// depend on M: the same token gives the same bits in any batch.  A result that is no finite number is formed
+// again by FMA from the operands (an infinity is no sum of three numbers).
+// (Distance from 64-bit sums at K = 1,024 .. 4,096: 0.97e-7 .. 1.1e-7 of the norm, where eight chains of FMA had 2.1e-7 ..
+// 4.1e-7.)
 #include "common.cuh"
 
 namespace {
 
-constexpr int WARPS = 8;             // k is divided over them: part of the order above
+constexpr int WARPS = 8;
 constexpr int THREADS = WARPS * 32;
+constexpr int TC_THREADS = THREADS + 32;       // (one more warp issues the products)
 
-template <int BM_, int BN_, int TM_, int TN_, int BK_, int STAGES_, int CTAS_>
-struct Tile {
-  static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, BK = BK_, STAGES = STAGES_, CTAS = CTAS_;
-  static constexpr int LM = BM / TM, LN = BN / TN;         // lanes over rows and columns
-  static constexpr int LD = BK + 4;                        // row of a stage: 8 rows start in 8 different bank groups
-  static constexpr int LDR = BN + 4;                       // row of a warp's sums
-  static constexpr int STAGE = (BM + BN) * LD;             // floats
-  static constexpr int SMEM = 4 * (STAGES * STAGE > WARPS * BM * LDR ? STAGES * STAGE : WARPS * BM * LDR);
-  static_assert(LM * LN == 32 && BK % (4 * WARPS) == 0, "a warp holds the tile; every warp has k in every stage");
-};
-
-// rows r0 .. r0 + ROWS - 1 (below `rows`), k0 .. k0 + BK - 1 (below K) of a [rows, K] matrix; zeros elsewhere
-template <int ROWS, int BK, int LD, bool VEC>
+// rows r0 .. r0 + ROWS - 1 (below `rows`), k0 .. k0 + COLS - 1 (below K) of a [rows, K] matrix; zeros elsewhere
+template <int ROWS, int COLS, int LD, bool VEC>
 __device__ __forceinline__ void copy_rows(float* dst, const float* __restrict__ src, int r0, int rows, int k0, int K) {
-  constexpr int E = VEC ? 4 : 1, PER = BK / E;             // elements a copy, copies a row
+  constexpr int E = VEC ? 4 : 1, PER = COLS / E;            // elements a copy, copies a row
   for (int i = threadIdx.x; i < ROWS * PER; i += THREADS) {
     const int r = i / PER, k = (i % PER) * E;
     const bool in = r0 + r < rows && k0 + k < K;
@@ -52,82 +36,262 @@ __device__ __forceinline__ void copy_rows(float* dst, const float* __restrict__ 
   }
 }
 
-template <typename C, bool VEC>
-__global__ void __launch_bounds__(THREADS, C::CTAS)
-gemm_fp32_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out,
-                 int M, int N, int K) {
-  extern __shared__ __align__(16) float smem[];
-  pdl_prologue(A, W);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ty = lane / C::LN, tx = lane % C::LN;
-  // row tiles lie next to one another: blocks that run together read the same weights
-  const int row_tiles = (M + C::BM - 1) / C::BM;
-  const int m0 = (int)(blockIdx.x % row_tiles) * C::BM, n0 = (int)(blockIdx.x / row_tiles) * C::BN;
-  const int steps = (K + C::BK - 1) / C::BK;
+// ---- tensor-core form.  A CTA takes 128 rows of W (the instruction's rows) by TOK rows of A (its columns) over a
+// run of k, the CTAs of a tile's runs are a thread-block cluster.  Per block of 64 k: every thread takes apart the
+// numbers it asked for a block earlier and leaves the three parts of both operands in shared memory in the layout
+// the instruction reads (rows of 128 bytes, 128-byte swizzle), one more thread issues the 24 products into one of two
+// accumulators in tensor memory (a warp of its own: it waits while the unit is busy), and while they run the accumulator of the block before is added to the sums in
+// registers.  At the end the cluster's CTAs add their sums through one another's shared memory, in run order.
+// Bound: by the trip of a block's operands to the registers (1.3 us a block of 16 to 64 rows; the products take
+// 0.8 us), then by taking them apart (1.9 us with 128 rows).  204 x 4,096 x 1,024: 74 us by FMA (52% of their rate), so 28;
+// 204 x 6,144 x 1,024 106 and 41; 204 x 1,024 x 3,072 57 and 22; one row of 1,024 x 3,072 21 and 18.
+constexpr int BN = 128, BK = 64, MAX_PARTS = 8;
+constexpr int PLANE_A = BN * BK * 2;                     // bytes of a part of W's rows
+__device__ int dib_gemm_fp32_error_word;
 
-  float acc[C::TM][C::TN];
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_commit(unsigned long long* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// D[tmem] (+)= A[smem] * B[smem]^T, both operands K-major
+__device__ __forceinline__ void tc_mma(unsigned tmem_d, unsigned long long desc_a, unsigned long long desc_b,
+                                       unsigned idesc, unsigned accum) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void tc_ld8(unsigned taddr, unsigned (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+// K-major bfloat16 tile of rows of 128 bytes with the 128-byte swizzle: 8-row groups lie 1024 bytes apart
+__device__ __forceinline__ unsigned long long smem_desc_sw128(unsigned addr) {
+  return (unsigned long long)((addr & 0x3FFFFu) >> 4) | (unsigned long long)(1024u >> 4) << 32 | 1ull << 46 | 2ull << 61;
+}
+__host__ __device__ constexpr unsigned make_idesc(int m, int n) {      // float32 accumulator, bfloat16 operands, both K-major
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(n >> 3) << 17) | ((unsigned)(m >> 4) << 24);
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_peer_smem(const float* local, unsigned rank) {
+  unsigned remote;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+// two float32 numbers as three pairs of bfloat16 numbers whose sums they are
+__device__ __forceinline__ void take_apart(float x, float y, unsigned (&part)[3]) {
 #pragma unroll
-  for (int i = 0; i < C::TM; ++i)
-#pragma unroll
-    for (int j = 0; j < C::TN; ++j) acc[i][j] = 0.f;
+  for (int i = 0; i < 3; ++i) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    part[i] = *reinterpret_cast<const unsigned*>(&h);
+    x = __fsub_rn(x, __uint_as_float(part[i] << 16));
+    y = __fsub_rn(y, __uint_as_float(part[i] & 0xffff0000u));
+  }
+}
 
-  auto fetch = [&](int s) {
-    if (s < steps) {
-      float* st = smem + (s % C::STAGES) * C::STAGE;
-      copy_rows<C::BM, C::BK, C::LD, VEC>(st, A, m0, M, s * C::BK, K);
-      copy_rows<C::BN, C::BK, C::LD, VEC>(st + C::BM * C::LD, W, n0, N, s * C::BK, K);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-#pragma unroll
-  for (int s = 0; s < C::STAGES - 1; ++s) fetch(s);
+template <int TOK> struct Tc {
+  static constexpr int PLANE_B = TOK * BK * 2;
+  static constexpr int STAGE = 3 * (PLANE_A + PLANE_B);
+  static constexpr int SUMS = TOK * BN * 4;              // the sums that a CTA leaves for its cluster
+  static constexpr int SMEM = (2 * STAGE > SUMS ? 2 * STAGE : SUMS) + 1024;      // (and the tiles' alignment)
+  static constexpr int CTAS = TOK <= 16 ? 2 : 1;
+  static constexpr int TMEM_COLS = 2 * TOK < 32 ? 32 : 2 * TOK;
+  static constexpr int ROWS_A = BN / 16, ROWS_B = TOK / 16;      // 16-byte pieces a thread has of a block's operands
+};
 
-  for (int s = 0; s < steps; ++s) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(C::STAGES - 2) : "memory");
-    __syncthreads();                 // stage s is there for all; stage s - 1 has been read by all
-    fetch(s + C::STAGES - 1);
-    const float* sa = smem + (s % C::STAGES) * C::STAGE;
-    const float* sw = sa + C::BM * C::LD;
-#pragma unroll
-    for (int k = 0; k < C::BK; k += 4 * WARPS) {
-      const int at = k + warp * 4;
-      float4 a[C::TM];
-#pragma unroll
-      for (int i = 0; i < C::TM; ++i)
-        a[i] = *reinterpret_cast<const float4*>(sa + (i * C::LM + ty) * C::LD + at);
-#pragma unroll
-      for (int j = 0; j < C::TN; ++j) {
-        const float4 b = *reinterpret_cast<const float4*>(sw + (j * C::LN + tx) * C::LD + at);
-#pragma unroll
-        for (int i = 0; i < C::TM; ++i) acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
-#pragma unroll
-        for (int i = 0; i < C::TM; ++i) acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
-#pragma unroll
-        for (int i = 0; i < C::TM; ++i) acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
-#pragma unroll
-        for (int i = 0; i < C::TM; ++i) acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+template <int TOK, bool VEC, bool FOLD>
+__global__ void __launch_bounds__(TC_THREADS, Tc<TOK>::CTAS)
+gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out, int M, int N,
+                    int K, int runs) {
+  using C = Tc<TOK>;
+  extern __shared__ unsigned char smem_dyn[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+  __shared__ unsigned long long done[2];                 // the products of the block in stage s have completed
+  __shared__ unsigned tmem_slot;
+  pdl_trigger();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.y * TOK, n0 = blockIdx.x * BN, part = blockIdx.z;
+  const int blocks = (K + BK - 1) / BK, per = (blocks + runs - 1) / runs, parts = FOLD ? 1 : runs;
+  const int kb0 = part * per, nkb = FOLD ? blocks : max(0, min(per, blocks - kb0));
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[0])));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[1])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"((unsigned)C::TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  // a thread's pieces: 4 k from 4 (tid % 16) of rows tid / 16 + 16 i
+  const int row = tid >> 4, c4 = tid & 15;
+  float4 a[C::ROWS_A], b[C::ROWS_B];
+  auto load = [&](const float* src, int r, int rows, int k) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < rows) {
+      const float* at = src + (size_t)r * K + k;
+      if (VEC) {
+        if (k < K) v = *reinterpret_cast<const float4*>(at);
+      } else {
+        if (k < K) v.x = at[0];
+        if (k + 1 < K) v.y = at[1];
+        if (k + 2 < K) v.z = at[2];
+        if (k + 3 < K) v.w = at[3];
       }
     }
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+    return v;
+  };
+  auto w_piece = [&](int kb, int i) { return load(W, n0 + row + 16 * i, N, (kb0 + kb) * BK + 4 * c4); };
+  auto a_piece = [&](int kb, int i) { return load(A, m0 + row + 16 * i, M, (kb0 + kb) * BK + 4 * c4); };
+  const bool mine = nkb > 0 && warp < WARPS;
+#pragma unroll
+  for (int i = 0; i < C::ROWS_A; ++i)
+    if (mine) a[i] = w_piece(0, i);    // (a constant: ahead of the wait)
+  pdl_wait(A);
+#pragma unroll
+  for (int i = 0; i < C::ROWS_B; ++i)
+    if (mine) b[i] = a_piece(0, i);
+  tc_fence_before();
   __syncthreads();
-  // the warps' sums meet in shared memory and are added in the warps' order
-  float* mine = smem + warp * C::BM * C::LDR;
+  tc_fence_after();
+  const unsigned tmem = tmem_slot;
+  // this thread's place in a part's tile: 8 bytes of row `row` (+ 16 i: the same swizzle)
+  const int at = row * 128 + (((c4 >> 1) ^ (row & 7)) << 4) + (c4 & 1) * 8;
+  constexpr unsigned idesc = make_idesc(BN, TOK);
+  constexpr int HALF = TOK / 2;        // a warp reads the rows 32 (warp % 4) .. of half of the columns
+  float sum[HALF];
 #pragma unroll
-  for (int i = 0; i < C::TM; ++i)
+  for (int j = 0; j < HALF; ++j) sum[j] = 0.f;
+  float total[FOLD ? HALF : 1];        // FOLD: of the runs before
+  bool dead = false;                   // a wait has run out: no more waits, the launch is reported as failed
+  auto add_block = [&](int kb) {
+    if (!dead && !mbar_wait(&done[kb & 1], (kb >> 1) & 1)) dead = true;
+    __syncwarp();
+    tc_fence_after();
+    const unsigned from = tmem + ((unsigned)((warp & 3) * 32) << 16) + (kb & 1) * TOK + (warp >> 2) * HALF;
 #pragma unroll
-    for (int j = 0; j < C::TN; ++j) {
-      mine[(i * C::LM + ty) * C::LDR + j * C::LN + tx] = acc[i][j];
+    for (int j = 0; j < HALF; j += 8) {
+      unsigned r[8];
+      tc_ld8(from + j, r);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sum[j + e] = __fadd_rn(sum[j + e], __uint_as_float(r[e]));
     }
-  __syncthreads();
-  for (int o = threadIdx.x; o < C::BM * C::BN; o += THREADS) {
-    const int r = o / C::BN, c = o % C::BN;
-    const float* p = smem + r * C::LDR + c;
-    float v = p[0];
+    tc_fence_before();
+    if (FOLD && ((kb + 1) % per == 0 || kb + 1 == nkb)) {
 #pragma unroll
-    for (int w = 1; w < WARPS; ++w) v = __fadd_rn(v, p[w * C::BM * C::LDR]);
-    if (m0 + r < M && n0 + c < N) out[(size_t)(m0 + r) * N + n0 + c] = v;
+      for (int j = 0; j < HALF; ++j) {
+        total[FOLD ? j : 0] = kb < per ? sum[j] : __fadd_rn(total[FOLD ? j : 0], sum[j]);
+        sum[j] = 0.f;
+      }
+    }
+  };
+  if (warp == WARPS) {
+    for (int kb = 0; kb < nkb; ++kb) {
+      __syncthreads();                 // block kb's parts are there; the accumulator of block kb - 2 has been read
+      if (lane == 0) {
+        tc_fence_after();
+        const unsigned stage = smem_u32(smem + (kb & 1) * C::STAGE);
+        const unsigned long long da = smem_desc_sw128(stage), db = smem_desc_sw128(stage + 3 * PLANE_A);
+        constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};      // the smallest products first
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+          for (int ks = 0; ks < BK / 16; ++ks)
+            tc_mma(tmem + (kb & 1) * TOK, da + ((PA[p] * PLANE_A + ks * 32) >> 4), db + ((PB[p] * C::PLANE_B + ks * 32) >> 4),
+                   idesc, p + ks > 0 ? 1u : 0u);
+        tc_commit(&done[kb & 1]);
+      }
+      __syncwarp();
+    }
+  } else {
+    for (int kb = 0; kb < nkb; ++kb) {
+      // the stage and the accumulator are free: the block before the last one has been added up
+      unsigned char* stage = smem + (kb & 1) * C::STAGE;
+      auto leave = [&](unsigned char* plane, int plane_bytes, const float4& v) {
+        unsigned lo[3], hi[3];
+        take_apart(v.x, v.y, lo);
+        take_apart(v.z, v.w, hi);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(plane + p * plane_bytes + at) = make_uint2(lo[p], hi[p]);
+      };
+#pragma unroll
+      for (int i = 0; i < C::ROWS_A; ++i) leave(stage + i * 16 * 128, PLANE_A, a[i]);
+#pragma unroll
+      for (int i = 0; i < C::ROWS_B; ++i) leave(stage + 3 * PLANE_A + i * 16 * 128, C::PLANE_B, b[i]);
+      if (kb + 1 < nkb) {
+#pragma unroll
+        for (int i = 0; i < C::ROWS_A; ++i) a[i] = w_piece(kb + 1, i);
+#pragma unroll
+        for (int i = 0; i < C::ROWS_B; ++i) b[i] = a_piece(kb + 1, i);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncthreads();
+      if (kb > 0) add_block(kb - 1);
+    }
+    if (nkb > 0) add_block(nkb - 1);
   }
+  if (dead) atomicExch(&dib_gemm_fp32_error_word, 1);
+  // the runs' sums, in run order; a CTA of the cluster takes a share of the tile's columns (rows of A)
+  __syncthreads();                     // (every product has completed: the stages are free)
+  float* sums = reinterpret_cast<float*>(smem);          // [TOK][128 rows of W]
+  if (warp < WARPS) {
+#pragma unroll
+    for (int j = 0; j < HALF; ++j) sums[((warp >> 2) * HALF + j) * BN + (warp & 3) * 32 + lane] = FOLD ? total[FOLD ? j : 0] : sum[j];
+  }
+  if (parts > 1) cluster_sync_all();
+  else __syncthreads();
+  const int cols = min(TOK, M - m0), share = (cols + parts - 1) / parts;
+  const int c_end = min(cols, (part + 1) * share);
+  for (int e = part * share * (BN / 4) + tid; e < c_end * (BN / 4); e += TC_THREADS) {
+    const int n = n0 + e % (BN / 4) * 4, m = m0 + e / (BN / 4);
+    const float* p = sums + 4 * e;
+    float4 v = *reinterpret_cast<const float4*>(p);
+    if (parts > 1) {
+      float4 run[MAX_PARTS];
+#pragma unroll
+      for (int r = 0; r < MAX_PARTS; ++r)
+        if (r < parts) run[r] = ld_peer_smem(p, r);
+      v = run[0];
+#pragma unroll
+      for (int r = 1; r < MAX_PARTS; ++r)
+        if (r < parts)
+          v = make_float4(__fadd_rn(v.x, run[r].x), __fadd_rn(v.y, run[r].y), __fadd_rn(v.z, run[r].z), __fadd_rn(v.w, run[r].w));
+    }
+    float o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n + i < N && !(fabsf(o[i]) <= 3.402823466e38f)) {      // an operand or a sum that bfloat16 parts cannot hold
+        const float *x = A + (size_t)m * K, *y = W + (size_t)(n + i) * K;
+        o[i] = 0.f;
+        for (int k = 0; k < K; ++k) o[i] = __fmaf_rn(x[k], y[k], o[i]);
+      }
+    float* to = out + (size_t)m * N + n;
+    if (n + 3 < N && (((uintptr_t)to) & 15) == 0) {
+      *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (n + i < N) to[i] = o[i];
+    }
+  }
+  __syncwarp();
+  if (parts > 1) cluster_sync_all();   // nobody leaves while a peer may still read its sums
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)C::TMEM_COLS));
 }
 
 // Short sums (K below SHORT_K): one chain over all k in index order, as there is little to divide; the
@@ -198,19 +362,36 @@ gemm_fp32_short_kernel(const float* __restrict__ A, const float* __restrict__ W,
     }
 }
 
-template <typename C, bool VEC>
-int launch_vec(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
+// Runs of k, a function of K alone (part of the order above).
+int runs_of(int K) { return K > 15 * BK ? 4 : 2; }
+template <int TOK, bool VEC, bool FOLD>
+int launch_form(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
+  using C = Tc<TOK>;
   static DeviceOnce once;
   if (!once.done()) {
-    if (cudaFuncSetAttribute(gemm_fp32_kernel<C, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(gemm_fp32_tc_kernel<TOK, VEC, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
+        cudaSuccess) {
       cudaGetLastError();
       return DIB_LAUNCH_FAILED;
     }
     once.mark();
   }
-  const long long blocks = (long long)ceil_div_host(M, C::BM) * ceil_div_host(N, C::BN);
-  if (blocks > 0x7fffffffll) return DIB_BAD_SIZE;
-  dib_launch(gemm_fp32_kernel<C, VEC>, dim3((unsigned)blocks), dim3(THREADS), C::SMEM, st, A, W, out, M, N, K);
+  const int runs = runs_of(K), parts = FOLD ? 1 : runs;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ceil_div_host(N, BN), ceil_div_host(M, TOK), parts);
+  cfg.blockDim = dim3(TC_THREADS);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = (unsigned)parts;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dib_pdl_enabled() ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, gemm_fp32_tc_kernel<TOK, VEC, FOLD>, A, W, out, M, N, K, runs);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
@@ -233,32 +414,31 @@ int launch_short(const float* A, const float* W, float* out, int M, int N, int K
 }
 // 16-byte copies want rows that start on 16 bytes
 bool takes_vectors(const float* A, const float* W, int K) { return K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0; }
-template <typename C>
+template <int TOK, bool FOLD>
 int launch(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
-  return takes_vectors(A, W, K) ? launch_vec<C, true>(A, W, out, M, N, K, st) : launch_vec<C, false>(A, W, out, M, N, K, st);
+  return takes_vectors(A, W, K) ? launch_form<TOK, true, FOLD>(A, W, out, M, N, K, st)
+                                : launch_form<TOK, false, FOLD>(A, W, out, M, N, K, st);
 }
-
-// The tiles, by rows and columns.  The choice: the tile whose fullest SM is done first.  With
-// q tiles on it that takes max(alone, q * busy): `alone` is one tile by itself (latency), `busy`
-// what a tile adds on an SM that has several; measured per 1024 k, in us.  (M = 64, N = 4096:
-// 8 x 32 38.9, 16 x 32 32.8, 32 x 32 28.7, 64 x 32 30.7 us a call; M = 212, N = 1024, K = 2048:
-// 16 x 32 57, 32 x 32 49, 64 x 32 51; a step of
-// 204 rows of a 28-layer model: 38.8 ms, against 67.1 ms with tiles of 64 x 64 x 16, one in flight.)  The rule
-// counts a B200's 148 SMs; every tile gives the same bits.
-using T64 = Tile<64, 32, 8, 8, 32, 3, 2>;
-using T32 = Tile<32, 32, 8, 4, 64, 3, 2>;
-using T16 = Tile<16, 32, 4, 4, 64, 3, 3>;
-using T8w = Tile<8, 64, 4, 4, 64, 4, 2>;
-using T8 = Tile<8, 32, 2, 4, 64, 4, 3>;
-
-template <typename C> float estimate(int M, int N, float alone, float busy) {
-  const long long tiles = (long long)ceil_div_host(M, C::BM) * ceil_div_host(N, C::BN);
-  const float q = (float)((tiles + 147) / 148);
-  return q * busy > alone ? q * busy : alone;
+// The rows of A a CTA takes: the tile whose last wave of CTAs is done first.  A CTA takes `fixed` us (launch, first
+// operands, the runs' sum) and `block` for each of its run's blocks; two CTAs of 16 rows fit an SM.  (204 rows, us with
+// 64 / 128 rows a CTA: N = 4,096, K = 1,024 42 / 28; 1,024, 2,048 17 / 21; 6,144, 1,024 63 / 41; 1,024, 3,072 22 / 28.)
+template <int TOK> float estimate(int M, int N, int K, float fixed, float block) {
+  const int runs = runs_of(K), per = (ceil_div_host(K, BK) + runs - 1) / runs;
+  const long long ctas = (long long)ceil_div_host(N, BN) * ceil_div_host(M, TOK) * runs, at_once = 148 * Tc<TOK>::CTAS;
+  return (float)((ctas + at_once - 1) / at_once) * (fixed + block * per);
 }
 
 }  // namespace
 
+// 0, or the code of a wait that ran out in a launch since the word was cleared (-1: it could not be read)
+extern "C" int dib_gemm_fp32_status() {
+  int v = 0;
+  return cudaMemcpyFromSymbol(&v, dib_gemm_fp32_error_word, sizeof(int)) == cudaSuccess ? v : -1;
+}
+extern "C" int dib_gemm_fp32_status_clear() {
+  const int zero = 0;
+  return cudaMemcpyToSymbol(dib_gemm_fp32_error_word, &zero, sizeof(int)) == cudaSuccess ? 0 : -1;
+}
 extern "C" int dib_gemm_fp32(const float* A, const float* W, float* out, int M, int N, int K,
                              cudaStream_t st) {
   if (M == 0 || N == 0) return DIB_OK;
@@ -266,16 +446,18 @@ extern "C" int dib_gemm_fp32(const float* A, const float* W, float* out, int M, 
   if (ceil_div_host(M, 64) > 65535) return DIB_BAD_SIZE;
   if (K < SHORT_K)
     return takes_vectors(A, W, K) ? launch_short<true>(A, W, out, M, N, K, st) : launch_short<false>(A, W, out, M, N, K, st);
-  const float cost[5] = {estimate<T8>(M, N, 7.f, 4.3f), estimate<T8w>(M, N, 10.f, 7.2f), estimate<T16>(M, N, 8.f, 6.3f),
-                         estimate<T32>(M, N, 13.f, 11.f), estimate<T64>(M, N, 22.f, 18.7f)};
+  // few rows of a wide product (the head): one CTA takes all runs, there are CTAs enough (5 x 151,936 x 1,024: 171 against
+  // 228 us)
+  if (M <= 16 && ceil_div_host(N, BN) >= 2 * 296) return launch<16, true>(A, W, out, M, N, K, st);
+  const float cost[4] = {estimate<16>(M, N, K, 3.2f, 1.25f), estimate<32>(M, N, K, 4.5f, 1.3f),
+                         estimate<64>(M, N, K, 5.7f, 1.4f), estimate<128>(M, N, K, 5.5f, 1.9f)};
   int best = 0;
-  for (int i = 1; i < 5; ++i)
+  for (int i = 1; i < 4; ++i)
     if (cost[i] < cost[best]) best = i;
   switch (best) {
-    case 0: return launch<T8>(A, W, out, M, N, K, st);
-    case 1: return launch<T8w>(A, W, out, M, N, K, st);
-    case 2: return launch<T16>(A, W, out, M, N, K, st);
-    case 3: return launch<T32>(A, W, out, M, N, K, st);
-    default: return launch<T64>(A, W, out, M, N, K, st);
+    case 0: return launch<16, false>(A, W, out, M, N, K, st);
+    case 1: return launch<32, false>(A, W, out, M, N, K, st);
+    case 2: return launch<64, false>(A, W, out, M, N, K, st);
+    default: return launch<128, false>(A, W, out, M, N, K, st);
   }
 }
