@@ -15,12 +15,12 @@
 // A block has 16 neighbouring (token, head of the group) queries of one key-value head,
 // or those of them that belong to one sequence: block (x, y) takes the y-th run of equal
 // sequences among the 16 and ends at once where there is none.  So the tile of keys and
-// values is read into shared memory once (the next one's copies are in flight meanwhile)
-// for up to 16 queries, four a warp: a prompt's queries share it, a decoding token has
-// a block of its own.  One warp per query with its keys read from global memory, a
-// 512-byte stride between lanes, was bound by the cache lines of those reads (4 decoding tokens and a
-// prompt's 200, up to 600 keys, 16 heads of 128: some 1,000 us a layer; so 22 us).
-// Bound now: the FMA and the shared-memory reads of its operands.
+// values is read into shared memory once (the next two tiles' copies are in flight meanwhile)
+// for up to 16 queries, two a warp: a prompt's queries share it, a decoding token has
+// a block of its own.  Bound: a warp's chain through a tile (dot products, two reductions over the
+// lanes, values), so the two queries of a warp go through it side by side and there are eight warps.  (16 heads
+// of 128, us a layer, with four warps of four queries one after the other and one tile under way / so: 200 tokens behind
+// 100 66 / 51, 300 behind 300 beside 8 of 1,000 keys 191 / 140, one token of 600 keys 50 / 46.)
 //
 // Cache layout of a layer: [num_pages, 2, num_kv_heads, page_size, head_dim].
 #include "common.cuh"
@@ -30,9 +30,9 @@
 namespace {
 
 constexpr int MAX_D = 256;
-constexpr int WARPS = 4, THREADS = WARPS * 32;
-constexpr int NQ = 4, ITEMS = WARPS * NQ;      // queries a warp, a block
-constexpr int KEYS = 32;
+constexpr int WARPS = 8, THREADS = WARPS * 32;
+constexpr int NQ = 2, ITEMS = WARPS * NQ;      // queries a warp, a block
+constexpr int KEYS = 32, BUFS = 3;             // keys of a tile; tiles in shared memory (two under way)
 constexpr float NEG_BIG = -1e30f;
 
 // floats between rows of a tile: rows padded to whole vectors, an odd number of vectors apart (the
@@ -42,7 +42,7 @@ __host__ __device__ __forceinline__ int row_stride(int D) {
   return 4 * (v + 1 + (v & 1));
 }
 __host__ __device__ __forceinline__ int smem_floats(int D) {
-  return 4 * KEYS * row_stride(D) + ITEMS * row_stride(D) + ITEMS * KEYS;
+  return 2 * BUFS * KEYS * row_stride(D) + ITEMS * row_stride(D) + ITEMS * KEYS;
 }
 
 // dot products of the lane's key with N queries, d in index order
@@ -66,7 +66,7 @@ __device__ __forceinline__ void dots(const float* krow, const float* q, int ld, 
 
 // NV: vectors of four dimensions a lane owns (1: D <= 128).  ASYNC: float32 rows on 16 bytes.
 template <typename T, int NV, bool ASYNC>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, NV == 1 ? 2 : 1)
 paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
                                const T* __restrict__ kv_cache,
                                const int* __restrict__ block_table, int max_blocks,
@@ -102,10 +102,10 @@ paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
   }
 
   const int ld = row_stride(D), vecs = (D + 3) / 4;
-  float* sk = smem;                                      // [2][KEYS][ld]
-  float* sv = sk + 2 * KEYS * ld;
-  float* sq = sv + 2 * KEYS * ld + warp * NQ * ld;       // this warp's queries
-  float* sp = smem + 4 * KEYS * ld + ITEMS * ld + warp * NQ * KEYS;
+  float* sk = smem;                                      // [BUFS][KEYS][ld]
+  float* sv = sk + BUFS * KEYS * ld;
+  float* sq = sv + BUFS * KEYS * ld + warp * NQ * ld;    // this warp's queries
+  float* sp = smem + 2 * BUFS * KEYS * ld + ITEMS * ld + warp * NQ * KEYS;
 
   // queries number warp, warp + WARPS, ... of the run are this warp's
   int nq = 0, first[NQ], pos[NQ];
@@ -130,12 +130,15 @@ paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
   const int row0 = threadIdx.x / vecs, col0 = threadIdx.x % vecs;
   const int row_step = THREADS / vecs, col_step = THREADS % vecs;
 
-  auto fetch = [&](int k0, int buf) {
+  // the lane's page of a tile, asked for a tile ahead of its copies
+  auto page_of = [&](int k0) {
     const int key = k0 + lane;
+    return key >= lo && key <= hi ? bt[key / page_size] : -1;
+  };
+  auto fetch = [&](int k0, int buf, int page) {
     long long off = -1;                                  // of the lane's key; rows nobody sees become zeros
-    if (key >= lo && key <= hi)
-      off = (long long)((size_t)bt[key / page_size] * page_stride + (size_t)kvh * head_stride +
-                        (size_t)(key % page_size) * D);
+    if (page >= 0)
+      off = (long long)((size_t)page * page_stride + (size_t)kvh * head_stride + (size_t)((k0 + lane) % page_size) * D);
     float* dk = sk + buf * KEYS * ld;
     float* dv = sv + buf * KEYS * ld;
     int r = row0, c = col0;
@@ -179,12 +182,21 @@ paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
   }
 
   const int begin = lo / KEYS * KEYS;
-  fetch(begin, 0);
+  const int page0 = page_of(begin), page1 = page_of(begin + KEYS);
+  int page = page_of(begin + 2 * KEYS);
+  fetch(begin, 0, page0);
+  fetch(begin + KEYS, 1, page1);                         // (a tile behind the last one: zeros)
   int buf = 0;
-  for (int k0 = begin; k0 <= hi; k0 += KEYS, buf ^= 1) {
-    if constexpr (ASYNC) asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                                     // tile k0 is there; the other buffer has been read
-    if (k0 + KEYS <= hi) fetch(k0 + KEYS, buf ^ 1);
+  for (int k0 = begin; k0 <= hi; k0 += KEYS, buf = buf + 1 == BUFS ? 0 : buf + 1) {
+    if constexpr (ASYNC) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();                                     // tile k0 is there; the one before has been read
+    if (k0 + KEYS <= hi) {
+      const int now = page;
+      page = page_of(k0 + 3 * KEYS);
+      fetch(k0 + 2 * KEYS, buf == 0 ? BUFS - 1 : buf - 1, now);
+    } else if constexpr (ASYNC) {
+      asm volatile("cp.async.commit_group;" ::: "memory");        // (keeps the count)
+    }
     if (nq == 0) continue;
     const float* krow = sk + (buf * KEYS + lane) * ld;
     float s[NQ];
@@ -192,26 +204,44 @@ paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
     else dots<NQ>(krow, sq, ld, vecs, s);
     const int key = k0 + lane;
     bool whole = true;                                   // every query of the warp sees the whole tile
+    // the queries side by side: one that sees none of the tile keeps its maximum and is scaled by one
+    float x[NQ], p[NQ], alpha[NQ];
 #pragma unroll
     for (int i = 0; i < NQ; ++i) {
-      if (i >= nq) break;
-      whole = whole && first[i] <= k0 && pos[i] >= k0 + KEYS - 1;
-      if (first[i] > k0 + KEYS - 1 || pos[i] < k0) continue;          // it sees none of it
-      const bool visible = key >= first[i] && key <= pos[i];
-      const float x = visible ? s[i] * scale : NEG_BIG;
-      const float m_new = fmaxf(m[i], warp_max(x));      // the tile holds at least one visible key
-      const float p = visible ? expf(x - m_new) : 0.f;
-      const float alpha = expf(m[i] - m_new);
-      l[i] = fmaf(l[i], alpha, warp_sum(p));
+      const bool live = i < nq;
+      whole = whole && (!live || (first[i] <= k0 && pos[i] >= k0 + KEYS - 1));
+      x[i] = live && key >= first[i] && key <= pos[i] ? s[i] * scale : NEG_BIG;
+      p[i] = x[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < NQ; ++i) p[i] = fmaxf(p[i], __shfl_xor_sync(0xffffffffu, p[i], o));
+    bool sees[NQ];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      sees[i] = i < nq && first[i] <= k0 + KEYS - 1 && pos[i] >= k0;
+      const float m_new = fmaxf(m[i], p[i]);             // (the tile holds a visible key where the query sees it)
+      p[i] = sees[i] && key >= first[i] && key <= pos[i] ? expf(x[i] - m_new) : 0.f;
+      alpha[i] = sees[i] ? expf(m[i] - m_new) : 1.f;
+      if (sees[i]) m[i] = m_new;
+      if (i < nq) sp[i * KEYS + lane] = p[i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < NQ; ++i) p[i] += __shfl_xor_sync(0xffffffffu, p[i], o);
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+      if (!sees[i]) continue;
+      l[i] = fmaf(l[i], alpha[i], p[i]);
 #pragma unroll
       for (int n = 0; n < NV; ++n) {
-        acc[i][n].x *= alpha;
-        acc[i][n].y *= alpha;
-        acc[i][n].z *= alpha;
-        acc[i][n].w *= alpha;
+        acc[i][n].x *= alpha[i];
+        acc[i][n].y *= alpha[i];
+        acc[i][n].z *= alpha[i];
+        acc[i][n].w *= alpha[i];
       }
-      m[i] = m_new;
-      sp[i * KEYS + lane] = p;
     }
     __syncwarp();
     // P.V: keys in order, a lane owns the dimensions 4 * lane ..
