@@ -512,6 +512,9 @@ decode_attention_stage1_kernel(const __nv_bfloat16* __restrict__ q,
 #ifndef DIB_LENGTHS_EARLY
 #define DIB_LENGTHS_EARLY 0
 #endif
+// UP: chunks whose partial results are asked for together.  Two (up to 32 splits, 4,096 keys, in one trip to memory)
+// where a step has few blocks; their registers would cost a step of many its blocks' places.
+template <int UP>
 __global__ void decode_attention_stage2_kernel(const float* __restrict__ part_o,
                                                const float* __restrict__ part_lse,
                                                const int* __restrict__ seq_lens,
@@ -529,10 +532,9 @@ __global__ void decode_attention_stage2_kernel(const float* __restrict__ part_o,
   merge_range(seq_lens[b], window, max_splits, s0, s1);
   const int c0 = s0 / CH, c1 = s1 / CH;
   if (DIB_LENGTHS_EARLY) pdl_wait(part_o, part_lse);
-  // the first two chunks' partial results together (up to 32 splits, 4,096 keys, in one trip to memory)
-  float lse_r[2][CH], o_r[2][CH][1];
+  float lse_r[UP][CH], o_r[UP][CH][1];
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+  for (int u = 0; u < UP; ++u)
 #pragma unroll
     for (int j = 0; j < CH; ++j) {
       const int s = (c0 + u) * CH + j;
@@ -542,17 +544,17 @@ __global__ void decode_attention_stage2_kernel(const float* __restrict__ part_o,
     }
   float M = NEG_BIG;
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+  for (int u = 0; u < UP; ++u)
 #pragma unroll
     for (int j = 0; j < CH; ++j) M = fmaxf(M, lse_r[u][j]);
-  for (int s = (c0 + 2) * CH; s <= s1; ++s) M = fmaxf(M, part_lse[row + s]);
+  for (int s = (c0 + UP) * CH; s <= s1; ++s) M = fmaxf(M, part_lse[row + s]);
   // a sink: exp(sink[head]) joins the denominator; without one the sum is left as it is (x + 0 = x)
   const float sink_w = sink != nullptr ? merge_weight(sink[h], M) : 0.f;
   bool first = true;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     float total[1] = {0.f}, total_den = 0.f, acc[1], den;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < UP; ++u) {
       if (c0 + u > c1) break;
       if (!first) {
 #pragma unroll
@@ -564,7 +566,7 @@ __global__ void decode_attention_stage2_kernel(const float* __restrict__ part_o,
       merge_chunk<1>(lse_r[u], o_r[u], c0 + u, s0, s1, M, acc, den);
       merge_add<1>(u == 0, acc, den, total, total_den);
     }
-    for (int c = c0 + 2; c <= c1; ++c) {
+    for (int c = c0 + UP; c <= c1; ++c) {
       float lse_c[CH], o_c[CH][1];
 #pragma unroll
       for (int j = 0; j < CH; ++j) {
@@ -687,7 +689,9 @@ static inline void launch_decode_merge(const float* part_o, const float* part_ls
                dim3(th, chunks < MERGE_GROUPS ? chunks : MERGE_GROUPS), 0, st,
                part_o, part_lse, seq_lens, (__nv_bfloat16*)out, max_splits, Hq, D, window, sink);
   else
-    dib_launch(decode_attention_stage2_kernel, dim3(num_seqs, Hq), dim3(th), 0, st, part_o, part_lse,
+    dib_launch(max_splits > MERGE_CH && (long long)num_seqs * Hq <= 4 * 148 ? &decode_attention_stage2_kernel<2>
+                                                                           : &decode_attention_stage2_kernel<1>,
+               dim3(num_seqs, Hq), dim3(th), 0, st, part_o, part_lse,
                seq_lens, (__nv_bfloat16*)out, max_splits, Hq, D, window, sink);
 }
 
