@@ -720,6 +720,7 @@ int dib_delta_recurrence_chunks(const void* proj, int kind, int splits, long lon
   if (T_ == 0 || B == 0) return DIB_OK;
   if (H < 1 || H > 65535 || R < 0 || R > 8192 || B > 0x7fffffff / 2 || !dib_delta_chunks_from(D, decay_scale)) return DIB_BAD_SIZE;
   if (w_dtype != 0 && w_dtype != 1) return DIB_BAD_DTYPE;
+  if (((uintptr_t)w2t | (uintptr_t)scratch) & 15) return DIB_BAD_ALIGN;
   const Source src = make_source(proj, kind, splits, stride);
   auto go = [&](auto size) -> int {
     constexpr int DD = decltype(size)::value;

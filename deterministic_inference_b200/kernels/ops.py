@@ -738,8 +738,8 @@ def gather_rows(x: torch.Tensor, index: torch.Tensor) -> torch.Tensor:
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None) -> torch.Tensor:
     """y = x @ weight^T; x [M, K], weight [N, K] (checkpoint layout), no bias.
 
-    float32: the package's own CUDA-core kernel (plain FMA, no TF32, fixed k
-    order, so a row's bits do not depend on the batch).  bfloat16: float32
+    float32: the package's own kernel (all bits of both operands, no TF32; the order of the
+    sums depends on K alone, so a row's bits do not depend on the batch).  bfloat16: float32
     accumulation on the tensor cores; ``out_dtype=torch.float32`` returns the
     accumulator unrounded (used for the logits).  With few rows and a split of k the
     bfloat16 product comes back as a ``SplitSum`` (see there)."""
@@ -1228,7 +1228,8 @@ def delta_rule(proj, w2_t: torch.Tensor, w0: torch.Tensor, a_bias, norm_weight: 
     o = torch.empty(t, num_heads, head_dim, dtype=torch.float32, device=dev)
     # portions of `start` tokens and more run in chunks, from the projection on; the others token by token.  Where a
     # step has both, each kernel leaves the other's sequences out by their length on the device
-    start = lib.dib_delta_chunks_from(c_int(head_dim), c_float(decay_scale)) if DELTA_FORM == "auto" else 0
+    start = lib.dib_delta_chunks_from(c_int(head_dim), c_float(decay_scale)) \
+        if DELTA_FORM == "auto" and w2_t.data_ptr() % 16 == 0 else 0
     forms, q_lens = delta_rule_forms(step), getattr(step, "q_lens", None)
     chunked = []
     for f in (f for f in forms if f[0] == 1 and start):
