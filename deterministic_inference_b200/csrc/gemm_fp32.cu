@@ -422,9 +422,14 @@ int launch(const float* A, const float* W, float* out, int M, int N, int K, cuda
 // The rows of A a CTA takes: the tile whose last wave of CTAs is done first.  A CTA takes `fixed` us (launch, first
 // operands, the runs' sum) and `block` for each of its run's blocks; two CTAs of 16 rows fit an SM.  (204 rows, us with
 // 64 / 128 rows a CTA: N = 4,096, K = 1,024 42 / 28; 1,024, 2,048 17 / 21; 6,144, 1,024 63 / 41; 1,024, 3,072 22 / 28.)
+// 16 rows are for 16 rows at most: above that another tile was the faster at each size measured (16 rows a CTA against the
+// best: 64 rows of 1,024, 3,072 26 / 20; 40 of 6,144, 1,024 30 / 21).  Their block takes longer in a grid of many CTAs; the
+// factor and the 74 are fitted, to 16 / 32 rows a CTA: one row of 1,024, 3,072 (32 CTAs) 18.2 / 19.0; of 4,096, 1,024 (128)
+// 10.7 / 9.5; 8 rows of 6,144, 1,024 (192) 12.0 / 18.1.
 template <int TOK> float estimate(int M, int N, int K, float fixed, float block) {
   const int runs = runs_of(K), per = (ceil_div_host(K, BK) + runs - 1) / runs;
   const long long ctas = (long long)ceil_div_host(N, BN) * ceil_div_host(M, TOK) * runs, at_once = 148 * Tc<TOK>::CTAS;
+  if (Tc<TOK>::CTAS == 2 && ctas > 74) block *= 1.55f;
   return (float)((ctas + at_once - 1) / at_once) * (fixed + block * per);
 }
 
@@ -446,10 +451,11 @@ extern "C" int dib_gemm_fp32(const float* A, const float* W, float* out, int M, 
   if (ceil_div_host(M, 64) > 65535) return DIB_BAD_SIZE;
   if (K < SHORT_K)
     return takes_vectors(A, W, K) ? launch_short<true>(A, W, out, M, N, K, st) : launch_short<false>(A, W, out, M, N, K, st);
-  // few rows of a wide product (the head): one CTA takes all runs, there are CTAs enough (5 x 151,936 x 1,024: 171 against
-  // 228 us)
+  // few rows of a wide product (the head): one CTA takes all runs, there are CTAs enough (5 x 151,936 x 1,024: 190 us; the
+  // two forms were chosen at 171 against 228 us, before the last change to the kernel.  All of the weights go through the
+  // registers to be split: the FMA kernel before took 126 us)
   if (M <= 16 && ceil_div_host(N, BN) >= 2 * 296) return launch<16, true>(A, W, out, M, N, K, st);
-  const float cost[4] = {estimate<16>(M, N, K, 3.2f, 1.25f), estimate<32>(M, N, K, 4.5f, 1.3f),
+  const float cost[4] = {M <= 16 ? estimate<16>(M, N, K, 3.2f, 1.25f) : 1e30f, estimate<32>(M, N, K, 4.5f, 1.3f),
                          estimate<64>(M, N, K, 5.7f, 1.4f), estimate<128>(M, N, K, 5.5f, 1.9f)};
   int best = 0;
   for (int i = 1; i < 4; ++i)
