@@ -18,7 +18,6 @@
 
 #include "source.cuh"
 #include "conv_tail.cuh"
-#include "delta_chunks.cuh"
 
 // proj row: [r | k | v | g | a_pre | lora hidden] = 5 * H * D + R columns; w2t [R][H * D] (the
 // decay map's second matrix, transposed: the threads of a block read consecutive elements).
@@ -283,7 +282,7 @@ template <int Q, int CPT> struct DeltaToken {      // a lane's part of a token's
 template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES, bool NEXT>
 __global__ void __launch_bounds__(32 * WARPS + 32)
 delta_recurrence_wide_kernel(const float* packed, float* state, long long slot_stride, float* o_out,
-                             const int* cu_q_lens, const int* state_slots, int below, int H, int D, int E) {
+                             const int* cu_q_lens, const int* state_slots, int H, int D, int E) {
   extern __shared__ __align__(16) float dr_smem[];           // [DR_STAGES][DR_TOKENS][6 Dp]
   constexpr int Q = MAXR / 4;
   constexpr int Dp = LANES * MAXR;             // D and E, padded with zeros
@@ -293,7 +292,7 @@ delta_recurrence_wide_kernel(const float* packed, float* state, long long slot_s
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_wait();                        // (launched in stream order; nothing is launched ahead of its end either)
   const int t0 = cu_q_lens[b], t1 = cu_q_lens[b + 1];
-  if (t1 <= t0 || t1 - t0 >= below) return;      // (longer portions run in chunks)
+  if (t1 <= t0) return;
   const int groups = (t1 - t0 + DR_TOKENS - 1) / DR_TOKENS;
   if (Dp != D || Dp != E) {
     for (int i = threadIdx.x; i < DR_STAGES * DR_TOKENS * SV; i += blockDim.x) dr_smem[i] = 0.f;   // the padding stays 0
@@ -620,7 +619,7 @@ static int launch_recurrence(const float* packed, float* state, long long slot_s
 
 template <int MAXR, int LANES, int CPT, int WARPS, int DR_TOKENS, int DR_STAGES, bool NEXT>
 static int launch_recurrence_wide(const float* packed, float* state, long long slot_stride, float* o_out,
-                                  const int* cu_q_lens, const int* state_slots, int below, int B, int H, int D, int E,
+                                  const int* cu_q_lens, const int* state_slots, int B, int H, int D, int E,
                                   cudaStream_t st) {
   constexpr int COLUMNS = 32 / LANES * CPT * WARPS;        // a block's
   constexpr size_t smem = sizeof(float) * DR_STAGES * DR_TOKENS * 6 * LANES * MAXR;    // 48 KB for 64, 96 for 128 and 256
@@ -640,7 +639,7 @@ static int launch_recurrence_wide(const float* packed, float* state, long long s
   cfg.blockDim = dim3(32 * WARPS + 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchKernelEx(&cfg, kernel, packed, state, slot_stride, o_out, cu_q_lens, state_slots, below, H, D, E);
+  cudaLaunchKernelEx(&cfg, kernel, packed, state, slot_stride, o_out, cu_q_lens, state_slots, H, D, E);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
@@ -678,83 +677,23 @@ int dib_delta_prepare(const void* proj, int kind, int splits, long long stride, 
 // sequence b of the step owns tokens cu_q_lens[b] .. cu_q_lens[b+1]-1 and the state slot
 // state_slots[b].  Slot 0 is no request's: a sequence on it starts from a zero state and leaves none.
 // packed [T][H][5 D + E].
-// form 1: a column's rows over 16 lanes (for steps of few sequences with many tokens; sequences of `below` tokens and
-// more are left out, 0: none), 0: over 4.
+// form 1: a column's rows over 16 lanes (for steps of few sequences with many tokens), 0: over 4.
 int dib_delta_recurrence(const float* packed, float* state, long long slot_stride, float* o_out,
-                         const int* cu_q_lens, const int* state_slots, int B, int H, int D, int E, int form, int below,
+                         const int* cu_q_lens, const int* state_slots, int B, int H, int D, int E, int form,
                          cudaStream_t st) {
   if (B == 0) return DIB_OK;
   if (H < 1 || H > 65535 || D < 1 || D > 256 || E < 1 || E > 256) return DIB_BAD_SIZE;
   const int big = D > E ? D : E;       // (the staging's pieces are counted for the larger of the two)
-  if (below <= 0) below = 0x7fffffff;
 #define DIB_DR(F, ...) return F<__VA_ARGS__>(packed, state, slot_stride, o_out, cu_q_lens, state_slots, B, H, D, E, st)
-#define DIB_DW(...) \
-  return launch_recurrence_wide<__VA_ARGS__>(packed, state, slot_stride, o_out, cu_q_lens, state_slots, below, B, H, D, E, st)
   if (form == 1) {
-    if (big <= 64) DIB_DW(4, 16, 1, 4, 16, 2, true);
-    if (big <= 128) DIB_DW(8, 16, 2, 4, 16, 2, true);
-    DIB_DW(16, 16, 2, 4, 8, 2, false);
+    if (big <= 64) DIB_DR(launch_recurrence_wide, 4, 16, 1, 4, 16, 2, true);
+    if (big <= 128) DIB_DR(launch_recurrence_wide, 8, 16, 2, 4, 16, 2, true);
+    DIB_DR(launch_recurrence_wide, 16, 16, 2, 4, 8, 2, false);
   }
   if (big <= 64) DIB_DR(launch_recurrence, 16, 8);
   if (big <= 128) DIB_DR(launch_recurrence, 32, 6);
   DIB_DR(launch_recurrence, 64, 4);
 #undef DIB_DR
-#undef DIB_DW
-}
-
-// Portions of prompts in chunks of 16 tokens (delta_chunks.cuh): the tokens from which on a portion takes that form with
-// heads of D and this decay; 0: none does.
-int dib_delta_chunks_from(int D, float decay_scale) {
-  return (D == 64 || D == 128) && fabsf(decay_scale) <= dchunks::CHUNK_DECAY ? dchunks::chunks_from(D) : 0;
-}
-// Their scratch: places for B sequences of T tokens in all, and float32 numbers of a place and head.
-int dib_delta_chunks_places(int T_, int B) { return T_ / dchunks::CH + B; }
-int dib_delta_chunks_floats(int D) { return D == 64 ? dchunks::Place<64>::FLOATS : dchunks::Place<128>::FLOATS; }
-// The per-token vectors and the recurrence of dib_delta_prepare and dib_delta_recurrence, from the projection to o_out,
-// for those of the B sequences of cu_q_lens (T tokens in all; the boundaries count tokens of the whole step, as proj and
-// o_out do) that have dib_delta_chunks_from tokens.
-int dib_delta_recurrence_chunks(const void* proj, int kind, int splits, long long stride, const void* w2t, int w_dtype,
-                                const float* w0, const float* a_bias, float* scratch, float* state, long long slot_stride,
-                                float* o_out, const int* cu_q_lens, const int* state_slots, int T_, int B, int H, int D,
-                                int R, float decay_scale, float key_eps, cudaStream_t st) {
-  if (T_ == 0 || B == 0) return DIB_OK;
-  if (H < 1 || H > 65535 || R < 0 || R > 8192 || B > 0x7fffffff / 2 || !dib_delta_chunks_from(D, decay_scale)) return DIB_BAD_SIZE;
-  if (w_dtype != 0 && w_dtype != 1) return DIB_BAD_DTYPE;
-  if (((uintptr_t)w2t | (uintptr_t)scratch) & 15) return DIB_BAD_ALIGN;
-  const Source src = make_source(proj, kind, splits, stride);
-  auto go = [&](auto size) -> int {
-    constexpr int DD = decltype(size)::value;
-    auto* prepare = kind == 1 ? (w_dtype == 1 ? &dchunks::chunk_prepare_kernel<DD, 1, 1> : &dchunks::chunk_prepare_kernel<DD, 1, 0>)
-                    : splits > 1 ? (w_dtype == 1 ? &dchunks::chunk_prepare_kernel<DD, 2, 1> : &dchunks::chunk_prepare_kernel<DD, 2, 0>)
-                                 : (w_dtype == 1 ? &dchunks::chunk_prepare_kernel<DD, 0, 1> : &dchunks::chunk_prepare_kernel<DD, 0, 0>);
-    dib_launch(prepare, dim3(dib_delta_chunks_places(T_, B), H), dim3(2 * DD), 0, st, src, w2t, w0, a_bias, scratch,
-               cu_q_lens, B, dchunks::chunks_from(DD), H, R, decay_scale, key_eps);
-    DIB_CHECK_LAUNCH();
-    auto walk = [&](auto cpt) -> int {
-      constexpr int CPT = decltype(cpt)::value;
-      auto* kernel = &dchunks::chunk_walk_kernel<DD, CPT>;
-      constexpr size_t smem = dchunks::walk_smem<DD, CPT>();
-      static DeviceOnce once;
-      if (!once.done()) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-          return DIB_LAUNCH_FAILED;
-        once.mark();
-      }
-      // (in plain stream order, as the walk token by token: see launch_recurrence_wide)
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(B, H, DD / (dchunks::COLS * CPT));
-      cfg.blockDim = dim3(2 * DD + 32);
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = st;
-      cudaLaunchKernelEx(&cfg, kernel, (const float*)scratch, state, slot_stride, o_out, cu_q_lens, state_slots,
-                         dchunks::chunks_from(DD), H);
-      DIB_CHECK_LAUNCH();
-      return DIB_OK;
-    };
-    // (one sequence of 2,048 tokens, 16 heads of 64: one column a thread 145 us, two 181; four of them 502 and 446)
-    return (long long)B * H * (DD / dchunks::COLS) > 148 ? walk(std::integral_constant<int, 2>{}) : walk(std::integral_constant<int, 1>{});
-  };
-  return D == 64 ? go(std::integral_constant<int, 64>{}) : go(std::integral_constant<int, 128>{});
 }
 
 int dib_delta_output(const float* o, const void* proj, int kind, int splits, long long stride,

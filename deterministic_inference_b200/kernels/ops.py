@@ -1225,42 +1225,18 @@ def delta_rule(proj, w2_t: torch.Tensor, w0: torch.Tensor, a_bias, norm_weight: 
     lib = _lib("delta_rule")
     src = _source_args(proj)
     dev = state.device
+    packed = torch.empty(t, num_heads, 6, head_dim, dtype=torch.float32, device=dev)
+    st = lib.dib_delta_prepare(*src, _ptr(w2_t), c_int(_dt(w2_t, "w2_t")), _ptr(w0), _ptr(a_bias), _ptr(packed),
+                               c_int(t), c_int(num_heads), c_int(head_dim), c_int(lora_rank),
+                               c_float(decay_scale), c_float(key_eps), _stream())
+    _check(st, "delta_rule(prepare)", f"heads {num_heads} of {head_dim}, rank {lora_rank}")
     o = torch.empty(t, num_heads, head_dim, dtype=torch.float32, device=dev)
-    # portions of `start` tokens and more run in chunks, from the projection on; the others token by token.  Where a
-    # step has both, each kernel leaves the other's sequences out by their length on the device
-    start = lib.dib_delta_chunks_from(c_int(head_dim), c_float(decay_scale)) \
-        if DELTA_FORM == "auto" and w2_t.data_ptr() % 16 == 0 else 0
-    forms, q_lens = delta_rule_forms(step), getattr(step, "q_lens", None)
-    chunked = []
-    for f in (f for f in forms if f[0] == 1 and start):
-        lens = q_lens[f[1]:f[1] + f[2]] if q_lens is not None else [0, start]
-        chunked += [f] if max(lens) >= start else []
-        forms = [x for x in forms if x != f or min(lens) < start]
-    # (a decoded sequence, in front of the portions, is one token)
-    decoded = sum(count for form, _, count in forms if form == 0) if chunked else 0
-    if forms:
-        vectors = decoded if chunked and all(form == 0 for form, _, _ in forms) else t
-        packed = torch.empty(vectors, num_heads, 6, head_dim, dtype=torch.float32, device=dev)
-        st = lib.dib_delta_prepare(*src, _ptr(w2_t), c_int(_dt(w2_t, "w2_t")), _ptr(w0), _ptr(a_bias), _ptr(packed),
-                                   c_int(vectors), c_int(num_heads), c_int(head_dim), c_int(lora_rank),
-                                   c_float(decay_scale), c_float(key_eps), _stream())
-        _check(st, "delta_rule(prepare)", f"heads {num_heads} of {head_dim}, rank {lora_rank}")
-    for form, first, count in forms:
+    for form, first, count in delta_rule_forms(step):
         st = lib.dib_delta_recurrence(_ptr(packed), _ptr(state), c_longlong(num_heads * head_dim * head_dim),
                                       _ptr(o), c_void_p(step.cu_q_lens.data_ptr() + 4 * first),
                                       c_void_p(step.state_slots.data_ptr() + 4 * first), c_int(count),
-                                      c_int(num_heads), c_int(head_dim), c_int(head_dim), c_int(form),
-                                      c_int(start), _stream())
+                                      c_int(num_heads), c_int(head_dim), c_int(head_dim), c_int(form), _stream())
         _check(st, "delta_rule(recurrence)", f"heads of {head_dim} (at most 256)")
-    for _, first, count in chunked:
-        scratch = torch.empty(lib.dib_delta_chunks_places(c_int(t - decoded), c_int(count)), num_heads,
-                              lib.dib_delta_chunks_floats(c_int(head_dim)), dtype=torch.float32, device=dev)
-        st = lib.dib_delta_recurrence_chunks(
-            *src, _ptr(w2_t), c_int(_dt(w2_t, "w2_t")), _ptr(w0), _ptr(a_bias), _ptr(scratch), _ptr(state),
-            c_longlong(num_heads * head_dim * head_dim), _ptr(o), c_void_p(step.cu_q_lens.data_ptr() + 4 * first),
-            c_void_p(step.state_slots.data_ptr() + 4 * first), c_int(t - decoded), c_int(count), c_int(num_heads),
-            c_int(head_dim), c_int(lora_rank), c_float(decay_scale), c_float(key_eps), _stream())
-        _check(st, "delta_rule(chunks)", f"heads {num_heads} of {head_dim}, rank {lora_rank}", kernels=2)
     out = torch.empty(t, hd, dtype=out_dtype, device=dev)
     st = lib.dib_delta_output(_ptr(o), *src, _ptr(norm_weight), _ptr(out), c_int(_DT[out_dtype]), c_int(t),
                               c_int(num_heads), c_int(head_dim), c_int(lora_rank), c_float(norm_eps), _stream())
@@ -1313,7 +1289,7 @@ def gated_delta_rule(proj, conv_weight: torch.Tensor, a_log: torch.Tensor, dt_bi
         st = lib.dib_delta_recurrence(_ptr(packed), _ptr(state), c_longlong(slot_stride), _ptr(o),
                                       c_void_p(step.cu_q_lens.data_ptr() + 4 * first),
                                       c_void_p(step.state_slots.data_ptr() + 4 * first), c_int(count),
-                                      c_int(h), c_int(d), c_int(e), c_int(form), c_int(0), _stream())
+                                      c_int(h), c_int(d), c_int(e), c_int(form), _stream())
         _check(st, "gated_delta_rule(recurrence)", f"heads of {d}/{e} (at most 256)")
     out = torch.empty(t, h * e, dtype=out_dtype, device=dev)
     st = lib.dib_gated_delta_output(_ptr(o), *src, c_longlong(width), _ptr(norm_weight), _ptr(out),

@@ -323,10 +323,9 @@ def test_delta_rule_alone(dtype, heads, dim, rank):
 @pytest.mark.parametrize("heads, dim, rank", [(3, 64, 16), (2, 64, 65), (2, 128, 5)])
 @pytest.mark.parametrize("fast", [False, True])
 @pytest.mark.parametrize("kind", ["bfloat16", "float32", "split"])
-def test_the_delta_rule_in_chunks(heads, dim, rank, fast, kind, monkeypatch):
-    """Portions in chunks of 16 tokens beside decoded tokens and shorter portions, from states that are not zero: at both
-    sides of a chunk's edge, against 64 bits and against the token-by-token form; a sequence's bits do not depend on the
-    others'.  (Heads of 128 run in chunks from 48 tokens on, heads of 64 from 112.)"""
+def test_the_delta_rule_of_portions(heads, dim, rank, fast, kind, monkeypatch):
+    """Portions of many lengths beside decoded tokens, from states that are not zero, against 64 bits, in the portions'
+    form for all sequences too; a sequence's bits do not depend on the others'."""
     from deterministic_inference_b200.kernels import ops
     g, dev, hd = torch.Generator().manual_seed(dim + rank), "cuda", heads * dim
     lens = (1, 1, 2, 47, 48, 49, 111, 112, 113, 129, 160, 150)   # the last one on the padding's slot
@@ -354,8 +353,6 @@ def test_the_delta_rule_in_chunks(heads, dim, rank, fast, kind, monkeypatch):
         step = SimpleNamespace(cu_q_lens=torch.tensor(cu, dtype=torch.int32, device=dev), num_seqs=len(who),
                                state_slots=torch.tensor([slots[i] for i in who], dtype=torch.int32, device=dev),
                                num_decode=sum(lens[i] == 1 for i in who))
-        if kind == "bfloat16":                                   # (with the lengths unknown on the host both forms are launched)
-            step.q_lens = [lens[i] for i in who]
         y = ops.delta_rule(x, w2.t().contiguous().to(dev), w0.to(dev), a_bias.to(dev), norm_w.to(dev), state, step, heads,
                            dim, rank, math.exp(-0.5), 1e-6, 2e-5, torch.float32)
         return [y[cu[j]:cu[j + 1]].cpu() for j in range(len(who))], state.cpu()
@@ -390,6 +387,67 @@ def test_the_delta_rule_in_chunks(heads, dim, rank, fast, kind, monkeypatch):
     assert torch.isnan(state[0]).all()
     for i in (6, 7, 10):
         assert torch.equal(run([i])[0][0], got[i]), i
+
+
+@pytest.mark.parametrize("heads, dim, rank", [(3, 64, 16), (2, 128, 5), (1, 200, 2)])
+@pytest.mark.parametrize("kind", ["bfloat16", "float32", "split"])
+def test_the_delta_rule_does_not_see_where_a_prompt_is_cut(heads, dim, rank, kind):
+    """A prompt in one portion and in portions of every kind (two tokens, odd ones, multiples of 16): equal bits of every
+    token's output and of the state.  The scheduler cuts a prompt to what other requests leave of a step's tokens."""
+    from deterministic_inference_b200.kernels import ops
+    g, dev, hd, n = torch.Generator().manual_seed(dim + rank), "cuda", heads * dim, 420
+    w2 = pg.as_stored_bf16(torch.randn(rank, hd, generator=g)).to(dev)
+    w0, a_bias, norm_w = ((torch.randn(hd, generator=g) + x).to(dev) for x in (-3.0, 0.0, 1.0))
+    proj = pg.as_stored_bf16(torch.randn(n, 5 * hd + rank, generator=g)).to(dev)
+    first = torch.randn(2, heads, dim, dim, generator=g).to(dev)
+
+    def run(cuts):
+        state, out = first.clone(), []
+        for a, b in zip(cuts, cuts[1:]):
+            x = proj[a:b].bfloat16() if kind == "bfloat16" else proj[a:b].contiguous()
+            if kind == "split":
+                x = ops.SplitSum(torch.stack([0.5 * x, 0.5 * x]), torch.float32)
+            step = SimpleNamespace(cu_q_lens=torch.tensor([0, b - a], dtype=torch.int32, device=dev), num_seqs=1,
+                                   state_slots=torch.tensor([1], dtype=torch.int32, device=dev), num_decode=0, q_lens=[b - a])
+            out.append(ops.delta_rule(x, w2, w0, a_bias, norm_w, state, step, heads, dim, rank, math.exp(-0.5), 1e-6, 2e-5,
+                                      torch.float32))
+        return torch.cat(out), state
+
+    whole, state = run([0, n])
+    for cuts in ([0, 256, n], [0, 100, 300, n], [0, 333, n], [0, 2, 5, 117, n], [0, 129, 131, 250, n]):
+        y, s = run(cuts)
+        assert torch.equal(y, whole) and torch.equal(s, state), cuts
+
+
+def test_bits_of_a_token_do_not_depend_on_its_portion_without_the_library(tmp_path):
+    """Under ``library_products=False`` the logits of a request in portions of 512 and of 100 are equal bit for bit."""
+    from deterministic_inference_b200 import EngineConfig
+    from deterministic_inference_b200.engine.batch import SequenceInput
+    from deterministic_inference_b200.engine.runner import ModelRunner
+    from deterministic_inference_b200.config import GamilornConfig
+    from deterministic_inference_b200.kernels import gemm_bf16
+    from deterministic_inference_b200.weights import write_random_model
+    layer = {"type": "parallel", "mlp": {"kind": "dense", "ff": 256},
+             "mixer": {"left": {"heads": 2, "kv_heads": 1, "dim": 64, "vdim": 64, "scale": 0.125,
+                                "mask": {"size": 150, "keep_first": 3}},
+                       "left_scale": 1.0, "right": {"heads": 4, "dim": 64, "decay_rank": 16}, "right_scale": 1.0}}
+    write_random_model(GamilornConfig.from_dict({"architecture": "Gamilorn", "vocab": 160, "width": 256, "max_positions": 1024,
+                                                 "norm": {"eps": 1e-5}, "logit_softcap": 30.0,
+                                                 "layers": [layer, layer]}), 57, tmp_path)
+    tokens = torch.randint(0, 160, (612,), generator=torch.Generator().manual_seed(58)).tolist()
+    rows = {}
+    try:
+        for portion in (512, 100):
+            r = ModelRunner(EngineConfig(model_path=str(tmp_path), dtype="bfloat16", kv_pool_tokens=2048, page_size=16,
+                                         max_reqs=4, max_seq_len=1024, cuda_graphs=False, library_products=False))
+            slot, got = r.cache.allocate_slot(), []
+            for c in range(0, len(tokens), portion):
+                n = min(portion, len(tokens) - c)
+                got.append(r.step([SequenceInput(slot, tokens[c:c + n], c, list(range(n)))])[0].clone())
+            rows[portion] = torch.cat(got)
+    finally:
+        gemm_bf16.set_library_products(True)
+    assert torch.equal(rows[512], rows[100])
 
 
 def prepared(proj, heads, dim, rank, w2_t, w0, a_bias):
