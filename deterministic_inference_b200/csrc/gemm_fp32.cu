@@ -110,6 +110,49 @@ template <int TOK> struct Tc {
   static constexpr int ROWS_A = BN / 16, ROWS_B = TOK / 16;      // 16-byte pieces a thread has of a block's operands
 };
 
+// The results that a CTA's `odd` marks (columns c0 .. c_end - 1 of its tile), by FMA from the operands.  A row of A that holds
+// a not-a-number has no other result; the others are sums over k by a warp for four columns, a chain a lane, the lanes by
+// the butterfly.  (us, 4,096 x 1,024, finite / one not-a-number in each row / an infinity in one row: 1 row 10 / 16 / 25, 204 rows
+// 27 / 75 / 39; all 204 rows with an infinity 476.  By the thread of each result 140, 3,730 and 156.)  A function of its own,
+// called: in the kernel it takes registers from the loop (204 rows 28 -> 30 us).
+__device__ __noinline__ void odd_results(const float* A, const float* W, float* out, unsigned char* odd, int m0, int n0,
+                                         int c0, int c_end, int N, int K) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int c = c0 + warp; c < c_end; c += TC_THREADS / 32) {
+    const unsigned bits = odd[c * (BN / 4) + lane];
+    if (!__any_sync(0xffffffffu, bits != 0)) continue;
+    const float* x = A + (size_t)(m0 + c) * K;
+    bool nan = false;
+#pragma unroll 8
+    for (int k = lane; k < K; k += 32) nan = nan || x[k] != x[k];
+    if (!__any_sync(0xffffffffu, nan)) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (bits >> i & 1) out[(size_t)(m0 + c) * N + n0 + lane * 4 + i] = __int_as_float(0x7fffffff);
+    odd[c * (BN / 4) + lane] = 0;
+  }
+  __syncthreads();
+  for (int e = c0 * (BN / 4) + warp; e < c_end * (BN / 4); e += TC_THREADS / 32) {
+    const unsigned bits = odd[e];
+    if (bits == 0) continue;
+    const int n = n0 + e % (BN / 4) * 4, m = m0 + e / (BN / 4);
+    const float *x = A + (size_t)m * K, *y[4];
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[i] = W + (size_t)min(n + i, N - 1) * K;
+#pragma unroll 4
+    for (int k = lane; k < K; k += 32) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] = __fmaf_rn(x[k], y[i][k], s[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      s[i] = warp_sum(s[i]);
+      if (lane == i && (bits >> i & 1)) out[(size_t)m * N + n + i] = s[i];
+    }
+  }
+}
+
 template <int TOK, bool VEC, bool FOLD>
 __global__ void __launch_bounds__(TC_THREADS, Tc<TOK>::CTAS)
 gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out, int M, int N,
@@ -119,6 +162,7 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
   __shared__ unsigned long long done[2];                 // the products of the block in stage s have completed
   __shared__ unsigned tmem_slot;
+  __shared__ unsigned char odd[TOK * (BN / 4)];          // of four neighbouring results: those that are no finite numbers
   pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * TOK, n0 = blockIdx.x * BN, part = blockIdx.z;
@@ -254,6 +298,7 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   else __syncthreads();
   const int cols = min(TOK, M - m0), share = (cols + parts - 1) / parts;
   const int c_end = min(cols, (part + 1) * share);
+  bool any = false;
   for (int e = part * share * (BN / 4) + tid; e < c_end * (BN / 4); e += TC_THREADS) {
     const int n = n0 + e % (BN / 4) * 4, m = m0 + e / (BN / 4);
     const float* p = sums + 4 * e;
@@ -269,14 +314,13 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
         if (r < parts)
           v = make_float4(__fadd_rn(v.x, run[r].x), __fadd_rn(v.y, run[r].y), __fadd_rn(v.z, run[r].z), __fadd_rn(v.w, run[r].w));
     }
-    float o[4] = {v.x, v.y, v.z, v.w};
+    const float o[4] = {v.x, v.y, v.z, v.w};
+    unsigned bits = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (n + i < N && !(fabsf(o[i]) <= 3.402823466e38f)) {      // an operand or a sum that bfloat16 parts cannot hold
-        const float *x = A + (size_t)m * K, *y = W + (size_t)(n + i) * K;
-        o[i] = 0.f;
-        for (int k = 0; k < K; ++k) o[i] = __fmaf_rn(x[k], y[k], o[i]);
-      }
+    for (int i = 0; i < 4; ++i)      // an operand or a sum that bfloat16 parts cannot hold
+      if (n + i < N && !(fabsf(o[i]) <= 3.402823466e38f)) bits |= 1u << i;
+    odd[e] = (unsigned char)bits;
+    any = any || bits != 0;
     float* to = out + (size_t)m * N + n;
     if (n + 3 < N && (((uintptr_t)to) & 15) == 0) {
       *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
@@ -292,6 +336,7 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((unsigned)C::TMEM_COLS));
+  if (__syncthreads_or(any)) odd_results(A, W, out, odd, m0, n0, part * share, c_end, N, K);
 }
 
 // Short sums (K below SHORT_K): one chain over all k in index order, as there is little to divide; the

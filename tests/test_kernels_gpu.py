@@ -1235,3 +1235,36 @@ def test_linear_fp32_numbers_that_bfloat16_cannot_hold(m, n, k):
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
     assert torch.equal(got[torch.isinf(got)], want[torch.isinf(want)])
     assert (got[:, 0].double() - (x.double() @ w.double().T)[:, 0]).abs().max() <= 3.4e38 * 2.0 ** -22
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 4096, 1024), (204, 4096, 1024), (8, 80000, 1024), (1, 1000, 3072)])
+def test_linear_fp32_rows_that_are_not_numbers_cost_no_multiple_of_the_time(m, n, k):
+    """All rows not-a-number, or one row with an infinity, at the sizes of a layer and of a wide head: the results, and at most
+    eight times the time of finite rows (one thread a result, all of k in a chain, took 6 to 128 times)."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    w = torch.randn(n, k, generator=g, device="cuda")
+    finite = torch.randn(m, k, generator=g, device="cuda")
+    nans, infinite = finite.clone(), finite.clone()
+    nans[:, k // 3] = float("nan")
+    infinite[m - 1, k // 2] = float("inf")
+    assert bool(torch.isnan(ops().linear(nans, w)).all())
+    got, want = ops().linear(infinite, w), ops().linear(finite, w)
+    assert torch.equal(got[m - 1], w[:, k // 2].sign() * float("inf"))
+    assert torch.equal(got[:m - 1], want[:m - 1])
+
+    def us(x):
+        best = float("inf")
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            for _ in range(10):
+                ops().linear(x, w)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 100)
+        return best
+
+    base = us(finite)
+    for x in (nans, infinite):
+        assert us(x) <= 8 * base
