@@ -1,15 +1,16 @@
 // True float32 matrix product: C[M,N] = A[M,K] * W[N,K]^T.
 //
 // This is the matrix product of the 32-bit path; no reduced-precision mode.  From K = 512 on the products run
-// on the tensor cores without giving up a bit of an operand: every float32 number is the exact sum of three
-// bfloat16 numbers (8 bits each; rounded to nearest, what is left, what is left of that), and of the nine
+// on the tensor cores without giving up a bit of an operand: every float32 number (times 2^16, see take_apart) is the
+// exact sum of three bfloat16 numbers (8 bits each; rounded to nearest, what is left, what is left of that), and of the nine
 // products of two such sums the six that matter are formed, the smallest first; the three left out are below
 // 2^-25 of the product.  k is cut into blocks of 64 and these into `parts(K)` runs.  The tensor core sums a
 // block from zero, in float32; a run adds its blocks up in index order with float32 additions outside the tensor
 // core, and the runs are added in order.  Below K = 512 an element is one chain of FMA over k in index order
 // (gemm_fp32_short_kernel).  The order is a function of K alone, whatever the tile, so a row's result does not
-// depend on M: the same token gives the same bits in any batch.  A result that is no finite number is formed
-// again by FMA from the operands (an infinity is no sum of three numbers).
+// depend on M: the same token gives the same bits in any batch.  A result that comes out as no finite number is formed
+// again by FMA from the operands: an infinity is no sum of three numbers, and neither are operands above 2^112 or sums above
+// 2^96, which the factor takes beyond float32's range.
 // (Distance from 64-bit sums at K = 1,024 .. 4,096: 0.97e-7 .. 1.1e-7 of the norm, where eight chains of FMA had 2.1e-7 ..
 // 4.1e-7.)
 #include "common.cuh"
@@ -89,14 +90,19 @@ __device__ __forceinline__ float4 ld_peer_smem(const float* local, unsigned rank
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
   return v;
 }
-// two float32 numbers as three pairs of bfloat16 numbers whose sums they are
+// two float32 numbers, times 2^SCALE, as three pairs of bfloat16 numbers whose sums they are.  The third part of a number
+// begins 16 bits below it: without the factor it would fall under bfloat16's smallest number, 2^-133, for numbers
+// below 2^-109; with it every number that float32 holds, subnormal ones included, keeps all its bits.
+constexpr int SCALE = 16;
 __device__ __forceinline__ void take_apart(float x, float y, unsigned (&part)[3]) {
+  float2 v = __fmul2_rn(make_float2(x, y), make_float2((float)(1 << SCALE), (float)(1 << SCALE)));
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
     part[i] = *reinterpret_cast<const unsigned*>(&h);
-    x = __fsub_rn(x, __uint_as_float(part[i] << 16));
-    y = __fsub_rn(y, __uint_as_float(part[i] & 0xffff0000u));
+    if (i < 2)       // (exact)
+      v = __ffma2_rn(make_float2(__uint_as_float(part[i] << 16), __uint_as_float(part[i] & 0xffff0000u)),
+                     make_float2(-1.f, -1.f), v);
   }
 }
 
@@ -314,10 +320,11 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
         if (r < parts)
           v = make_float4(__fadd_rn(v.x, run[r].x), __fadd_rn(v.y, run[r].y), __fadd_rn(v.z, run[r].z), __fadd_rn(v.w, run[r].w));
     }
-    const float o[4] = {v.x, v.y, v.z, v.w};
+    constexpr float DOWN = 1.0f / (1 << SCALE);
+    const float o[4] = {v.x * DOWN * DOWN, v.y * DOWN * DOWN, v.z * DOWN * DOWN, v.w * DOWN * DOWN};
     unsigned bits = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)      // an operand or a sum that bfloat16 parts cannot hold
+    for (int i = 0; i < 4; ++i)      // an operand or a sum that the scaled parts cannot hold
       if (n + i < N && !(fabsf(o[i]) <= 3.402823466e38f)) bits |= 1u << i;
     odd[e] = (unsigned char)bits;
     any = any || bits != 0;
