@@ -270,8 +270,8 @@ struct DeviceOnce {
 // while the kernel before it on the stream is still draining (its blocks are
 // scheduled, its prologue runs), and every kernel waits with griddepcontrol.wait for
 // that predecessor to have finished and flushed its memory before it reads or writes
-// anything the predecessor may touch.  Only constants (weights, tables, tensor maps)
-// are read before the wait.  In a chain A, B, C each kernel waits for the one before
+// anything the predecessor may touch.  Only constants (tables, tensor maps, the bfloat16 products' weights) and the
+// step's metadata, which host copies alone write, are read before the wait.  In a chain A, B, C each kernel waits for the one before
 // it, which itself only finished after its own wait, so C also sees A complete.  Set
 // DIB200_PDL=0 to launch the plain way.
 //
@@ -286,6 +286,10 @@ template <typename... P> __device__ __forceinline__ void pdl_wait(P&... p) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   (pdl_fresh(p), ...);
 }
+// Bring what lies at p (global memory) into L2.  A value read after the wait that is asked for so ahead of it is as fresh as
+// any other, as L2 is where all writes meet; only its trip to memory is over.  For arguments that a caller may have
+// computed just before (a weight that is an activation).
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // Ask for a tensor map (a kernel parameter) ahead of the first copy that uses it.
 __device__ __forceinline__ void prefetch_tensormap(const void* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");

@@ -269,8 +269,8 @@ __global__ void qk_norm_rope_cache_vec_kernel(
 
   // A warp takes ITEMS consecutive (token, head) items and issues the loads of all of
   // them before it works on any, so their memory round-trips overlap.  The step's positions and cache slots do
-  // not change while its kernels run, and the rotation table and the norms' weights never: with one item a
-  // warp (decoded tokens) all of them are there before the projection is, whose trip to memory is the only one then.
+  // not change while its kernels run, and the rotation table never: with one item a warp (decoded tokens) they are
+  // there before the projection is, and the norms' weights are in L2, so that one trip to memory is left.
   float v[ITEMS][EPL];
   int tok[ITEMS], head[ITEMS], pos[ITEMS], slot[ITEMS];
   bool act[ITEMS];
@@ -291,17 +291,21 @@ __global__ void qk_norm_rope_cache_vec_kernel(
     }
     if (head[it] >= Hq && kv_cache != nullptr) slot[it] = slot_mapping[tok[it]];
   }
+  const bool normed = EARLY && head[0] < Hq + Hkv && (head[0] < Hq ? q_norm_w : k_norm_w) != nullptr;
   if (EARLY && head[0] < Hq + Hkv) {
-    const float* nw = head[0] < Hq ? q_norm_w : k_norm_w;
+    if (normed) prefetch_l2((head[0] < Hq ? q_norm_w : k_norm_w) + lane * EPL);
     const float* tab = cos_sin + (size_t)pos[0] * D + (lane & 15) * EPL;
 #pragma unroll
     for (int k = 0; k < EPL; ++k) {
-      wn[k] = nw != nullptr ? nw[lane * EPL + k] : 0.f;
       cc[k] = cos_sin != nullptr ? tab[k] : 0.f;
       sn[k] = cos_sin != nullptr ? tab[D / 2 + k] : 0.f;
     }
   }
-  pdl_wait(qkv, parts);
+  pdl_wait(qkv, parts, q_norm_w, k_norm_w);
+  if (normed) {
+#pragma unroll
+    for (int k = 0; k < EPL; ++k) wn[k] = (head[0] < Hq ? q_norm_w : k_norm_w)[lane * EPL + k];
+  }
 #pragma unroll
   for (int it = 0; it < ITEMS; ++it) {
     if (!act[it]) continue;
@@ -564,13 +568,18 @@ add_rms_norm_split_kernel(const float* __restrict__ parts, int S,
                                           float eps) {
   pdl_trigger();
   __shared__ float scratch[128];
-  float4 ww[ITERS];     // (a constant: its trip to memory is over before the partials are there)
+  float4 ww[ITERS];     // (in L2 by then, and asked for together with the partials)
+#pragma unroll
+  for (int it = 0; it < ITERS; ++it) {
+    const int i = (it * blockDim.x + threadIdx.x) * 4;
+    if (i < H) prefetch_l2(w + i);
+  }
+  pdl_wait(parts, residual, w);
 #pragma unroll
   for (int it = 0; it < ITERS; ++it) {
     const int i = (it * blockDim.x + threadIdx.x) * 4;
     ww[it] = i < H ? *reinterpret_cast<const float4*>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  pdl_wait(parts, residual);
   const size_t base = (size_t)blockIdx.x * H;
   float v[ITERS][4];
   float ss[ITERS][1];

@@ -205,10 +205,15 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   auto w_piece = [&](int kb, int i) { return load(W, n0 + row + 16 * i, N, (kb0 + kb) * BK + 4 * c4); };
   auto a_piece = [&](int kb, int i) { return load(A, m0 + row + 16 * i, M, (kb0 + kb) * BK + 4 * c4); };
   const bool mine = nkb > 0 && warp < WARPS;
+  // W may have been computed just before (another activation): its first block is only brought into L2 ahead of the wait
 #pragma unroll
   for (int i = 0; i < C::ROWS_A; ++i)
-    if (mine) a[i] = w_piece(0, i);    // (a constant: ahead of the wait)
-  pdl_wait(A);
+    if (mine && (c4 & 1) == 0 && n0 + row + 16 * i < N && kb0 * BK + 4 * c4 < K)
+      prefetch_l2(W + (size_t)(n0 + row + 16 * i) * K + kb0 * BK + 4 * c4);
+  pdl_wait(A, W);
+#pragma unroll
+  for (int i = 0; i < C::ROWS_A; ++i)
+    if (mine) a[i] = w_piece(0, i);
 #pragma unroll
   for (int i = 0; i < C::ROWS_B; ++i)
     if (mine) b[i] = a_piece(0, i);

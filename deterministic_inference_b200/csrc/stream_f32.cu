@@ -143,7 +143,15 @@ __global__ void stream_norm_kernel(float* residual, Source x0, float a0, Source 
   __shared__ float scratch[32];
   constexpr int N = VPT > 0 ? VPT : 1;
   pdl_trigger();
-  float wv[N];                       // (a constant: its trip to memory is over before the row is there)
+  float wv[N];                       // (in L2 by then, and asked for together with the row)
+  if (VPT > 0) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int c = threadIdx.x + i * blockDim.x;
+      if (c < W && out != nullptr) prefetch_l2(w + c);
+    }
+  }
+  pdl_wait(x0.p, x1.p, residual, w);
   if (VPT > 0) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -151,7 +159,6 @@ __global__ void stream_norm_kernel(float* residual, Source x0, float a0, Source 
       wv[i] = c < W && out != nullptr ? w[c] : 0.f;
     }
   }
-  pdl_wait(x0.p, x1.p, residual);
   const long long base = (long long)blockIdx.x * W;
   float ss = 0.f;
   if (VPT > 0) {

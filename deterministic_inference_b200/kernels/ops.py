@@ -565,7 +565,8 @@ def qk_norm_rope_cache(qkv: torch.Tensor, num_heads: int, num_kv_heads: int, hea
     the token's position (when a table [max_pos, rotary_dim] = [cos | sin] is
     given), q to the returned tensor [T, Hq, D], k and v into the token's slot of
     the paged cache [pages, 2, Hkv, page_size, D] (when a cache is given;
-    slot = page * page_size + offset, negative = skip)."""
+    slot = page * page_size + offset, negative = skip).  ``cos_sin``, ``positions`` and ``slot_mapping`` are the
+    step's constants: no kernel of this package that is still running when this one is launched may write them."""
     parts = None
     if isinstance(qkv, SplitSum):
         if head_dim in (64, 128, 256) and (cos_sin is None or cos_sin.shape[1] == head_dim):
@@ -740,7 +741,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype=None) -> torch.Tenso
 
     float32: the package's own kernel (all bits of both operands, no TF32; the order of the
     sums depends on K alone, so a row's bits do not depend on the batch).  bfloat16: float32
-    accumulation on the tensor cores; ``out_dtype=torch.float32`` returns the
+    accumulation on the tensor cores, and ``weight`` is a constant: a kernel of this package that is still running
+    when the product is launched must not write it; ``out_dtype=torch.float32`` returns the
     accumulator unrounded (used for the logits).  With few rows and a split of k the
     bfloat16 product comes back as a ``SplitSum`` (see there)."""
     if isinstance(x, (GatedSplit, SplitAttention)) and weight.dtype == torch.bfloat16 \

@@ -1282,3 +1282,46 @@ def test_linear_fp32_rows_that_are_not_numbers_cost_no_multiple_of_the_time(m, n
     base = us(finite)
     for x in (nans, infinite):
         assert us(x) <= 8 * base
+
+
+@pytest.mark.parametrize("m,n,k", [(4, 512, 1024), (200, 512, 1024), (8, 76000, 512)])
+def test_linear_fp32_takes_a_weight_that_the_kernel_in_front_has_made(m, n, k):
+    """A weight that is itself an activation, written by the kernel just in front into memory that held other numbers: every
+    pass as with a weight that has lain there."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(m, k, generator=g, device="cuda")
+    table = torch.randn(n + 7, k, generator=g, device="cuda")
+    index = [torch.arange(i, n + i, dtype=torch.int32, device="cuda") for i in range(8)]
+    want = [ops().linear(x, table[i:n + i].contiguous()) for i in range(8)]
+    torch.cuda.synchronize()
+    got = [ops().linear(x, ops().gather_rows(table, i)) for i in index]
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("rows", [1, 3])
+def test_norms_take_weights_that_the_kernel_in_front_has_made(rows):
+    """The norms of decoded tokens with a weight written by the kernel just in front."""
+    o, g, h = ops(), torch.Generator(device="cuda").manual_seed(rows), 1024
+    table = torch.randn(8, h, generator=g, device="cuda")
+    index = [torch.tensor([i], dtype=torch.int32, device="cuda") for i in range(8)]
+    parts = torch.randn(4, rows, h, generator=g, device="cuda")
+    qkv = torch.randn(rows, 3 * 256, generator=g, device="cuda")
+    pos = torch.arange(rows, dtype=torch.int32, device="cuda")
+    start = torch.randn(rows, h, generator=g, device="cuda")
+
+    def passes(weight_of):
+        out = []
+        for i in range(8):
+            res = start.bfloat16()
+            out.append(o.add_rms_norm(o.SplitSum(parts, torch.bfloat16), res, weight_of(i), 1e-6)[0])
+            out.append(o.stream_rms_norm(start.clone(), weight_of(i), 1e-6, torch.float32, add=o.SplitSum(parts, torch.float32)))
+            w = weight_of(i).view(8, 128)
+            out.append(o.qk_norm_rope_cache(qkv, 2, 2, 128, w[0], w[1], 1e-6, None, pos, None, None, 16))
+        return out
+
+    kept = [table[i].clone() for i in range(8)]
+    torch.cuda.synchronize()
+    want = passes(lambda i: kept[i])
+    torch.cuda.synchronize()
+    got = passes(lambda i: o.gather_rows(table, index[i]).view(h))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
