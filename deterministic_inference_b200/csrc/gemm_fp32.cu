@@ -4,7 +4,7 @@
 // on the tensor cores without giving up a bit of an operand: every float32 number (times 2^16, see take_apart) is the
 // exact sum of three bfloat16 numbers (8 bits each; rounded to nearest, what is left, what is left of that), and of the nine
 // products of two such sums the six that matter are formed, the smallest first; the three left out are below
-// 2^-25 of the product.  k is cut into blocks of 64 and these into `parts(K)` runs.  The tensor core sums a
+// 2^-25 of the product.  k is cut into blocks of 64 and these into four runs.  The tensor core sums a
 // block from zero, in float32; a run adds its blocks up in index order with float32 additions outside the tensor
 // core, and the runs are added in order.  Below K = 512 an element is one chain of FMA over k in index order
 // (gemm_fp32_short_kernel).  The order is a function of K alone, whatever the tile, so a row's result does not
@@ -19,7 +19,6 @@ namespace {
 
 constexpr int WARPS = 8;
 constexpr int THREADS = WARPS * 32;
-constexpr int TC_THREADS = THREADS + 32;       // (one more warp issues the products)
 
 // rows r0 .. r0 + ROWS - 1 (below `rows`), k0 .. k0 + COLS - 1 (below K) of a [rows, K] matrix; zeros elsewhere
 template <int ROWS, int COLS, int LD, bool VEC>
@@ -38,15 +37,16 @@ __device__ __forceinline__ void copy_rows(float* dst, const float* __restrict__ 
 }
 
 // ---- tensor-core form.  A CTA takes 128 rows of W (the instruction's rows) by TOK rows of A (its columns) over a
-// run of k, the CTAs of a tile's runs are a thread-block cluster.  Per block of 64 k: every thread takes apart the
-// numbers it asked for a block earlier and leaves the three parts of both operands in shared memory in the layout
-// the instruction reads (rows of 128 bytes, 128-byte swizzle), one more thread issues the 24 products into one of two
-// accumulators in tensor memory (a warp of its own: it waits while the unit is busy), and while they run the accumulator of the block before is added to the sums in
+// run of k or all of them (Form).  Per block of 64 k: every thread takes apart the numbers it asked for one or two blocks
+// earlier and leaves the three parts of both operands in shared memory in the layout the instruction reads (rows of 128
+// bytes, 128-byte swizzle), one more thread issues the 24 products into one of two accumulators in tensor memory (a warp of
+// its own: it waits while the unit is busy), and while they run the accumulator of the block before is added to the sums in
 // registers.  At the end the cluster's CTAs add their sums through one another's shared memory, in run order.
-// Bound: by the trip of a block's operands to the registers (1.3 us a block of 16 to 64 rows; the products take
-// 0.8 us), then by taking them apart (1.9 us with 128 rows).  204 x 4,096 x 1,024: 74 us by FMA (52% of their rate), so 28;
-// 204 x 6,144 x 1,024 106 and 41; 204 x 1,024 x 3,072 57 and 22; one row of 1,024 x 3,072 21 and 18.
-constexpr int BN = 128, BK = 64, MAX_PARTS = 8;
+// Bound: by the tensor unit, 1.05 us a block of 16 rows, 1.3 of 64, 2 of 128, whatever the depth and the number of the warps that
+// feed it (a product of 128 x 16 x 16 takes it 57 cycles).  204 x 4,096 x 1,024: 74 us by FMA (52% of their rate), so 27;
+// 204 x 6,144 x 1,024 106 and 41; 204 x 1,024 x 3,072 57 and 21; one row of 1,024 x 3,072 21 and 16.  The head of 151,936 x 1,024 is
+// slower at up to 8 rows (127 and 163), whose bits may not differ from those of 64 rows (596 and 232).
+constexpr int BN = 128, BK = 64, MAX_PARTS = 4;
 constexpr int PLANE_A = BN * BK * 2;                     // bytes of a part of W's rows
 __device__ int dib_gemm_fp32_error_word;
 
@@ -68,7 +68,12 @@ __device__ __forceinline__ void tc_mma(unsigned tmem_d, unsigned long long desc_
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
       : "memory");
 }
-__device__ __forceinline__ void tc_ld8(unsigned taddr, unsigned (&r)[8]) {
+__device__ __forceinline__ void tc_ld(unsigned taddr, unsigned (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+__device__ __forceinline__ void tc_ld(unsigned taddr, unsigned (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr));
@@ -106,25 +111,32 @@ __device__ __forceinline__ void take_apart(float x, float y, unsigned (&part)[3]
   }
 }
 
-template <int TOK> struct Tc {
+// How a tile's runs of k are divided (the order of the sums is the same).  RUNS: a CTA of the cluster takes a run.  FOLD: one
+// CTA takes all runs, one after the other (no cluster), for grids that fill the GPU without the division.
+enum Form { RUNS, FOLD };
+
+// TOK rows of A a CTA, NW warps that take operands apart, DEPTH blocks that a thread has asked for and not yet taken apart
+template <int TOK, int NW, int DEPTH> struct Tc {
   static constexpr int PLANE_B = TOK * BK * 2;
   static constexpr int STAGE = 3 * (PLANE_A + PLANE_B);
   static constexpr int SUMS = TOK * BN * 4;              // the sums that a CTA leaves for its cluster
   static constexpr int SMEM = (2 * STAGE > SUMS ? 2 * STAGE : SUMS) + 1024;      // (and the tiles' alignment)
-  static constexpr int CTAS = TOK <= 16 ? 2 : 1;
+  static constexpr int CTAS = TOK <= 16 && NW == 8 && DEPTH == 1 ? 2 : 1;
+  static constexpr int THREADS = NW * 32 + 32;           // (one more warp issues the products)
   static constexpr int TMEM_COLS = 2 * TOK < 32 ? 32 : 2 * TOK;
-  static constexpr int ROWS_A = BN / 16, ROWS_B = TOK / 16;      // 16-byte pieces a thread has of a block's operands
+  static constexpr int STEP = 2 * NW;                    // rows between a thread's pieces of a block
+  static constexpr int ROWS_A = BN / STEP, ROWS_B = TOK / STEP;     // its 16-byte pieces of the operands
 };
 
 // The results that a CTA's `odd` marks (columns c0 .. c_end - 1 of its tile), by FMA from the operands.  A row of A that holds
 // a not-a-number has no other result; the others are sums over k by a warp for four columns, a chain a lane, the lanes by
 // the butterfly.  (us, 4,096 x 1,024, finite / one not-a-number in each row / an infinity in one row: 1 row 10 / 16 / 25, 204 rows
-// 27 / 75 / 39; all 204 rows with an infinity 476.  By the thread of each result 140, 3,730 and 156.)  A function of its own,
+// 27 / 54 / 38; all 204 rows with an infinity 295.  By the thread of each result 140, 3,730 and 156.)  A function of its own,
 // called: in the kernel it takes registers from the loop (204 rows 28 -> 30 us).
 __device__ __noinline__ void odd_results(const float* A, const float* W, float* out, unsigned char* odd, int m0, int n0,
                                          int c0, int c_end, int N, int K) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int c = c0 + warp; c < c_end; c += TC_THREADS / 32) {
+  for (int c = c0 + warp; c < c_end; c += blockDim.x >> 5) {
     const unsigned bits = odd[c * (BN / 4) + lane];
     if (!__any_sync(0xffffffffu, bits != 0)) continue;
     const float* x = A + (size_t)(m0 + c) * K;
@@ -138,7 +150,7 @@ __device__ __noinline__ void odd_results(const float* A, const float* W, float* 
     odd[c * (BN / 4) + lane] = 0;
   }
   __syncthreads();
-  for (int e = c0 * (BN / 4) + warp; e < c_end * (BN / 4); e += TC_THREADS / 32) {
+  for (int e = c0 * (BN / 4) + warp; e < c_end * (BN / 4); e += blockDim.x >> 5) {
     const unsigned bits = odd[e];
     if (bits == 0) continue;
     const int n = n0 + e % (BN / 4) * 4, m = m0 + e / (BN / 4);
@@ -159,11 +171,13 @@ __device__ __noinline__ void odd_results(const float* A, const float* W, float* 
   }
 }
 
-template <int TOK, bool VEC, bool FOLD>
-__global__ void __launch_bounds__(TC_THREADS, Tc<TOK>::CTAS)
+template <int TOK, int NW, int DEPTH, bool VEC, Form FORM>
+__global__ void __launch_bounds__((Tc<TOK, NW, DEPTH>::THREADS), (Tc<TOK, NW, DEPTH>::CTAS))
 gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out, int M, int N,
-                    int K, int runs) {
-  using C = Tc<TOK>;
+                    int K, int runs, int tile0) {
+  using C = Tc<TOK, NW, DEPTH>;
+  constexpr bool FOLDS = FORM == FOLD;
+  constexpr int TC_THREADS = C::THREADS, WARPS = NW;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
   __shared__ unsigned long long done[2];                 // the products of the block in stage s have completed
@@ -171,9 +185,10 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   __shared__ unsigned char odd[TOK * (BN / 4)];          // of four neighbouring results: those that are no finite numbers
   pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * TOK, n0 = blockIdx.x * BN, part = blockIdx.z;
-  const int blocks = (K + BK - 1) / BK, per = (blocks + runs - 1) / runs, parts = FOLD ? 1 : runs;
-  const int kb0 = part * per, nkb = FOLD ? blocks : max(0, min(per, blocks - kb0));
+  const int m0 = blockIdx.y * TOK, n0 = (tile0 + blockIdx.x) * BN, part = blockIdx.z;
+  const int n_end = min(N, n0 + BN);
+  const int blocks = (K + BK - 1) / BK, per = (blocks + runs - 1) / runs, parts = FOLDS ? 1 : runs;
+  const int kb0 = part * per, nkb = FOLDS ? blocks : max(0, min(per, blocks - kb0));
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[0])));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[1])));
@@ -184,9 +199,9 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
                  "r"((unsigned)C::TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
-  // a thread's pieces: 4 k from 4 (tid % 16) of rows tid / 16 + 16 i
+  // a thread's pieces: 4 k from 4 (tid % 16) of rows tid / 16 + STEP i
   const int row = tid >> 4, c4 = tid & 15;
-  float4 a[C::ROWS_A], b[C::ROWS_B];
+  float4 a[DEPTH][C::ROWS_A], b[DEPTH][C::ROWS_B];
   auto load = [&](const float* src, int r, int rows, int k) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < rows) {
@@ -202,33 +217,53 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
     }
     return v;
   };
-  auto w_piece = [&](int kb, int i) { return load(W, n0 + row + 16 * i, N, (kb0 + kb) * BK + 4 * c4); };
-  auto a_piece = [&](int kb, int i) { return load(A, m0 + row + 16 * i, M, (kb0 + kb) * BK + 4 * c4); };
+  // A block that lies within K, rows on 16 bytes: a uniform base and a thread's offset, rows behind the last one's standing
+  // in for it (their results go nowhere).  (Addresses and bounds apiece were half of the kernel's instructions.)
+  const unsigned row_bytes = 4u * (unsigned)K, skip = C::STEP * row_bytes;
+  const unsigned w_off = row * row_bytes + c4 * 16, w_last = (unsigned)(n_end - n0 - 1) * row_bytes + c4 * 16;
+  const unsigned a_last = (unsigned)(min(TOK, M - m0) - 1) * row_bytes + c4 * 16;
+  const bool near = VEC && K <= (1 << 22);               // (offsets within 32 bits)
+  auto w_piece = [&](int kb, int i) { return load(W, n0 + row + C::STEP * i, n_end, (kb0 + kb) * BK + 4 * c4); };
+  auto a_piece = [&](int kb, int i) { return load(A, m0 + row + C::STEP * i, M, (kb0 + kb) * BK + 4 * c4); };
   const bool mine = nkb > 0 && warp < WARPS;
-  // W may have been computed just before (another activation): its first block is only brought into L2 ahead of the wait
+  // W may have been computed just before (another activation): its first blocks are only brought into L2 ahead of the wait
 #pragma unroll
-  for (int i = 0; i < C::ROWS_A; ++i)
-    if (mine && (c4 & 1) == 0 && n0 + row + 16 * i < N && kb0 * BK + 4 * c4 < K)
-      prefetch_l2(W + (size_t)(n0 + row + 16 * i) * K + kb0 * BK + 4 * c4);
+  for (int d = 0; d < DEPTH; ++d)
+#pragma unroll
+    for (int i = 0; i < C::ROWS_A; ++i)
+      if (mine && d < nkb && (c4 & 1) == 0 && n0 + row + C::STEP * i < n_end && (kb0 + d) * BK + 4 * c4 < K)
+        prefetch_l2(W + (size_t)(n0 + row + C::STEP * i) * K + (kb0 + d) * BK + 4 * c4);
   pdl_wait(A, W);
+  auto ask = [&](int kb, int d) {
+    if (near && (kb0 + kb + 1) * BK <= K) {
+      const char* wt = reinterpret_cast<const char*>(W + (size_t)n0 * K + (kb0 + kb) * BK);
+      const char* at = reinterpret_cast<const char*>(A + (size_t)m0 * K + (kb0 + kb) * BK);
 #pragma unroll
-  for (int i = 0; i < C::ROWS_A; ++i)
-    if (mine) a[i] = w_piece(0, i);
+      for (int i = 0; i < C::ROWS_A; ++i) a[d][i] = *reinterpret_cast<const float4*>(wt + min(w_off + i * skip, w_last));
 #pragma unroll
-  for (int i = 0; i < C::ROWS_B; ++i)
-    if (mine) b[i] = a_piece(0, i);
+      for (int i = 0; i < C::ROWS_B; ++i) b[d][i] = *reinterpret_cast<const float4*>(at + min(w_off + i * skip, a_last));
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < C::ROWS_A; ++i) a[d][i] = w_piece(kb, i);
+#pragma unroll
+    for (int i = 0; i < C::ROWS_B; ++i) b[d][i] = a_piece(kb, i);
+  };
+#pragma unroll
+  for (int d = 0; d < DEPTH; ++d)
+    if (mine && d < nkb) ask(d, d);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const unsigned tmem = tmem_slot;
-  // this thread's place in a part's tile: 8 bytes of row `row` (+ 16 i: the same swizzle)
+  // this thread's place in a part's tile: 8 bytes of row `row` (+ STEP i: the same swizzle)
   const int at = row * 128 + (((c4 >> 1) ^ (row & 7)) << 4) + (c4 & 1) * 8;
   constexpr unsigned idesc = make_idesc(BN, TOK);
-  constexpr int HALF = TOK / 2;        // a warp reads the rows 32 (warp % 4) .. of half of the columns
+  constexpr int HALF = TOK * 4 / NW, LD = HALF < 8 ? HALF : 8;   // a warp reads the rows 32 (warp % 4) .. of HALF columns
   float sum[HALF];
 #pragma unroll
   for (int j = 0; j < HALF; ++j) sum[j] = 0.f;
-  float total[FOLD ? HALF : 1];        // FOLD: of the runs before
+  float total[FOLDS ? HALF : 1];       // FOLD: of the runs before
   bool dead = false;                   // a wait has run out: no more waits, the launch is reported as failed
   auto add_block = [&](int kb) {
     if (!dead && !mbar_wait(&done[kb & 1], (kb >> 1) & 1)) dead = true;
@@ -236,18 +271,18 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
     tc_fence_after();
     const unsigned from = tmem + ((unsigned)((warp & 3) * 32) << 16) + (kb & 1) * TOK + (warp >> 2) * HALF;
 #pragma unroll
-    for (int j = 0; j < HALF; j += 8) {
-      unsigned r[8];
-      tc_ld8(from + j, r);
+    for (int j = 0; j < HALF; j += LD) {
+      unsigned r[LD];
+      tc_ld(from + j, r);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int e = 0; e < 8; ++e) sum[j + e] = __fadd_rn(sum[j + e], __uint_as_float(r[e]));
+      for (int e = 0; e < LD; ++e) sum[j + e] = __fadd_rn(sum[j + e], __uint_as_float(r[e]));
     }
     tc_fence_before();
-    if (FOLD && ((kb + 1) % per == 0 || kb + 1 == nkb)) {
+    if (FOLDS && ((kb + 1) % per == 0 || kb + 1 == nkb)) {
 #pragma unroll
       for (int j = 0; j < HALF; ++j) {
-        total[FOLD ? j : 0] = kb < per ? sum[j] : __fadd_rn(total[FOLD ? j : 0], sum[j]);
+        total[FOLDS ? j : 0] = kb < per ? sum[j] : __fadd_rn(total[FOLDS ? j : 0], sum[j]);
         sum[j] = 0.f;
       }
     }
@@ -271,29 +306,29 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
       __syncwarp();
     }
   } else {
-    for (int kb = 0; kb < nkb; ++kb) {
-      // the stage and the accumulator are free: the block before the last one has been added up
-      unsigned char* stage = smem + (kb & 1) * C::STAGE;
-      auto leave = [&](unsigned char* plane, int plane_bytes, const float4& v) {
-        unsigned lo[3], hi[3];
-        take_apart(v.x, v.y, lo);
-        take_apart(v.z, v.w, hi);
+    for (int k0 = 0; k0 < nkb; k0 += DEPTH) {
 #pragma unroll
-        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(plane + p * plane_bytes + at) = make_uint2(lo[p], hi[p]);
-      };
+      for (int d = 0; d < DEPTH; ++d) {
+        const int kb = k0 + d;
+        if (kb >= nkb) break;
+        // the stage and the accumulator are free: the block before the last one has been added up
+        unsigned char* stage = smem + (kb & 1) * C::STAGE;
+        auto leave = [&](unsigned char* plane, int plane_bytes, const float4& v) {
+          unsigned lo[3], hi[3];
+          take_apart(v.x, v.y, lo);
+          take_apart(v.z, v.w, hi);
 #pragma unroll
-      for (int i = 0; i < C::ROWS_A; ++i) leave(stage + i * 16 * 128, PLANE_A, a[i]);
+          for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(plane + p * plane_bytes + at) = make_uint2(lo[p], hi[p]);
+        };
 #pragma unroll
-      for (int i = 0; i < C::ROWS_B; ++i) leave(stage + 3 * PLANE_A + i * 16 * 128, C::PLANE_B, b[i]);
-      if (kb + 1 < nkb) {
+        for (int i = 0; i < C::ROWS_A; ++i) leave(stage + i * C::STEP * 128, PLANE_A, a[d][i]);
 #pragma unroll
-        for (int i = 0; i < C::ROWS_A; ++i) a[i] = w_piece(kb + 1, i);
-#pragma unroll
-        for (int i = 0; i < C::ROWS_B; ++i) b[i] = a_piece(kb + 1, i);
+        for (int i = 0; i < C::ROWS_B; ++i) leave(stage + 3 * PLANE_A + i * C::STEP * 128, C::PLANE_B, b[d][i]);
+        if (kb + DEPTH < nkb) ask(kb + DEPTH, d);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (kb > 0) add_block(kb - 1);
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncthreads();
-      if (kb > 0) add_block(kb - 1);
     }
     if (nkb > 0) add_block(nkb - 1);
   }
@@ -303,7 +338,7 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   float* sums = reinterpret_cast<float*>(smem);          // [TOK][128 rows of W]
   if (warp < WARPS) {
 #pragma unroll
-    for (int j = 0; j < HALF; ++j) sums[((warp >> 2) * HALF + j) * BN + (warp & 3) * 32 + lane] = FOLD ? total[FOLD ? j : 0] : sum[j];
+    for (int j = 0; j < HALF; ++j) sums[((warp >> 2) * HALF + j) * BN + (warp & 3) * 32 + lane] = FOLDS ? total[FOLDS ? j : 0] : sum[j];
   }
   if (parts > 1) cluster_sync_all();
   else __syncthreads();
@@ -330,16 +365,16 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
     unsigned bits = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i)      // an operand or a sum that the scaled parts cannot hold
-      if (n + i < N && !(fabsf(o[i]) <= 3.402823466e38f)) bits |= 1u << i;
+      if (n + i < n_end && !(fabsf(o[i]) <= 3.402823466e38f)) bits |= 1u << i;
     odd[e] = (unsigned char)bits;
     any = any || bits != 0;
     float* to = out + (size_t)m * N + n;
-    if (n + 3 < N && (((uintptr_t)to) & 15) == 0) {
+    if (n + 3 < n_end && (((uintptr_t)to) & 15) == 0) {
       *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
     } else {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (n + i < N) to[i] = o[i];
+        if (n + i < n_end) to[i] = o[i];
     }
   }
   __syncwarp();
@@ -419,24 +454,24 @@ gemm_fp32_short_kernel(const float* __restrict__ A, const float* __restrict__ W,
     }
 }
 
-// Runs of k, a function of K alone (part of the order above).
-int runs_of(int K) { return K > 15 * BK ? 4 : 2; }
-template <int TOK, bool VEC, bool FOLD>
-int launch_form(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
-  using C = Tc<TOK>;
+// Part of the order above.  (8 and 204 rows of 1,536, 512, us: two runs 8.2 and 10.1, four 5.7 and 9.5, eight 5.4 and 14.5.)
+constexpr int RUNS_OF_K = 4;
+template <int TOK, int NW, int DEPTH, bool VEC, Form FORM>
+int launch_form(const float* A, const float* W, float* out, int M, int N, int K, int tile0, int tiles, cudaStream_t st) {
+  using C = Tc<TOK, NW, DEPTH>;
   static DeviceOnce once;
   if (!once.done()) {
-    if (cudaFuncSetAttribute(gemm_fp32_tc_kernel<TOK, VEC, FOLD>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
+    if (cudaFuncSetAttribute(gemm_fp32_tc_kernel<TOK, NW, DEPTH, VEC, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
         cudaSuccess) {
       cudaGetLastError();
       return DIB_LAUNCH_FAILED;
     }
     once.mark();
   }
-  const int runs = runs_of(K), parts = FOLD ? 1 : runs;
+  constexpr int runs = RUNS_OF_K, parts = FORM == FOLD ? 1 : runs;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ceil_div_host(N, BN), ceil_div_host(M, TOK), parts);
-  cfg.blockDim = dim3(TC_THREADS);
+  cfg.gridDim = dim3(tiles, ceil_div_host(M, TOK), parts);
+  cfg.blockDim = dim3(C::THREADS);
   cfg.dynamicSmemBytes = C::SMEM;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -448,7 +483,7 @@ int launch_form(const float* A, const float* W, float* out, int M, int N, int K,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = dib_pdl_enabled() ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, gemm_fp32_tc_kernel<TOK, VEC, FOLD>, A, W, out, M, N, K, runs);
+  cudaLaunchKernelEx(&cfg, gemm_fp32_tc_kernel<TOK, NW, DEPTH, VEC, FORM>, A, W, out, M, N, K, runs, tile0);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
@@ -471,23 +506,56 @@ int launch_short(const float* A, const float* W, float* out, int M, int N, int K
 }
 // 16-byte copies want rows that start on 16 bytes
 bool takes_vectors(const float* A, const float* W, int K) { return K % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0; }
-template <int TOK, bool FOLD>
-int launch(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st) {
-  return takes_vectors(A, W, K) ? launch_form<TOK, true, FOLD>(A, W, out, M, N, K, st)
-                                : launch_form<TOK, false, FOLD>(A, W, out, M, N, K, st);
+template <int TOK, int NW, int DEPTH, Form FORM>
+int launch(const float* A, const float* W, float* out, int M, int N, int K, cudaStream_t st, int tile0 = 0, int tiles = -1) {
+  if (tiles < 0) tiles = ceil_div_host(N, BN);
+  return takes_vectors(A, W, K) ? launch_form<TOK, NW, DEPTH, true, FORM>(A, W, out, M, N, K, tile0, tiles, st)
+                                : launch_form<TOK, NW, DEPTH, false, FORM>(A, W, out, M, N, K, tile0, tiles, st);
 }
-// The rows of A a CTA takes: the tile whose last wave of CTAs is done first.  A CTA takes `fixed` us (launch, first
-// operands, the runs' sum) and `block` for each of its run's blocks; two CTAs of 16 rows fit an SM.  (204 rows, us with
-// 64 / 128 rows a CTA: N = 4,096, K = 1,024 42 / 28; 1,024, 2,048 17 / 21; 6,144, 1,024 63 / 41; 1,024, 3,072 22 / 28.)
-// 16 rows are for 16 rows at most: above that another tile was the faster at each size measured (16 rows a CTA against the
-// best: 64 rows of 1,024, 3,072 26 / 20; 40 of 6,144, 1,024 30 / 21).  Their block takes longer in a grid of many CTAs; the
-// factor and the 74 are fitted, to 16 / 32 rows a CTA: one row of 1,024, 3,072 (32 CTAs) 18.2 / 19.0; of 4,096, 1,024 (128)
-// 10.7 / 9.5; 8 rows of 6,144, 1,024 (192) 12.0 / 18.1.
-template <int TOK> float estimate(int M, int N, int K, float fixed, float block) {
-  const int runs = runs_of(K), per = (ceil_div_host(K, BK) + runs - 1) / runs;
-  const long long ctas = (long long)ceil_div_host(N, BN) * ceil_div_host(M, TOK) * runs, at_once = 148 * Tc<TOK>::CTAS;
-  if (Tc<TOK>::CTAS == 2 && ctas > 74) block *= 1.55f;
-  return (float)((ctas + at_once - 1) / at_once) * (fixed + block * per);
+
+// Which tile and form: the one whose last wave of CTAs is done first.  A CTA takes `fixed` us (launch, first operands, the
+// runs' sum) and `block` us for each of its blocks of 64 k; `at_once` CTAs fit the GPU.  Fitted to single products with weights from
+// memory, us (tile rows and form: measured): 1 row of 1,024, 3,072 and 1,024, 2,048 (16 RUNS) 16.1, 12.1; 17 rows (32 RUNS) 18.1, 13.5;
+// 204 rows (64 RUNS) 20.6, 15.5; 204 x 4,096 x 1,024 (64 FOLD, 128 RUNS, 64 RUNS) 26, 27, 41; 500 x 4,096 x 1,024 (128 FOLD, 128
+// RUNS) 44, 54; the head of 151,936 x 1,024 at 8, 17, 64 and 204 rows (16, 32, 64, 128 FOLD) 163, 194, 232, 776, where the RUNS took
+// 209, 335, 387 and 1,030.  Below 16 rows two CTAs share an SM with a block asked for ahead, or one has it with two:
+// 8 rows of 6,144, 1,024 (192 CTAs) 13.3 / 17.3, of 4,096, 1,024 (128) 12.4 / 9.2.  What waits is the tensor unit: a product of 128 x 16 x 16
+// takes it 57 cycles as one of 128 x 32 x 16 nearly does, 24 of them a block.
+struct Choice {
+  int form = -1;
+  float time = 1e30f;
+  void consider(int id, float t) {
+    if (t < time) form = id, time = t;
+  }
+};
+struct Sizes {
+  int M, N, K;
+  int blocks() const { return ceil_div_host(K, BK); }
+  long long tiles(int tok) const { return (long long)ceil_div_host(N, BN) * ceil_div_host(M, tok); }
+  bool fits(int tok) const { return ceil_div_host(M, tok) <= 65535; }
+  float runs(int tok, int at_once, float fixed, float block) const {
+    if (!fits(tok)) return 1e30f;
+    const int per = (blocks() + RUNS_OF_K - 1) / RUNS_OF_K;
+    return (float)((tiles(tok) * RUNS_OF_K + at_once - 1) / at_once) * (fixed + block * per);
+  }
+  // FOLD: a last wave of a few tiles (the head of 151,936: 1,187 tiles, 8 waves of 148 and 3) is a grid of RUNS of its own
+  int tail(int tok, int at_once) const {
+    const long long all = tiles(tok), left = all % at_once;
+    return M <= tok && all > at_once && left * RUNS_OF_K <= 148 ? (int)left : 0;
+  }
+  float fold(int tok, int at_once, float fixed, float block) const {
+    if (!fits(tok)) return 1e30f;
+    const long long all = tiles(tok);
+    const int left = tail(tok, at_once);
+    return (float)((all - left + at_once - 1) / at_once) * (fixed + block * blocks()) + (left > 0 ? 6.f : 0.f);
+  }
+};
+template <int TOK, int NW, int DEPTH, int RUNS_NW, int RUNS_DEPTH>
+int launch_fold(const float* A, const float* W, float* out, const Sizes& z, int at_once, cudaStream_t st) {
+  const int left = z.tail(TOK, at_once), tiles = ceil_div_host(z.N, BN);
+  const int status = launch<TOK, NW, DEPTH, FOLD>(A, W, out, z.M, z.N, z.K, st, 0, tiles - left);
+  if (status != DIB_OK || left == 0) return status;
+  return launch<TOK, RUNS_NW, RUNS_DEPTH, RUNS>(A, W, out, z.M, z.N, z.K, st, tiles - left, left);
 }
 
 }  // namespace
@@ -508,19 +576,28 @@ extern "C" int dib_gemm_fp32(const float* A, const float* W, float* out, int M, 
   if (ceil_div_host(M, 64) > 65535) return DIB_BAD_SIZE;
   if (K < SHORT_K)
     return takes_vectors(A, W, K) ? launch_short<true>(A, W, out, M, N, K, st) : launch_short<false>(A, W, out, M, N, K, st);
-  // few rows of a wide product (the head): one CTA takes all runs, there are CTAs enough (5 x 151,936 x 1,024: 190 us; the
-  // two forms were chosen at 171 against 228 us, before the last change to the kernel.  All of the weights go through the
-  // registers to be split: the FMA kernel before took 126 us)
-  if (M <= 16 && ceil_div_host(N, BN) >= 2 * 296) return launch<16, true>(A, W, out, M, N, K, st);
-  const float cost[4] = {M <= 16 ? estimate<16>(M, N, K, 3.2f, 1.25f) : 1e30f, estimate<32>(M, N, K, 4.5f, 1.3f),
-                         estimate<64>(M, N, K, 5.7f, 1.4f), estimate<128>(M, N, K, 5.5f, 1.9f)};
-  int best = 0;
-  for (int i = 1; i < 4; ++i)
-    if (cost[i] < cost[best]) best = i;
-  switch (best) {
-    case 0: return launch<16, false>(A, W, out, M, N, K, st);
-    case 1: return launch<32, false>(A, W, out, M, N, K, st);
-    case 2: return launch<64, false>(A, W, out, M, N, K, st);
-    default: return launch<128, false>(A, W, out, M, N, K, st);
+  const Sizes z{M, N, K};
+  Choice best;
+  if (M <= 16) {
+    best.consider(0, z.runs(16, 148, 3.8f, 1.04f));
+    best.consider(1, z.runs(16, 296, 3.5f, 2.4f));
+    best.consider(2, z.fold(16, 296, 3.5f, z.tiles(16) > 148 ? 2.1f : 1.4f));
+  }
+  best.consider(3, z.runs(32, 148, 4.6f, 1.13f));
+  best.consider(4, z.fold(32, 148, 4.5f, 1.12f));
+  best.consider(5, z.runs(64, 148, 5.3f, 1.25f));
+  best.consider(6, z.fold(64, 148, 5.1f, 1.32f));
+  best.consider(7, z.runs(128, 148, 4.9f, 1.98f));
+  best.consider(8, z.fold(128, 148, 10.5f, 2.07f));
+  switch (best.form) {
+    case 0: return launch<16, 8, 2, RUNS>(A, W, out, M, N, K, st);
+    case 1: return launch<16, 8, 1, RUNS>(A, W, out, M, N, K, st);
+    case 2: return launch_fold<16, 8, 1, 8, 2>(A, W, out, z, 296, st);
+    case 3: return launch<32, 8, 1, RUNS>(A, W, out, M, N, K, st);
+    case 4: return launch_fold<32, 8, 2, 8, 1>(A, W, out, z, 148, st);
+    case 5: return launch<64, 16, 1, RUNS>(A, W, out, M, N, K, st);
+    case 6: return launch_fold<64, 8, 1, 16, 1>(A, W, out, z, 148, st);
+    case 7: return launch<128, 16, 1, RUNS>(A, W, out, M, N, K, st);
+    default: return launch_fold<128, 16, 1, 16, 1>(A, W, out, z, 148, st);
   }
 }

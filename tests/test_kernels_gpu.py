@@ -178,12 +178,12 @@ def test_linear_fp32_is_true_fp32(m, n, k):
 
 @pytest.mark.parametrize("n,k", [(31, 33), (33, 64), (65, 130), (4096, 260), (100, 511), (100, 512),
                                  (4096, 513), (65, 578), (1024, 1028), (40003, 516), (4099, 1028), (40003, 517),
-                                 (4099, 1030)])
+                                 (4099, 1030), (75700, 512), (75649, 1028), (38200, 1025), (6144, 1024), (1000, 640)])
 def test_linear_fp32_tiles_give_the_same_bits(n, k):
-    """Every tile the row count and the width may choose adds in one order: the row's bits are those of the
-    row alone, at the edges of the tiles; against 64 bits the error is that of eight chains of k / 8, or of one
-    below 512.  (The last four widths, no multiple of a tile's, reach all five tiles from K = 512 on, each with
-    copies of 16 and of 4 bytes.)"""
+    """Every tile and form the row count and the width may choose adds in one order: the row's bits are those of the
+    row alone, at the edges of the tiles; against 64 bits the error is that of a chain of k terms below 512, and
+    from there on of a few roundings.  (The wide ones reach all tiles and both forms from K = 512 on, a last wave of a few
+    tiles too, each with copies of 16 and of 4 bytes.)"""
     torch.manual_seed(16)
     x = torch.randn(400, k, device="cuda")
     w = torch.randn(n, k, device="cuda")
@@ -193,9 +193,35 @@ def test_linear_fp32_tiles_give_the_same_bits(n, k):
         for r, one in zip((0, 7, 8, 16, 33), rows):
             if r < m:
                 assert torch.equal(got[r], one[0]), (m, r)
-        # a chain of c terms: at most c * 2^-24 of the sum of the terms' sizes, and 8 partials more
-        bound = ((k / 8 if k >= 512 else k) + 16) * 2.0 ** -24 * (x[:m].abs().double() @ w.abs().double().T)
-        assert ((got.double() - x[:m].double() @ w.double().T).abs() <= bound).all(), m
+        # a chain of c terms: at most c * 2^-24 of the sum of the terms' sizes; blocks of 64 that the tensor unit
+        # sums, a run's blocks and four runs: at most blocks / 4 + 4 roundings of partial sums, and as much again for
+        # what the unit and the parts leave out
+        want = x[:m].double() @ w.double().T
+        bound = ((k / 32 + 16) if k >= 512 else k + 16) * 2.0 ** -24 * (x[:m].abs().double() @ w.abs().double().T)
+        assert ((got.double() - want).abs() <= bound).all(), m
+        # measured 0.9e-7 .. 1.0e-7 of the norm; two of an operand's three parts, or one of the six products of parts left
+        # out, 2.6e-6 and more; chains of FMA 1.5e-7 .. 2.1e-7
+        if k >= 512:
+            assert float((got.double() - want).norm() / want.norm()) <= 3e-7, m
+
+
+@pytest.mark.parametrize("n,k", [(200, 512), (200, 1028), (75700, 517)])
+@pytest.mark.parametrize("m", [1, 16, 17, 64, 65, 200])
+def test_linear_fp32_products_of_the_parts(m, n, k):
+    """Sums in which all cancels but one product of parts: x = 1 + 2^-9 + 2^-20 has the parts 1, 2^-9 and 2^-20.  Each of the
+    six products that are formed carries a result alone, exact; with W and x in each other's place too."""
+    at = k // 2
+    thin, thick = 1 + 2.0 ** -9, 1 + 2.0 ** -9 + 2.0 ** -20
+    cases = [([thick, -thin], [1.0, 1.0], 2.0 ** -20),              # third part times first
+             ([thin, -1.0], [1.0, 1.0], 2.0 ** -9),                 # second times first
+             ([thin, -1.0, -1.0], [thin, 1.0, 2.0 ** -8], 2.0 ** -18),      # second times second
+             ([1.0], [1.0], 1.0)]
+    for a, b, want in cases:
+        for xs, ws in ((a, b), (b, a)):
+            x, w = torch.zeros(m, k, device="cuda"), torch.zeros(n, k, device="cuda")
+            x[:, at:at + len(xs)] = torch.tensor(xs, device="cuda")
+            w[:, at:at + len(ws)] = torch.tensor(ws, device="cuda")
+            assert bool((ops().linear(x, w) == want).all()), (xs, ws)
 
 
 def test_linear_fp32_row_does_not_depend_on_batch():
@@ -1232,7 +1258,8 @@ def test_linear_fp32_numbers_of_all_sizes_keep_their_bits(m, n, k, exponent):
         assert float((ops().linear(x, w).double() - want).norm() / want.norm()) <= 5e-7
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 40, 512), (5, 64, 1024), (70, 100, 1028)])
+@pytest.mark.parametrize("m,n,k", [(1, 40, 512), (5, 64, 1024), (70, 100, 1028), (1, 75700, 1028), (16, 75700, 517),
+                                   (17, 75700, 512), (65, 75700, 512)])
 def test_linear_fp32_numbers_that_bfloat16_cannot_hold(m, n, k):
     """Infinities, not-a-numbers and the largest numbers come out as FMA gives them; numbers of all sizes keep float32's
     accuracy."""
@@ -1240,8 +1267,8 @@ def test_linear_fp32_numbers_that_bfloat16_cannot_hold(m, n, k):
     x = torch.randn(m, k, generator=g, device="cuda") * 2.0 ** torch.randint(-40, 40, (m, 1), generator=g, device="cuda")
     w = torch.randn(n, k, generator=g, device="cuda") * 2.0 ** torch.randint(-40, 40, (n, 1), generator=g, device="cuda")
     want = x.double() @ w.double().T
-    # the eight partials' chains of k / 128 sums and what the parts leave out, as in the test of the tiles
-    bound = (k / 8 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    # as in the test of the tiles
+    bound = (k / 32 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     assert ((ops().linear(x, w).double() - want).abs() <= bound).all()
     x[:, 3], w[:, 3], w[0, 3] = 3.4e38, 0.0, 1.0                      # rounds up beyond bfloat16's range
     w[1, 5], w[2, 7] = float("inf"), float("nan")
