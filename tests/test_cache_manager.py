@@ -199,3 +199,30 @@ def test_pages_for_a_byte_budget_are_shared_by_bytes_per_page_and_window_groups_
     m.check_invariants()
     m.release_slot(s)
     m.check_invariants()
+
+
+@pytest.mark.parametrize("slots", [[5], [4, 5, 6, 9], list(range(1, 60, 3)), [2, 9, 30, 31, 33]])
+def test_state_is_zeroed_by_a_few_operations_whatever_slots_come(slots):
+    """A busy engine's free slots lie in any order: the number of operations does not grow with the runs that a batch's
+    slots form, and nobody else's state is touched."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Count(TorchDispatchMode):
+        writes = 0
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.writes += func.__name__.split(".")[0] in ("zero_", "index_fill_", "fill_", "index_put_", "copy_", "_to_copy")
+            return func(*args, **(kwargs or {}))
+
+    c = CacheManager({"a": StateSpec((2, 3)), "b": StateSpec((4,)), "c": StateSpec((2, 3))}, 4, 8, 64, 64, device="cpu")
+    for g in c.state_groups.values():
+        g.array.fill_(1.0)
+    c.fresh_slots = list(reversed(slots))
+    with Count() as count:
+        c.reset_fresh_state()
+    assert count.writes <= 2 * len(c.state_groups) + 2
+    for g in c.state_groups.values():
+        want = torch.ones_like(g.array)
+        want[:, slots] = 0
+        assert torch.equal(g.array, want)
+    assert c.fresh_slots == []
