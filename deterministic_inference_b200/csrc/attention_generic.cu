@@ -15,12 +15,13 @@
 // A block has 16 neighbouring (token, head of the group) queries of one key-value head,
 // or those of them that belong to one sequence: block (x, y) takes the y-th run of equal
 // sequences among the 16 and ends at once where there is none.  So the tile of keys and
-// values is read into shared memory once (the next two tiles' copies are in flight meanwhile)
+// values is read into shared memory once (the next tile's copies are in flight meanwhile)
 // for up to 16 queries, two a warp: a prompt's queries share it, a decoding token has
 // a block of its own.  Bound: a warp's chain through a tile (dot products, two reductions over the
 // lanes, values), so the two queries of a warp go through it side by side and there are eight warps.  (16 heads
-// of 128, us a layer, with four warps of four queries one after the other and one tile under way / so: 200 tokens behind
-// 100 66 / 51, 300 behind 300 beside 8 of 1,000 keys 191 / 140, one token of 600 keys 50 / 46.)
+// of 128, us a layer, with four warps of four queries one after the other / so: 200 tokens behind
+// 100 63 / 45, 300 behind 300 beside 8 of 1,000 keys 182 / 156, one token of 600 keys 49 / 44.  With three buffers of two tiles under way
+// the same or slower: 45, 160, 45, and fewer blocks an SM: bfloat16 heads of 192, 1,000 tokens 939 / 659.)
 //
 // Cache layout of a layer: [num_pages, 2, num_kv_heads, page_size, head_dim].
 #include "common.cuh"
@@ -30,9 +31,8 @@
 namespace {
 
 constexpr int MAX_D = 256;
-constexpr int WARPS = 8, THREADS = WARPS * 32;
-constexpr int NQ = 2, ITEMS = WARPS * NQ;      // queries a warp, a block
-constexpr int KEYS = 32, BUFS = 3;             // keys of a tile; tiles in shared memory (two under way)
+constexpr int ITEMS = 16;                      // queries a block
+constexpr int KEYS = 32, BUFS = 2;             // keys of a tile; tiles in shared memory (one under way)
 constexpr float NEG_BIG = -1e30f;
 
 // floats between rows of a tile: rows padded to whole vectors, an odd number of vectors apart (the
@@ -46,7 +46,7 @@ __host__ __device__ __forceinline__ int smem_floats(int D) {
 }
 
 // dot products of the lane's key with N queries, d in index order
-template <int N>
+template <int N, int NQ>
 __device__ __forceinline__ void dots(const float* krow, const float* q, int ld, int vecs, float (&s)[NQ]) {
 #pragma unroll
   for (int i = 0; i < N; ++i) s[i] = 0.f;
@@ -65,14 +65,15 @@ __device__ __forceinline__ void dots(const float* krow, const float* q, int ld, 
 }
 
 // NV: vectors of four dimensions a lane owns (1: D <= 128).  ASYNC: float32 rows on 16 bytes.
-template <typename T, int NV, bool ASYNC>
-__global__ void __launch_bounds__(THREADS, NV == 1 ? 2 : 1)
+template <typename T, int NV, bool ASYNC, int WARPS, int BLOCKS>
+__global__ void __launch_bounds__(WARPS * 32, BLOCKS)
 paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
                                const T* __restrict__ kv_cache,
                                const int* __restrict__ block_table, int max_blocks,
                                const int* __restrict__ token_seq,
                                const int* __restrict__ positions, int T_tokens, int Hq, int Hkv,
                                int D, int page_size, float scale, int window) {
+  constexpr int THREADS = WARPS * 32, NQ = ITEMS / WARPS;      // (queries a warp)
   extern __shared__ __align__(16) float smem[];
   pdl_prologue(q, kv_cache, block_table, token_seq, positions);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -182,20 +183,17 @@ paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
   }
 
   const int begin = lo / KEYS * KEYS;
-  const int page0 = page_of(begin), page1 = page_of(begin + KEYS);
-  int page = page_of(begin + 2 * KEYS);
+  const int page0 = page_of(begin);
+  int page = page_of(begin + KEYS);
   fetch(begin, 0, page0);
-  fetch(begin + KEYS, 1, page1);                         // (a tile behind the last one: zeros)
   int buf = 0;
-  for (int k0 = begin; k0 <= hi; k0 += KEYS, buf = buf + 1 == BUFS ? 0 : buf + 1) {
-    if constexpr (ASYNC) asm volatile("cp.async.wait_group 1;" ::: "memory");
+  for (int k0 = begin; k0 <= hi; k0 += KEYS, buf ^= 1) {
+    if constexpr (ASYNC) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                     // tile k0 is there; the one before has been read
     if (k0 + KEYS <= hi) {
       const int now = page;
-      page = page_of(k0 + 3 * KEYS);
-      fetch(k0 + 2 * KEYS, buf == 0 ? BUFS - 1 : buf - 1, now);
-    } else if constexpr (ASYNC) {
-      asm volatile("cp.async.commit_group;" ::: "memory");        // (keeps the count)
+      page = page_of(k0 + 2 * KEYS);
+      fetch(k0 + KEYS, buf ^ 1, now);
     }
     if (nq == 0) continue;
     const float* krow = sk + (buf * KEYS + lane) * ld;
@@ -307,52 +305,72 @@ paged_attention_generic_kernel(const T* __restrict__ q, T* __restrict__ out,
   }
 }
 
-template <typename T, int NV, bool ASYNC>
-int launch(const T* q, T* out, const T* kv, const int* bt, int max_blocks, const int* token_seq, const int* positions,
-           int tokens, int Hq, int Hkv, int D, int page_size, float scale, int window, cudaStream_t st) {
+struct Args {
+  const void *q, *kv;
+  void* out;
+  const int *bt, *token_seq, *positions;
+  int max_blocks, tokens, Hq, Hkv, D, page_size, window;
+  float scale;
+};
+template <typename T, int NV, bool ASYNC, int WARPS, int BLOCKS>
+int launch(const Args& a, cudaStream_t st) {
   static DeviceOnce once;
   if (!once.done()) {
-    if (cudaFuncSetAttribute(paged_attention_generic_kernel<T, NV, ASYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             4 * smem_floats(MAX_D)) != cudaSuccess) {
+    if (cudaFuncSetAttribute(paged_attention_generic_kernel<T, NV, ASYNC, WARPS, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             4 * smem_floats(NV == 1 ? 128 : MAX_D)) != cudaSuccess) {
       cudaGetLastError();
       return DIB_LAUNCH_FAILED;
     }
     once.mark();
   }
-  const int group = Hq / Hkv;
-  const long long blocks = ((long long)tokens * group + ITEMS - 1) / ITEMS;
+  const int group = a.Hq / a.Hkv;
+  const long long blocks = ((long long)a.tokens * group + ITEMS - 1) / ITEMS;
   // 16 neighbouring queries touch at most this many tokens, and as many sequences
   int runs = (ITEMS + group - 2) / group + 1;
   if (runs > ITEMS) runs = ITEMS;
-  if (runs > tokens) runs = tokens;
-  dib_launch(paged_attention_generic_kernel<T, NV, ASYNC>, dim3((unsigned)(blocks * Hkv), runs), dim3(THREADS),
-             4 * smem_floats(D), st, q, out, kv, bt, max_blocks, token_seq, positions, tokens, Hq, Hkv, D, page_size,
-             scale, window);
+  if (runs > a.tokens) runs = a.tokens;
+  dib_launch(paged_attention_generic_kernel<T, NV, ASYNC, WARPS, BLOCKS>, dim3((unsigned)(blocks * a.Hkv), runs), dim3(WARPS * 32),
+             4 * smem_floats(a.D), st, (const T*)a.q, (T*)a.out, (const T*)a.kv, a.bt, a.max_blocks, a.token_seq, a.positions,
+             a.tokens, a.Hq, a.Hkv, a.D, a.page_size, a.scale, a.window);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
 
+// Warps a block and blocks an SM, with the same bits.  The blocks that hold queries, some `busy` of them, come in waves of
+// what the SMs hold; eight warps with all registers take the shortest time for one, fewer registers 1.04 of it, four
+// warps of four queries 1.2, for groups of at most four heads (a decoding token's queries, one or two of the warps).  Heads
+// above 128: one block an SM 1.0, two 1.08.  (us a layer, two / three blocks of eight warps / four of four: 64 sequences of 200 keys,
+// 8 heads of 64 30 / 31 / 21, 128 of 300 82 / 68 / 55; 32 of 1,000, 12 heads of 96 133 / 80 / 87; a prompt of 1,000, bfloat16, 32 heads of
+// 64 on one 570 / 493 / -.  Heads of 192, one / two blocks: 8 of 600, 16 heads 55 / 61, 32 of 1,000 337 / 196.)
+template <typename T, bool ASYNC>
+int choose(const Args& a, int decoded, cudaStream_t st) {
+  const int group = a.Hq / a.Hkv, fit = 227 * 1024 / (4 * smem_floats(a.D) + 1024);
+  const long long busy = ((long long)decoded + ((long long)(a.tokens - decoded) * group + ITEMS - 1) / ITEMS) * a.Hkv;
+  auto time = [&](int blocks, float wave) {
+    const long long at_once = 148ll * (blocks < fit ? blocks : fit);
+    return (float)((busy + at_once - 1) / at_once) * wave;
+  };
+  if (a.D > 128) return time(2, 1.08f) < time(1, 1.f) ? launch<T, 2, ASYNC, 8, 2>(a, st) : launch<T, 2, ASYNC, 8, 1>(a, st);
+  const float two = time(2, 1.f), three = time(3, 1.04f), four = group <= 4 && decoded == a.tokens ? time(4, 1.2f) : 1e30f;
+  if (four < two && four < three) return launch<T, 1, ASYNC, 4, 4>(a, st);
+  return three < two ? launch<T, 1, ASYNC, 8, 3>(a, st) : launch<T, 1, ASYNC, 8, 2>(a, st);
+}
+
 }  // namespace
 
+// decoded: how many of the tokens are a sequence's only one in the step (for the choice of a form; any number is right)
 extern "C" int dib_paged_attention_generic(const void* q, void* out, const void* kv_cache,
                                            const int* block_table, int max_blocks,
-                                           const int* token_seq, const int* positions, int T,
+                                           const int* token_seq, const int* positions, int T, int decoded,
                                            int Hq, int Hkv, int D, int page_size, float scale,
                                            int window, int dtype, cudaStream_t st) {
   if (T == 0) return DIB_OK;
   if (D < 1 || D > MAX_D || Hkv < 1 || Hq % Hkv != 0 || page_size < 1) return DIB_BAD_SIZE;
   if (((long long)T * (Hq / Hkv) + ITEMS - 1) / ITEMS * Hkv > 0x7fffffffll) return DIB_BAD_SIZE;
-  auto go = [&](auto* tag, auto async) {
-    using E = std::remove_pointer_t<decltype(tag)>;
-    constexpr bool A = decltype(async)::value;
-    return D <= 128 ? launch<E, 1, A>((const E*)q, (E*)out, (const E*)kv_cache, block_table, max_blocks, token_seq,
-                                      positions, T, Hq, Hkv, D, page_size, scale, window, st)
-                    : launch<E, 2, A>((const E*)q, (E*)out, (const E*)kv_cache, block_table, max_blocks, token_seq,
-                                      positions, T, Hq, Hkv, D, page_size, scale, window, st);
-  };
+  const Args a{q, kv_cache, out, block_table, token_seq, positions, max_blocks, T, Hq, Hkv, D, page_size, window, scale};
+  decoded = decoded < 0 ? 0 : decoded > T ? T : decoded;
   if (dtype == 0)     // (rows of the cache start on 16 bytes when D is a multiple of 4)
-    return D % 4 == 0 && ((uintptr_t)kv_cache & 15) == 0 ? go((float*)nullptr, std::true_type{})
-                                                         : go((float*)nullptr, std::false_type{});
-  if (dtype == 1) return go((__nv_bfloat16*)nullptr, std::false_type{});
+    return D % 4 == 0 && ((uintptr_t)kv_cache & 15) == 0 ? choose<float, true>(a, decoded, st) : choose<float, false>(a, decoded, st);
+  if (dtype == 1) return choose<__nv_bfloat16, false>(a, decoded, st);
   return DIB_BAD_DTYPE;
 }

@@ -684,8 +684,8 @@ def paged_attention(q: torch.Tensor, kv_cache: torch.Tensor, meta, scale: float,
             return deferred if deferred is not None else out
     st = _lib("attention_generic").dib_paged_attention_generic(
         _ptr(q), _ptr(out), _ptr(kv_cache), _ptr(meta.block_table), c_int(meta.block_table.shape[1]),
-        _ptr(meta.token_seq), _ptr(meta.positions), c_int(t), c_int(hq), c_int(hkv), c_int(d),
-        c_int(page_size), c_float(scale), c_int(win), c_int(_dt(q, "q")), _stream())
+        _ptr(meta.token_seq), _ptr(meta.positions), c_int(t), c_int(int(getattr(meta, "num_decode", 0) or 0)), c_int(hq),
+        c_int(hkv), c_int(d), c_int(page_size), c_float(scale), c_int(win), c_int(_dt(q, "q")), _stream())
     _check(st, "paged_attention", f"head_dim {d} (at most 256), heads {hq}/{hkv}")
     return out
 

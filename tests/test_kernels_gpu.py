@@ -7,6 +7,8 @@ test_03_extend_attention.py, test_04_reshape_and_cache.py, test_07_sampler.py)."
 import pytest
 import torch
 
+from types import SimpleNamespace
+
 from tests import torch_kernels as ref
 from tests.attn_util import PagedCase, dense_reference
 
@@ -1352,3 +1354,42 @@ def test_norms_take_weights_that_the_kernel_in_front_has_made(rows):
     torch.cuda.synchronize()
     got = passes(lambda i: o.gather_rows(table, index[i]).view(h))
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("dtype,hq,hkv,d", [(torch.float32, 8, 8, 64), (torch.float32, 16, 8, 96), (torch.float32, 16, 16, 192),
+                                            (torch.float32, 8, 8, 63), (torch.bfloat16, 32, 1, 64), (torch.bfloat16, 8, 4, 192)])
+def test_generic_attention_forms_give_the_same_bits(dtype, hq, hkv, d):
+    """Many decoding tokens (four warps a block, or three or two blocks an SM), each of them alone (eight warps, two blocks or
+    one), what the step says of its decoded tokens left out or wrong, and a prompt whole and in portions: the same bits; some
+    rows against 64 bits."""
+    g = torch.Generator(device="cuda").manual_seed(d)
+    page, per, seqs = 16, 11, 150
+    kv = torch.randn(seqs * per + 1, 2, hkv, page, d, generator=g, device="cuda").to(dtype)
+    table = (torch.randperm(seqs * per, generator=g, device="cuda").int() + 1).view(seqs, per).contiguous()
+    lens = torch.randint(1, page * per + 1, (seqs,), generator=g, device="cuda").int()
+    q = torch.randn(seqs, hq, d, generator=g, device="cuda").to(dtype)
+
+    def run(who, pos, queries, decode):
+        meta = SimpleNamespace(block_table=table, token_seq=who.int().contiguous(), positions=pos.int().contiguous())
+        if decode is not None:
+            meta.num_decode = decode
+        return ops().paged_attention(queries.contiguous(), kv, meta, d ** -0.5)
+
+    everyone = torch.arange(seqs, device="cuda")
+    many = run(everyone, lens - 1, q, seqs)
+    for decode in (None, 0, 70, seqs + 5):
+        assert torch.equal(run(everyone, lens - 1, q, decode), many), decode
+    for i in (0, 1, 77, seqs - 1):
+        assert torch.equal(run(everyone[i:i + 1], lens[i:i + 1] - 1, q[i:i + 1], 1)[0], many[i]), i
+    for i in (0, 77):
+        n = int(lens[i])
+        rows = kv[table[i].long()].double().transpose(0, 1)                    # [2, pages, Hkv, page, D]
+        k, v = (rows[j].permute(1, 0, 2, 3).reshape(hkv, -1, d)[:, :n].repeat_interleave(hq // hkv, 0) for j in (0, 1))
+        p = torch.softmax(torch.einsum("hd,hnd->hn", q[i].double(), k) * d ** -0.5, -1)
+        tol = 1e-5 if dtype == torch.float32 else 1e-2
+        torch.testing.assert_close(many[i].double(), torch.einsum("hn,hnd->hd", p, v), atol=tol, rtol=tol)
+    n = page * per
+    prompt = torch.randn(n, hq, d, generator=g, device="cuda").to(dtype)
+    whole = run(torch.zeros(n, device="cuda"), torch.arange(n, device="cuda"), prompt, 0)
+    for a, b in ((0, 1), (1, 50), (50, n)):
+        assert torch.equal(run(torch.zeros(b - a, device="cuda"), torch.arange(a, b, device="cuda"), prompt[a:b], None), whole[a:b])
