@@ -365,7 +365,7 @@ moe_product_mma_kernel(const __nv_bfloat16* __restrict__ a_rows, const int* __re
 // as two of four, wait for one another less and share the items out more evenly: sort to combine, 16 experts
 // of 1,024 x 1,536, 8 tokens 30 against 38 us, 64 tokens 40 against 50; 8 of 4,096 x 4,096, 64 tokens 187 against 199.)  A row's sum is the same as above:
 // steps of 32 k, ascending, in the same permutation.  (Which of the two runs, and what both take:
-// product_times.)
+// streams_weights.)
 constexpr int ST_THREADS = 128, ST_B = 32, ST_A = 16, ST_K = 256, ST_STAGES = 2;
 constexpr int ST_LD = ST_K + GP_PAD;
 constexpr int ST_CTAS = 4 * 148;          // four an SM
@@ -617,22 +617,19 @@ int launch_product_stream(const void* a_rows, const int* order, int max_tiles, i
 }
 
 // Tiles of 16 rows: streamed weights for few tiles, whose other form has too few CTAs to fill the GPU and walks all
-// of K in one chain; that form for many small ones, where its CTAs hide one another's start and end.  Both give
-// the same bits, and a layer's two products take the same form.  The times are fits, in us with weights from memory;
-// measured from the sort to the combination (registers / streamed): 16 experts of 1,024 x 1,536, 8 tokens 51 / 30, 64 tokens
-// 61 / 40; 64 of 2,048 x 512, 4 tokens 55 / 49, 16 tokens 79 / 87, 64 tokens 92 / 99; 8 of 4,096 x 4,096, 8 tokens
-// 158 / 127, 64 tokens 257 / 187; 128 of 2,048 x 768, 4 tokens 64 / 65, 64 tokens 228 / 253; 512 of 512 x 256, 8 tokens
-// 19 / 21, 64 tokens 64 / 75.
-void product_times(int tiles, int K, int rows_b, float& registers, float& streamed) {
-  const float megabytes = 2e-6f * tiles * (float)K * (float)rows_b;
-  const float items = (float)tiles * ((rows_b + ST_B - 1) / ST_B);
-  const float chain = 1.0f + 0.0137f * K + megabytes / 10.5f, bytes = 3.0f + megabytes / 5.0f;
-  streamed += 5.5f + megabytes / 5.9f + 0.0015f * items;
-  registers += chain > bytes ? chain : bytes;
-}
+// of K in one chain; that form for many, where its CTAs hide one another's start and end and read more evenly.  Both give
+// the same bits, and a layer's two products take the same form.  The line is the number of tiles in use: streamed took 0.62 to
+// 0.99 of the other's time up to 57 tiles (26 of 28 sizes), 1.01 to 1.20 of it from 59 on (14 of 17).  Long rows (W from 4,096 on) pay for a
+// walker's items to the 64 tiles of a small model's experts (62 of 6,144 x 2,048 0.89, 63 of 4,096 x 1,408 0.87; 82 of it 1.02, 125 1.09); with
+// F from 2 W on the down product has few and long items, whose last round leaves most walkers idle (44 of 1,024 x 4,096
+// 1.10, of 2,048 x 4,096 1.08, 38 of 1,024 x 2,048 1.03, 31 of 1,024 x 4,096 0.94).  (us from the sort to the combination with weights
+// from memory, registers / streamed: 16 experts of 1,024 x 1,536, 8 tokens 48 / 30; 64 of 2,048 x 512, 16 tokens 79 / 75, 64 tokens
+// 94 / 105; 128 of 2,048 x 768, 8 tokens 124 / 102, 16 158 / 162, 64 228 / 244; 8 of 4,096 x 4,096, 64 tokens 255 / 176; 64 of 2,880 x
+// 2,880, 16 tokens 352 / 325, 64 558 / 658.  Products of bytes and latencies fitted to these were wrong more often.)
+bool streams_weights(int tiles, int F, int W) { return tiles <= (W >= 4096 ? 64 : F >= 2 * W ? 36 : 57); }
 
 // mode 0: gate and up; 1: down; 2: up alone.  dtype 0 float32, 1 bfloat16.  streams: tiles of 16 rows stream
-// their weights (see dib_moe_streams).
+// their weights (see streams_weights).
 int moe_product(const void* a_rows, int dtype, const int* order, int max_tiles, int tile, int streams, int top,
                 const void* w, void* out, int K, int N, int mode, float limit, float alpha, cudaStream_t st) {
   if (max_tiles == 0) return DIB_OK;
@@ -739,12 +736,7 @@ int dib_moe_sort(const int* ids, const int* table, int top, int V, int pairs, in
 }
 
 // Do tiles of 16 rows, about `tiles` of them in use, stream their weights (both products of a layer)?
-int dib_moe_streams(int tiles, int F, int W, int gated) {
-  float registers = 0.f, streamed = 0.f;
-  product_times(tiles, W, gated ? 2 * F : F, registers, streamed);
-  product_times(tiles, F, W, registers, streamed);
-  return streamed <= registers ? 1 : 0;
-}
+int dib_moe_streams(int tiles, int F, int W) { return streams_weights(tiles, F, W) ? 1 : 0; }
 
 // limit > 0: the limited gate (limit, alpha); else silu
 int dib_moe_gate_up(const void* x, int dtype, const int* order, int max_tiles, int tile, int streams, int top,

@@ -1689,8 +1689,7 @@ def routed_experts(x: torch.Tensor, ids, weights, w_gate_up: torch.Tensor,
         hidden = torch.empty(max_tiles * tile, f, dtype=x.dtype, device=dev)
         # the experts that tokens' choices at random name, and tiles that are not full
         named = n_exp * (1.0 - (1.0 - min(top, n_exp) / n_exp) ** t)
-        streams = lib.dib_moe_streams(c_int(int(max(named, pairs / tile + named / 2))), c_int(f), c_int(w),
-                                      c_int(1 if gated else 0))
+        streams = lib.dib_moe_streams(c_int(int(max(named, pairs / tile + named / 2))), c_int(f), c_int(w))
         if gated:
             st = lib.dib_moe_gate_up(_ptr(x), c_int(_dt(x, "x")), _ptr(order), c_int(max_tiles), c_int(tile),
                                      c_int(streams), c_int(top), _ptr(w_gate_up), _ptr(hidden), c_int(f), c_int(w),

@@ -245,3 +245,33 @@ def test_the_command_line_writes_a_model_folder_the_registry_reads_back(tmp_path
     assert back.to_dict() == cfg.to_dict()
     model = build_model(back, torch.float32, "cpu")
     load_weights(out, model.tensor_specs(), model.plan, torch.float32, "cpu")
+
+
+# experts, W, F, tokens, choices a token: us of the form with weights in registers and of the streamed one, measured from the sort to
+# the combination with weights from memory (gated experts, one B200)
+EXPERT_FORMS = [
+    (128, 2048, 768, 64, 8, 228.3, 244.2), (128, 2048, 768, 32, 8, 214.1, 222.9), (128, 2048, 768, 8, 8, 123.7, 101.8),
+    (64, 2048, 512, 4, 8, 55.5, 45.5), (64, 2048, 512, 16, 8, 78.6, 74.6), (64, 2048, 512, 64, 8, 94.4, 104.9),
+    (16, 1024, 1536, 8, 2, 48.3, 30.0), (16, 1024, 1536, 64, 2, 62.0, 41.7), (8, 4096, 4096, 8, 2, 167.3, 140.9),
+    (8, 4096, 4096, 64, 2, 254.9, 176.0), (512, 512, 256, 64, 8, 67.6, 75.1), (32, 1024, 512, 16, 4, 37.1, 30.9),
+    (32, 1024, 512, 64, 4, 42.8, 33.9), (256, 1024, 512, 64, 8, 155.3, 180.0), (64, 2048, 1408, 8, 6, 127.1, 115.9),
+    (64, 2048, 1408, 64, 6, 221.8, 237.5), (64, 512, 256, 8, 8, 22.5, 20.9), (64, 4096, 1408, 8, 6, 252.7, 214.7),
+    (64, 4096, 1408, 64, 6, 425.3, 371.7), (96, 2048, 768, 8, 8, 94.1, 86.3), (60, 2048, 1408, 16, 4, 154.6, 126.9),
+    (60, 2048, 1408, 64, 4, 210.7, 221.4), (48, 1024, 4096, 64, 2, 220.2, 243.0), (72, 1024, 1024, 64, 4, 93.0, 103.5),
+    (64, 2880, 2880, 64, 4, 558.3, 657.7), (64, 2880, 2880, 16, 4, 352.1, 324.9), (128, 2880, 2880, 4, 4, 181.3, 150.6),
+    (128, 2880, 2880, 16, 4, 515.1, 466.0), (160, 5120, 1536, 8, 6, 391.1, 358.6), (256, 7168, 2048, 8, 8, 898.2, 786.4),
+    (128, 4096, 1408, 64, 8, 739.1, 803.4), (256, 7168, 2048, 16, 8, 1463.8, 1754.2), (64, 6144, 2048, 64, 4, 828.0, 737.5),
+    (32, 4096, 8192, 64, 2, 1035.4, 947.9), (48, 2048, 4096, 64, 2, 410.7, 444.0), (64, 3072, 1024, 64, 4, 226.7, 251.7),
+    (32, 1024, 4096, 64, 2, 181.8, 170.3)]
+
+
+@pytest.mark.parametrize("experts, w, f, tokens, top, registers, streamed", EXPERT_FORMS)
+def test_the_form_of_few_rows_an_expert_is_the_quicker_one(experts, w, f, tokens, top, registers, streamed):
+    """The rule that picks a form, as the launch asks it, against measured times.  (Three measured sizes of forty are on the wrong
+    side of its lines: 256 of 1,024 x 512, 16 tokens, 5%; 64 of 4,096 x 1,408, 16 tokens, 4%; 32 of 2,048 x 8,192, 64 tokens, 19%.)"""
+    from ctypes import c_int
+    from deterministic_inference_b200.kernels import build
+    lib = build.load_library("routed_experts")
+    named = experts * (1.0 - (1.0 - min(top, experts) / experts) ** tokens)
+    tiles = int(max(named, tokens * top / 16 + named / 2))
+    assert bool(lib.dib_moe_streams(c_int(tiles), c_int(f), c_int(w))) == (streamed < registers)
