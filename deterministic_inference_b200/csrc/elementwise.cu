@@ -293,7 +293,7 @@ __global__ void qk_norm_rope_cache_vec_kernel(
   }
   const bool normed = EARLY && head[0] < Hq + Hkv && (head[0] < Hq ? q_norm_w : k_norm_w) != nullptr;
   if (EARLY && head[0] < Hq + Hkv) {
-    if (normed) prefetch_l2((head[0] < Hq ? q_norm_w : k_norm_w) + lane * EPL);
+    if (normed && lane * EPL % 8 == 0) prefetch_l2((head[0] < Hq ? q_norm_w : k_norm_w) + lane * EPL);
     const float* tab = cos_sin + (size_t)pos[0] * D + (lane & 15) * EPL;
 #pragma unroll
     for (int k = 0; k < EPL; ++k) {
@@ -569,10 +569,12 @@ add_rms_norm_split_kernel(const float* __restrict__ parts, int S,
   pdl_trigger();
   __shared__ float scratch[128];
   float4 ww[ITERS];     // (in L2 by then, and asked for together with the partials)
+  if (gridDim.x <= PREFETCH_BLOCKS && (threadIdx.x & 1) == 0) {
 #pragma unroll
-  for (int it = 0; it < ITERS; ++it) {
-    const int i = (it * blockDim.x + threadIdx.x) * 4;
-    if (i < H) prefetch_l2(w + i);
+    for (int it = 0; it < ITERS; ++it) {
+      const int i = (it * blockDim.x + threadIdx.x) * 4;
+      if (i < H) prefetch_l2(w + i);
+    }
   }
   pdl_wait(parts, residual, w);
 #pragma unroll

@@ -144,7 +144,7 @@ __global__ void stream_norm_kernel(float* residual, Source x0, float a0, Source 
   constexpr int N = VPT > 0 ? VPT : 1;
   pdl_trigger();
   float wv[N];                       // (in L2 by then, and asked for together with the row)
-  if (VPT > 0) {
+  if (VPT > 0 && gridDim.x <= PREFETCH_BLOCKS && (threadIdx.x & 7) == 0) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
