@@ -293,7 +293,8 @@ __global__ void qk_norm_rope_cache_vec_kernel(
   }
   const bool normed = EARLY && head[0] < Hq + Hkv && (head[0] < Hq ? q_norm_w : k_norm_w) != nullptr;
   if (EARLY && head[0] < Hq + Hkv) {
-    if (normed && lane * EPL % 8 == 0) prefetch_l2((head[0] < Hq ? q_norm_w : k_norm_w) + lane * EPL);
+    if (normed && gridDim.x <= PREFETCH_BLOCKS && lane * EPL % 8 == 0)
+      prefetch_l2((head[0] < Hq ? q_norm_w : k_norm_w) + lane * EPL);
     const float* tab = cos_sin + (size_t)pos[0] * D + (lane & 15) * EPL;
 #pragma unroll
     for (int k = 0; k < EPL; ++k) {
