@@ -46,7 +46,7 @@ __device__ __forceinline__ void copy_rows(float* dst, const float* __restrict__ 
 // feed it (a product of 128 x 16 x 16 takes it 57 cycles).  204 x 4,096 x 1,024: 74 us by FMA (52% of their rate), so 27;
 // 204 x 6,144 x 1,024 106 and 41; 204 x 1,024 x 3,072 57 and 21; one row of 1,024 x 3,072 21 and 16.  The head of 151,936 x 1,024 is
 // slower at up to 8 rows (127 and 163), whose bits may not differ from those of 64 rows (596 and 232).
-constexpr int BN = 128, BK = 64, MAX_PARTS = 4;
+constexpr int BN = 128, BK = 64;
 constexpr int PLANE_A = BN * BK * 2;                     // bytes of a part of W's rows
 __device__ int dib_gemm_fp32_error_word;
 
@@ -111,16 +111,20 @@ __device__ __forceinline__ void take_apart(float x, float y, unsigned (&part)[3]
   }
 }
 
-// How a tile's runs of k are divided (the order of the sums is the same).  RUNS: a CTA of the cluster takes a run.  FOLD: one
-// CTA takes all runs, one after the other (no cluster), for grids that fill the GPU without the division.
-enum Form { RUNS, FOLD };
+// How a tile's four runs of k are divided (the order of the sums is the same).  RUNS: a CTA of the cluster takes a run.  PAIRS: two
+// CTAs take two runs each, the first adds its two up, the second leaves both.  FOLD: one CTA takes all runs, one after
+// the other (no cluster).  For grids that fill the GPU with less division.
+constexpr int RUNS_OF_K = 4;         // (8 and 204 rows of 1,536, 512, us: two runs 8.2 and 10.1, four 5.7 and 9.5, eight 5.4 and 14.5)
+enum Form { RUNS, PAIRS, FOLD };
+constexpr int ctas_of(Form form) { return form == RUNS ? RUNS_OF_K : form == PAIRS ? 2 : 1; }
 
 // TOK rows of A a CTA, NW warps that take operands apart, DEPTH blocks that a thread has asked for and not yet taken apart
 template <int TOK, int NW, int DEPTH> struct Tc {
   static constexpr int PLANE_B = TOK * BK * 2;
   static constexpr int STAGE = 3 * (PLANE_A + PLANE_B);
   static constexpr int SUMS = TOK * BN * 4;              // the sums that a CTA leaves for its cluster
-  static constexpr int SMEM = (2 * STAGE > SUMS ? 2 * STAGE : SUMS) + 1024;      // (and the tiles' alignment)
+  static constexpr int SMEM = 2 * STAGE + 1024;          // (and the tiles' alignment)
+  static_assert(2 * STAGE >= 2 * SUMS, "the sums of two runs fit the stages");
   static constexpr int CTAS = TOK <= 16 && NW == 8 && DEPTH == 1 ? 2 : 1;
   static constexpr int THREADS = NW * 32 + 32;           // (one more warp issues the products)
   static constexpr int TMEM_COLS = 2 * TOK < 32 ? 32 : 2 * TOK;
@@ -174,9 +178,10 @@ __device__ __noinline__ void odd_results(const float* A, const float* W, float* 
 template <int TOK, int NW, int DEPTH, bool VEC, Form FORM>
 __global__ void __launch_bounds__((Tc<TOK, NW, DEPTH>::THREADS), (Tc<TOK, NW, DEPTH>::CTAS))
 gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ out, int M, int N,
-                    int K, int runs, int tile0) {
+                    int K, int tile0) {
   using C = Tc<TOK, NW, DEPTH>;
-  constexpr bool FOLDS = FORM == FOLD;
+  constexpr int PARTS = ctas_of(FORM), RUNS_EACH = RUNS_OF_K / PARTS;
+  constexpr bool FOLDS = FORM != RUNS;
   constexpr int TC_THREADS = C::THREADS, WARPS = NW;
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
@@ -187,8 +192,8 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * TOK, n0 = (tile0 + blockIdx.x) * BN, part = blockIdx.z;
   const int n_end = min(N, n0 + BN);
-  const int blocks = (K + BK - 1) / BK, per = (blocks + runs - 1) / runs, parts = FOLDS ? 1 : runs;
-  const int kb0 = part * per, nkb = FOLDS ? blocks : max(0, min(per, blocks - kb0));
+  const int blocks = (K + BK - 1) / BK, per = (blocks + RUNS_OF_K - 1) / RUNS_OF_K;
+  const int kb0 = part * RUNS_EACH * per, nkb = max(0, min(RUNS_EACH * per, blocks - kb0));
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[0])));
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&done[1])));
@@ -263,7 +268,7 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   float sum[HALF];
 #pragma unroll
   for (int j = 0; j < HALF; ++j) sum[j] = 0.f;
-  float total[FOLDS ? HALF : 1];       // FOLD: of the runs before
+  float total[FOLDS ? HALF : 1];       // of the runs before (PAIRS, second CTA: the first run, next to the second in `sum`)
   bool dead = false;                   // a wait has run out: no more waits, the launch is reported as failed
   auto add_block = [&](int kb) {
     if (!dead && !mbar_wait(&done[kb & 1], (kb >> 1) & 1)) dead = true;
@@ -279,7 +284,7 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
       for (int e = 0; e < LD; ++e) sum[j + e] = __fadd_rn(sum[j + e], __uint_as_float(r[e]));
     }
     tc_fence_before();
-    if (FOLDS && ((kb + 1) % per == 0 || kb + 1 == nkb)) {
+    if (FOLDS && ((kb + 1) % per == 0 || kb + 1 == nkb) && !(FORM == PAIRS && part == 1 && kb >= per)) {
 #pragma unroll
       for (int j = 0; j < HALF; ++j) {
         total[FOLDS ? j : 0] = kb < per ? sum[j] : __fadd_rn(total[FOLDS ? j : 0], sum[j]);
@@ -335,30 +340,35 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
   if (dead) atomicExch(&dib_gemm_fp32_error_word, 1);
   // the runs' sums, in run order; a CTA of the cluster takes a share of the tile's columns (rows of A)
   __syncthreads();                     // (every product has completed: the stages are free)
-  float* sums = reinterpret_cast<float*>(smem);          // [TOK][128 rows of W]
+  float* sums = reinterpret_cast<float*>(smem);          // [TOK][128 rows of W] (PAIRS: two of them)
   if (warp < WARPS) {
 #pragma unroll
-    for (int j = 0; j < HALF; ++j) sums[((warp >> 2) * HALF + j) * BN + (warp & 3) * 32 + lane] = FOLDS ? total[FOLDS ? j : 0] : sum[j];
+    for (int j = 0; j < HALF; ++j) {
+      float* to = sums + ((warp >> 2) * HALF + j) * BN + (warp & 3) * 32 + lane;
+      *to = FOLDS ? total[FOLDS ? j : 0] : sum[j];
+      if (FORM == PAIRS) to[TOK * BN] = sum[j];
+    }
   }
-  if (parts > 1) cluster_sync_all();
+  if (PARTS > 1) cluster_sync_all();
   else __syncthreads();
-  const int cols = min(TOK, M - m0), share = (cols + parts - 1) / parts;
+  const int cols = min(TOK, M - m0), share = (cols + PARTS - 1) / PARTS;
   const int c_end = min(cols, (part + 1) * share);
   bool any = false;
   for (int e = part * share * (BN / 4) + tid; e < c_end * (BN / 4); e += TC_THREADS) {
     const int n = n0 + e % (BN / 4) * 4, m = m0 + e / (BN / 4);
     const float* p = sums + 4 * e;
-    float4 v = *reinterpret_cast<const float4*>(p);
-    if (parts > 1) {
-      float4 run[MAX_PARTS];
+    float4 v;
+    if (PARTS > 1) {
+      float4 run[PARTS + 1];
 #pragma unroll
-      for (int r = 0; r < MAX_PARTS; ++r)
-        if (r < parts) run[r] = ld_peer_smem(p, r);
+      for (int r = 0; r < PARTS; ++r) run[r] = ld_peer_smem(p, r);
+      if (FORM == PAIRS) run[PARTS] = ld_peer_smem(p + TOK * BN, 1);
       v = run[0];
 #pragma unroll
-      for (int r = 1; r < MAX_PARTS; ++r)
-        if (r < parts)
-          v = make_float4(__fadd_rn(v.x, run[r].x), __fadd_rn(v.y, run[r].y), __fadd_rn(v.z, run[r].z), __fadd_rn(v.w, run[r].w));
+      for (int r = 1; r < (FORM == PAIRS ? PARTS + 1 : PARTS); ++r)
+        v = make_float4(__fadd_rn(v.x, run[r].x), __fadd_rn(v.y, run[r].y), __fadd_rn(v.z, run[r].z), __fadd_rn(v.w, run[r].w));
+    } else {
+      v = *reinterpret_cast<const float4*>(p);
     }
     constexpr float DOWN = 1.0f / (1 << SCALE);
     const float o[4] = {v.x * DOWN * DOWN, v.y * DOWN * DOWN, v.z * DOWN * DOWN, v.w * DOWN * DOWN};
@@ -378,7 +388,7 @@ gemm_fp32_tc_kernel(const float* __restrict__ A, const float* __restrict__ W, fl
     }
   }
   __syncwarp();
-  if (parts > 1) cluster_sync_all();   // nobody leaves while a peer may still read its sums
+  if (PARTS > 1) cluster_sync_all();   // nobody leaves while a peer may still read its sums
   tc_fence_before();
   __syncthreads();
   if (warp == 0)
@@ -454,8 +464,6 @@ gemm_fp32_short_kernel(const float* __restrict__ A, const float* __restrict__ W,
     }
 }
 
-// Part of the order above.  (8 and 204 rows of 1,536, 512, us: two runs 8.2 and 10.1, four 5.7 and 9.5, eight 5.4 and 14.5.)
-constexpr int RUNS_OF_K = 4;
 template <int TOK, int NW, int DEPTH, bool VEC, Form FORM>
 int launch_form(const float* A, const float* W, float* out, int M, int N, int K, int tile0, int tiles, cudaStream_t st) {
   using C = Tc<TOK, NW, DEPTH>;
@@ -468,7 +476,7 @@ int launch_form(const float* A, const float* W, float* out, int M, int N, int K,
     }
     once.mark();
   }
-  constexpr int runs = RUNS_OF_K, parts = FORM == FOLD ? 1 : runs;
+  constexpr int parts = ctas_of(FORM);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles, ceil_div_host(M, TOK), parts);
   cfg.blockDim = dim3(C::THREADS);
@@ -483,7 +491,7 @@ int launch_form(const float* A, const float* W, float* out, int M, int N, int K,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = dib_pdl_enabled() ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, gemm_fp32_tc_kernel<TOK, NW, DEPTH, VEC, FORM>, A, W, out, M, N, K, runs, tile0);
+  cudaLaunchKernelEx(&cfg, gemm_fp32_tc_kernel<TOK, NW, DEPTH, VEC, FORM>, A, W, out, M, N, K, tile0);
   DIB_CHECK_LAUNCH();
   return DIB_OK;
 }
@@ -518,7 +526,8 @@ int launch(const float* A, const float* W, float* out, int M, int N, int K, cuda
 // memory, us (tile rows and form: measured): 1 row of 1,024, 3,072 and 1,024, 2,048 (16 RUNS) 16.1, 12.1; 17 rows (32 RUNS) 18.1, 13.5;
 // 204 rows (64 RUNS) 20.6, 15.5; 204 x 4,096 x 1,024 (64 FOLD, 128 RUNS, 64 RUNS) 26, 27, 41; 500 x 4,096 x 1,024 (128 FOLD, 128
 // RUNS) 44, 54; the head of 151,936 x 1,024 at 8, 17, 64 and 204 rows (16, 32, 64, 128 FOLD) 163, 194, 232, 776, where the RUNS took
-// 209, 335, 387 and 1,030.  Below 16 rows two CTAs share an SM with a block asked for ahead, or one has it with two:
+// 209, 335, 387 and 1,030; 17, 64 and 46 rows of 6,144, 1,024, 1,024 and 512 (32, 64, 64 PAIRS; RUNS have two waves there) 14.5, 18.2, 11.5
+// against 18.3, 20.5, 13.3.  Up to 16 rows two CTAs share an SM with a block asked for ahead, or one has it with two:
 // 8 rows of 6,144, 1,024 (192 CTAs) 13.3 / 17.3, of 4,096, 1,024 (128) 12.4 / 9.2.  What waits is the tensor unit: a product of 128 x 16 x 16
 // takes it 57 cycles as one of 128 x 32 x 16 nearly does, 24 of them a block.
 struct Choice {
@@ -533,10 +542,10 @@ struct Sizes {
   int blocks() const { return ceil_div_host(K, BK); }
   long long tiles(int tok) const { return (long long)ceil_div_host(N, BN) * ceil_div_host(M, tok); }
   bool fits(int tok) const { return ceil_div_host(M, tok) <= 65535; }
-  float runs(int tok, int at_once, float fixed, float block) const {
+  float divided(Form form, int tok, int at_once, float fixed, float block) const {
     if (!fits(tok)) return 1e30f;
-    const int per = (blocks() + RUNS_OF_K - 1) / RUNS_OF_K;
-    return (float)((tiles(tok) * RUNS_OF_K + at_once - 1) / at_once) * (fixed + block * per);
+    const int per = (blocks() + RUNS_OF_K - 1) / RUNS_OF_K * (RUNS_OF_K / ctas_of(form));
+    return (float)((tiles(tok) * ctas_of(form) + at_once - 1) / at_once) * (fixed + block * per);
   }
   // FOLD: a last wave of a few tiles (the head of 151,936: 1,187 tiles, 8 waves of 148 and 3) is a grid of RUNS of its own
   int tail(int tok, int at_once) const {
@@ -579,16 +588,20 @@ extern "C" int dib_gemm_fp32(const float* A, const float* W, float* out, int M, 
   const Sizes z{M, N, K};
   Choice best;
   if (M <= 16) {
-    best.consider(0, z.runs(16, 148, 3.8f, 1.04f));
-    best.consider(1, z.runs(16, 296, 3.5f, 2.4f));
+    best.consider(0, z.divided(RUNS, 16, 148, 3.8f, 1.04f));
+    best.consider(1, z.divided(RUNS, 16, 296, 3.5f, 2.4f));
     best.consider(2, z.fold(16, 296, 3.5f, z.tiles(16) > 148 ? 2.1f : 1.4f));
   }
-  best.consider(3, z.runs(32, 148, 4.6f, 1.13f));
+  best.consider(3, z.divided(RUNS, 32, 148, 4.6f, 1.13f));
   best.consider(4, z.fold(32, 148, 4.5f, 1.12f));
-  best.consider(5, z.runs(64, 148, 5.3f, 1.25f));
+  best.consider(5, z.divided(RUNS, 64, 148, 5.3f, 1.25f));
   best.consider(6, z.fold(64, 148, 5.1f, 1.32f));
-  best.consider(7, z.runs(128, 148, 4.9f, 1.98f));
+  best.consider(7, z.divided(RUNS, 128, 148, 4.9f, 1.98f));
   best.consider(8, z.fold(128, 148, 10.5f, 2.07f));
+  if (M <= 16) best.consider(9, z.divided(PAIRS, 16, 148, 4.6f, 1.08f));
+  best.consider(10, z.divided(PAIRS, 32, 148, 5.2f, 1.17f));
+  best.consider(11, z.divided(PAIRS, 64, 148, 5.0f, 1.62f));
+  best.consider(12, z.divided(PAIRS, 128, 148, 8.2f, 2.2f));
   switch (best.form) {
     case 0: return launch<16, 8, 2, RUNS>(A, W, out, M, N, K, st);
     case 1: return launch<16, 8, 1, RUNS>(A, W, out, M, N, K, st);
@@ -598,6 +611,10 @@ extern "C" int dib_gemm_fp32(const float* A, const float* W, float* out, int M, 
     case 5: return launch<64, 16, 1, RUNS>(A, W, out, M, N, K, st);
     case 6: return launch_fold<64, 8, 1, 16, 1>(A, W, out, z, 148, st);
     case 7: return launch<128, 16, 1, RUNS>(A, W, out, M, N, K, st);
-    default: return launch_fold<128, 16, 1, 16, 1>(A, W, out, z, 148, st);
+    case 8: return launch_fold<128, 16, 1, 16, 1>(A, W, out, z, 148, st);
+    case 9: return launch<16, 8, 2, PAIRS>(A, W, out, M, N, K, st);
+    case 10: return launch<32, 8, 1, PAIRS>(A, W, out, M, N, K, st);
+    case 11: return launch<64, 16, 1, PAIRS>(A, W, out, M, N, K, st);
+    default: return launch<128, 16, 1, PAIRS>(A, W, out, M, N, K, st);
   }
 }

@@ -180,11 +180,12 @@ def test_linear_fp32_is_true_fp32(m, n, k):
 
 @pytest.mark.parametrize("n,k", [(31, 33), (33, 64), (65, 130), (4096, 260), (100, 511), (100, 512),
                                  (4096, 513), (65, 578), (1024, 1028), (40003, 516), (4099, 1028), (40003, 517),
-                                 (4099, 1030), (75700, 512), (75649, 1028), (38200, 1025), (6144, 1024), (1000, 640)])
+                                 (4099, 1030), (75700, 512), (75649, 1028), (38200, 1025), (6144, 1024), (6144, 1025), (6100, 577),
+                                 (1000, 640)])
 def test_linear_fp32_tiles_give_the_same_bits(n, k):
     """Every tile and form the row count and the width may choose adds in one order: the row's bits are those of the
     row alone, at the edges of the tiles; against 64 bits the error is that of a chain of k terms below 512, and
-    from there on of a few roundings.  (The wide ones reach all tiles and both forms from K = 512 on, a last wave of a few
+    from there on of a few roundings.  (The wide ones reach all tiles and forms from K = 512 on, a last wave of a few
     tiles too, each with copies of 16 and of 4 bytes.)"""
     torch.manual_seed(16)
     x = torch.randn(400, k, device="cuda")
